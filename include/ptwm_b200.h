@@ -226,6 +226,15 @@ typedef struct ptwm_b200_encode_options {
 
 typedef struct ptwm_b200_encoded ptwm_b200_encoded;
 
+/* Where ptwm_b200_encode_model takes its device memory from (work memory and the container itself): the program's own pool
+ * instead of cudaMalloc / cudaFree, which cost many times the encode.  alloc returns the address of `bytes` bytes on the
+ * device, 256-byte aligned, for use on `stream`, or 0; free takes a block back when everything that used it has been
+ * enqueued on that stream.  Both may be called from any thread that calls into the library.  NULL, NULL: cudaMalloc again.
+ * A block is always returned to the allocator that handed it out. */
+typedef uint64_t (*ptwm_b200_alloc_fn)(uint64_t bytes, uint32_t device_ordinal, uint64_t stream);
+typedef void (*ptwm_b200_free_fn)(uint64_t ptr, uint32_t device_ordinal, uint64_t stream);
+int64_t ptwm_b200_set_allocator(ptwm_b200_alloc_fn alloc, ptwm_b200_free_fn free);
+
 /* compress_model (compressor.rs:972-1200) for the production split / passthrough
  * chains, compact \x89PTWC layout: split + reorder, histograms, table build and
  * stream encoding (identity, huffman, rans, tans, order1_scale_ac) run on the

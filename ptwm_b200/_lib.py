@@ -53,7 +53,11 @@ class EncodeOptions(C.Structure):
                 ("emit_payload_hash", C.c_uint8), ("candidates", C.c_uint8), ("reserved", C.c_uint8 * 1)]
 
 
+ALLOC_FN = C.CFUNCTYPE(C.c_uint64, C.c_uint64, C.c_uint32, C.c_uint64)
+FREE_FN = C.CFUNCTYPE(None, C.c_uint64, C.c_uint32, C.c_uint64)
+
 _SIGNATURES = {
+    "ptwm_b200_set_allocator": (C.c_int64, [ALLOC_FN, FREE_FN]),
     "ptwm_b200_encode_model": (C.c_int64, [C.POINTER(EncodeTensor), C.c_size_t, C.POINTER(EncodeOptions), C.c_uint32, C.c_uint64, C.POINTER(C.c_void_p)]),
     "ptwm_b200_encoded_size": (C.c_uint64, [C.c_void_p]),
     "ptwm_b200_encoded_device_ptr": (C.c_uint64, [C.c_void_p]),

@@ -52,6 +52,38 @@ class CompressionConfig:
     emit_payload_hash: bool = False
 
 
+@_lib.ALLOC_FN
+def _torch_alloc(nbytes: int, device: int, stream: int) -> int:
+    try:
+        return torch.cuda.caching_allocator_alloc(nbytes, device, 0 if stream == 1 else stream)  # 1 is the legacy default stream, torch's 0
+    except Exception:  # out of memory: the library reports it
+        return 0
+
+
+@_lib.FREE_FN
+def _torch_free(ptr: int, device: int, stream: int) -> None:
+    try:
+        torch.cuda.caching_allocator_delete(ptr)
+    except Exception:  # only while the interpreter goes down
+        pass
+
+
+_allocator_set = False
+
+
+def _library():
+    """The library, drawing the encoder's device memory from torch's allocator: recycled between calls, visible in torch's
+    statistics and given back by ``torch.cuda.empty_cache()``."""
+    global _allocator_set
+    L = _lib.lib()
+    if not _allocator_set:
+        for fn in (_torch_alloc, _torch_free):  # the library may call them for containers that outlive this module at exit
+            C.pythonapi.Py_IncRef(C.py_object(fn))
+        _check(L.ptwm_b200_set_allocator(_torch_alloc, _torch_free))
+        _allocator_set = True
+    return L
+
+
 class EncodedContainer:
     """A container held in device memory by the library."""
 
@@ -151,5 +183,5 @@ def compress_model(tensors: Mapping[str, torch.Tensor], config: Optional[Compres
                              int(cfg.emit_payload_hash), tries)
     torch.cuda.current_stream(dev).synchronize()
     h = C.c_void_p()
-    _check(_lib.lib().ptwm_b200_encode_model(arr, len(names), C.byref(opt), dev, stream_handle(dev), C.byref(h)))
+    _check(_library().ptwm_b200_encode_model(arr, len(names), C.byref(opt), dev, stream_handle(dev), C.byref(h)))
     return EncodedContainer(h, names, n_planes, dev)

@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -192,26 +193,56 @@ struct Piece { uint64_t dst; std::vector<uint8_t> bytes; };
 
 }  // namespace
 
+namespace {
+
+// Device memory comes from the allocator the program registered (ptwm_b200_set_allocator), else from cudaMalloc.  An encode
+// takes work memory several times the size of the tensors; handed out and taken back by the driver that was 55 of the 64 ms
+// of a 1.7 GB model.  The blocks belong to the stream the encode runs on, which is all an allocator that recycles memory in
+// stream order has to know.
+struct Allocator { ptwm_b200_alloc_fn alloc = nullptr; ptwm_b200_free_fn free = nullptr; };
+std::mutex g_alloc_mu;
+Allocator g_alloc;
+Allocator current_allocator() { std::lock_guard<std::mutex> g(g_alloc_mu); return g_alloc; }
+
+struct DeviceBuf {
+    void* p = nullptr;
+    Allocator from;
+    int device = 0;
+    cudaStream_t stream = nullptr;
+    DeviceBuf() = default;
+    DeviceBuf(const DeviceBuf&) = delete;
+    DeviceBuf& operator=(const DeviceBuf&) = delete;
+    ~DeviceBuf() {
+        if (!p) return;
+        if (from.free) from.free(uint64_t(reinterpret_cast<uintptr_t>(p)), uint32_t(device), uint64_t(reinterpret_cast<uintptr_t>(stream)));
+        else { DeviceGuard g{device}; cudaFree(p); }
+    }
+    template <class T> T* as() { return static_cast<T*>(p); }
+    cudaError_t alloc(size_t n, cudaStream_t st, bool registered = true) {
+        stream = st;
+        cudaError_t e = cudaGetDevice(&device);
+        if (e != cudaSuccess) return e;
+        from = registered ? current_allocator() : Allocator{};
+        if (!from.alloc) return cudaMalloc(&p, n ? n : 1);
+        p = reinterpret_cast<void*>(uintptr_t(from.alloc(n ? n : 1, uint32_t(device), uint64_t(reinterpret_cast<uintptr_t>(st)))));
+        return p ? cudaSuccess : cudaErrorMemoryAllocation;
+    }
+};
+
+}  // namespace
+
 struct ptwm_b200_encoded {
-    uint8_t* d_out = nullptr;
+    DeviceBuf out;
     uint64_t size = 0;
     int device = 0;
     std::vector<std::vector<int>> plane_codecs;
-    ~ptwm_b200_encoded() { if (d_out) { DeviceGuard g{device}; cudaFree(d_out); } }
 };
 
 namespace {
 
-struct DeviceBuf {
-    void* p = nullptr;
-    ~DeviceBuf() { if (p) cudaFree(p); }
-    template <class T> T* as() { return static_cast<T*>(p); }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, n ? n : 1); }
-};
-
 template <class T>
 cudaError_t upload_vec(DeviceBuf& b, const std::vector<T>& v, cudaStream_t st) {
-    cudaError_t e = b.alloc(v.size() * sizeof(T));
+    cudaError_t e = b.alloc(v.size() * sizeof(T), st);
     if (e != cudaSuccess || v.empty()) return e;
     return cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
 }
@@ -306,16 +337,16 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     prof("plan (host)");
     // ---- device pipeline: split, histograms ---------------------------------
     DeviceBuf d_planes, d_splits, d_chunks, d_hist, d_plane_hist, d_codec, d_tables, d_results, d_slots;
-    CUDA_TRY(d_planes.alloc(planes_bytes));
+    CUDA_TRY(d_planes.alloc(planes_bytes, st));
     CUDA_TRY(upload_vec(d_splits, splits, st));
     CUDA_TRY(upload_vec(d_chunks, chunks, st));
-    CUDA_TRY(d_hist.alloc(uint64_t(n_chunks) * 1024));
-    CUDA_TRY(d_plane_hist.alloc(uint64_t(n_planes) * 256 * 8));
+    CUDA_TRY(d_hist.alloc(uint64_t(n_chunks) * 1024, st));
+    CUDA_TRY(d_plane_hist.alloc(uint64_t(n_planes) * 256 * 8, st));
     CUDA_TRY(cudaMemsetAsync(d_plane_hist.p, 0, uint64_t(n_planes) * 256 * 8 + (n_planes ? 0 : 1), st));
     if (tile) { split_kernel<<<tile, 256, 0, st>>>(d_splits.as<SplitItem>(), uint32_t(splits.size()), d_planes.as<uint8_t>()); CUDA_TRY(cudaGetLastError()); }
     DeviceBuf d_or;
     std::vector<uint32_t> or_words(n_or_words);
-    if (n_or_words) { CUDA_TRY(d_or.alloc(uint64_t(n_or_words) * 4)); CUDA_TRY(cudaMemsetAsync(d_or.p, 0, uint64_t(n_or_words) * 4, st)); }
+    if (n_or_words) { CUDA_TRY(d_or.alloc(uint64_t(n_or_words) * 4, st)); CUDA_TRY(cudaMemsetAsync(d_or.p, 0, uint64_t(n_or_words) * 4, st)); }
     for (auto& tp : plan) {
         auto blocks = [](uint64_t n) { return unsigned(std::min<uint64_t>((n + 4095) / 4096, 2368)); };
         if (tp.has_delta) { delta_kernel<<<blocks(tp.delta.len), 256, 0, st>>>(d_planes.as<uint8_t>() + tp.planes.back().buf_off, d_planes.as<uint8_t>() + tp.delta.buf_off, tp.delta.len); CUDA_TRY(cudaGetLastError()); }
@@ -339,7 +370,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             if (tp.has_delta) add(tp.delta, tp.delta_index);
         }
         CUDA_TRY(upload_vec(d_verify, verify, st));
-        CUDA_TRY(d_acc.alloc(uint64_t(n_planes) * 4));
+        CUDA_TRY(d_acc.alloc(uint64_t(n_planes) * 4, st));
         CUDA_TRY(cudaMemsetAsync(d_acc.p, 0, uint64_t(n_planes) * 4 + (n_planes ? 0 : 1), st));
         if (n_runs) {
             Bases b{nullptr, 0, 0, nullptr, d_planes.as<uint8_t>()};
@@ -350,7 +381,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     std::vector<uint64_t> hashes(hash_items.size());
     if (!hash_items.empty()) {
         CUDA_TRY(upload_vec(d_hitems, hash_items, st));
-        CUDA_TRY(d_hout.alloc(hash_items.size() * 8));
+        CUDA_TRY(d_hout.alloc(hash_items.size() * 8, st));
         Bases b{nullptr, 0, 0, nullptr, nullptr};
         xxh64_kernel<<<uint32_t(hash_items.size()), 32, 0, st>>>(d_hitems.as<HashItem>(), uint32_t(hash_items.size()), b, d_hout.as<uint64_t>());
         CUDA_TRY(cudaGetLastError());
@@ -379,7 +410,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             DeviceBuf d_whole, d_list, d_counts;
             CUDA_TRY(upload_vec(d_whole, whole, st));
             CUDA_TRY(upload_vec(d_list, list, st));
-            CUDA_TRY(d_counts.alloc(whole.size() * size_t(O1E_PRESENT)));
+            CUDA_TRY(d_counts.alloc(whole.size() * size_t(O1E_PRESENT), st));
             CUDA_TRY(cudaMemsetAsync(d_counts.p, 0, whole.size() * size_t(O1E_PRESENT), st));
             o1sac_count_kernel<<<uint32_t(whole.size()), 256, 0, st>>>(d_whole.as<EncChunk>(), d_list.as<uint32_t>(), d_planes.as<uint8_t>(), d_counts.as<uint8_t>());
             CUDA_TRY(cudaGetLastError());
@@ -413,7 +444,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             for (size_t k = 0; k < own.size(); ++k) fit_dense_rows(own[k], dense.data() + k * size_t(257 * 256));
             DeviceBuf d_dense, d_pairs, d_dist;
             if ((fit_err = upload_vec(d_dense, dense, st)) != cudaSuccess || (fit_err = upload_vec(d_pairs, pairs, st)) != cudaSuccess ||
-                (fit_err = d_dist.alloc(d.size() * sizeof(double))) != cudaSuccess) return d;
+                (fit_err = d_dist.alloc(d.size() * sizeof(double), st)) != cudaSuccess) return d;
             fit_pair_distance_kernel<<<uint32_t(d.size()), 256, 0, st>>>(d_dense.as<uint16_t>(), d_pairs.as<uint32_t>(), d_dist.as<double>());
             if ((fit_err = cudaGetLastError()) != cudaSuccess) return d;
             if ((fit_err = cudaMemcpyAsync(d.data(), d_dist.p, d.size() * sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return d;
@@ -559,10 +590,10 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     // ---- tables and streams ---------------------------------------------------
     CUDA_TRY(upload_vec(d_codec, plane_codec, st));
     if (n_chunks) CUDA_TRY(cudaMemcpyAsync(d_chunks.p, chunks.data(), chunks.size() * sizeof(EncChunk), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(d_tables.alloc(tables_bytes));
-    CUDA_TRY(d_results.alloc(uint64_t(n_chunks) * sizeof(EncResult)));
+    CUDA_TRY(d_tables.alloc(tables_bytes, st));
+    CUDA_TRY(d_results.alloc(uint64_t(n_chunks) * sizeof(EncResult), st));
     CUDA_TRY(cudaMemsetAsync(d_results.p, 0, uint64_t(n_chunks) * sizeof(EncResult) + (n_chunks ? 0 : 1), st));
-    CUDA_TRY(d_slots.alloc(slots_bytes));
+    CUDA_TRY(d_slots.alloc(slots_bytes, st));
     std::vector<EncResult> results(n_chunks);
     prof("  work memory for tables and streams");
     DeviceBuf d_o1list, d_tanslist;
@@ -833,16 +864,16 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     prof("layout and records (host)");
     // ---- write the container ----------------------------------------------------
     enc.size = pos; enc.device = device;
-    CUDA_TRY(cudaMalloc(&enc.d_out, pos));
+    CUDA_TRY(enc.out.alloc(pos, st));
     DeviceBuf d_staged, d_triples, d_gathers;
     CUDA_TRY(upload_vec(d_staged, staged, st));
     CUDA_TRY(upload_vec(d_triples, triples, st));
     CUDA_TRY(upload_vec(d_gathers, gathers, st));
-    scatter_kernel<<<uint32_t(triples.size() / 3), 128, 0, st>>>(d_staged.as<uint8_t>(), d_triples.as<uint64_t>(), enc.d_out);
+    scatter_kernel<<<uint32_t(triples.size() / 3), 128, 0, st>>>(d_staged.as<uint8_t>(), d_triples.as<uint64_t>(), enc.out.as<uint8_t>());
     CUDA_TRY(cudaGetLastError());
     if (!gathers.empty()) {
         gather_kernel<<<uint32_t(gathers.size()), 128, 0, st>>>(d_gathers.as<GatherItem>(), d_chunks.as<EncChunk>(), d_results.as<EncResult>(), d_planes.as<uint8_t>(),
-                                                                d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), enc.d_out);
+                                                                d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), enc.out.as<uint8_t>());
         CUDA_TRY(cudaGetLastError());
     }
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -891,11 +922,11 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         for (uint32_t ctx = 0; ctx < 256; ++ctx)
             if (state[ctx >> 3] & (1u << (ctx & 7))) { tab[O1E_PRESENT + ctx] = 1; load_row(1 + ctx, state + 32 + 512 + 512 * size_t(k)); ++k; }
         const uint32_t zero = 0;
-        CUDA_TRY(d_chunk.alloc(sizeof(EncChunk)));
-        CUDA_TRY(d_tables.alloc(tab.size()));
-        CUDA_TRY(d_results.alloc(sizeof(EncResult)));
-        CUDA_TRY(d_slots.alloc(4 * slot_cap));
-        CUDA_TRY(d_list.alloc(4));
+        CUDA_TRY(d_chunk.alloc(sizeof(EncChunk), st, false));
+        CUDA_TRY(d_tables.alloc(tab.size(), st, false));
+        CUDA_TRY(d_results.alloc(sizeof(EncResult), st, false));
+        CUDA_TRY(d_slots.alloc(4 * slot_cap, st, false));
+        CUDA_TRY(d_list.alloc(4, st, false));
         CUDA_TRY(cudaMemcpyAsync(d_chunk.p, &chunk, sizeof(chunk), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(d_tables.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(d_list.p, &zero, 4, cudaMemcpyHostToDevice, st));
@@ -919,15 +950,15 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
     }
     uint32_t mode = 1;
     uint64_t size = 1 + uint64_t(n);
-    CUDA_TRY(d_chunk.alloc(sizeof(EncChunk)));
-    CUDA_TRY(d_results.alloc(sizeof(EncResult)));
-    CUDA_TRY(d_tables.alloc(enc_table_bytes(codec)));
+    CUDA_TRY(d_chunk.alloc(sizeof(EncChunk), st, false));
+    CUDA_TRY(d_results.alloc(sizeof(EncResult), st, false));
+    CUDA_TRY(d_tables.alloc(enc_table_bytes(codec), st, false));
     if (n <= 0xFFFFFFFFull) {  // the length prefix is a u32; longer planes stay raw
         if (slot_cap > 0x3FFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
-        CUDA_TRY(d_codec.alloc(1));
-        CUDA_TRY(d_hist.alloc(256 * sizeof(uint32_t)));
-        CUDA_TRY(d_phist.alloc(256 * sizeof(unsigned long long)));
-        CUDA_TRY(d_slots.alloc(4 * slot_cap));
+        CUDA_TRY(d_codec.alloc(1, st, false));
+        CUDA_TRY(d_hist.alloc(256 * sizeof(uint32_t), st, false));
+        CUDA_TRY(d_phist.alloc(256 * sizeof(unsigned long long), st, false));
+        CUDA_TRY(d_slots.alloc(4 * slot_cap, st, false));
         CUDA_TRY(cudaMemcpyAsync(d_chunk.p, &chunk, sizeof(chunk), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(d_codec.p, &codec_byte, 1, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemsetAsync(d_phist.p, 0, 256 * sizeof(unsigned long long), st));
@@ -935,7 +966,7 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         table_kernel<<<1, 64, 0, st>>>(d_chunk.as<EncChunk>(), 1, d_codec.as<uint8_t>(), d_hist.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
         encode_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), 1, d_codec.as<uint8_t>(), in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
         if (codec == C_TANS) {
-            CUDA_TRY(d_tlist.alloc(4));
+            CUDA_TRY(d_tlist.alloc(4, st, false));
             CUDA_TRY(cudaMemsetAsync(d_tlist.p, 0, 4, st));  // the list of chunks to code: chunk 0
             CUDA_TRY(cudaFuncSetAttribute(tans_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TENC_SMEM));
             tans_encode_kernel<<<1, 32, TENC_SMEM, st>>>(d_chunk.as<EncChunk>(), d_tlist.as<uint32_t>(), 1, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
@@ -953,7 +984,7 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         const bool coded = r.coded && blob < n && (codec == C_HUFFMAN || n <= (1ull << 30) || n <= blob * 64);
         if (coded) { mode = codec == C_RANS ? 2 : codec == C_HUFFMAN ? 3 : 4; size = 1 + 4 + blob; }
     } else {
-        CUDA_TRY(d_slots.alloc(16));
+        CUDA_TRY(d_slots.alloc(16, st, false));
     }
     if (need(size) > out_cap) return fail(PTWM_RC_BUFFER_TOO_SMALL, "output buffer too small");
     if (mode == 1 && n > 0xFFFFFFFFull) {  // raw: tag byte, then the plane
@@ -961,7 +992,7 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         CUDA_TRY(cudaMemcpyAsync(out + 1, in, n, cudaMemcpyDeviceToDevice, st));
     } else {
         const GatherItem g{0, 0, mode | GATHER_BARE};
-        CUDA_TRY(d_gather.alloc(sizeof(g)));
+        CUDA_TRY(d_gather.alloc(sizeof(g), st, false));
         CUDA_TRY(cudaMemcpyAsync(d_gather.p, &g, sizeof(g), cudaMemcpyHostToDevice, st));
         gather_kernel<<<1, 128, 0, st>>>(d_gather.as<GatherItem>(), d_chunk.as<EncChunk>(), d_results.as<EncResult>(), in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), out);
         CUDA_TRY(cudaGetLastError());
@@ -972,6 +1003,12 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
 
 extern "C" {
 
+int64_t ptwm_b200_set_allocator(ptwm_b200_alloc_fn alloc, ptwm_b200_free_fn free) {
+    if ((alloc == nullptr) != (free == nullptr)) return fail(PTWM_RC_INVALID_INPUT, "an allocator is a pair of functions");
+    std::lock_guard<std::mutex> g(g_alloc_mu);
+    g_alloc = Allocator{alloc, free};
+    return 0;
+}
 int64_t ptwm_b200_encode_model(const ptwm_b200_encode_tensor* tensors, size_t n, const ptwm_b200_encode_options* options, uint32_t device_ordinal, uint64_t stream,
                                ptwm_b200_encoded** out) {
     if ((!tensors && n) || !out) return fail(PTWM_RC_INVALID_INPUT, "null argument");
@@ -1040,12 +1077,12 @@ int64_t ptwm_b200_fit_shared_states_host(const uint8_t* const* planes, const uin
     } catch (const std::exception& ex) { return fail(PTWM_RC_INTERNAL, ex.what()); }
 }
 uint64_t ptwm_b200_encoded_size(const ptwm_b200_encoded* e) { return e ? e->size : 0; }
-uint64_t ptwm_b200_encoded_device_ptr(const ptwm_b200_encoded* e) { return e ? uint64_t(reinterpret_cast<uintptr_t>(e->d_out)) : 0; }
+uint64_t ptwm_b200_encoded_device_ptr(const ptwm_b200_encoded* e) { return e ? uint64_t(reinterpret_cast<uintptr_t>(e->out.p)) : 0; }
 int64_t ptwm_b200_encoded_copy(const ptwm_b200_encoded* e, uint8_t* host_dst, size_t cap) {
     if (!e || !host_dst) return fail(PTWM_RC_INVALID_INPUT, "null argument");
     if (cap < e->size) return fail(PTWM_RC_BUFFER_TOO_SMALL, "host buffer smaller than the container");
     DeviceGuard guard{e->device};
-    CUDA_TRY(cudaMemcpy(host_dst, e->d_out, e->size, cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(host_dst, e->out.p, e->size, cudaMemcpyDeviceToHost));
     return int64_t(e->size);
 }
 int64_t ptwm_b200_encoded_copy_to_device(const ptwm_b200_encoded* e, uint64_t dst_dev_ptr, uint64_t cap, uint64_t stream) {
@@ -1053,7 +1090,7 @@ int64_t ptwm_b200_encoded_copy_to_device(const ptwm_b200_encoded* e, uint64_t ds
     if (cap < e->size) return fail(PTWM_RC_BUFFER_TOO_SMALL, "device buffer smaller than the container");
     DeviceGuard guard{e->device};
     cudaStream_t st = reinterpret_cast<cudaStream_t>(uintptr_t(stream));
-    CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<void*>(uintptr_t(dst_dev_ptr)), e->d_out, e->size, cudaMemcpyDeviceToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<void*>(uintptr_t(dst_dev_ptr)), e->out.p, e->size, cudaMemcpyDeviceToDevice, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     return int64_t(e->size);
 }
