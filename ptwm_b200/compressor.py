@@ -52,6 +52,10 @@ class CompressionConfig:
     emit_payload_hash: bool = False
 
 
+_new_bytes = C.PYFUNCTYPE(C.py_object, C.c_void_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
+_bytes_address = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
+
+
 @_lib.ALLOC_FN
 def _torch_alloc(nbytes: int, device: int, stream: int) -> int:
     try:
@@ -101,9 +105,11 @@ class EncodedContainer:
             self._e = None
 
     def to_bytes(self) -> bytes:
-        buf = C.create_string_buffer(max(self.size, 1))
-        _check(_lib.lib().ptwm_b200_encoded_copy(self._e, buf, self.size))
-        return buf.raw[:self.size]
+        # the library writes straight into the new object; nobody else has seen it yet
+        data = _new_bytes(None, self.size)
+        if self.size:
+            _check(_lib.lib().ptwm_b200_encoded_copy(self._e, _bytes_address(data), self.size))
+        return data
 
     def to_tensor(self) -> torch.Tensor:
         """The container bytes as a CUDA uint8 tensor (a copy owned by torch)."""

@@ -217,7 +217,7 @@ struct DeviceBuf {
         if (from.free) from.free(uint64_t(reinterpret_cast<uintptr_t>(p)), uint32_t(device), uint64_t(reinterpret_cast<uintptr_t>(stream)));
         else { DeviceGuard g{device}; cudaFree(p); }
     }
-    template <class T> T* as() { return static_cast<T*>(p); }
+    template <class T> T* as() const { return static_cast<T*>(p); }
     cudaError_t alloc(size_t n, cudaStream_t st, bool registered = true) {
         stream = st;
         cudaError_t e = cudaGetDevice(&device);
@@ -1082,7 +1082,10 @@ int64_t ptwm_b200_encoded_copy(const ptwm_b200_encoded* e, uint8_t* host_dst, si
     if (!e || !host_dst) return fail(PTWM_RC_INVALID_INPUT, "null argument");
     if (cap < e->size) return fail(PTWM_RC_BUFFER_TOO_SMALL, "host buffer smaller than the container");
     DeviceGuard guard{e->device};
-    CUDA_TRY(cudaMemcpy(host_dst, e->out.p, e->size, cudaMemcpyDeviceToHost));
+    DeviceState* ds;
+    int64_t rc = device_state(e->device, &ds);
+    if (rc < 0) return rc;
+    if ((rc = copy_to_host(host_dst, e->out.as<uint8_t>(), e->size, *ds)) < 0) return rc;
     return int64_t(e->size);
 }
 int64_t ptwm_b200_encoded_copy_to_device(const ptwm_b200_encoded* e, uint64_t dst_dev_ptr, uint64_t cap, uint64_t stream) {

@@ -41,6 +41,9 @@ struct DeviceState {
 int64_t device_state(int dev, DeviceState** out);
 const CrcTables& crc_tables();
 
+// Device bytes into ordinary host memory (`src` complete, or ordered before ds.stream).
+int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds);
+
 inline uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }
 
 // One plane into one payload on the device (encoder.cu); body of ptwm_plane_codec_v1_encode_cuda.

@@ -1,12 +1,16 @@
 // Host side of libptwm_b200.so: the planner that flattens a parsed container
 // into kernel work lists, the runner that launches them, and the C ABI
 // declared in include/ptwm_b200.h.
+#include <sys/mman.h>
+
 #include <algorithm>
+#include <condition_variable>
 #include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "format.hpp"
@@ -33,7 +37,85 @@ CrcTables host_crc_tables() {
     for (int k = 0; k < 64; ++k) { t.x2n[k] = p; p = gf2_mulmod(p, p); }
     return t;
 }
+std::mutex g_stage_mu;  // one staging buffer per device, used under this lock
+// Caller holds the lock.
+int64_t stage_reserve(DeviceState& ds, size_t bytes) {
+    if (ds.stage_cap >= bytes) return 0;
+    // grows only on the first large plan of a process: pinning synchronises with the device
+    if (ds.stage) CUDA_TRY(cudaFreeHost(ds.stage));
+    ds.stage = nullptr; ds.stage_cap = 0;
+    const size_t cap = std::max<size_t>(bytes + bytes / 2, size_t(32) << 20);
+    CUDA_TRY(cudaMallocHost(&ds.stage, cap));
+    ds.stage_cap = cap;
+    return 0;
+}
 }  // namespace
+
+// Through the pinned staging buffer in slices: the copy engine fills slice k + 4 while host threads move slice k on.  A copy
+// into pageable memory by the driver runs at 5 - 10 GB/s, and memory nobody has touched yet costs a page fault per 4 KiB on
+// top of that, so the slices are taken by four threads, on huge pages where the system grants them.
+int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds) {
+    constexpr size_t SLICE = size_t(2) << 20, RING = 8;
+    if (n < SLICE) {
+        CUDA_TRY(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, ds.stream));
+        CUDA_TRY(cudaStreamSynchronize(ds.stream));
+        return 0;
+    }
+    const uintptr_t page = uintptr_t(1) << 21, lo = (reinterpret_cast<uintptr_t>(dst) + page - 1) & ~(page - 1), hi = (reinterpret_cast<uintptr_t>(dst) + n) & ~(page - 1);
+    if (hi > lo) madvise(reinterpret_cast<void*>(lo), hi - lo, MADV_HUGEPAGE);  // a hint; refused is fine
+    std::lock_guard<std::mutex> g(g_stage_mu);
+    int64_t rc = stage_reserve(ds, SLICE * RING);
+    if (rc < 0) return rc;
+    struct Events {
+        cudaEvent_t ev[RING] = {nullptr};
+        ~Events() { for (auto e : ev) if (e) cudaEventDestroy(e); }
+    } events;
+    for (auto& e : events.ev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const size_t slices = (n + SLICE - 1) / SLICE;
+    uint8_t* stage = static_cast<uint8_t*>(ds.stage);
+    std::mutex mu;
+    std::condition_variable cv;
+    size_t sent = 0;                       // slices handed to the copy engine
+    std::vector<char> moved(slices, 0);    // slices that have left the staging buffer
+    cudaError_t failed = cudaSuccess;
+    int device = 0;
+    CUDA_TRY(cudaGetDevice(&device));
+    auto worker = [&](size_t first, size_t step) {
+        cudaSetDevice(device);
+        for (size_t k = first; k < slices; k += step) {
+            {
+                std::unique_lock<std::mutex> l(mu);
+                cv.wait(l, [&] { return sent > k || failed != cudaSuccess; });
+                if (failed != cudaSuccess) return;
+            }
+            const cudaError_t e = cudaEventSynchronize(events.ev[k % RING]);
+            if (e == cudaSuccess) std::memcpy(dst + k * SLICE, stage + (k % RING) * SLICE, std::min(SLICE, n - k * SLICE));
+            std::lock_guard<std::mutex> l(mu);
+            if (e != cudaSuccess) failed = e;
+            moved[k] = 1;
+            cv.notify_all();
+        }
+    };
+    const size_t n_threads = std::min<size_t>(slices, 4);
+    std::vector<std::thread> threads;
+    for (size_t t = 0; t < n_threads; ++t) threads.emplace_back(worker, t, n_threads);
+    for (size_t k = 0; k < slices; ++k) {
+        if (k >= RING) {
+            std::unique_lock<std::mutex> l(mu);
+            cv.wait(l, [&] { return moved[k - RING] || failed != cudaSuccess; });
+        }
+        cudaError_t e = cudaMemcpyAsync(stage + (k % RING) * SLICE, src + k * SLICE, std::min(SLICE, n - k * SLICE), cudaMemcpyDeviceToHost, ds.stream);
+        if (e == cudaSuccess) e = cudaEventRecord(events.ev[k % RING], ds.stream);
+        std::lock_guard<std::mutex> l(mu);
+        if (e != cudaSuccess) failed = e;
+        sent = k + 1;
+        cv.notify_all();
+        if (failed != cudaSuccess) break;
+    }
+    for (auto& t : threads) t.join();
+    CUDA_TRY(failed);
+    return 0;
+}
 
 const CrcTables& crc_tables() { static CrcTables t = host_crc_tables(); return t; }
 
@@ -303,19 +385,13 @@ void finish_lists(ptwm_b200_plan& pl) {
 // host-to-device copy: a caller that streams a container to the GPU has tens of large copies queued on the copy
 // engine, and a small copy issued now would only run after all of them (the plan of the first piece would be ready
 // when the last byte of the container has arrived).  The kernel runs on the library's stream beside those copies.
-std::mutex g_stage_mu;  // one staging buffer per device, used under this lock
 template <class T>
 int64_t upload(T* dst, const std::vector<T>& v, DeviceState& ds) {
     if (v.empty()) return 0;
     const size_t bytes = v.size() * sizeof(T), padded = (bytes + 15) & ~size_t(15);
     std::lock_guard<std::mutex> g(g_stage_mu);
-    if (ds.stage_cap < padded) {  // grows only on the first large plan of a process: pinning synchronises with the device
-        if (ds.stage) CUDA_TRY(cudaFreeHost(ds.stage));
-        ds.stage = nullptr; ds.stage_cap = 0;
-        const size_t cap = std::max<size_t>(padded + padded / 2, size_t(32) << 20);
-        CUDA_TRY(cudaMallocHost(&ds.stage, cap));
-        ds.stage_cap = cap;
-    }
+    const int64_t rc = stage_reserve(ds, padded);
+    if (rc < 0) return rc;
     std::memcpy(ds.stage, v.data(), bytes);
     const size_t n16 = padded / 16;
     stage_in_kernel<<<unsigned(std::min<size_t>((n16 + 255) / 256, 1184)), 256, 0, ds.stream>>>(static_cast<const uint4*>(ds.stage), reinterpret_cast<uint4*>(dst), n16);
