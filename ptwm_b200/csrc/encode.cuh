@@ -24,6 +24,8 @@ struct SplitItem {
 };
 constexpr uint32_t SPLIT_TILE = 8192;
 
+constexpr uint64_t ENC_PAD = 64;  // bytes behind the planes and the slots that a 16-byte access may reach
+
 struct EncChunk {
     uint64_t plane_off;  // this chunk's bytes in the planes buffer
     uint64_t slot_off;   // four stream slots of slot_cap bytes each in the slot buffer (tANS / O1SAC: one stream over all four)
@@ -47,54 +49,19 @@ struct GatherItem {
 constexpr uint32_t GATHER_BARE = 0x100;
 constexpr uint32_t GATHER_NOFRAME = 0x200;  // an unchunked plane: inline state (if the codec has one) and payload, no frame header
 
-// layout of the table area of a chunk
-//   rANS:    freqs u16[256] | per symbol {reciprocal u32, bias u32, 2048 - freq u32, reciprocal shift u32}   (4.5 KiB)
-//   Huffman: lengths u8[256] | unused[256] | rev codes u16[256]                            (1 KiB)
-//   tANS:    norm u16[256] | delta_nb u32[256] | delta_find_state i32[256] | next-state u16[2048] | spread symbols u8[2048]
+// layout of the table area of a chunk (what the gather and the encoder need of it; the rest is rebuilt in shared memory)
+//   rANS:    freqs u16[256]
+//   Huffman: lengths u8[256] | codes u32[256]: reversed code | length << 16                 (1280 bytes)
+//   tANS:    norm u16[256]
 //   O1SAC:   joint counts u32[256][256] | row-start counts u32[256] | present u8[256] | rank u16[256] |
 //            pmf u16[257][256] (row 0 marginal, row 1 + c for context c) | cum u16[257][256]
-constexpr uint32_t ENC_TABLE_BYTES = 1024;
-constexpr uint32_t ENC_RANS_TABLE_BYTES = 512 + 4096;
-constexpr uint32_t ENC_TANS_TABLE_BYTES = 512 + 1024 + 1024 + 4096 + 2048;
+constexpr uint32_t ENC_FREQ_TABLE_BYTES = 512;
+constexpr uint32_t ENC_HUFF_TABLE_BYTES = 256 + 1024;
 constexpr uint32_t O1E_JOINT = 0, O1E_MARG = 262144, O1E_PRESENT = O1E_MARG + 1024, O1E_RANK = O1E_PRESENT + 256, O1E_PMF = O1E_RANK + 512,
                    O1E_CUM = O1E_PMF + 257 * 512, ENC_O1SAC_TABLE_BYTES = O1E_CUM + 257 * 512;
 constexpr uint32_t O1SAC_TOTAL = 4096;
 __host__ __device__ inline uint32_t enc_table_bytes(int codec) {
-    return codec == C_RANS ? ENC_RANS_TABLE_BYTES : codec == C_TANS ? ENC_TANS_TABLE_BYTES : codec == C_O1SAC ? ENC_O1SAC_TABLE_BYTES : ENC_TABLE_BYTES;
-}
-
-// The bytes of [p, p + n) handed to `f` one at a time, last to first (BACKWARD) or first to last, read from memory
-// in aligned 16-byte blocks wherever a whole block lies inside the range.  An encoding thread walks its own stream:
-// with single-byte loads every byte costs a 32-byte sector fetch of its own once the lines have left the L1.
-template <bool BACKWARD, class F>
-__device__ __forceinline__ void for_each_byte(const uint8_t* p, uint32_t n, F&& f) {
-    const uintptr_t lo = reinterpret_cast<uintptr_t>(p), hi = lo + n;
-    const uintptr_t first_block = (lo + 15) & ~uintptr_t(15), last_block = hi & ~uintptr_t(15);  // whole blocks: [first_block, last_block)
-    if (first_block >= last_block) {
-        if (BACKWARD) for (uint32_t k = n; k-- > 0;) f(uint32_t(p[k]));
-        else for (uint32_t k = 0; k < n; ++k) f(uint32_t(p[k]));
-        return;
-    }
-    if (BACKWARD) {
-        for (uintptr_t a = hi; a-- > last_block;) f(uint32_t(*reinterpret_cast<const uint8_t*>(a)));
-        for (uintptr_t b = last_block; b > first_block;) {
-            b -= 16;
-            const uint4 v = *reinterpret_cast<const uint4*>(b);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int k = 15; k >= 0; --k) f((w[k >> 2] >> (8 * (k & 3))) & 0xFFu);
-        }
-        for (uintptr_t a = first_block; a-- > lo;) f(uint32_t(*reinterpret_cast<const uint8_t*>(a)));
-    } else {
-        for (uintptr_t a = lo; a < first_block; ++a) f(uint32_t(*reinterpret_cast<const uint8_t*>(a)));
-        for (uintptr_t b = first_block; b < last_block; b += 16) {
-            const uint4 v = *reinterpret_cast<const uint4*>(b);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int k = 0; k < 16; ++k) f((w[k >> 2] >> (8 * (k & 3))) & 0xFFu);
-        }
-        for (uintptr_t a = last_block; a < hi; ++a) f(uint32_t(*reinterpret_cast<const uint8_t*>(a)));
-    }
+    return codec == C_HUFFMAN ? ENC_HUFF_TABLE_BYTES : codec == C_O1SAC ? ENC_O1SAC_TABLE_BYTES : ENC_FREQ_TABLE_BYTES;
 }
 
 __global__ void __launch_bounds__(256) split_kernel(const SplitItem* __restrict__ items, uint32_t n_items, uint8_t* __restrict__ planes) {
@@ -230,249 +197,605 @@ __global__ void __launch_bounds__(128) hist_kernel(const EncChunk* __restrict__ 
     }
 }
 
-// One thread per chunk builds the chunk's table for the codec its plane uses.
-__global__ void __launch_bounds__(64) table_kernel(const EncChunk* __restrict__ chunks, uint32_t n_chunks, const uint8_t* __restrict__ plane_codec,
-                                                   const uint32_t* __restrict__ hist, uint8_t* __restrict__ tables, EncResult* __restrict__ results) {
-    uint32_t ci = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ci >= n_chunks) return;
-    const EncChunk c = chunks[ci];
-    const uint32_t* raw = hist + uint64_t(ci) * 256;
-    uint8_t* tab = tables + c.table_off;
-    EncResult r{{0, 0, 0, 0}, 0, 0};
-    int codec = plane_codec[c.plane];
-    if (codec == C_O1SAC) return;  // fitted by its own kernels
-    if (codec == C_RANS && c.n) {
-        uint16_t* freqs = reinterpret_cast<uint16_t*>(tab);
-        uint4* sym = reinterpret_cast<uint4*>(tab + 512);
-        int ms = rans_normalize(raw, c.n, freqs);
-        if (ms >= 0) {
-            // x' = x + bias + floor(x / f) * (2048 - f) with the quotient from a rounded-up reciprocal: exact for every
-            // state below 2^31, i.e. identical to (x / f) * 2048 + x % f + start (entropy/rans/compress.rs:140-185)
-            uint32_t run = 0;
-            for (int i = 0; i < 256; ++i) {
-                const uint32_t f = freqs[i];
-                uint4 e = make_uint4(0, 0, 0, 0);
-                if (f == 1) e = make_uint4(0xFFFFFFFFu, run + 2047u, 2047u, 0u);
-                else if (f > 1) {
-                    uint32_t shift = 0;
-                    while (f > (1u << shift)) ++shift;
-                    e = make_uint4(uint32_t(((1ull << (shift + 31)) + f - 1) / f), run, 2048u - f, shift - 1);
-                }
-                sym[i] = e;
-                run += f;
-            }
-            r.hdr_n = uint32_t(ms); r.coded = 1;
-            // A chunk that cannot come out smaller than it is gets no encoding pass: the coder's output is at least the
-            // information content of the chunk under its table, less the four initial states, so when that alone (with a
-            // margin for the float logarithm) reaches the chunk's size the result would be discarded anyway
-            // (compress.rs: NotBeneficial).  Sign / mantissa planes are the usual case.
-            float bits = 0.f;
-            for (int i = 0; i <= ms; ++i) if (raw[i]) bits += float(raw[i]) * (11.f - log2f(float(freqs[i])));
-            const float lower = bits * (1.f - 1e-4f) / 8.f - 16.f + float(1 + 2 * (ms + 1) + 16);
-            if (lower >= float(c.n) + 64.f) r.coded = 0;
-        }
-    } else if (codec == C_HUFFMAN && c.n) {
-        uint32_t nf[512]; uint16_t parent[512]; uint8_t alive[512]; uint8_t sym_of[256];
-        uint8_t* lengths = tab;
-        int nw = huffman_lengths<uint32_t>(raw, lengths, nf, parent, alive, sym_of);
-        if (nw > 0) {
-            huffman_codes(lengths, reinterpret_cast<uint16_t*>(tab + 512));
-            r.hdr_n = uint32_t(nw); r.coded = 1;
-            // the four streams together hold at least ceil(total bits / 8) bytes: no encoding pass for a chunk that cannot shrink
-            uint64_t total_bits = 0;
-            for (int i = 0; i < nw; ++i) total_bits += uint64_t(raw[i]) * lengths[i];
-            if ((total_bits + 7) / 8 + (nw <= 127 ? 1 : 2) + (uint32_t(nw) + 1) / 2 + 16 >= c.n) r.coded = 0;
-        }
-    } else if (codec == C_TANS && c.n) {  // entropy/tans/mod.rs:199-266
-        uint16_t* norm = reinterpret_cast<uint16_t*>(tab);
-        uint32_t* dnb = reinterpret_cast<uint32_t*>(tab + 512);
-        int32_t* dfs = reinterpret_cast<int32_t*>(tab + 1536);
-        uint16_t* next_state = reinterpret_cast<uint16_t*>(tab + 2560);
-        uint8_t* spread = tab + 6656;
-        const int nsym = tans_normalize(raw, c.n, norm);
-        if (nsym >= 2) {
-            uint32_t pos = 0;
-            for (int s = 0; s < 256; ++s)
-                for (uint32_t k = 0; k < norm[s]; ++k) { spread[pos] = uint8_t(s); pos = (pos + 1283u) & 2047u; }
-            uint16_t fill[256];
-            uint32_t running = 0;
-            int32_t tot = 0;
-            for (int s = 0; s < 256; ++s) {
-                fill[s] = uint16_t(running); running += norm[s];
-                const uint32_t cnt = norm[s];
-                dnb[s] = 0; dfs[s] = 0;
-                if (cnt == 1) { dnb[s] = (11u << 16) - 2048u; dfs[s] = tot - 1; tot += 1; }
-                else if (cnt > 1) {
-                    const uint32_t max_bits = 11u - (31u - uint32_t(__clz(cnt - 1)));
-                    dnb[s] = (max_bits << 16) - (cnt << max_bits);
-                    dfs[s] = tot - int32_t(cnt); tot += int32_t(cnt);
-                }
-            }
-            for (uint32_t u = 0; u < 2048; ++u) { const int s = spread[u]; next_state[fill[s]++] = uint16_t(2048u + u); }
-            r.hdr_n = uint32_t(nsym); r.coded = 1;
-        }
+// ---- tables --------------------------------------------------------------------------------------------
+// One warp per chunk turns its histogram into the table of the codec its plane uses; lane l owns the symbols 8 l .. 8 l + 7.
+// The same choices as rans_normalize, tans_normalize, huffman_lengths of encode_tables.cuh, made by all
+// lanes together: with one thread per chunk the 256-step loops and the Huffman tree took 0.6 - 1.1 ms however few chunks
+// there were.
+__device__ __forceinline__ uint32_t warp_prefix(uint32_t v, uint32_t lane) {  // exclusive
+    uint32_t incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d); if (lane >= uint32_t(d)) incl += t; }
+    return incl - v;
+}
+// The first index at which the largest of all values stands.
+__device__ __forceinline__ uint32_t warp_first_argmax(const uint32_t v[8], uint32_t lane, uint32_t& best) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m = max(m, v[k]);
+    best = __reduce_max_sync(0xFFFFFFFFu, m);
+    uint32_t at = 0xFFFFFFFFu;
+#pragma unroll
+    for (int k = 7; k >= 0; --k) if (v[k] == best) at = lane * 8 + k;
+    return __reduce_min_sync(0xFFFFFFFFu, at);
+}
+// floor(c * 2048 / n), at least one where c is not zero; returns the sum over all symbols
+__device__ __forceinline__ uint32_t warp_scale_counts(const uint32_t c[8], uint32_t n, uint32_t f[8]) {
+    uint32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        f[k] = 0;
+        if (c[k]) { f[k] = uint32_t(uint64_t(c[k]) * 2048u / n); if (f[k] == 0) f[k] = 1; }
+        sum += f[k];
     }
-    results[ci] = r;
+    return __reduce_add_sync(0xFFFFFFFFu, sum);
+}
+__device__ __forceinline__ void warp_add_at(uint32_t f[8], uint32_t lane, uint32_t at, uint32_t d) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) if (lane * 8 + k == at) f[k] += d;
+}
+__device__ __forceinline__ void warp_store_freqs(uint8_t* tab, uint32_t lane, const uint32_t f[8]) {
+    *reinterpret_cast<uint4*>(tab + 16 * lane) = make_uint4(f[0] | f[1] << 16, f[2] | f[3] << 16, f[4] | f[5] << 16, f[6] | f[7] << 16);
+}
+__device__ __forceinline__ void warp_load_freqs(const uint8_t* tab, uint32_t lane, uint32_t f[8]) {
+    const uint4 v = *reinterpret_cast<const uint4*>(tab + 16 * lane);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) f[k] = (w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
 }
 
-// tANS (entropy/tans/mod.rs:268-318): one stream per chunk, so one lane per chunk; the symbols are walked last to first and the
-// bits go upward from the start of the chunk's slot area.  A symbol is two table look-ups that depend on the running
-// state, so the tables of the 32 chunks of a block sit in shared memory, laid out [entry][lane] like the decoder's:
-// next state (u16 x 2048), and per symbol the bit-count term (u32) and the state offset (i16).  With the tables in global
-// memory every symbol waited for the L2 twice.
-constexpr int TENC_CHUNKS = 32;
-constexpr int TENC_NEXT_BYTES = 2048 * 32 * 2, TENC_DNB_BYTES = 256 * 32 * 4, TENC_DFS_BYTES = 256 * 32 * 2;
-constexpr int TENC_SMEM = TENC_NEXT_BYTES + TENC_DNB_BYTES + TENC_DFS_BYTES;
-__global__ void __launch_bounds__(32, 1) tans_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
-                                                            const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
-                                                            EncResult* __restrict__ results) {
-    extern __shared__ __align__(16) uint8_t tenc_smem[];
-    const uint32_t lane = threadIdx.x, li = blockIdx.x * TENC_CHUNKS + lane;
-    if (li >= n_list) return;
-    const uint32_t ci = list[li];
-    const EncChunk c = chunks[ci];
-    if (!results[ci].coded || !c.n) return;  // lanes do not depend on one another
-    uint16_t* next_state = reinterpret_cast<uint16_t*>(tenc_smem) + lane;                                 // entry e at next_state[e * 32]
-    uint32_t* dnb = reinterpret_cast<uint32_t*>(tenc_smem + TENC_NEXT_BYTES) + lane;                       // symbol s at dnb[s * 32]
-    int16_t* dfs = reinterpret_cast<int16_t*>(tenc_smem + TENC_NEXT_BYTES + TENC_DNB_BYTES) + lane;       // symbol s at dfs[s * 32]
-    {
-        const uint8_t* tab = tables + c.table_off;  // table areas start on 16-byte boundaries
-        const uint4* g_dnb = reinterpret_cast<const uint4*>(tab + 512);
-        const uint4* g_dfs = reinterpret_cast<const uint4*>(tab + 1536);
-        const uint4* g_next = reinterpret_cast<const uint4*>(tab + 2560);
-        for (uint32_t k = 0; k < 64; ++k) {
-            const uint4 a = g_dnb[k], b = g_dfs[k];
-            dnb[(4 * k + 0) * 32] = a.x; dnb[(4 * k + 1) * 32] = a.y; dnb[(4 * k + 2) * 32] = a.z; dnb[(4 * k + 3) * 32] = a.w;
-            dfs[(4 * k + 0) * 32] = int16_t(int32_t(b.x)); dfs[(4 * k + 1) * 32] = int16_t(int32_t(b.y));
-            dfs[(4 * k + 2) * 32] = int16_t(int32_t(b.z)); dfs[(4 * k + 3) * 32] = int16_t(int32_t(b.w));
-        }
-        for (uint32_t k = 0; k < 256; ++k) {
-            const uint4 v = g_next[k];
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+struct HuffWork {             // shared memory of one warp while it builds a Huffman code
+    uint32_t leaf_f[256];     // count of leaf i (leaves numbered in symbol order)
+    uint32_t sorted_f[257];   // counts in increasing (count, leaf) order
+    uint32_t node_f[256];     // internal nodes in the order they are made; later their depth
+    uint16_t leaf_parent[256], node_parent[256];  // by place in sorted order / by node
+    uint8_t leaf_sym[256], sorted_leaf[256], len[256];
+};
+// Code lengths: the two smallest nodes under the (count, node id) order are merged again and again.  With the leaves sorted
+// that is the two-queue method: merged nodes come out in increasing count order, and on equal counts a leaf goes first
+// because its id is smaller.  Returns the number of weights to store; the lengths end up in w.len.
+__device__ __forceinline__ uint32_t warp_huffman_lengths(const uint32_t c[8], uint32_t lane, HuffWork& w) {
+    uint32_t mine = 0;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) next_state[(8 * k + j) * 32] = uint16_t(w[j >> 1] >> (16 * (j & 1)));
+    for (int k = 0; k < 8; ++k) mine += c[k] != 0;
+    uint32_t at = warp_prefix(mine, lane), last = 0;
+    const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, mine);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        w.len[lane * 8 + k] = 0;
+        if (c[k]) { w.leaf_f[at] = c[k]; w.leaf_sym[at] = uint8_t(lane * 8 + k); ++at; last = lane * 8 + k; }
+    }
+    last = __reduce_max_sync(0xFFFFFFFFu, last);
+    if (n == 0) return 0;
+    __syncwarp();
+    if (n == 1) { if (lane == 0) w.len[w.leaf_sym[0]] = 1; __syncwarp(); return last + 1; }
+    for (uint32_t i = lane; i < n; i += 32) {
+        const uint32_t f = w.leaf_f[i];
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < n; ++j) { const uint32_t g = w.leaf_f[j]; rank += (g < f) || (g == f && j < i); }
+        w.sorted_f[rank] = f; w.sorted_leaf[rank] = uint8_t(i);
+    }
+    __syncwarp();
+    if (lane == 0) {
+        uint32_t i = 0, j = 0, made = 0;  // next leaf, next merged node, merged nodes made
+        uint32_t fi = w.sorted_f[0], fj = 0;
+        while (made < n - 1) {
+            uint32_t sum = 0;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (i < n && (j >= made || fi <= fj)) { sum += fi; w.leaf_parent[i] = uint16_t(made); ++i; fi = i < n ? w.sorted_f[i] : 0u; }
+                else { sum += fj; w.node_parent[j] = uint16_t(made); ++j; fj = j < made ? w.node_f[j] : 0u; }
+            }
+            w.node_f[made] = sum;
+            if (j == made) fj = sum;
+            ++made;
+        }
+        w.node_f[n - 2] = 0;  // depths, from the root down: a parent is always made after its children
+        for (uint32_t k = n - 2; k-- > 0;) w.node_f[k] = w.node_f[w.node_parent[k]] + 1;
+    }
+    __syncwarp();
+    bool clamped = false;
+    for (uint32_t r = lane; r < n; r += 32) {
+        uint32_t d = w.node_f[w.leaf_parent[r]] + 1;
+        if (d > 11) { d = 11; clamped = true; }
+        w.len[w.leaf_sym[w.sorted_leaf[r]]] = uint8_t(d);
+    }
+    __syncwarp();
+    if (__any_sync(0xFFFFFFFFu, clamped)) {  // lengthen the first of the shortest codes until the lengths fit a prefix code
+        uint32_t len[8], kraft = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { len[k] = w.len[lane * 8 + k]; kraft += len[k] ? 1u << (11 - len[k]) : 0u; }
+        kraft = __reduce_add_sync(0xFFFFFFFFu, kraft);
+        while (kraft > 2048) {
+            uint32_t key = 0xFFFFFFFFu;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) if (len[k] && len[k] < 11) key = min(key, len[k] << 8 | (lane * 8 + k));
+            key = __reduce_min_sync(0xFFFFFFFFu, key);
+            if (key == 0xFFFFFFFFu) break;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) if (lane * 8 + k == (key & 0xFFu)) ++len[k];
+            kraft -= 1u << (10 - (key >> 8));  // 2^(11 - len) becomes half of that
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) w.len[lane * 8 + k] = uint8_t(len[k]);
+        __syncwarp();
+    }
+    return last + 1;
+}
+
+__global__ void __launch_bounds__(128) table_kernel(const EncChunk* __restrict__ chunks, uint32_t n_chunks, const uint8_t* __restrict__ plane_codec,
+                                                    const uint32_t* __restrict__ hist, uint8_t* __restrict__ tables, EncResult* __restrict__ results) {
+    __shared__ HuffWork huff[4];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ci = blockIdx.x * 4 + warp;
+    if (ci >= n_chunks) return;
+    const EncChunk c = chunks[ci];
+    const int codec = plane_codec[c.plane];
+    if (codec == C_O1SAC) return;  // fitted by its own kernels
+    EncResult r{{0, 0, 0, 0}, 0, 0};
+    if (codec != C_IDENTITY && c.n) {
+        uint8_t* tab = tables + c.table_off;
+        const uint4* raw = reinterpret_cast<const uint4*>(hist + uint64_t(ci) * 256) + 2 * lane;
+        const uint4 a = raw[0], b = raw[1];
+        const uint32_t cnt[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        if (codec == C_HUFFMAN) {
+            HuffWork& w = huff[warp];
+            const uint32_t nw = warp_huffman_lengths(cnt, lane, w);
+            if (nw) {
+                // canonical codes: first code of every length, then symbols in order (tree.rs:119-170), bit-reversed for the LSB-first stream
+                uint32_t len[8], code[8] = {0, 0, 0, 0, 0, 0, 0, 0}, next = 0, bits = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) { len[k] = w.len[lane * 8 + k]; bits += cnt[k] * len[k]; }
+                for (uint32_t l = 1; l < 12; ++l) {
+                    uint32_t mine = 0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) mine += len[k] == l;
+                    uint32_t at = next + warp_prefix(mine, lane);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) if (len[k] == l) code[k] = __brev(at++) >> (32 - l);
+                    next = (next + __reduce_add_sync(0xFFFFFFFFu, mine)) << 1;
+                }
+                *reinterpret_cast<uint2*>(tab + 8 * lane) = make_uint2(len[0] | len[1] << 8 | len[2] << 16 | len[3] << 24, len[4] | len[5] << 8 | len[6] << 16 | len[7] << 24);
+                uint4* out = reinterpret_cast<uint4*>(tab + 256) + 2 * lane;
+                out[0] = make_uint4(code[0] | len[0] << 16, code[1] | len[1] << 16, code[2] | len[2] << 16, code[3] | len[3] << 16);
+                out[1] = make_uint4(code[4] | len[4] << 16, code[5] | len[5] << 16, code[6] | len[6] << 16, code[7] | len[7] << 16);
+                r.hdr_n = nw; r.coded = 1;
+                // the four streams together hold at least ceil(total bits / 8) bytes: no encoding pass for a chunk that cannot shrink
+                uint64_t total_bits = bits;  // a lane's share stays below 2^32 only for chunks below 2^28 symbols
+                if (c.n >= (1u << 28)) { total_bits = 0; for (int k = 0; k < 8; ++k) total_bits += uint64_t(cnt[k]) * len[k]; }
+#pragma unroll
+                for (int d = 16; d; d >>= 1) total_bits += __shfl_xor_sync(0xFFFFFFFFu, total_bits, d);
+                if ((total_bits + 7) / 8 + (nw <= 127 ? 1 : 2) + (nw + 1) / 2 + 16 >= c.n) r.coded = 0;
+            }
+        } else {
+            uint32_t f[8], best, present = 0;
+            const uint32_t sum = warp_scale_counts(cnt, c.n, f), top = warp_first_argmax(cnt, lane, best);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) present |= uint32_t(cnt[k] != 0) << k;
+            if (codec == C_RANS) {
+                bool ok = true;
+                if (sum > 2048) {  // the excess comes off the most frequent symbol, or the chunk stays raw
+                    uint32_t ft = 0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) if (lane * 8 + k == top) ft = f[k];
+                    ft = __reduce_max_sync(0xFFFFFFFFu, ft);
+                    ok = ft > sum - 2048;
+                }
+                if (ok) {
+                    warp_add_at(f, lane, top, 2048 - sum);
+                    warp_store_freqs(tab, lane, f);
+                    const uint32_t ms = __reduce_max_sync(0xFFFFFFFFu, present ? lane * 8 + 31 - __clz(present) : 0u);
+                    r.hdr_n = ms; r.coded = 1;
+                    // A chunk that cannot come out smaller than it is gets no encoding pass: the coder's output is at least the
+                    // information content of the chunk under its table, less the four initial states, so when that alone (with a
+                    // margin for the float logarithm) reaches the chunk's size the result would be discarded anyway
+                    // (compress.rs: NotBeneficial).  Sign / mantissa planes are the usual case.
+                    float bits = 0.f;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) if (cnt[k]) bits += float(cnt[k]) * (11.f - log2f(float(f[k])));
+#pragma unroll
+                    for (int d = 16; d; d >>= 1) bits += __shfl_xor_sync(0xFFFFFFFFu, bits, d);
+                    const float lower = bits * (1.f - 1e-4f) / 8.f - 16.f + float(1 + 2 * (ms + 1) + 16);
+                    if (lower >= float(c.n) + 64.f) r.coded = 0;
+                }
+            } else {  // tANS (entropy/tans/mod.rs:153-194)
+                uint32_t left = sum;
+                while (left > 2048) {  // one at a time from the first largest entry above one
+                    uint32_t most;
+                    const uint32_t at = warp_first_argmax(f, lane, most);
+                    if (most <= 1) break;
+                    warp_add_at(f, lane, at, 0xFFFFFFFFu);
+                    --left;
+                }
+                if (left < 2048) warp_add_at(f, lane, top, 2048 - left);
+                const uint32_t nsym = __reduce_add_sync(0xFFFFFFFFu, __popc(present));
+                warp_store_freqs(tab, lane, f);
+                if (nsym >= 2) { r.hdr_n = nsym; r.coded = 1; }
+            }
         }
     }
-    uint32_t* w32 = reinterpret_cast<uint32_t*>(slots + c.slot_off);  // slot areas start on 16-byte boundaries
-    uint64_t acc = 0, total_bits = 0;
-    uint32_t nb_acc = 0, words = 0, value = 2048;
-    auto add_bits = [&](uint32_t v, uint32_t nb) {
-        acc |= uint64_t(v & ((1u << nb) - 1u)) << nb_acc;
-        nb_acc += nb; total_bits += nb;
-        if (nb_acc >= 32) { w32[words++] = uint32_t(acc); acc >>= 32; nb_acc -= 32; }
-    };
-    auto step = [&](uint32_t b) {
-        const uint32_t nb = (value + dnb[b * 32]) >> 16;
-        add_bits(value, nb);
-        value = next_state[uint32_t(int32_t(value >> nb) + int32_t(dfs[b * 32])) * 32];
-    };
-    // the plane's bytes last to first: single bytes down to a 16-byte boundary, then aligned blocks, each requested while the
-    // one before it is coded, then the bytes below the first boundary
-    const uintptr_t lo = reinterpret_cast<uintptr_t>(planes + c.plane_off), hi = lo + c.n;
+    if (lane == 0) results[ci] = r;
+}
+
+// ---- streams -------------------------------------------------------------------------------------------
+// The bytes of rANS and Huffman streams are made last to first.  They are appended upward from the start of the stream's slot
+// in the order they are made, and the gather turns them around.
+// f(sym) for the bytes of [lo, hi), last to first, out of aligned 16-byte blocks, each requested while the one above it is
+// worked on; `block` gets the sixteen bytes of a whole block, highest first.
+template <class Byte, class Block>
+__device__ __forceinline__ void walk_down(uintptr_t lo, uintptr_t hi, Byte&& byte, Block&& block) {
     const uintptr_t first_block = (lo + 15) & ~uintptr_t(15), last_block = hi & ~uintptr_t(15);
     if (first_block >= last_block) {
-        for (uintptr_t a = hi; a-- > lo;) step(*reinterpret_cast<const uint8_t*>(a));
-    } else {
-        for (uintptr_t a = hi; a-- > last_block;) step(*reinterpret_cast<const uint8_t*>(a));
-        uintptr_t b = last_block - 16;
-        uint4 ahead = *reinterpret_cast<const uint4*>(b);
-        for (;;) {
-            const uint4 v = ahead;
-            const bool more = b > first_block;
-            if (more) ahead = *reinterpret_cast<const uint4*>(b - 16);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int k = 15; k >= 0; --k) step((w[k >> 2] >> (8 * (k & 3))) & 0xFFu);
-            if (!more) break;
-            b -= 16;
-        }
-        for (uintptr_t a = first_block; a-- > lo;) step(*reinterpret_cast<const uint8_t*>(a));
+        for (uintptr_t a = hi; a-- > lo;) byte(uint32_t(*reinterpret_cast<const uint8_t*>(a)));
+        return;
     }
-    add_bits(value, 11);
-    uint8_t* tail = reinterpret_cast<uint8_t*>(w32 + words);
-    uint32_t bytes = words * 4;
-    while (nb_acc > 0) { *tail++ = uint8_t(acc); acc >>= 8; nb_acc = nb_acc > 8 ? nb_acc - 8 : 0; ++bytes; }
-    results[ci].stream_len[0] = bytes;
-    results[ci].stream_len[1] = uint32_t(total_bits);
-    results[ci].stream_len[2] = uint32_t(total_bits >> 32);
+    for (uintptr_t a = hi; a-- > last_block;) byte(uint32_t(*reinterpret_cast<const uint8_t*>(a)));
+    uintptr_t b = last_block - 16;
+    uint4 ahead = *reinterpret_cast<const uint4*>(b);
+    for (;;) {
+        const uint4 v = ahead;
+        const bool more = b > first_block;
+        if (more) ahead = *reinterpret_cast<const uint4*>(b - 16);
+        block(v);
+        if (!more) break;
+        b -= 16;
+    }
+    for (uintptr_t a = first_block; a-- > lo;) byte(uint32_t(*reinterpret_cast<const uint8_t*>(a)));
 }
 
-// One thread per stream.  Bytes are produced last-to-first for both codecs, so
-// each stream is written downward from the end of its slot and ends up in
-// decode order; stream_len tells the gather where it starts.
-__global__ void __launch_bounds__(128) encode_kernel(const EncChunk* __restrict__ chunks, uint32_t n_chunks, const uint8_t* __restrict__ plane_codec,
-                                                     const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
-                                                     EncResult* __restrict__ results) {
-    uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t ci = gi >> 2, s = gi & 3;
-    if (ci >= n_chunks) return;
+// rANS: one lane per stream, eight chunks per warp.  A symbol is a serial step of the coder's state: its chain is kept short
+// (what the symbol's step needs sits in shared memory, 16 bytes per symbol, read ahead of use because it depends on the data
+// alone; the number of bytes that leave is 0, 1 or 2 by two compares) and so is the number of instructions, because the
+// integer pipe is what bounds a launch that fills the GPU: the bytes that leave are shifted into a register pair from above,
+// and every two symbols the oldest word of the pair is put into a ring in shared memory whether it is full or not (only the
+// write position moves on a full word), from where sixteen bytes at a time go out.  A branch with a store per full word was
+// taken by some lane in nearly every step.  The rows cover `range` symbols from the chunk's first one on: the host knows the
+// span of a plane's alphabet and sends planes of similar span together, so that exponent planes (some 40 values) keep 22
+// blocks on an SM.  With 16-byte entries in global memory and a loop per byte a symbol took 330 ns.
+// x' = x + bias + floor(x / f) * (2048 - f) with the quotient from a rounded-up reciprocal: exact for every state below 2^31,
+// i.e. identical to (x / f) * 2048 + x % f + start (entropy/rans/compress.rs:140-185).
+constexpr uint32_t RENC_RING = 16;  // words per lane: up to 3 waiting, up to 8 more in sixteen symbols, one being filled
+__host__ __device__ inline uint32_t renc_smem_bytes(uint32_t range) { return RANS_WARP_CHUNKS * (range + 1) * 16 + RENC_RING * 32 * 4; }  // a row is one entry longer: rows shifted in the banks
+__global__ void __launch_bounds__(32) rans_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list, uint32_t range,
+                                                         const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
+                                                         EncResult* __restrict__ results) {
+    extern __shared__ __align__(16) uint8_t renc_smem[];
+    uint4* entries = reinterpret_cast<uint4*>(renc_smem);
+    uint32_t* ring_all = reinterpret_cast<uint32_t*>(renc_smem + RANS_WARP_CHUNKS * (range + 1) * 16);
+    const uint32_t lane = threadIdx.x, c8 = lane >> 2, s = lane & 3, li = blockIdx.x * RANS_WARP_CHUNKS + c8;
+    const uint32_t ci = li < n_list ? list[li] : 0xFFFFFFFFu;
+    EncChunk c{};
+    if (li < n_list) c = chunks[ci];
+    const bool live = li < n_list && c.n && results[ci].coded;
+    uint32_t first_sym = 0;
+    for (uint32_t k = 0; k < RANS_WARP_CHUNKS; ++k) {  // entry: reciprocal, bias << 8 | reciprocal shift, 2048 - frequency, frequency << 20
+        if (!__shfl_sync(0xFFFFFFFFu, uint32_t(live), 4 * k)) continue;
+        uint32_t f[8], sum = 0, lowest = 0xFFFFFFFFu;
+        warp_load_freqs(tables + __shfl_sync(0xFFFFFFFFu, c.table_off, 4 * k), lane, f);
+#pragma unroll
+        for (int j = 7; j >= 0; --j) { sum += f[j]; if (f[j]) lowest = lane * 8 + j; }
+        lowest = __reduce_min_sync(0xFFFFFFFFu, lowest);
+        if (c8 == k) first_sym = lowest;
+        uint32_t start = warp_prefix(sum, lane);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t at = lane * 8 + j - lowest;  // (wraps for the symbols below the first)
+            uint4 e = make_uint4(0xFFFFFFFFu, (start + 2047u) << 8, 2047u, 1u << 20);  // f = 1: the quotient comes out one short of x
+            if (f[j] > 1) {
+                const uint32_t shift = 32 - __clz(f[j] - 1);  // smallest with f <= 2^shift
+                e = make_uint4(uint32_t(((1ull << (shift + 31)) + f[j] - 1) / f[j]), start << 8 | (shift - 1), 2048u - f[j], f[j] << 20);
+            }
+            if (f[j] && at < range) entries[k * (range + 1) + at] = e;
+            start += f[j];
+        }
+    }
+    __syncwarp();
+    if (!live) return;
+    uint32_t start, len;
+    split_four_dev(c.n, s, start, len);
+    uint8_t* slot = slots + c.slot_off + uint64_t(s) * c.slot_cap;
+    const uint4* row = entries + c8 * (range + 1) - first_sym;
+    uint32_t* ring = ring_all + lane;
+    uint32_t x = 1u << 23;
+    uint32_t b_lo = 0, b_hi = 0, have = 0;  // the youngest `have` bits wait at the top of b_hi:b_lo; below 32 between pairs of symbols
+    uint32_t put = 0, sent = 0;             // words made / stored
+    auto step = [&](const uint4& e) {
+        // bytes leave while x >= f << 20 (= ((L >> 11) << 8) * f): at most two, the state being below 2^31
+        uint32_t sh = x >= e.w ? 8u : 0u;
+        sh = (x >> 8) >= e.w ? 16u : sh;
+        b_lo = __funnelshift_r(b_lo, b_hi, sh);
+        b_hi = __funnelshift_r(b_hi, x, sh);
+        have += sh;
+        x >>= sh;
+        x = x + (e.y >> 8) + __funnelshift_r(__umulhi(x, e.x), 0u, e.y) * e.z;  // shift by the low five bits of e.y
+    };
+    auto settle = [&]() {
+        ring[(put & (RENC_RING - 1)) * 32] = __funnelshift_rc(b_lo, b_hi, 64 - have);  // the oldest word when there is one
+        const bool full = have >= 32;
+        put += full; have -= full ? 32u : 0u;
+    };
+    auto drain = [&]() {  // sixteen bytes out for every lane that has them, when any has
+        if (__any_sync(__activemask(), put - sent >= 4)) {
+            if (put - sent >= 4) {
+                uint32_t w[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) w[k] = ring[((sent + k) & (RENC_RING - 1)) * 32];
+                *reinterpret_cast<uint4*>(slot + 4 * size_t(sent)) = make_uint4(w[0], w[1], w[2], w[3]);
+                sent += 4;
+            }
+        }
+    };
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(planes + c.plane_off) + start;
+    walk_down(lo, lo + len, [&](uint32_t b) { step(row[b]); settle(); drain(); },
+              [&](const uint4& v) {
+                  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                  for (int h = 3; h >= 0; --h) {
+                      uint4 e[4];
+#pragma unroll
+                      for (int k = 0; k < 4; ++k) e[k] = row[(w[h] >> (8 * k)) & 0xFFu];
+                      step(e[3]); step(e[2]); settle();
+                      step(e[1]); step(e[0]); settle();
+                  }
+                  drain();
+                  drain();
+              });
+    // the final state, little-endian once the bytes are turned around, then what waits
+    for (int k = 3; k >= 0; --k) {
+        b_lo = __funnelshift_r(b_lo, b_hi, 8);
+        b_hi = __funnelshift_r(b_hi, x >> (8 * k), 8);
+        have += 8;
+        settle();
+    }
+    for (; sent < put; ++sent) *reinterpret_cast<uint32_t*>(slot + 4 * size_t(sent)) = ring[(sent & (RENC_RING - 1)) * 32];
+    if (have) *reinterpret_cast<uint32_t*>(slot + 4 * size_t(put)) = b_hi >> (32 - have);
+    results[ci].stream_len[s] = 4 * put + (have + 7) / 8;
+}
+
+// Huffman: the place of a symbol's bits follows from the lengths before it, so a warp codes a stream 512 symbols at a time:
+// every lane strings its sixteen codes together, a prefix sum over the lanes gives the bit each string starts at, and the
+// strings are put together in shared memory.  (One thread per stream took 107 ns per symbol.)
+constexpr uint32_t HENC_LANE = 16, HENC_WORDS = (32 * HENC_LANE * 11 + 31) / 32 + 2;
+__global__ void __launch_bounds__(128) huffman_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
+                                                             const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
+                                                             EncResult* __restrict__ results) {
+    __shared__ uint32_t codes[256];
+    __shared__ uint32_t words_all[4][HENC_WORDS];
+    const uint32_t ci = list[blockIdx.x], lane = threadIdx.x & 31, s = threadIdx.x >> 5;
     const EncChunk c = chunks[ci];
-    int codec = plane_codec[c.plane];
-    if (codec == C_O1SAC || codec == C_TANS || !results[ci].coded) return;  // those two have kernels of their own
+    if (!c.n || !results[ci].coded) return;
+    const uint32_t* g_codes = reinterpret_cast<const uint32_t*>(tables + c.table_off + 256);
+    for (uint32_t i = threadIdx.x; i < 256; i += 128) codes[i] = g_codes[i];
+    uint32_t* words = words_all[s];
+    for (uint32_t i = lane; i < HENC_WORDS; i += 32) words[i] = 0;
+    __syncthreads();
     uint32_t start, len;
     split_four_dev(c.n, s, start, len);
     const uint8_t* src = planes + c.plane_off + start;
-    uint8_t* slot_end = slots + c.slot_off + uint64_t(s + 1) * c.slot_cap;
-    uint8_t* w = slot_end;
-    // Bytes go out downward.  Single byte stores to global memory are what this kernel used to wait for, so
-    // once the write position is 8-byte aligned eight bytes are collected (the first produced ends up highest,
-    // as in memory) and stored as one word.
-    uint64_t acc = 0;
-    uint32_t have = 0;
-    auto put = [&](uint32_t b) {
-        if (have == 0 && (reinterpret_cast<uintptr_t>(w) & 7)) { *--w = uint8_t(b); return; }
-        acc = (acc << 8) | (b & 0xFFu);
-        if (++have == 8) { w -= 8; *reinterpret_cast<uint64_t*>(w) = acc; have = 0; acc = 0; }
+    uint8_t* slot = slots + c.slot_off + uint64_t(s) * c.slot_cap;
+    uint32_t* out = reinterpret_cast<uint32_t*>(slot);
+    uint32_t have = 0;  // bits of the word that is not full yet, which stays in words[0]
+    auto fetch = [&](uint32_t at, uint32_t n, uint64_t& a, uint64_t& b) {  // up to sixteen bytes from src + at
+        a = b = 0;
+        if (n == HENC_LANE) { a = ld8_unaligned(src + at); b = ld8_unaligned(src + at + 8); }
+        else { a = ld_bytes(src + at, n < 8 ? n : 8); if (n > 8) b = ld_bytes(src + at + 8, n - 8); }
     };
-    auto flush = [&]() { while (have) { --have; *--w = uint8_t(acc >> (8 * have)); } };
-    const uint8_t* tab = tables + c.table_off;
-    if (codec == C_RANS) {
-        const uint4* syms = reinterpret_cast<const uint4*>(tab + 512);
-        uint32_t x = 1u << 23;
-        for_each_byte<true>(src, len, [&](uint32_t sym) {
-            const uint4 e = __ldg(syms + sym);
-            const uint32_t max_state = (2048u - e.z) << 20;  // ((L >> 11) << 8) * freq
-            while (x >= max_state) { put(x); x >>= 8; }
-            x = x + e.y + (__umulhi(x, e.x) >> e.w) * e.z;
-        });
-        put(x >> 24); put(x >> 16); put(x >> 8); put(x);  // the final state, little-endian, below the renormalisation bytes
-    } else {
-        const uint8_t* lengths = tab;
-        const uint16_t* rev = reinterpret_cast<const uint16_t*>(tab + 512);
-        uint64_t bits = 0; uint32_t cnt = 0;
-        for_each_byte<false>(src, len, [&](uint32_t sym) {
-            bits |= uint64_t(rev[sym]) << cnt;
-            cnt += lengths[sym];
-            while (cnt >= 8) { put(uint32_t(bits)); bits >>= 8; cnt -= 8; }
-        });
-        if (cnt) put(uint32_t(bits));
+    auto count_at = [&](uint32_t base) -> uint32_t { const uint32_t at = base + lane * HENC_LANE; return at >= len ? 0u : len - at < HENC_LANE ? len - at : HENC_LANE; };
+    uint64_t na, nb;
+    fetch(lane * HENC_LANE, count_at(0), na, nb);
+    for (uint32_t base = 0; base < len; base += 32 * HENC_LANE) {
+        const uint32_t n = count_at(base);
+        const uint64_t ca = na, cb = nb;
+        if (base + 32 * HENC_LANE < len) fetch(base + (32 + lane) * HENC_LANE, count_at(base + 32 * HENC_LANE), na, nb);  // the next round's symbols
+        uint32_t e[HENC_LANE], bits = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < HENC_LANE; ++k) {
+            const uint32_t sy = uint32_t((k < 8 ? ca : cb) >> (8 * (k & 7))) & 0xFFu;
+            e[k] = k < n ? codes[sy] : 0u;
+            bits += e[k] >> 16;
+        }
+        const uint32_t before = warp_prefix(bits, lane), total = __shfl_sync(0xFFFFFFFFu, before + bits, 31);
+        const uint32_t at = have + before;
+        uint32_t w = at >> 5, fill = at & 31, lo = 0;
+        bool first = true;  // the word the lane before this one may also write into
+#pragma unroll
+        for (uint32_t k = 0; k < HENC_LANE; ++k) {
+            const uint32_t cd = e[k] & 0xFFFFu, l = e[k] >> 16;
+            lo |= cd << fill;
+            fill += l;
+            if (fill >= 32) {
+                if (first) atomicOr(&words[w], lo); else words[w] = lo;
+                first = false;
+                ++w; fill -= 32;
+                lo = fill ? cd >> (l - fill) : 0u;
+            }
+        }
+        if (fill && lo) atomicOr(&words[w], lo);
+        __syncwarp();
+        const uint32_t full = (have + total) >> 5;
+        have = (have + total) & 31;
+        const uint32_t rest = words[full];
+        for (uint32_t i = lane; i < full; i += 32) out[i] = words[i];
+        __syncwarp();
+        for (uint32_t i = lane; i <= full; i += 32) words[i] = i == 0 ? rest : 0u;
+        if (lane == 0 && full == 0) words[0] = rest;
+        out += full;
+        __syncwarp();
     }
-    flush();
-    results[ci].stream_len[s] = uint32_t(slot_end - w);
+    if (lane == 0) {
+        if (have) *out = words[0];
+        results[ci].stream_len[s] = uint32_t(reinterpret_cast<uint8_t*>(out) - slot) + (have + 7) / 8;
+    }
 }
 
-// n bytes from s to d by the threads of a block: d is brought to a 16-byte boundary, then every thread moves 16 bytes at
-// a time, the source words taken aligned and shifted into place (a word that holds a needed byte is read whole; device
-// allocations are padded beyond that).
+// tANS (entropy/tans/mod.rs:268-318): one serial stream per chunk, its symbols walked last to first, its bits going upward.
+// One warp per chunk all the same: the chunk is cut into 32 runs of symbols and every lane codes its run from a guessed state.
+// Two coders with different states that see the same symbols meet after a while (both states of a pair fall into the few
+// states of a rare symbol; about 1,100 symbols on an exponent plane) and then stay together, so most lanes leave their run in
+// the state the serial coder has there.  The state a lane leaves in is where the lane below must start: lanes whose start
+// was not that go again until nobody's changes.  Each round settles at least one more lane, so the worst case is the serial
+// chain.  A last pass writes the bits at the places the runs' bit counts give.
+constexpr uint32_t TENC_MIN_RUN = 256;  // shorter runs would hardly ever end in the right state
+__global__ void __launch_bounds__(32) tans_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
+                                                         const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
+                                                         EncResult* __restrict__ results) {
+    __shared__ uint16_t next_state[2048];
+    __shared__ uint2 sym[256];        // bit-count term, offset into next_state
+    __shared__ uint16_t fill[256];
+    __shared__ uint8_t spread[2048];
+    const uint32_t lane = threadIdx.x, ci = list[blockIdx.x];
+    const EncChunk c = chunks[ci];
+    if (!results[ci].coded || !c.n) return;
+    {
+        uint32_t f[8], sum = 0;
+        warp_load_freqs(tables + c.table_off, lane, f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum += f[k];
+        uint32_t run = warp_prefix(sum, lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            uint2 e = make_uint2(0, 0);
+            if (f[k] == 1) e = make_uint2((11u << 16) - 2048u, run - 1);
+            else if (f[k] > 1) {
+                const uint32_t max_bits = 11u - (31u - uint32_t(__clz(f[k] - 1)));
+                e = make_uint2((max_bits << 16) - (f[k] << max_bits), run - f[k]);
+            }
+            sym[lane * 8 + k] = e;
+            fill[lane * 8 + k] = uint16_t(run);
+            run += f[k];
+        }
+        __syncwarp();
+        // position k of the symbols in order goes to state 1283 k mod 2048; lane l places positions 64 l .. 64 l + 63
+        uint32_t sy = 0;
+        for (uint32_t d = 128; d; d >>= 1) if (sy + d < 256 && fill[sy + d] <= 64 * lane) sy += d;  // the last symbol that starts at or below 64 l
+        for (uint32_t k = 64 * lane; k < 64 * lane + 64; ++k) {
+            while (sy < 255 && fill[sy + 1] <= k) ++sy;
+            spread[(k * 1283u) & 2047u] = uint8_t(sy);
+        }
+        __syncwarp();
+        for (uint32_t u0 = 0; u0 < 2048; u0 += 32) {  // the states of a symbol, in increasing order
+            const uint32_t t = spread[u0 + lane], same = __match_any_sync(0xFFFFFFFFu, t), before = same & ((1u << lane) - 1u), at = fill[t];
+            __syncwarp();
+            next_state[at + __popc(before)] = uint16_t(2048u + u0 + lane);
+            if (!before) fill[t] = uint16_t(at + __popc(same));
+            __syncwarp();
+        }
+    }
+    const uintptr_t base = reinterpret_cast<uintptr_t>(planes + c.plane_off);
+    uint32_t per = (c.n + 31) / 32;
+    if (per < TENC_MIN_RUN) per = TENC_MIN_RUN;
+    const uint64_t first = uint64_t(lane) * per;
+    const uint32_t r_lo = first < c.n ? uint32_t(first) : c.n, r_hi = first + per < c.n ? uint32_t(first + per) : c.n;
+    auto entry = [&](uint32_t b) { return sym[b]; };
+    // the run from `state`: state at its end; emit(bits, count) for every symbol
+    auto code_run = [&](uint32_t value, auto&& emit) -> uint32_t {
+        auto step = [&](uint2 e) {
+            const uint32_t nb = (value + e.x) >> 16;
+            emit(value & ((1u << nb) - 1u), nb);
+            value = next_state[(value >> nb) + e.y];
+        };
+        walk_down(base + r_lo, base + r_hi, [&](uint32_t b) { step(entry(b)); },
+                  [&](const uint4& v) {
+                      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                      for (int h = 3; h >= 0; --h) {
+                          uint2 e[4];
+#pragma unroll
+                          for (int k = 0; k < 4; ++k) e[k] = entry((w[h] >> (8 * k)) & 0xFFu);
+#pragma unroll
+                          for (int k = 3; k >= 0; --k) step(e[k]);
+                      }
+                  });
+        return value;
+    };
+    const uint32_t last = (c.n - 1) / per;  // the lane that starts the chain, in state 2048
+    uint32_t from = 2048, end = 0;
+    uint64_t bits = 0;
+    bool go = lane <= last;
+    for (;;) {
+        if (go) { bits = 0; end = code_run(from, [&](uint32_t, uint32_t nb) { bits += nb; }); }
+        uint32_t want = __shfl_down_sync(0xFFFFFFFFu, end, 1);
+        if (lane >= last) want = 2048;
+        go = lane <= last && want != from;
+        from = want;
+        if (!__any_sync(0xFFFFFFFFu, go)) break;
+    }
+    // bits go upward from the run that is coded first, i.e. the highest lane's
+    uint64_t incl = bits;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { const uint64_t t = __shfl_down_sync(0xFFFFFFFFu, incl, d); if (lane + d < 32) incl += t; }
+    const uint64_t at = incl - bits, all = __shfl_sync(0xFFFFFFFFu, incl, 0);
+    uint32_t* out = reinterpret_cast<uint32_t*>(slots + c.slot_off);  // slot areas start on 16-byte boundaries
+    // the words where two runs meet are put together with atomics, from zero
+    uint32_t* w = out + (at >> 5);
+    if (lane <= last) { *w = 0; out[(at + bits) >> 5] = 0; }
+    if (lane == 0) { out[all >> 5] = 0; out[(all + 11) >> 5] = 0; }
+    __threadfence_block();
+    __syncwarp();
+    if (lane <= last) {
+        uint32_t lo = 0, hi = 0, have = uint32_t(at & 31);
+        bool shared_word = true;
+        auto flush = [&]() { if (shared_word) atomicOr(w, lo); else *w = lo; shared_word = false; ++w; lo = hi; hi = 0; have -= 32; };
+        const uint32_t value = code_run(from, [&](uint32_t v, uint32_t nb) {
+            lo |= v << have;
+            hi |= __funnelshift_l(v, 0u, have);
+            have += nb;
+            if (have >= 32) flush();
+        });
+        if (lane == 0) {
+            const uint32_t v = value & 2047u;
+            lo |= v << have; hi |= __funnelshift_l(v, 0u, have);
+            have += 11;
+            if (have >= 32) flush();
+        }
+        if (have) atomicOr(w, lo);
+    }
+    if (lane == 0) {
+        const uint64_t total = all + 11;
+        results[ci].stream_len[0] = uint32_t((total + 7) / 8);
+        results[ci].stream_len[1] = uint32_t(total);
+        results[ci].stream_len[2] = uint32_t(total >> 32);
+    }
+}
+
+// n bytes from s to d by the threads of a block.  d is brought to a 16-byte boundary, then every thread stores 16 bytes at a
+// time, taken from the two aligned blocks that hold them (a block that holds a needed byte is read whole: the planes and slot
+// buffers are padded for that).
 __device__ __forceinline__ void block_copy(uint8_t* d, const uint8_t* s, uint32_t n, uint32_t t, uint32_t nt) {
     uint32_t head = uint32_t((16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15);
     if (head > n) head = n;
-    for (uint32_t i = t; i < head; i += nt) d[i] = s[i];
+    if (t < head) d[t] = s[t];
     d += head; s += head; n -= head;
-    const uint32_t blocks = n >> 4;
-    const uint32_t sh = uint32_t(reinterpret_cast<uintptr_t>(s) & 3) * 8;
-    const uint32_t* sw = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(s) & ~uintptr_t(3));
+    const uint32_t blocks = n >> 4, off = uint32_t(reinterpret_cast<uintptr_t>(s) & 15);
+    const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<uintptr_t>(s) & ~uintptr_t(15));
     for (uint32_t b = t; b < blocks; b += nt) {
-        const uint32_t* q = sw + 4 * size_t(b);
-        const uint32_t w0 = q[0], w1 = q[1], w2 = q[2], w3 = q[3];
-        uint4 v = make_uint4(w0, w1, w2, w3);
-        if (sh) {
-            const uint32_t w4 = q[4];
-            v = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
-        }
+        uint4 v = q[b];
+        if (off) { uint32_t w[4]; extract16(v, q[b + 1], off, w); v = make_uint4(w[0], w[1], w[2], w[3]); }
         *reinterpret_cast<uint4*>(d + 16 * size_t(b)) = v;
     }
-    for (uint32_t i = blocks * 16 + t; i < n; i += nt) d[i] = s[i];
+    const uint32_t i = blocks * 16 + t;
+    if (i < n) d[i] = s[i];
+}
+// The same with the bytes in opposite order: d[i] = s[n - 1 - i].
+__device__ __forceinline__ void block_copy_reversed(uint8_t* d, const uint8_t* s, uint32_t n, uint32_t t, uint32_t nt) {
+    uint32_t head = uint32_t((16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15);
+    if (head > n) head = n;
+    if (t < head) d[t] = s[n - 1 - t];
+    d += head; n -= head;
+    const uint32_t blocks = n >> 4;
+    if (t < blocks) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(s) + n - 16;  // the source bytes of block 0; block b sits 16 b below
+        const uint32_t off = uint32_t(a & 15);
+        const uint4* q = reinterpret_cast<const uint4*>(a & ~uintptr_t(15));
+        for (uint32_t b = t; b < blocks; b += nt) {
+            const uint4 v = *(q - b);
+            uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            if (off) extract16(v, *(q - b + 1), off, w);
+            *reinterpret_cast<uint4*>(d + 16 * size_t(b)) =
+                make_uint4(__byte_perm(w[3], 0, 0x0123), __byte_perm(w[2], 0, 0x0123), __byte_perm(w[1], 0, 0x0123), __byte_perm(w[0], 0, 0x0123));
+        }
+    }
+    const uint32_t i = blocks * 16 + t;
+    if (i < n) d[i] = s[n - 1 - i];
 }
 // One CTA per chunk frame: [state_version 0][state_len 0 u32] then the codec
 // payload, written at its final place in the container.
@@ -556,8 +879,7 @@ __global__ void __launch_bounds__(128) gather_kernel(const GatherItem* __restric
     if (t < 16) d[t] = uint8_t(r.stream_len[t >> 2] >> (8 * (t & 3)));
     d += 16;
     for (uint32_t s = 0; s < 4; ++s) {
-        const uint8_t* sp = slots + c.slot_off + uint64_t(s + 1) * c.slot_cap - r.stream_len[s];
-        block_copy(d, sp, r.stream_len[s], t, blockDim.x);
+        block_copy_reversed(d, slots + c.slot_off + uint64_t(s) * c.slot_cap, r.stream_len[s], t, blockDim.x);
         d += r.stream_len[s];
     }
 }

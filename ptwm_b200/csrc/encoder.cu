@@ -122,9 +122,8 @@ int select_codec(const unsigned long long* hist, uint64_t n, uint32_t menu, doub
     if ((menu & PTWM_B200_MENU_HUFFMAN)) {
         double size = 1;
         if (n) {
-            uint8_t lengths[256], alive[512], sym_of[256]; uint16_t parent[512]; uint64_t nf[512], raw[256];
-            for (int i = 0; i < 256; ++i) raw[i] = hist[i];
-            int nw = huffman_lengths<uint64_t>(raw, lengths, nf, parent, alive, sym_of);
+            uint8_t lengths[256];
+            const int nw = huffman_lengths(hist, lengths);
             double bits = 0;
             for (int i = 0; i < 256; ++i) bits += double(hist[i]) * lengths[i];
             double blob = (nw <= 127 ? 1 : 2) + (nw + 1) / 2 + 16 + std::ceil(bits / 8) + 2;
@@ -247,6 +246,38 @@ cudaError_t upload_vec(DeviceBuf& b, const std::vector<T>& v, cudaStream_t st) {
     return cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
 }
 
+// Chunks by the codec of their plane, for the kernels that code them; rANS chunks also by the span of their plane's alphabet,
+// which sizes the shared memory of a block: 64 symbols for exponent planes, 128 and 256 for the others.
+struct EncodeLists {
+    std::vector<uint32_t> rans[3], huff, tans;
+    static int span_class(uint32_t span) { return span <= 64 ? 0 : span <= 128 ? 1 : 2; }
+    static uint32_t class_span(int k) { return 64u << k; }
+};
+// The stream encoders over chunks whose tables are built.  `d_lists` keeps the lists on the device.
+int64_t launch_encoders(const EncChunk* chunks, const EncodeLists& lists, DeviceBuf& d_lists, const uint8_t* planes, const uint8_t* tables, uint8_t* slots,
+                        EncResult* results, cudaStream_t st) {
+    std::vector<uint32_t> all;
+    for (auto& v : lists.rans) all.insert(all.end(), v.begin(), v.end());
+    all.insert(all.end(), lists.huff.begin(), lists.huff.end());
+    all.insert(all.end(), lists.tans.begin(), lists.tans.end());
+    if (all.empty()) return 0;
+    CUDA_TRY(upload_vec(d_lists, all, st));
+    const uint32_t* list = d_lists.as<uint32_t>();
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t n = uint32_t(lists.rans[k].size()), span = EncodeLists::class_span(k);
+        if (!n) continue;
+        rans_encode_kernel<<<(n + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, renc_smem_bytes(span), st>>>(chunks, list, n, span, planes, tables, slots, results);
+        CUDA_TRY(cudaGetLastError());
+        list += n;
+    }
+    const uint32_t n_h = uint32_t(lists.huff.size()), n_t = uint32_t(lists.tans.size());
+    if (n_h) huffman_encode_kernel<<<n_h, 128, 0, st>>>(chunks, list, n_h, planes, tables, slots, results);
+    CUDA_TRY(cudaGetLastError());
+    if (n_t) tans_encode_kernel<<<n_t, 32, 0, st>>>(chunks, list + n_h, n_t, planes, tables, slots, results);
+    CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
 int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, const ptwm_b200_encode_options& opt, int device, cudaStream_t st,
                     CrcTables* d_tabs, ptwm_b200_encoded& enc) {
     const bool chunked = opt.chunk_size != PTWM_B200_CHUNK_NONE;
@@ -337,7 +368,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     prof("plan (host)");
     // ---- device pipeline: split, histograms ---------------------------------
     DeviceBuf d_planes, d_splits, d_chunks, d_hist, d_plane_hist, d_codec, d_tables, d_results, d_slots;
-    CUDA_TRY(d_planes.alloc(planes_bytes, st));
+    CUDA_TRY(d_planes.alloc(planes_bytes + ENC_PAD, st));
     CUDA_TRY(upload_vec(d_splits, splits, st));
     CUDA_TRY(upload_vec(d_chunks, chunks, st));
     CUDA_TRY(d_hist.alloc(uint64_t(n_chunks) * 1024, st));
@@ -458,7 +489,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     prof("shared-state fit");
     // ---- codec per plane ------------------------------------------------------
     std::vector<uint8_t> plane_codec(n_planes);
-    std::vector<uint32_t> tans_chunks;  // chunks of tANS planes, for the kernel that codes them
+    EncodeLists lists;
     std::vector<uint32_t> o1sac_chunks, o1shared_chunks, o1shared_state;  // chunks that fit their own state / that code against shared state o1shared_state[k]
     uint64_t tables_bytes = 0;
     std::vector<std::pair<uint32_t, uint32_t>> recrc;  // (tensor, accumulator) of planes shifted by MantissaZeroStrip: their CRC is taken again below
@@ -550,13 +581,24 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
                 plane_codec[pi] = uint8_t(pp.codec);
                 enc.plane_codecs.back().push_back(pp.codec);
                 if (opt.emit_plane_crc) pp.crc = pp.len ? ~(accs[pi] ^ gf2_mulmod(x_pow_8n(T.x2n, pp.len), 0xFFFFFFFFu)) : 0u;
+                int span = 0;
+                if (pp.codec == C_RANS && pp.len) {
+                    const unsigned long long* h = &plane_hist[size_t(pi) * 256];
+                    int lo = 0, hi = 255;
+                    while (lo < 255 && !h[lo]) ++lo;
+                    while (hi > lo && !h[hi]) --hi;
+                    if (tp.post_op == 2 && p == 0) { lo >>= tp.post_k; hi >>= tp.post_k; }  // counted before the shift
+                    span = EncodeLists::span_class(uint32_t(hi - lo + 1));
+                }
                 if (pp.codec != C_IDENTITY)  // stream slots and table areas only for planes that get coded
                     for (uint32_t k = 0; k < pp.n_chunks; ++k) {
                         EncChunk& ch = chunks[pp.first_chunk + k];
                         ch.slot_off = slots_bytes; slots_bytes += uint64_t(ch.slot_cap) * 4;
                         ch.table_off = tables_bytes; tables_bytes += enc_table_bytes(pp.codec);
                         if (pp.codec == C_O1SAC) (pp.shared >= 0 ? o1shared_chunks : o1sac_chunks).push_back(pp.first_chunk + k);
-                        if (pp.codec == C_TANS) tans_chunks.push_back(pp.first_chunk + k);
+                        if (pp.codec == C_RANS) lists.rans[span].push_back(pp.first_chunk + k);
+                        if (pp.codec == C_HUFFMAN) lists.huff.push_back(pp.first_chunk + k);
+                        if (pp.codec == C_TANS) lists.tans.push_back(pp.first_chunk + k);
                         if (pp.codec == C_O1SAC && pp.shared >= 0) o1shared_state.push_back(uint32_t(pp.shared));
                     }
             }
@@ -593,10 +635,11 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     CUDA_TRY(d_tables.alloc(tables_bytes, st));
     CUDA_TRY(d_results.alloc(uint64_t(n_chunks) * sizeof(EncResult), st));
     CUDA_TRY(cudaMemsetAsync(d_results.p, 0, uint64_t(n_chunks) * sizeof(EncResult) + (n_chunks ? 0 : 1), st));
-    CUDA_TRY(d_slots.alloc(slots_bytes, st));
+    CUDA_TRY(d_slots.alloc(slots_bytes + ENC_PAD, st));
     std::vector<EncResult> results(n_chunks);
     prof("  work memory for tables and streams");
-    DeviceBuf d_o1list, d_tanslist;
+    DeviceBuf d_o1list, d_lists;
+    int64_t rc;
     if (!o1sac_chunks.empty()) {  // Order1ScaleAC: counts, rows, then the range coder, one chunk per block / thread
         CUDA_TRY(upload_vec(d_o1list, o1sac_chunks, st));
         for (uint32_t ci : o1sac_chunks) CUDA_TRY(cudaMemsetAsync(d_tables.as<uint8_t>() + chunks[ci].table_off, 0, O1E_PRESENT, st));
@@ -643,20 +686,12 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     }
     prof("  order1_scale_ac chunks");
     if (n_chunks) {
-        table_kernel<<<(n_chunks + 63) / 64, 64, 0, st>>>(d_chunks.as<EncChunk>(), n_chunks, d_codec.as<uint8_t>(), d_hist.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
+        table_kernel<<<(n_chunks + 3) / 4, 128, 0, st>>>(d_chunks.as<EncChunk>(), n_chunks, d_codec.as<uint8_t>(), d_hist.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
         CUDA_TRY(cudaGetLastError());
         prof("  table_kernel");
-        encode_kernel<<<(n_chunks * 4 + 127) / 128, 128, 0, st>>>(d_chunks.as<EncChunk>(), n_chunks, d_codec.as<uint8_t>(), d_planes.as<uint8_t>(), d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
-        CUDA_TRY(cudaGetLastError());
-        if (!tans_chunks.empty()) {
-            CUDA_TRY(upload_vec(d_tanslist, tans_chunks, st));
-            const uint32_t n_t = uint32_t(tans_chunks.size());
-            CUDA_TRY(cudaFuncSetAttribute(tans_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TENC_SMEM));  // per device; cheap to repeat
-            tans_encode_kernel<<<(n_t + TENC_CHUNKS - 1) / TENC_CHUNKS, 32, TENC_SMEM, st>>>(d_chunks.as<EncChunk>(), d_tanslist.as<uint32_t>(), n_t, d_planes.as<uint8_t>(),
-                                                                                         d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
-            CUDA_TRY(cudaGetLastError());
-        }
-        prof("  encode_kernel");
+        if ((rc = launch_encoders(d_chunks.as<EncChunk>(), lists, d_lists, d_planes.as<uint8_t>(), d_tables.as<uint8_t>(), d_slots.as<uint8_t>(),
+                                  d_results.as<EncResult>(), st)) < 0) return rc;
+        prof("  stream encoders");
         CUDA_TRY(cudaMemcpyAsync(results.data(), d_results.p, results.size() * sizeof(EncResult), cudaMemcpyDeviceToHost, st));
     }
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -900,8 +935,8 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         return int64_t(n);
     }
     if (n > 0xFFFFFFFFull && codec == C_O1SAC) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
-    DeviceBuf d_chunk, d_codec, d_hist, d_phist, d_tables, d_results, d_slots, d_gather, d_list, d_tlist;
-    const uint64_t slot_cap = ((n / 4 + 1) * 12 + 7) / 8 + 64;  // a symbol takes at most 12 bits in any of the codecs
+    DeviceBuf d_chunk, d_codec, d_hist, d_phist, d_tables, d_results, d_slots, d_gather, d_list;
+    const uint64_t slot_cap = align_up(((n / 4 + 1) * 12 + 7) / 8 + 64, 16);  // a symbol takes at most 12 bits in any of the codecs; slots are written in aligned words
     EncChunk chunk{0, 0, 0, uint32_t(n), uint32_t(slot_cap), 0, 0};
     const uint8_t codec_byte = uint8_t(codec);
     if (codec == C_O1SAC) {
@@ -925,7 +960,7 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         CUDA_TRY(d_chunk.alloc(sizeof(EncChunk), st, false));
         CUDA_TRY(d_tables.alloc(tab.size(), st, false));
         CUDA_TRY(d_results.alloc(sizeof(EncResult), st, false));
-        CUDA_TRY(d_slots.alloc(4 * slot_cap, st, false));
+        CUDA_TRY(d_slots.alloc(4 * slot_cap + ENC_PAD, st, false));
         CUDA_TRY(d_list.alloc(4, st, false));
         CUDA_TRY(cudaMemcpyAsync(d_chunk.p, &chunk, sizeof(chunk), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(d_tables.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, st));
@@ -956,21 +991,20 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
     if (n <= 0xFFFFFFFFull) {  // the length prefix is a u32; longer planes stay raw
         if (slot_cap > 0x3FFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
         CUDA_TRY(d_codec.alloc(1, st, false));
+        CUDA_TRY(d_list.alloc(4, st, false));
         CUDA_TRY(d_hist.alloc(256 * sizeof(uint32_t), st, false));
         CUDA_TRY(d_phist.alloc(256 * sizeof(unsigned long long), st, false));
-        CUDA_TRY(d_slots.alloc(4 * slot_cap, st, false));
+        CUDA_TRY(d_slots.alloc(4 * slot_cap + ENC_PAD, st, false));
         CUDA_TRY(cudaMemcpyAsync(d_chunk.p, &chunk, sizeof(chunk), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(d_codec.p, &codec_byte, 1, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemsetAsync(d_phist.p, 0, 256 * sizeof(unsigned long long), st));
         hist_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), in, d_hist.as<uint32_t>(), d_phist.as<unsigned long long>());
-        table_kernel<<<1, 64, 0, st>>>(d_chunk.as<EncChunk>(), 1, d_codec.as<uint8_t>(), d_hist.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
-        encode_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), 1, d_codec.as<uint8_t>(), in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
-        if (codec == C_TANS) {
-            CUDA_TRY(d_tlist.alloc(4, st, false));
-            CUDA_TRY(cudaMemsetAsync(d_tlist.p, 0, 4, st));  // the list of chunks to code: chunk 0
-            CUDA_TRY(cudaFuncSetAttribute(tans_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TENC_SMEM));
-            tans_encode_kernel<<<1, 32, TENC_SMEM, st>>>(d_chunk.as<EncChunk>(), d_tlist.as<uint32_t>(), 1, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
-        }
+        table_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), 1, d_codec.as<uint8_t>(), d_hist.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
+        CUDA_TRY(cudaMemsetAsync(d_list.p, 0, 4, st));  // the list of chunks to code: chunk 0
+        const uint32_t* list = d_list.as<uint32_t>();
+        if (codec == C_RANS) rans_encode_kernel<<<1, 32, renc_smem_bytes(256), st>>>(d_chunk.as<EncChunk>(), list, 1, 256, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
+        else if (codec == C_HUFFMAN) huffman_encode_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), list, 1, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
+        else tans_encode_kernel<<<1, 32, 0, st>>>(d_chunk.as<EncChunk>(), list, 1, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
         CUDA_TRY(cudaGetLastError());
         EncResult r;
         CUDA_TRY(cudaMemcpyAsync(&r, d_results.p, sizeof(r), cudaMemcpyDeviceToHost, st));
