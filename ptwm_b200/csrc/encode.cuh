@@ -15,15 +15,6 @@
 
 namespace ptwm {
 
-struct SplitItem {
-    const uint8_t* src;  // raw tensor bytes (device)
-    uint64_t plane_off[4];  // where each plane starts in the planes buffer
-    uint64_t n;          // elements (= bytes per plane)
-    uint32_t kind;
-    uint32_t first_tile;
-};
-constexpr uint32_t SPLIT_TILE = 8192;
-
 constexpr uint64_t ENC_PAD = 64;  // bytes behind the planes and the slots that a 16-byte access may reach
 
 struct EncChunk {
@@ -40,12 +31,29 @@ struct EncResult {       // per chunk, read back by the host
     uint32_t hdr_n;      // rANS: max_sym; Huffman: number of weights; tANS: present symbols; O1SAC: context rows
     uint32_t coded;      // 0: no table could be built, store raw
 };
-struct GatherItem {
-    uint64_t dst;        // absolute offset of the chunk frame in the container
-    uint32_t chunk;
+// One plane as the host lays it out; chunk k of it starts k * chunk bytes into the plane.
+struct EncPlane {
+    uint64_t buf_off;    // the plane's bytes in the planes buffer
+    uint64_t len, chunk;
+    uint64_t slot_off, slot_stride, table_off;  // areas of the first chunk, distance between chunks
+    uint32_t first_chunk, n_chunks;
+    uint32_t table_bytes, row_len;
+    uint32_t codec;
+    uint32_t shared;     // Order1ScaleAC against a shared state: no state of its own
+    uint32_t list_off;   // where the plane's chunks go in the encoders' lists, ENC_NO_LIST for nowhere
+    uint32_t reserved;
+};
+constexpr uint32_t ENC_NO_LIST = 0xFFFFFFFFu;
+__host__ __device__ inline uint32_t enc_slot_cap(uint64_t n) { return uint32_t((((n + 3) / 4) * 3 / 2 + 16 + 15) / 16 * 16); }  // <= 12 bits per symbol plus the rANS state
+struct ChunkPlace {
+    uint64_t frame;      // offset of the chunk frame from the plane's first
+    uint32_t entry;      // offset of the chunk's entry in the plane's chunk table
     uint32_t mode;       // 0 identity (bare bytes), 1 raw-tagged, 2 rANS, 3 Huffman, 4 tANS, 5 Order1ScaleAC (state inside the frame);
                          // + GATHER_BARE: the payload alone, no chunk frame header (and no state)
 };
+struct PlaneSizes { uint64_t frames; uint32_t entries, state_len; };  // bytes of all frames / of the chunk table / of an unchunked Order1ScaleAC plane's state
+struct PlaneDst { uint64_t frames, table; };                         // where they go in the container; frames = ENC_NOWHERE: the plane is not written
+constexpr uint64_t ENC_NOWHERE = ~0ull;
 constexpr uint32_t GATHER_BARE = 0x100;
 constexpr uint32_t GATHER_NOFRAME = 0x200;  // an unchunked plane: inline state (if the codec has one) and payload, no frame header
 
@@ -64,137 +72,277 @@ __host__ __device__ inline uint32_t enc_table_bytes(int codec) {
     return codec == C_HUFFMAN ? ENC_HUFF_TABLE_BYTES : codec == C_O1SAC ? ENC_O1SAC_TABLE_BYTES : ENC_FREQ_TABLE_BYTES;
 }
 
-__global__ void __launch_bounds__(256) split_kernel(const SplitItem* __restrict__ items, uint32_t n_items, uint8_t* __restrict__ planes) {
-    uint32_t tile = blockIdx.x;
-    uint32_t lo = 0, hi = n_items;
-    while (lo + 1 < hi) { uint32_t mid = (lo + hi) >> 1; if (items[mid].first_tile <= tile) lo = mid; else hi = mid; }
-    const SplitItem it = items[lo];
-    uint64_t base = uint64_t(tile - it.first_tile) * SPLIT_TILE;
-    uint32_t n = it.n - base < SPLIT_TILE ? uint32_t(it.n - base) : SPLIT_TILE;
-    const int eb = kind_elem_bytes(int(it.kind));
-    const uint8_t* src = it.src + base * uint64_t(eb);
-    // Sixteen elements per thread and step where the source is 16-byte aligned: 128-bit loads, one 128-bit store per
-    // plane.  (Plane offsets and tile bases are multiples of 16 by construction.)  The rest goes element by element.
-    uint32_t done = 0;
-    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && it.kind != K_PASS) {
-        const uint32_t groups = n / 16;
-        for (uint32_t g = threadIdx.x; g < groups; g += blockDim.x) {
-            const uint64_t at = base + uint64_t(g) * 16;
-            if (it.kind == K_M16) {
-                const uint4 a = reinterpret_cast<const uint4*>(src)[2 * g], b = reinterpret_cast<const uint4*>(src)[2 * g + 1];
-                const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                uint32_t lo[4], hi[4];
+__device__ __forceinline__ uint32_t warp_prefix(uint32_t v, uint32_t lane) {  // exclusive
+    uint32_t incl = v;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {  // two words = four elements -> one word per plane
-                    const uint32_t r0 = ((w[2 * k] << 1) & 0xFF00FF00u) | ((w[2 * k] >> 8) & 0x00800080u) | (w[2 * k] & 0x007F007Fu);
-                    const uint32_t r1 = ((w[2 * k + 1] << 1) & 0xFF00FF00u) | ((w[2 * k + 1] >> 8) & 0x00800080u) | (w[2 * k + 1] & 0x007F007Fu);
-                    lo[k] = __byte_perm(r0, r1, 0x6420);
-                    hi[k] = __byte_perm(r0, r1, 0x7531);
-                }
-                *reinterpret_cast<uint4*>(planes + it.plane_off[0] + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                *reinterpret_cast<uint4*>(planes + it.plane_off[1] + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            } else if (it.kind == K_M32) {
-                uint32_t pl[4][4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {  // four elements -> one word per plane
-                    const uint4 v = reinterpret_cast<const uint4*>(src)[4 * g + q];
-                    const uint32_t e[4] = {v.x, v.y, v.z, v.w};
-                    uint32_t r[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) r[k] = ((e[k] << 1) & 0xFF000000u) | ((e[k] >> 8) & 0x00800000u) | (e[k] & 0x007FFFFFu);
-                    const uint32_t t0 = __byte_perm(r[0], r[1], 0x5140), t1 = __byte_perm(r[2], r[3], 0x5140);  // bytes 0,1 of the pairs
-                    const uint32_t t2 = __byte_perm(r[0], r[1], 0x7362), t3 = __byte_perm(r[2], r[3], 0x7362);  // bytes 2,3
-                    pl[0][q] = __byte_perm(t0, t1, 0x5410); pl[1][q] = __byte_perm(t0, t1, 0x7632);
-                    pl[2][q] = __byte_perm(t2, t3, 0x5410); pl[3][q] = __byte_perm(t2, t3, 0x7632);
-                }
-#pragma unroll
-                for (int p = 0; p < 4; ++p) *reinterpret_cast<uint4*>(planes + it.plane_off[p] + at) = make_uint4(pl[p][0], pl[p][1], pl[p][2], pl[p][3]);
-            } else {
-                const uint4 v = reinterpret_cast<const uint4*>(src)[g];
-                const uint32_t e[4] = {v.x, v.y, v.z, v.w};
-                uint32_t hi[4], lo[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint32_t r = it.kind == K_E4M3 ? (((e[k] & 0x78787878u) << 1) | ((e[k] & 0x80808080u) >> 4) | (e[k] & 0x07070707u))
-                                                        : (((e[k] & 0x7C7C7C7Cu) << 1) | ((e[k] & 0x80808080u) >> 5) | (e[k] & 0x03030303u));
-                    hi[k] = (r >> 4) & 0x0F0F0F0Fu; lo[k] = r & 0x0F0F0F0Fu;
-                }
-                *reinterpret_cast<uint4*>(planes + it.plane_off[0] + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(planes + it.plane_off[1] + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            }
-        }
-        done = groups * 16;
-    } else if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-        const uint32_t groups = n / 16;
-        for (uint32_t g = threadIdx.x; g < groups; g += blockDim.x)
-            *reinterpret_cast<uint4*>(planes + it.plane_off[0] + base + uint64_t(g) * 16) = reinterpret_cast<const uint4*>(src)[g];
-        done = groups * 16;
+    for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d); if (lane >= uint32_t(d)) incl += t; }
+    return incl - v;
+}
+
+// Forward bit reorder and byte split, with the histogram of every plane taken on the way: a block owns a chunk of a tensor (or
+// SPLIT_TILE elements of a longer one), reads its elements once and writes the planes' bytes.  Sixteen elements per thread and
+// step where the source is 16-byte aligned: 128-bit loads, one 128-bit store per plane.  (Plane offsets are multiples of 16;
+// the groups start at multiples of 16 elements of the tensor, what lies outside them at either end of the block's range goes
+// element by element.)
+//
+// COPIES histograms per plane, laid out [symbol][copy], lane l counting in copy l mod COPIES: with 32 a lane has a bank of its
+// own and no atomic waits for another lane's (eight copies took three passes: the lanes that share a copy mostly meet in the
+// same few symbols of an exponent plane, or in the same bank).  Clearing and adding up 32 copies costs as much as counting
+// 16 Ki symbols, so chunks below SPLIT_WIDE_FROM keep eight.  COPIES = 0: no counts.
+struct SplitItem {
+    const uint8_t* src;     // raw tensor bytes (device)
+    uint64_t plane_off[4];  // where each plane starts in the planes buffer
+    uint64_t n;             // elements (= bytes per plane)
+    uint64_t chunk;         // elements per chunk
+    uint32_t kind;
+    uint32_t first_tile;
+    uint32_t first_chunk[4];  // of each plane
+};
+constexpr uint32_t SPLIT_TILE = 32768, SPLIT_WIDE_FROM = 8192, SPLIT_THREADS = 512;
+__host__ __device__ inline uint32_t split_tiles_per_chunk(uint64_t n, uint64_t chunk) { return uint32_t(((n < chunk ? n : chunk) + SPLIT_TILE - 1) / SPLIT_TILE); }
+inline uint64_t split_tiles(uint64_t n, uint64_t chunk) { return (n + chunk - 1) / chunk * split_tiles_per_chunk(n, chunk); }
+inline uint32_t split_smem_bytes(uint32_t planes, uint32_t copies) { return planes * copies * 1024; }
+
+template <int COPIES>
+__global__ void __launch_bounds__(SPLIT_THREADS) split_kernel(const SplitItem* __restrict__ items, uint32_t n_items, uint8_t* __restrict__ planes, uint32_t* __restrict__ hist) {
+    extern __shared__ uint32_t counts[];
+    uint32_t first = 0, after = n_items;
+    while (first + 1 < after) { const uint32_t mid = (first + after) >> 1; if (items[mid].first_tile <= blockIdx.x) first = mid; else after = mid; }
+    const SplitItem it = items[first];
+    const uint32_t tile = blockIdx.x - it.first_tile, per_chunk = split_tiles_per_chunk(it.n, it.chunk), chunk = tile / per_chunk;
+    const uint64_t chunk_at = uint64_t(chunk) * it.chunk, chunk_end = chunk_at + it.chunk < it.n ? chunk_at + it.chunk : it.n;
+    const uint64_t begin = chunk_at + uint64_t(tile % per_chunk) * SPLIT_TILE;
+    if (begin >= chunk_end) return;  // the last chunk of a tensor can have fewer tiles
+    const uint64_t end = begin + SPLIT_TILE < chunk_end ? begin + SPLIT_TILE : chunk_end;
+    const int np = kind_planes(int(it.kind)), eb = kind_elem_bytes(int(it.kind));
+    if (COPIES) {
+        for (uint32_t i = threadIdx.x; i < uint32_t(np) * 64 * COPIES; i += SPLIT_THREADS) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
     }
-    for (uint32_t i = done + threadIdx.x; i < n; i += blockDim.x) {
+    auto count = [&](int p, uint32_t byte) { if (COPIES) atomicAdd(&counts[(uint32_t(p) * 256 + byte) * COPIES + (threadIdx.x & (COPIES - 1))], 1u); };
+    auto count_words = [&](int p, const uint32_t w[4]) {
+        if (COPIES) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) count(p, (w[k >> 2] >> (8 * (k & 3))) & 0xFFu);
+        }
+    };
+    auto put = [&](int p, uint64_t at, const uint32_t w[4]) {
+        *reinterpret_cast<uint4*>(planes + it.plane_off[p] + at) = make_uint4(w[0], w[1], w[2], w[3]);
+        count_words(p, w);
+    };
+    auto one = [&](uint64_t i) {
+        uint32_t r;
         switch (it.kind) {
-            case K_PASS: planes[it.plane_off[0] + base + i] = src[i]; break;
+            case K_PASS: r = it.src[i]; break;
             case K_M16: {
-                uint32_t v = uint32_t(src[2 * i]) | uint32_t(src[2 * i + 1]) << 8;
-                uint32_t r = ((v << 1) & 0xFF00u) | ((v >> 8) & 0x0080u) | (v & 0x007Fu);
-                planes[it.plane_off[0] + base + i] = uint8_t(r);
-                planes[it.plane_off[1] + base + i] = uint8_t(r >> 8);
+                const uint32_t v = uint32_t(it.src[2 * i]) | uint32_t(it.src[2 * i + 1]) << 8;
+                r = ((v << 1) & 0xFF00u) | ((v >> 8) & 0x0080u) | (v & 0x007Fu);
                 break;
             }
             case K_M32: {
-                uint32_t v = ld_u32_unaligned(src + 4 * i);
-                uint32_t r = ((v << 1) & 0xFF000000u) | ((v >> 8) & 0x00800000u) | (v & 0x007FFFFFu);
-#pragma unroll
-                for (int p = 0; p < 4; ++p) planes[it.plane_off[p] + base + i] = uint8_t(r >> (8 * p));
+                const uint32_t v = ld_u32_unaligned(it.src + 4 * i);
+                r = ((v << 1) & 0xFF000000u) | ((v >> 8) & 0x00800000u) | (v & 0x007FFFFFu);
                 break;
             }
-            default: {
-                uint32_t v = src[i];
-                uint32_t r = it.kind == K_E4M3 ? (((v & 0x78) << 1) | ((v & 0x80) >> 4) | (v & 0x07)) : (((v & 0x7C) << 1) | ((v & 0x80) >> 5) | (v & 0x03));
-                planes[it.plane_off[0] + base + i] = uint8_t(r >> 4);
-                planes[it.plane_off[1] + base + i] = uint8_t(r & 0x0F);
+            default: {  // plane 0 holds the high nibble
+                const uint32_t v = it.src[i];
+                const uint32_t x = it.kind == K_E4M3 ? (((v & 0x78) << 1) | ((v & 0x80) >> 4) | (v & 0x07)) : (((v & 0x7C) << 1) | ((v & 0x80) >> 5) | (v & 0x03));
+                r = x >> 4 | (x & 0x0Fu) << 8;
                 break;
             }
         }
+        for (int p = 0; p < np; ++p) { planes[it.plane_off[p] + i] = uint8_t(r >> (8 * p)); count(p, (r >> (8 * p)) & 0xFFu); }
+    };
+    uint64_t lo = end, hi = end;  // whole groups of sixteen: [lo, hi)
+    if ((reinterpret_cast<uintptr_t>(it.src) & 15) == 0) {
+        lo = (begin + 15) & ~uint64_t(15); hi = end & ~uint64_t(15);
+        if (lo >= hi) lo = hi = end;
+    }
+    for (uint64_t i = begin + threadIdx.x; i < lo; i += SPLIT_THREADS) one(i);
+    for (uint64_t i = hi + threadIdx.x; i < end; i += SPLIT_THREADS) one(i);
+    const uint32_t groups = uint32_t((hi - lo) >> 4);
+    const uint4* src = reinterpret_cast<const uint4*>(it.src + lo * uint64_t(eb));
+    if (it.kind == K_M16) {
+        for (uint32_t g = threadIdx.x; g < groups; g += SPLIT_THREADS) {
+            const uint4 a = src[2 * g], b = src[2 * g + 1];
+            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            uint32_t l[4], h[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {  // two words = four elements -> one word per plane
+                const uint32_t r0 = ((w[2 * k] << 1) & 0xFF00FF00u) | ((w[2 * k] >> 8) & 0x00800080u) | (w[2 * k] & 0x007F007Fu);
+                const uint32_t r1 = ((w[2 * k + 1] << 1) & 0xFF00FF00u) | ((w[2 * k + 1] >> 8) & 0x00800080u) | (w[2 * k + 1] & 0x007F007Fu);
+                l[k] = __byte_perm(r0, r1, 0x6420);
+                h[k] = __byte_perm(r0, r1, 0x7531);
+            }
+            put(0, lo + 16 * uint64_t(g), l);
+            put(1, lo + 16 * uint64_t(g), h);
+        }
+    } else if (it.kind == K_M32) {
+        for (uint32_t g = threadIdx.x; g < groups; g += SPLIT_THREADS) {
+            uint32_t pl[4][4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {  // four elements -> one word per plane
+                const uint4 v = src[4 * g + q];
+                const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+                uint32_t r[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) r[k] = ((e[k] << 1) & 0xFF000000u) | ((e[k] >> 8) & 0x00800000u) | (e[k] & 0x007FFFFFu);
+                const uint32_t t0 = __byte_perm(r[0], r[1], 0x5140), t1 = __byte_perm(r[2], r[3], 0x5140);  // bytes 0,1 of the pairs
+                const uint32_t t2 = __byte_perm(r[0], r[1], 0x7362), t3 = __byte_perm(r[2], r[3], 0x7362);  // bytes 2,3
+                pl[0][q] = __byte_perm(t0, t1, 0x5410); pl[1][q] = __byte_perm(t0, t1, 0x7632);
+                pl[2][q] = __byte_perm(t2, t3, 0x5410); pl[3][q] = __byte_perm(t2, t3, 0x7632);
+            }
+#pragma unroll
+            for (int p = 0; p < 4; ++p) put(p, lo + 16 * uint64_t(g), pl[p]);
+        }
+    } else if (it.kind == K_PASS) {
+        for (uint32_t g = threadIdx.x; g < groups; g += SPLIT_THREADS) {
+            const uint4 v = src[g];
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            put(0, lo + 16 * uint64_t(g), w);
+        }
+    } else {
+        for (uint32_t g = threadIdx.x; g < groups; g += SPLIT_THREADS) {
+            const uint4 v = src[g];
+            const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+            uint32_t h[4], l[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t r = it.kind == K_E4M3 ? (((e[k] & 0x78787878u) << 1) | ((e[k] & 0x80808080u) >> 4) | (e[k] & 0x07070707u))
+                                                    : (((e[k] & 0x7C7C7C7Cu) << 1) | ((e[k] & 0x80808080u) >> 5) | (e[k] & 0x03030303u));
+                h[k] = (r >> 4) & 0x0F0F0F0Fu; l[k] = r & 0x0F0F0F0Fu;
+            }
+            put(0, lo + 16 * uint64_t(g), h);
+            put(1, lo + 16 * uint64_t(g), l);
+        }
+    }
+    if (!COPIES) return;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < uint32_t(np) * 256; i += SPLIT_THREADS) {
+        uint32_t total = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < uint32_t(COPIES); ++k) total += counts[i * COPIES + ((k + i) & (COPIES - 1))];  // rotated: the threads of a warp in different banks
+        uint32_t* out = hist + uint64_t(it.first_chunk[i >> 8] + chunk) * 256 + (i & 255);
+        if (per_chunk == 1) *out = total; else if (total) atomicAdd(out, total);
     }
 }
 
-// One CTA of 128 threads per chunk: shared-memory histogram, then the chunk's
-// counts go to global memory and are added to the plane's totals.
-__global__ void __launch_bounds__(128) hist_kernel(const EncChunk* __restrict__ chunks, const uint8_t* __restrict__ planes, uint32_t* __restrict__ hist,
-                                                   unsigned long long* __restrict__ plane_hist) {
-    // Eight copies of the histogram, laid out [symbol][copy]: the lanes of a warp spread over the copies (an exponent plane
-    // sends most of them to the same three or four symbols) and the copies of a symbol sit in different banks.  The plane
-    // is read 16 bytes at a time.
+// Counts of every plane from those of its chunks: blocks of 64 chunks, one thread per symbol.
+__global__ void __launch_bounds__(256) plane_hist_kernel(const EncPlane* __restrict__ enc_planes, const uint32_t* __restrict__ hist, unsigned long long* __restrict__ plane_hist) {
+    const EncPlane& p = enc_planes[blockIdx.y];
+    const uint32_t first = blockIdx.x * 64;
+    if (first >= p.n_chunks) return;
+    const uint32_t last = first + 64 < p.n_chunks ? first + 64 : p.n_chunks;
+    unsigned long long total = 0;
+    for (uint32_t k = first; k < last; ++k) total += hist[uint64_t(p.first_chunk + k) * 256 + threadIdx.x];
+    if (total) atomicAdd(&plane_hist[uint64_t(blockIdx.y) * 256 + threadIdx.x], total);
+}
+// Counts of bytes that are already there (the IntDelta planes, a single plane): the blocks of a chunk (the grid's second
+// dimension) take SPLIT_TILE bytes at a time.  The count areas were cleared.
+inline uint32_t hist_blocks(uint64_t n) { const uint64_t t = (n + SPLIT_TILE - 1) / SPLIT_TILE; return uint32_t(t < 1024 ? t : 1024); }
+__global__ void __launch_bounds__(256) hist_kernel(const EncChunk* __restrict__ chunks, const uint8_t* __restrict__ planes, uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[256 * 8];
     const EncChunk c = chunks[blockIdx.x];
     for (uint32_t i = threadIdx.x; i < 256 * 8; i += blockDim.x) h[i] = 0;
     __syncthreads();
-    const uint8_t* p = planes + c.plane_off;
     uint32_t* mine = h + (threadIdx.x & 7);
-    const uintptr_t lo = reinterpret_cast<uintptr_t>(p), hi = lo + c.n;
-    const uintptr_t first_block = (lo + 15) & ~uintptr_t(15), last_block = hi & ~uintptr_t(15);
-    if (first_block >= last_block) {
-        for (uint32_t i = threadIdx.x; i < c.n; i += blockDim.x) atomicAdd(&mine[uint32_t(p[i]) * 8], 1u);
-    } else {
-        const uint32_t head = uint32_t(first_block - lo), tail = uint32_t(hi - last_block);
-        if (threadIdx.x < head) atomicAdd(&mine[uint32_t(p[threadIdx.x]) * 8], 1u);
-        if (threadIdx.x < tail) atomicAdd(&mine[uint32_t(*reinterpret_cast<const uint8_t*>(last_block + threadIdx.x)) * 8], 1u);
-        const uint32_t blocks = uint32_t((last_block - first_block) >> 4);
-        for (uint32_t b = threadIdx.x; b < blocks; b += blockDim.x) {
-            const uint4 v = *reinterpret_cast<const uint4*>(first_block + 16 * uintptr_t(b));
+    const uintptr_t start = reinterpret_cast<uintptr_t>(planes + c.plane_off);
+    for (uint64_t begin = uint64_t(blockIdx.y) * SPLIT_TILE; begin < c.n; begin += uint64_t(gridDim.y) * SPLIT_TILE) {
+        const uintptr_t lo = start + begin, hi = start + (begin + SPLIT_TILE < c.n ? begin + SPLIT_TILE : c.n);
+        const uintptr_t first_block = (lo + 15) & ~uintptr_t(15), last_block = hi & ~uintptr_t(15);
+        if (first_block >= last_block) {
+            for (uintptr_t a = lo + threadIdx.x; a < hi; a += blockDim.x) atomicAdd(&mine[uint32_t(*reinterpret_cast<const uint8_t*>(a)) * 8], 1u);
+            continue;
+        }
+        if (lo + threadIdx.x < first_block) atomicAdd(&mine[uint32_t(*reinterpret_cast<const uint8_t*>(lo + threadIdx.x)) * 8], 1u);
+        if (last_block + threadIdx.x < hi) atomicAdd(&mine[uint32_t(*reinterpret_cast<const uint8_t*>(last_block + threadIdx.x)) * 8], 1u);
+        for (uintptr_t b = first_block + 16 * uintptr_t(threadIdx.x); b < last_block; b += 16 * uintptr_t(blockDim.x)) {
+            const uint4 v = *reinterpret_cast<const uint4*>(b);
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int k = 0; k < 16; ++k) atomicAdd(&mine[((w[k >> 2] >> (8 * (k & 3))) & 0xFFu) * 8], 1u);
         }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
-        uint32_t total = 0;
+    uint32_t total = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) total += h[i * 8 + k];
-        hist[uint64_t(blockIdx.x) * 256 + i] = total;
-        if (total) atomicAdd(&plane_hist[uint64_t(c.plane) * 256 + i], (unsigned long long)total);
+    for (int k = 0; k < 8; ++k) total += h[threadIdx.x * 8 + k];
+    if (total) atomicAdd(&hist[uint64_t(blockIdx.x) * 256 + threadIdx.x], total);
+}
+
+// The chunk descriptors of all planes, and the lists of chunks the stream encoders walk.
+__global__ void __launch_bounds__(256) expand_chunks_kernel(const EncPlane* __restrict__ enc_planes, uint32_t n_planes, uint32_t n_chunks, EncChunk* __restrict__ chunks, uint32_t* __restrict__ lists) {
+    const uint32_t ci = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ci >= n_chunks) return;
+    uint32_t lo = 0, hi = n_planes;  // the last plane that starts at or before the chunk (planes without chunks start where the next one does)
+    while (lo + 1 < hi) { const uint32_t mid = (lo + hi) >> 1; if (enc_planes[mid].first_chunk <= ci) lo = mid; else hi = mid; }
+    const EncPlane& p = enc_planes[lo];
+    const uint32_t k = ci - p.first_chunk;
+    const uint64_t at = uint64_t(k) * p.chunk;
+    const uint32_t n = uint32_t(p.len - at < p.chunk ? p.len - at : p.chunk);
+    chunks[ci] = EncChunk{p.buf_off + at, p.slot_off + uint64_t(k) * p.slot_stride, p.table_off + uint64_t(k) * p.table_bytes, n, enc_slot_cap(n), lo, p.row_len};
+    if (p.list_off != ENC_NO_LIST) lists[p.list_off + k] = ci;
+}
+
+// ---- layout --------------------------------------------------------------------------------------------
+// Frame size and form of every chunk, running offsets over a plane's chunks, and the bytes of the plane's chunk table (a varint
+// offset and a varint length per chunk).  One block per plane; what the host needs for the records is one PlaneSizes each.
+__host__ __device__ inline uint32_t varint_bytes(uint64_t v) { uint32_t n = 1; while (v >= 0x80) { v >>= 7; ++n; } return n; }
+__device__ __forceinline__ uint32_t put_varint_dev(uint8_t* d, uint64_t v) {
+    uint32_t n = 0;
+    while (v >= 0x80) { d[n++] = uint8_t(v) | 0x80; v >>= 7; }
+    d[n++] = uint8_t(v);
+    return n;
+}
+// Payload bytes (without a chunk frame header) and the gather's form of one chunk.
+__host__ __device__ inline uint64_t enc_payload(int codec, bool shared, uint32_t n, const EncResult& r, uint32_t& mode) {
+    if (codec == C_IDENTITY) { mode = 0; return n; }
+    if (codec == C_O1SAC) { mode = shared ? (5 | GATHER_BARE) : 5; return (shared ? 0 : r.stream_len[1]) + uint64_t(r.stream_len[0]); }  // a plane's own state sits in front of the coder's bytes
+    uint64_t blob;
+    if (codec == C_TANS) blob = 3 + 3 * uint64_t(r.hdr_n) + 8 + r.stream_len[0];
+    else {
+        const uint64_t hdr = codec == C_RANS ? 1 + 2 * (uint64_t(r.hdr_n) + 1) : (r.hdr_n <= 127 ? 1 : 2) + (uint64_t(r.hdr_n) + 1) / 2;
+        blob = hdr + 16 + uint64_t(r.stream_len[0]) + r.stream_len[1] + r.stream_len[2] + r.stream_len[3];
     }
+    // stored raw when coding does not shrink the chunk (compress.rs NotBeneficial) or the length rule refuses it (length_prefix.rs:29-33)
+    const bool coded = r.coded && blob < n && (codec == C_HUFFMAN || n <= (1u << 30) || n <= blob * 64);
+    mode = coded ? (codec == C_RANS ? 2 : codec == C_HUFFMAN ? 3 : 4) : 1;
+    return coded ? 5 + blob : 1 + uint64_t(n);
+}
+__global__ void __launch_bounds__(256) layout_kernel(const EncPlane* __restrict__ enc_planes, const EncChunk* __restrict__ chunks, const EncResult* __restrict__ results, uint32_t framed,
+                                                     ChunkPlace* __restrict__ places, PlaneSizes* __restrict__ sizes) {
+    __shared__ uint64_t warp_frames[8];
+    __shared__ uint32_t warp_entries[8];
+    const EncPlane& p = enc_planes[blockIdx.x];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t frames = 0;   // bytes of the chunks before the current 256
+    uint32_t entries = 0;  // bytes of their table entries
+    for (uint32_t base = 0; base < p.n_chunks; base += 256) {
+        const uint32_t k = base + threadIdx.x, ci = p.first_chunk + k;
+        uint64_t size = 0;
+        uint32_t mode = 0, n = 0;
+        if (k < p.n_chunks) {
+            n = chunks[ci].n;
+            size = enc_payload(int(p.codec), p.shared != 0, n, results[ci], mode) + (framed ? 5 : 0);
+        }
+        uint64_t incl = size;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) { const uint64_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d); if (lane >= uint32_t(d)) incl += t; }
+        __syncthreads();
+        if (lane == 31) warp_frames[warp] = incl;
+        __syncthreads();
+        uint64_t before = frames + incl - size, all = 0;
+        for (uint32_t w = 0; w < 8; ++w) { if (w < warp) before += warp_frames[w]; all += warp_frames[w]; }
+        const uint32_t e = k < p.n_chunks ? varint_bytes(before) + varint_bytes(n) : 0u;
+        const uint32_t e_excl = warp_prefix(e, lane);
+        if (lane == 31) warp_entries[warp] = e_excl + e;
+        __syncthreads();
+        uint32_t e_before = entries + e_excl, e_all = 0;
+        for (uint32_t w = 0; w < 8; ++w) { if (w < warp) e_before += warp_entries[w]; e_all += warp_entries[w]; }
+        if (k < p.n_chunks) places[ci] = ChunkPlace{before, e_before, mode | (framed ? 0u : GATHER_NOFRAME)};
+        frames += all; entries += e_all;
+    }
+    if (threadIdx.x == 0) sizes[blockIdx.x] = PlaneSizes{frames, entries, p.codec == C_O1SAC && p.n_chunks == 1 && !p.shared ? results[p.first_chunk].stream_len[1] : 0u};
 }
 
 // ---- tables --------------------------------------------------------------------------------------------
@@ -202,12 +350,6 @@ __global__ void __launch_bounds__(128) hist_kernel(const EncChunk* __restrict__ 
 // The same choices as rans_normalize, tans_normalize, huffman_lengths of encode_tables.cuh, made by all
 // lanes together: with one thread per chunk the 256-step loops and the Huffman tree took 0.6 - 1.1 ms however few chunks
 // there were.
-__device__ __forceinline__ uint32_t warp_prefix(uint32_t v, uint32_t lane) {  // exclusive
-    uint32_t incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d); if (lane >= uint32_t(d)) incl += t; }
-    return incl - v;
-}
 // The first index at which the largest of all values stands.
 __device__ __forceinline__ uint32_t warp_first_argmax(const uint32_t v[8], uint32_t lane, uint32_t& best) {
     uint32_t m = 0;
@@ -323,13 +465,13 @@ __device__ __forceinline__ uint32_t warp_huffman_lengths(const uint32_t c[8], ui
     return last + 1;
 }
 
-__global__ void __launch_bounds__(128) table_kernel(const EncChunk* __restrict__ chunks, uint32_t n_chunks, const uint8_t* __restrict__ plane_codec,
+__global__ void __launch_bounds__(128) table_kernel(const EncPlane* __restrict__ enc_planes, const EncChunk* __restrict__ chunks, uint32_t n_chunks,
                                                     const uint32_t* __restrict__ hist, uint8_t* __restrict__ tables, EncResult* __restrict__ results) {
     __shared__ HuffWork huff[4];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ci = blockIdx.x * 4 + warp;
     if (ci >= n_chunks) return;
     const EncChunk c = chunks[ci];
-    const int codec = plane_codec[c.plane];
+    const int codec = int(enc_planes[c.plane].codec);
     if (codec == C_O1SAC) return;  // fitted by its own kernels
     EncResult r{{0, 0, 0, 0}, 0, 0};
     if (codec != C_IDENTITY && c.n) {
@@ -797,18 +939,12 @@ __device__ __forceinline__ void block_copy_reversed(uint8_t* d, const uint8_t* s
     const uint32_t i = blocks * 16 + t;
     if (i < n) d[i] = s[n - 1 - i];
 }
-// One CTA per chunk frame: [state_version 0][state_len 0 u32] then the codec
-// payload, written at its final place in the container.
-__global__ void __launch_bounds__(128) gather_kernel(const GatherItem* __restrict__ items, const EncChunk* __restrict__ chunks, const EncResult* __restrict__ results,
-                                                     const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, const uint8_t* __restrict__ slots,
-                                                     uint8_t* __restrict__ out) {
-    const GatherItem g = items[blockIdx.x];
-    const EncChunk c = chunks[g.chunk];
-    const EncResult r = results[g.chunk];
-    uint8_t* d = out + g.dst;
+// One chunk frame by the threads of a block: [state_version 0][state_len 0 u32] then the codec payload, at its final place.
+__device__ __forceinline__ void gather_frame(uint8_t* d, const EncChunk& c, const EncResult& r, uint32_t form, const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables,
+                                             const uint8_t* __restrict__ slots) {
     const uint32_t t = threadIdx.x;
-    const uint32_t mode = g.mode & 0xFFu;
-    const bool framed = !(g.mode & (GATHER_BARE | GATHER_NOFRAME));
+    const uint32_t mode = form & 0xFFu;
+    const bool framed = !(form & (GATHER_BARE | GATHER_NOFRAME));
     if (framed) {
         if (t < 5 && mode != 5) d[t] = 0;
         d += 5;
@@ -824,7 +960,7 @@ __global__ void __launch_bounds__(128) gather_kernel(const GatherItem* __restric
         const uint8_t* present = tab + O1E_PRESENT;
         const uint16_t* rank = reinterpret_cast<const uint16_t*>(tab + O1E_RANK);
         const uint16_t* pmf = reinterpret_cast<const uint16_t*>(tab + O1E_PMF);
-        if (!(g.mode & GATHER_BARE)) {
+        if (!(form & GATHER_BARE)) {
             const uint32_t state_len = r.stream_len[1];
             if (framed && t == 0) {  // frame header: state_version 1, state length
                 uint8_t* fh = d - 5;
@@ -847,12 +983,19 @@ __global__ void __launch_bounds__(128) gather_kernel(const GatherItem* __restric
     if (t == 0) { d[0] = 1; d[1] = uint8_t(c.n); d[2] = uint8_t(c.n >> 8); d[3] = uint8_t(c.n >> 16); d[4] = uint8_t(c.n >> 24); }
     d += 5;
     if (mode == 4) {  // tANS blob: [11][nsym u16][(symbol, freq u16) per present symbol][total bits u64][bits]
-        const uint16_t* norm = reinterpret_cast<const uint16_t*>(tab);
-        if (t == 0) {
-            d[0] = 11; d[1] = uint8_t(r.hdr_n); d[2] = uint8_t(r.hdr_n >> 8);
-            uint8_t* q = d + 3;
-            for (int sy = 0; sy < 256; ++sy) if (norm[sy]) { q[0] = uint8_t(sy); q[1] = uint8_t(norm[sy]); q[2] = uint8_t(norm[sy] >> 8); q += 3; }
-            for (int k = 0; k < 4; ++k) { q[k] = uint8_t(r.stream_len[1] >> (8 * k)); q[4 + k] = uint8_t(r.stream_len[2] >> (8 * k)); }
+        if (t < 32) {
+            if (t == 0) {
+                d[0] = 11; d[1] = uint8_t(r.hdr_n); d[2] = uint8_t(r.hdr_n >> 8);
+                uint8_t* q = d + 3 + 3 * r.hdr_n;
+                for (int k = 0; k < 4; ++k) { q[k] = uint8_t(r.stream_len[1] >> (8 * k)); q[4 + k] = uint8_t(r.stream_len[2] >> (8 * k)); }
+            }
+            uint32_t f[8], present = 0;
+            warp_load_freqs(tab, t, f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) present += f[k] != 0;
+            uint8_t* q = d + 3 + 3 * warp_prefix(present, t);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) if (f[k]) { q[0] = uint8_t(8 * t + k); q[1] = uint8_t(f[k]); q[2] = uint8_t(f[k] >> 8); q += 3; }
         }
         d += 3 + 3 * r.hdr_n + 8;
         const uint8_t* sp = slots + c.slot_off;
@@ -882,6 +1025,25 @@ __global__ void __launch_bounds__(128) gather_kernel(const GatherItem* __restric
         block_copy_reversed(d, slots + c.slot_off + uint64_t(s) * c.slot_cap, r.stream_len[s], t, blockDim.x);
         d += r.stream_len[s];
     }
+}
+
+__global__ void __launch_bounds__(128) gather_kernel(const EncChunk* __restrict__ chunks, const EncResult* __restrict__ results, const ChunkPlace* __restrict__ places,
+                                                     const PlaneDst* __restrict__ dsts, const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables,
+                                                     const uint8_t* __restrict__ slots, uint8_t* __restrict__ out) {
+    const EncChunk c = chunks[blockIdx.x];
+    const PlaneDst dst = dsts[c.plane];
+    if (dst.frames == ENC_NOWHERE) return;
+    const ChunkPlace place = places[blockIdx.x];
+    if (dst.table != ENC_NOWHERE && threadIdx.x == 127) {  // the chunk's entry in the plane's table: frame offset, decoded length
+        uint8_t* e = out + dst.table + place.entry;
+        e += put_varint_dev(e, place.frame);
+        put_varint_dev(e, c.n);
+    }
+    gather_frame(out + dst.frames + place.frame, c, results[blockIdx.x], place.mode, planes, tables, slots);
+}
+__global__ void __launch_bounds__(512) gather_one_kernel(const EncChunk* __restrict__ chunk, const EncResult* __restrict__ result, uint32_t form, const uint8_t* __restrict__ planes,
+                                                         const uint8_t* __restrict__ tables, const uint8_t* __restrict__ slots, uint8_t* __restrict__ out) {
+    gather_frame(out, *chunk, *result, form, planes, tables, slots);
 }
 
 // ---- ops between a byte split and a terminal (transforms/int_delta.rs:36-44, transforms/mantissa_zero.rs) ------

@@ -86,15 +86,13 @@ struct PlanePlan {
     uint8_t role = 0;        // compact terminal role byte of the chain
     uint32_t row_len = 0;    // rows layout of the plane (last dimension of a passthrough tensor), 0 = flat
     // layout
-    std::vector<uint64_t> frame_size;  // per chunk (or one entry for an empty plane)
-    uint64_t payload_len = 0, state_len = 0;  // state_len: inline state of an unchunked Order1ScaleAC plane
+    uint64_t payload_len = 0, state_len = 0, table_len = 0;  // state_len: inline state of an unchunked Order1ScaleAC plane; table_len: bytes of the chunk table
     int shared = -1;         // Order1ScaleAC against this shared state of the prelude instead of a state of its own
 };
 struct TensorPlan {
     ChainDef chain;
     uint32_t chain_id = 0;
     std::vector<PlanePlan> planes;
-    uint64_t hash = 0;
     // candidate chains: the exponent plane after IntDelta lives in a plane of its own until the choice is made
     bool has_delta = false;
     PlanePlan delta;          // plane index = delta_index
@@ -102,6 +100,9 @@ struct TensorPlan {
     uint32_t try_mzs = 0;     // word index of the OR of mantissa plane 0's bytes, + 1 (0 = not looked at)
     int post_op = 0, post_k = 0;  // what was chosen (or given): 1 IntDelta on the last plane, 2 MantissaZeroStrip(post_k) on plane 0
 };
+
+// Global plane index of plane p as it is written: the delta plane stands in for the exponent plane where IntDelta was chosen.
+uint32_t plane_index(const TensorPlan& tp, size_t p) { return tp.post_op == 1 && p + 1 == tp.planes.size() ? tp.delta_index : tp.first_plane + uint32_t(p); }
 
 // Size of the whole plane under each codec of the menu, the way the reference's
 // trial encode compares them (select.rs:27-64: smallest state + payload, the
@@ -248,38 +249,50 @@ cudaError_t upload_vec(DeviceBuf& b, const std::vector<T>& v, cudaStream_t st) {
 
 // Chunks by the codec of their plane, for the kernels that code them; rANS chunks also by the span of their plane's alphabet,
 // which sizes the shared memory of a block: 64 symbols for exponent planes, 128 and 256 for the others.
-struct EncodeLists {
-    std::vector<uint32_t> rans[3], huff, tans;
-    static int span_class(uint32_t span) { return span <= 64 ? 0 : span <= 128 ? 1 : 2; }
-    static uint32_t class_span(int k) { return 64u << k; }
-};
-// The stream encoders over chunks whose tables are built.  `d_lists` keeps the lists on the device.
-int64_t launch_encoders(const EncChunk* chunks, const EncodeLists& lists, DeviceBuf& d_lists, const uint8_t* planes, const uint8_t* tables, uint8_t* slots,
+enum { LIST_RANS = 0 /* and 1, 2 */, LIST_HUFFMAN = 3, LIST_TANS = 4, LIST_KINDS = 5 };
+int rans_list(uint32_t span) { return span <= 64 ? 0 : span <= 128 ? 1 : 2; }
+uint32_t rans_list_span(int k) { return 64u << k; }
+// The stream encoders over chunks whose tables are built; `lists` holds the chunks of all kinds, one kind after the other.
+int64_t launch_encoders(const EncChunk* chunks, const uint32_t* lists, const uint32_t n[LIST_KINDS], const uint8_t* planes, const uint8_t* tables, uint8_t* slots,
                         EncResult* results, cudaStream_t st) {
-    std::vector<uint32_t> all;
-    for (auto& v : lists.rans) all.insert(all.end(), v.begin(), v.end());
-    all.insert(all.end(), lists.huff.begin(), lists.huff.end());
-    all.insert(all.end(), lists.tans.begin(), lists.tans.end());
-    if (all.empty()) return 0;
-    CUDA_TRY(upload_vec(d_lists, all, st));
-    const uint32_t* list = d_lists.as<uint32_t>();
-    for (int k = 0; k < 3; ++k) {
-        const uint32_t n = uint32_t(lists.rans[k].size()), span = EncodeLists::class_span(k);
-        if (!n) continue;
-        rans_encode_kernel<<<(n + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, renc_smem_bytes(span), st>>>(chunks, list, n, span, planes, tables, slots, results);
+    for (int k = 0; k < LIST_KINDS; ++k) {
+        if (!n[k]) continue;
+        if (k < LIST_HUFFMAN) {
+            const uint32_t span = rans_list_span(k);
+            rans_encode_kernel<<<(n[k] + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, renc_smem_bytes(span), st>>>(chunks, lists, n[k], span, planes, tables, slots, results);
+        } else if (k == LIST_HUFFMAN) huffman_encode_kernel<<<n[k], 128, 0, st>>>(chunks, lists, n[k], planes, tables, slots, results);
+        else tans_encode_kernel<<<n[k], 32, 0, st>>>(chunks, lists, n[k], planes, tables, slots, results);
         CUDA_TRY(cudaGetLastError());
-        list += n;
+        lists += n[k];
     }
-    const uint32_t n_h = uint32_t(lists.huff.size()), n_t = uint32_t(lists.tans.size());
-    if (n_h) huffman_encode_kernel<<<n_h, 128, 0, st>>>(chunks, list, n_h, planes, tables, slots, results);
-    CUDA_TRY(cudaGetLastError());
-    if (n_t) tans_encode_kernel<<<n_t, 32, 0, st>>>(chunks, list + n_h, n_t, planes, tables, slots, results);
-    CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
+// Parts of one block of device memory: add() in any number, then alloc() once.
+struct Arena {
+    DeviceBuf buf;
+    uint64_t size = 0;
+    uint64_t add(uint64_t bytes) { const uint64_t at = size; size += align_up(bytes, 256); return at; }
+    cudaError_t alloc(cudaStream_t st) { return buf.alloc(size + ENC_PAD, st); }
+    template <class T> T* at(uint64_t off) const { return reinterpret_cast<T*>(buf.as<uint8_t>() + off); }
+};
+// Host tables on their way to an arena in one copy.
+struct Upload {
+    std::vector<uint8_t> bytes;
+    template <class T>
+    uint64_t add(const std::vector<T>& v) {
+        const uint64_t at = bytes.size();
+        bytes.resize(at + align_up(v.size() * sizeof(T), 256));
+        if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
+    }
+};
+template <class T>
+cudaError_t to_host(std::vector<T>& v, const T* src, cudaStream_t st) { return v.empty() ? cudaSuccess : cudaMemcpyAsync(v.data(), src, v.size() * sizeof(T), cudaMemcpyDeviceToHost, st); }
+
 int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, const ptwm_b200_encode_options& opt, int device, cudaStream_t st,
-                    CrcTables* d_tabs, ptwm_b200_encoded& enc) {
+                    DeviceState& ds, ptwm_b200_encoded& enc) {
+    CrcTables* d_tabs = ds.d_tabs;
     const bool chunked = opt.chunk_size != PTWM_B200_CHUNK_NONE;
     const uint64_t chunk_size = !chunked ? (1ull << 32) : opt.chunk_size ? opt.chunk_size : 65536u;
     const uint32_t menu = opt.menu ? opt.menu : 31u;
@@ -301,10 +314,18 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     std::vector<TensorPlan> plan(n_tensors);
     std::vector<ChainDef> registry;
     std::vector<SplitItem> splits;
-    std::vector<EncChunk> chunks;
+    std::vector<EncPlane> ep;  // by global plane index
     std::vector<HashItem> hash_items;
-    uint64_t planes_bytes = 0, slots_bytes = 0;
-    uint32_t n_planes = 0, tile = 0, n_or_words = 0;
+    uint64_t planes_bytes = 0, slots_bytes = 0, n_chunks64 = 0, tiles64 = 0;
+    uint32_t n_or_words = 0;
+    int most_planes = 1;
+    auto new_plane = [&](PlanePlan& pp, uint32_t row_len) {
+        const uint64_t n = (pp.len + chunk_size - 1) / chunk_size;
+        pp.buf_off = planes_bytes; pp.first_chunk = uint32_t(n_chunks64); pp.n_chunks = uint32_t(n);
+        planes_bytes += align_up(pp.len, 16);
+        n_chunks64 += n;
+        ep.push_back(EncPlane{pp.buf_off, pp.len, chunk_size, 0, 0, 0, pp.first_chunk, pp.n_chunks, 0, row_len, C_IDENTITY, 0, ENC_NO_LIST, 0});
+    };
     for (size_t i = 0; i < n_tensors; ++i) {
         const ptwm_b200_encode_tensor& t = tensors[i];
         std::string why;
@@ -322,29 +343,22 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             if (t.post_op == 2 && (t.post_plane != 0 || t.post_k < 1 || t.post_k > 7)) return fail(PTWM_RC_UNSUPPORTED, std::string(t.name) + ": MantissaZeroStrip(1..7) goes on mantissa plane 0");
             if (t.post_op > 2) return fail(PTWM_RC_UNSUPPORTED, std::string(t.name) + ": unknown per-plane op");
         }
-        plan[i].first_plane = n_planes;
+        plan[i].first_plane = uint32_t(ep.size());
+        most_planes = std::max(most_planes, np);
         const uint64_t plane_len = t.nbytes / uint64_t(kind_elem_bytes(kind));
         if (plane_len > 0xFFFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "plane longer than 4 GiB");
-        SplitItem sp{reinterpret_cast<const uint8_t*>(uintptr_t(t.dev_ptr)), {0, 0, 0, 0}, plane_len, uint32_t(kind), tile};
+        SplitItem sp{reinterpret_cast<const uint8_t*>(uintptr_t(t.dev_ptr)), {0, 0, 0, 0}, plane_len, chunk_size, uint32_t(kind), uint32_t(tiles64), {0, 0, 0, 0}};
         plan[i].planes.resize(size_t(np));
         for (int p = 0; p < np; ++p) {
             PlanePlan& pp = plan[i].planes[size_t(p)];
-            pp.len = plane_len; pp.buf_off = planes_bytes; pp.first_chunk = uint32_t(chunks.size());
+            pp.len = plane_len;
             pp.role = plan[i].chain.roles[size_t(p)];
             // a passthrough plane keeps the tensor's rows (its last dimension); split planes are flat (transforms/byte_split.rs:76)
             pp.row_len = kind == K_PASS && t.ndim >= 1 && t.shape[t.ndim - 1] && plane_len ? uint32_t(t.shape[t.ndim - 1]) : 0u;
-            sp.plane_off[p] = planes_bytes;
-            planes_bytes += align_up(plane_len, 16);
-            for (uint64_t off = 0; off < plane_len; off += chunk_size) {
-                uint32_t n = uint32_t(std::min<uint64_t>(chunk_size, plane_len - off));
-                uint32_t cap = uint32_t(align_up(uint64_t((n + 3) / 4) * 3 / 2 + 16, 16));  // <= 12 bits per symbol plus the rANS state
-                // chunks are coded flat (compressor.rs:352-355); a whole plane keeps its rows
-                chunks.push_back(EncChunk{pp.buf_off + off, 0, 0, n, cap, n_planes, chunked ? 0u : pp.row_len});
-            }
-            pp.n_chunks = uint32_t(chunks.size()) - pp.first_chunk;
-            ++n_planes;
+            new_plane(pp, chunked ? 0u : pp.row_len);  // chunks are coded flat (compressor.rs:352-355); a whole plane keeps its rows
+            sp.plane_off[p] = pp.buf_off; sp.first_chunk[p] = pp.first_chunk;
         }
-        if (plane_len) { splits.push_back(sp); tile += uint32_t((plane_len + SPLIT_TILE - 1) / SPLIT_TILE); }
+        if (plane_len) { splits.push_back(sp); tiles64 += split_tiles(plane_len, chunk_size); }
         if (opt.emit_payload_hash) hash_items.push_back(HashItem{make_ref(SP_BLOB, t.dev_ptr), t.nbytes});
         const bool split_kind = (kind == K_M16 || kind == K_M32) && plane_len;
         plan[i].post_op = t.post_op; plan[i].post_k = t.post_k;
@@ -352,44 +366,17 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
         if (split_kind && (t.post_op == 2 || (!t.post_op && (opt.candidates & PTWM_B200_TRY_MZS)))) plan[i].try_mzs = ++n_or_words;
     }
     // the IntDelta candidates' exponent planes: planes of their own behind the others
+    bool any_delta = false;
     for (size_t i = 0; i < n_tensors; ++i) {
         TensorPlan& tp = plan[i];
         if (!tp.has_delta) continue;
-        const PlanePlan& ex = tp.planes.back();
-        PlanePlan& pp = tp.delta;
-        pp.len = ex.len; pp.buf_off = planes_bytes; pp.first_chunk = uint32_t(chunks.size()); pp.role = ex.role; pp.row_len = 0;
-        planes_bytes += align_up(pp.len, 16);
-        for (uint32_t k = 0; k < ex.n_chunks; ++k) { EncChunk c = chunks[ex.first_chunk + k]; c.plane_off = pp.buf_off + (c.plane_off - ex.buf_off); c.plane = n_planes; chunks.push_back(c); }
-        pp.n_chunks = ex.n_chunks;
-        tp.delta_index = n_planes++;
+        tp.delta.len = tp.planes.back().len; tp.delta.role = tp.planes.back().role; tp.delta.row_len = 0;
+        tp.delta_index = uint32_t(ep.size());
+        new_plane(tp.delta, 0);
+        any_delta |= tp.delta.len != 0;
     }
-    const uint32_t n_chunks = uint32_t(chunks.size());
-
-    prof("plan (host)");
-    // ---- device pipeline: split, histograms ---------------------------------
-    DeviceBuf d_planes, d_splits, d_chunks, d_hist, d_plane_hist, d_codec, d_tables, d_results, d_slots;
-    CUDA_TRY(d_planes.alloc(planes_bytes + ENC_PAD, st));
-    CUDA_TRY(upload_vec(d_splits, splits, st));
-    CUDA_TRY(upload_vec(d_chunks, chunks, st));
-    CUDA_TRY(d_hist.alloc(uint64_t(n_chunks) * 1024, st));
-    CUDA_TRY(d_plane_hist.alloc(uint64_t(n_planes) * 256 * 8, st));
-    CUDA_TRY(cudaMemsetAsync(d_plane_hist.p, 0, uint64_t(n_planes) * 256 * 8 + (n_planes ? 0 : 1), st));
-    if (tile) { split_kernel<<<tile, 256, 0, st>>>(d_splits.as<SplitItem>(), uint32_t(splits.size()), d_planes.as<uint8_t>()); CUDA_TRY(cudaGetLastError()); }
-    DeviceBuf d_or;
-    std::vector<uint32_t> or_words(n_or_words);
-    if (n_or_words) { CUDA_TRY(d_or.alloc(uint64_t(n_or_words) * 4, st)); CUDA_TRY(cudaMemsetAsync(d_or.p, 0, uint64_t(n_or_words) * 4, st)); }
-    for (auto& tp : plan) {
-        auto blocks = [](uint64_t n) { return unsigned(std::min<uint64_t>((n + 4095) / 4096, 2368)); };
-        if (tp.has_delta) { delta_kernel<<<blocks(tp.delta.len), 256, 0, st>>>(d_planes.as<uint8_t>() + tp.planes.back().buf_off, d_planes.as<uint8_t>() + tp.delta.buf_off, tp.delta.len); CUDA_TRY(cudaGetLastError()); }
-        if (tp.try_mzs) { or_bytes_kernel<<<blocks(tp.planes[0].len), 256, 0, st>>>(d_planes.as<uint8_t>() + tp.planes[0].buf_off, tp.planes[0].len, d_or.as<uint32_t>() + tp.try_mzs - 1); CUDA_TRY(cudaGetLastError()); }
-    }
-    if (n_or_words) CUDA_TRY(cudaMemcpyAsync(or_words.data(), d_or.p, uint64_t(n_or_words) * 4, cudaMemcpyDeviceToHost, st));
-    if (n_chunks) { hist_kernel<<<n_chunks, 128, 0, st>>>(d_chunks.as<EncChunk>(), d_planes.as<uint8_t>(), d_hist.as<uint32_t>(), d_plane_hist.as<unsigned long long>()); CUDA_TRY(cudaGetLastError()); }
-    std::vector<unsigned long long> plane_hist(size_t(n_planes) * 256);
-    if (n_planes) CUDA_TRY(cudaMemcpyAsync(plane_hist.data(), d_plane_hist.p, plane_hist.size() * 8, cudaMemcpyDeviceToHost, st));
-
-    // plane CRCs and payload hashes run on the same stream meanwhile
-    DeviceBuf d_verify, d_acc, d_hitems, d_hout;
+    if (n_chunks64 > 0x7FFFFFFFull || tiles64 > 0x7FFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "too many chunks");
+    const uint32_t n_chunks = uint32_t(n_chunks64), n_planes = uint32_t(ep.size()), tile = uint32_t(tiles64);
     std::vector<VerifyTensor> verify;
     uint64_t n_runs = 0;
     if (opt.emit_plane_crc) {
@@ -400,26 +387,91 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             for (size_t p = 0; p < tp.planes.size(); ++p) add(tp.planes[p], tp.first_plane + uint32_t(p));
             if (tp.has_delta) add(tp.delta, tp.delta_index);
         }
-        CUDA_TRY(upload_vec(d_verify, verify, st));
-        CUDA_TRY(d_acc.alloc(uint64_t(n_planes) * 4, st));
-        CUDA_TRY(cudaMemsetAsync(d_acc.p, 0, uint64_t(n_planes) * 4 + (n_planes ? 0 : 1), st));
-        if (n_runs) {
-            Bases b{nullptr, 0, 0, nullptr, d_planes.as<uint8_t>()};
-            crc_planes_kernel<<<uint32_t((n_runs + 127) / 128), 128, 0, st>>>(d_verify.as<VerifyTensor>(), uint32_t(verify.size()), n_runs, b, d_tabs, d_acc.as<uint32_t>());
+    }
+
+    prof("plan (host)");
+    // ---- device pipeline: split, histograms ---------------------------------
+    const bool counted = opt.forced_codec != C_IDENTITY || opt.candidates;  // an Identity container needs no counts
+    Arena wa;
+    const uint64_t a_planes = wa.add(planes_bytes + ENC_PAD), a_hist = wa.add(counted ? uint64_t(n_chunks) * 1024 : 0), a_plane_hist = wa.add(uint64_t(n_planes) * 256 * 8),
+                   a_or = wa.add(uint64_t(n_or_words) * 4), a_acc = wa.add(uint64_t(n_planes) * 4), a_hashes = wa.add(hash_items.size() * 8),
+                   a_chunks = wa.add(uint64_t(n_chunks) * sizeof(EncChunk));
+    Upload up;
+    const uint64_t u_splits = up.add(splits), u_ep = up.add(ep), u_verify = up.add(verify), u_hitems = up.add(hash_items);
+    const uint64_t a_up = wa.add(up.bytes.size());
+    CUDA_TRY(wa.alloc(st));
+    uint8_t* d_planes = wa.at<uint8_t>(a_planes);
+    uint32_t* d_hist = wa.at<uint32_t>(a_hist);
+    unsigned long long* d_plane_hist = wa.at<unsigned long long>(a_plane_hist);
+    uint32_t *d_or = wa.at<uint32_t>(a_or), *d_acc = wa.at<uint32_t>(a_acc);
+    EncChunk* d_chunks = wa.at<EncChunk>(a_chunks);
+    EncPlane* d_ep = wa.at<EncPlane>(a_up + u_ep);
+    CUDA_TRY(cudaMemcpyAsync(wa.at<uint8_t>(a_up), up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice, st));
+    // The payload hashes only need the tensors; each is a serial chain, so they run beside everything else.
+    struct Side {
+        cudaStream_t s = nullptr;
+        cudaEvent_t ready = nullptr;
+        ~Side() { if (s) cudaStreamSynchronize(s); if (ready) cudaEventDestroy(ready); }  // nothing of it may outlive the work memory
+    } side;
+    if (!hash_items.empty()) {
+        side.s = ds.stream;
+        if (side.s != st) {
+            CUDA_TRY(cudaEventCreateWithFlags(&side.ready, cudaEventDisableTiming));
+            CUDA_TRY(cudaEventRecord(side.ready, st));
+            CUDA_TRY(cudaStreamWaitEvent(side.s, side.ready, 0));
+        }
+        Bases b{nullptr, 0, 0, nullptr, nullptr};
+        xxh64_kernel<<<uint32_t(hash_items.size()), 32, 0, side.s>>>(wa.at<HashItem>(a_up + u_hitems), uint32_t(hash_items.size()), b, wa.at<uint64_t>(a_hashes));
+        CUDA_TRY(cudaGetLastError());
+    }
+    CUDA_TRY(cudaMemsetAsync(d_plane_hist, 0, (a_hashes - a_plane_hist) + (n_planes ? 0 : 1), st));  // plane counts, OR words, CRC accumulators
+    const bool wide_chunks = chunk_size > SPLIT_TILE;
+    if (counted && n_chunks && wide_chunks) CUDA_TRY(cudaMemsetAsync(d_hist, 0, uint64_t(n_chunks) * 1024, st));  // chunks of several blocks add up
+    if (tile) {
+        const SplitItem* items = wa.at<SplitItem>(a_up + u_splits);
+        const uint32_t n = uint32_t(splits.size());
+        if (!counted) split_kernel<0><<<tile, SPLIT_THREADS, 0, st>>>(items, n, d_planes, d_hist);
+        else if (chunk_size < SPLIT_WIDE_FROM) split_kernel<8><<<tile, SPLIT_THREADS, split_smem_bytes(uint32_t(most_planes), 8), st>>>(items, n, d_planes, d_hist);
+        else {
+            CUDA_TRY(cudaFuncSetAttribute(split_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(split_smem_bytes(4, 32))));  // per device; cheap to repeat
+            split_kernel<32><<<tile, SPLIT_THREADS, split_smem_bytes(uint32_t(most_planes), 32), st>>>(items, n, d_planes, d_hist);
+        }
+        CUDA_TRY(cudaGetLastError());
+    }
+    if (any_delta) {
+        expand_chunks_kernel<<<(n_chunks + 255) / 256, 256, 0, st>>>(d_ep, n_planes, n_chunks, d_chunks, nullptr);
+        CUDA_TRY(cudaGetLastError());
+    }
+    std::vector<uint32_t> or_words(n_or_words);
+    for (auto& tp : plan) {
+        auto blocks = [](uint64_t n) { return unsigned(std::min<uint64_t>((n + 4095) / 4096, 2368)); };
+        if (tp.has_delta) {
+            delta_kernel<<<blocks(tp.delta.len), 256, 0, st>>>(d_planes + tp.planes.back().buf_off, d_planes + tp.delta.buf_off, tp.delta.len);
+            CUDA_TRY(cudaGetLastError());
+            CUDA_TRY(cudaMemsetAsync(d_hist + uint64_t(tp.delta.first_chunk) * 256, 0, uint64_t(tp.delta.n_chunks) * 1024, st));
+            hist_kernel<<<dim3(tp.delta.n_chunks, hist_blocks(std::min<uint64_t>(chunk_size, tp.delta.len))), 256, 0, st>>>(
+                d_chunks + tp.delta.first_chunk, d_planes, d_hist + uint64_t(tp.delta.first_chunk) * 256);
             CUDA_TRY(cudaGetLastError());
         }
+        if (tp.try_mzs) { or_bytes_kernel<<<blocks(tp.planes[0].len), 256, 0, st>>>(d_planes + tp.planes[0].buf_off, tp.planes[0].len, d_or + tp.try_mzs - 1); CUDA_TRY(cudaGetLastError()); }
     }
-    std::vector<uint64_t> hashes(hash_items.size());
-    if (!hash_items.empty()) {
-        CUDA_TRY(upload_vec(d_hitems, hash_items, st));
-        CUDA_TRY(d_hout.alloc(hash_items.size() * 8, st));
-        Bases b{nullptr, 0, 0, nullptr, nullptr};
-        xxh64_kernel<<<uint32_t(hash_items.size()), 32, 0, st>>>(d_hitems.as<HashItem>(), uint32_t(hash_items.size()), b, d_hout.as<uint64_t>());
+    uint32_t most_chunks = 0;
+    for (auto& e : ep) most_chunks = std::max(most_chunks, e.n_chunks);
+    if (counted && n_chunks) {
+        for (uint32_t p0 = 0; p0 < n_planes; p0 += 65535)  // the grid's second dimension is 16 bits
+            plane_hist_kernel<<<dim3((most_chunks + 63) / 64, std::min(n_planes - p0, 65535u)), 256, 0, st>>>(d_ep + p0, d_hist, d_plane_hist + uint64_t(p0) * 256);
         CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemcpyAsync(hashes.data(), d_hout.p, hashes.size() * 8, cudaMemcpyDeviceToHost, st));
     }
+    std::vector<unsigned long long> plane_hist(size_t(n_planes) * 256);
+    CUDA_TRY(to_host(or_words, d_or, st));
+    CUDA_TRY(to_host(plane_hist, d_plane_hist, st));
     std::vector<uint32_t> accs(n_planes);
-    if (opt.emit_plane_crc && n_planes) CUDA_TRY(cudaMemcpyAsync(accs.data(), d_acc.p, accs.size() * 4, cudaMemcpyDeviceToHost, st));
+    if (n_runs) {
+        Bases b{nullptr, 0, 0, nullptr, d_planes};
+        crc_planes_kernel<<<uint32_t((n_runs + 127) / 128), 128, 0, st>>>(wa.at<VerifyTensor>(a_up + u_verify), uint32_t(verify.size()), n_runs, b, d_tabs, d_acc);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(to_host(accs, d_acc, st));
+    }
 
     // Lag-1 counts of every plane Order1ScaleAC accepts, with the plane's rows, for the size comparison below.
     std::vector<double> o1sac_size(n_planes, -1.0);
@@ -443,7 +495,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             CUDA_TRY(upload_vec(d_list, list, st));
             CUDA_TRY(d_counts.alloc(whole.size() * size_t(O1E_PRESENT), st));
             CUDA_TRY(cudaMemsetAsync(d_counts.p, 0, whole.size() * size_t(O1E_PRESENT), st));
-            o1sac_count_kernel<<<uint32_t(whole.size()), 256, 0, st>>>(d_whole.as<EncChunk>(), d_list.as<uint32_t>(), d_planes.as<uint8_t>(), d_counts.as<uint8_t>());
+            o1sac_count_kernel<<<uint32_t(whole.size()), 256, 0, st>>>(d_whole.as<EncChunk>(), d_list.as<uint32_t>(), d_planes, d_counts.as<uint8_t>());
             CUDA_TRY(cudaGetLastError());
             counts.resize(whole.size() * size_t(O1E_PRESENT / 4));
             CUDA_TRY(cudaMemcpyAsync(counts.data(), d_counts.p, counts.size() * 4, cudaMemcpyDeviceToHost, st));
@@ -457,7 +509,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     }
     CUDA_TRY(cudaStreamSynchronize(st));
 
-    prof("split, histograms, CRC / hash, counts");
+    prof("split, histograms, CRC, counts");
     // ---- shared states (compressor.rs:834-881): only whole planes can use one (a chunked plane carries its states inline,
     //      compressor.rs:324-381), and only when the codec is chosen, not forced
     FitResult shared;
@@ -488,8 +540,8 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
 
     prof("shared-state fit");
     // ---- codec per plane ------------------------------------------------------
-    std::vector<uint8_t> plane_codec(n_planes);
-    EncodeLists lists;
+    uint32_t list_sizes[LIST_KINDS] = {0};
+    std::vector<int> list_kind(n_planes, -1);
     std::vector<uint32_t> o1sac_chunks, o1shared_chunks, o1shared_state;  // chunks that fit their own state / that code against shared state o1shared_state[k]
     uint64_t tables_bytes = 0;
     std::vector<std::pair<uint32_t, uint32_t>> recrc;  // (tensor, accumulator) of planes shifted by MantissaZeroStrip: their CRC is taken again below
@@ -555,9 +607,9 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             } else if (tp.post_op == 2) {
                 tp.planes[0].codec = stripped(tp.post_k, nullptr);
                 const uint64_t n = tp.planes[0].len;
-                shift_right_kernel<<<unsigned(std::min<uint64_t>((n + 4095) / 4096, 2368)), 256, 0, st>>>(d_planes.as<uint8_t>() + tp.planes[0].buf_off, n, uint32_t(tp.post_k));
+                shift_right_kernel<<<unsigned(std::min<uint64_t>((n + 4095) / 4096, 2368)), 256, 0, st>>>(d_planes + tp.planes[0].buf_off, n, uint32_t(tp.post_k));
                 CUDA_TRY(cudaGetLastError());
-                relabel_hist_kernel<<<tp.planes[0].n_chunks, 256, 0, st>>>(d_hist.as<uint32_t>(), tp.planes[0].first_chunk, uint32_t(tp.post_k));
+                relabel_hist_kernel<<<tp.planes[0].n_chunks, 256, 0, st>>>(d_hist, tp.planes[0].first_chunk, uint32_t(tp.post_k));
                 CUDA_TRY(cudaGetLastError());
                 tp.chain.nodes.push_back({uint16_t(detail::OP_MZS), {uint8_t(tp.post_k)}});
                 tp.chain.post_plane = 0;
@@ -578,33 +630,29 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
                 PlanePlan& pp = tp.planes[p];
                 const uint32_t pi = (tp.post_op == 1 && p == np - 1) ? tp.delta_index : tp.first_plane + uint32_t(p);
                 if (pp.codec == C_O1SAC && !chunked && pp.row_len && pp.len % pp.row_len) return fail(PTWM_RC_INVALID_INPUT, "order1_scale_ac: the row length does not divide the plane");
-                plane_codec[pi] = uint8_t(pp.codec);
+                EncPlane& e = ep[pi];
+                e.codec = uint32_t(pp.codec); e.shared = pp.shared >= 0;
                 enc.plane_codecs.back().push_back(pp.codec);
                 if (opt.emit_plane_crc) pp.crc = pp.len ? ~(accs[pi] ^ gf2_mulmod(x_pow_8n(T.x2n, pp.len), 0xFFFFFFFFu)) : 0u;
-                int span = 0;
-                if (pp.codec == C_RANS && pp.len) {
+                if (pp.codec == C_IDENTITY || !pp.n_chunks) continue;  // stream slots and table areas only for planes that get coded
+                e.slot_off = slots_bytes; e.slot_stride = uint64_t(enc_slot_cap(std::min(chunk_size, pp.len))) * 4;
+                e.table_off = tables_bytes; e.table_bytes = enc_table_bytes(pp.codec);
+                slots_bytes += e.slot_stride * pp.n_chunks; tables_bytes += uint64_t(e.table_bytes) * pp.n_chunks;
+                if (pp.codec == C_O1SAC) {
+                    for (uint32_t k = 0; k < pp.n_chunks; ++k) (pp.shared >= 0 ? o1shared_chunks : o1sac_chunks).push_back(pp.first_chunk + k);
+                    if (pp.shared >= 0) o1shared_state.insert(o1shared_state.end(), pp.n_chunks, uint32_t(pp.shared));
+                } else if (pp.codec == C_RANS) {
                     const unsigned long long* h = &plane_hist[size_t(pi) * 256];
                     int lo = 0, hi = 255;
                     while (lo < 255 && !h[lo]) ++lo;
                     while (hi > lo && !h[hi]) --hi;
                     if (tp.post_op == 2 && p == 0) { lo >>= tp.post_k; hi >>= tp.post_k; }  // counted before the shift
-                    span = EncodeLists::span_class(uint32_t(hi - lo + 1));
-                }
-                if (pp.codec != C_IDENTITY)  // stream slots and table areas only for planes that get coded
-                    for (uint32_t k = 0; k < pp.n_chunks; ++k) {
-                        EncChunk& ch = chunks[pp.first_chunk + k];
-                        ch.slot_off = slots_bytes; slots_bytes += uint64_t(ch.slot_cap) * 4;
-                        ch.table_off = tables_bytes; tables_bytes += enc_table_bytes(pp.codec);
-                        if (pp.codec == C_O1SAC) (pp.shared >= 0 ? o1shared_chunks : o1sac_chunks).push_back(pp.first_chunk + k);
-                        if (pp.codec == C_RANS) lists.rans[span].push_back(pp.first_chunk + k);
-                        if (pp.codec == C_HUFFMAN) lists.huff.push_back(pp.first_chunk + k);
-                        if (pp.codec == C_TANS) lists.tans.push_back(pp.first_chunk + k);
-                        if (pp.codec == C_O1SAC && pp.shared >= 0) o1shared_state.push_back(uint32_t(pp.shared));
-                    }
+                    list_kind[pi] = rans_list(uint32_t(hi - lo + 1));
+                } else list_kind[pi] = pp.codec == C_HUFFMAN ? int(LIST_HUFFMAN) : int(LIST_TANS);
+                if (list_kind[pi] >= 0) list_sizes[list_kind[pi]] += pp.n_chunks;
             }
-            if (opt.emit_payload_hash) tp.hash = hashes[i];
         }
-        // planes that are not written (the exponent plane or its delta twin, whichever lost) get no encoding pass: plane_codec stays Identity
+        // planes that are not written (the exponent plane or its delta twin, whichever lost) get no encoding pass: their codec stays Identity
         if (!recrc.empty()) {  // CRC of the shifted planes
             std::vector<VerifyTensor> again;
             uint64_t runs = 0;
@@ -612,14 +660,14 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
                 const PlanePlan& pp = plan[rc.first].planes[0];
                 again.push_back(VerifyTensor{make_ref(SP_OUT, pp.buf_off), pp.len, runs, K_PASS, rc.second});
                 runs += (pp.len + VERIFY_RUN - 1) / VERIFY_RUN;
-                CUDA_TRY(cudaMemsetAsync(d_acc.as<uint32_t>() + rc.second, 0, 4, st));
+                CUDA_TRY(cudaMemsetAsync(d_acc + rc.second, 0, 4, st));
             }
             DeviceBuf d_again;
             CUDA_TRY(upload_vec(d_again, again, st));
-            Bases b{nullptr, 0, 0, nullptr, d_planes.as<uint8_t>()};
-            crc_planes_kernel<<<uint32_t((runs + 127) / 128), 128, 0, st>>>(d_again.as<VerifyTensor>(), uint32_t(again.size()), runs, b, d_tabs, d_acc.as<uint32_t>());
+            Bases b{nullptr, 0, 0, nullptr, d_planes};
+            crc_planes_kernel<<<uint32_t((runs + 127) / 128), 128, 0, st>>>(d_again.as<VerifyTensor>(), uint32_t(again.size()), runs, b, d_tabs, d_acc);
             CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cudaMemcpyAsync(accs.data(), d_acc.p, accs.size() * 4, cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(to_host(accs, d_acc, st));
             CUDA_TRY(cudaStreamSynchronize(st));
             for (auto& rc : recrc) {
                 PlanePlan& pp = plan[rc.first].planes[0];
@@ -630,26 +678,34 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
 
     prof("codec and chain choice (host)");
     // ---- tables and streams ---------------------------------------------------
-    CUDA_TRY(upload_vec(d_codec, plane_codec, st));
-    if (n_chunks) CUDA_TRY(cudaMemcpyAsync(d_chunks.p, chunks.data(), chunks.size() * sizeof(EncChunk), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(d_tables.alloc(tables_bytes, st));
-    CUDA_TRY(d_results.alloc(uint64_t(n_chunks) * sizeof(EncResult), st));
-    CUDA_TRY(cudaMemsetAsync(d_results.p, 0, uint64_t(n_chunks) * sizeof(EncResult) + (n_chunks ? 0 : 1), st));
-    CUDA_TRY(d_slots.alloc(slots_bytes + ENC_PAD, st));
-    std::vector<EncResult> results(n_chunks);
-    prof("  work memory for tables and streams");
-    DeviceBuf d_o1list, d_lists;
+    uint32_t n_listed = 0, list_at[LIST_KINDS];
+    for (int k = 0; k < LIST_KINDS; ++k) { list_at[k] = n_listed; n_listed += list_sizes[k]; }
+    for (uint32_t p = 0; p < n_planes; ++p) if (list_kind[p] >= 0) { ep[p].list_off = list_at[list_kind[p]]; list_at[list_kind[p]] += ep[p].n_chunks; }
+    Arena wb;
+    const uint64_t b_tables = wb.add(tables_bytes), b_results = wb.add(uint64_t(n_chunks) * sizeof(EncResult)), b_lists = wb.add(uint64_t(n_listed) * 4),
+                   b_places = wb.add(uint64_t(n_chunks) * sizeof(ChunkPlace)), b_sizes = wb.add(uint64_t(n_planes) * sizeof(PlaneSizes)),
+                   b_slots = wb.add(slots_bytes + ENC_PAD);
+    CUDA_TRY(wb.alloc(st));
+    uint8_t *d_tables = wb.at<uint8_t>(b_tables), *d_slots = wb.at<uint8_t>(b_slots);
+    EncResult* d_results = wb.at<EncResult>(b_results);
+    uint32_t* d_lists = wb.at<uint32_t>(b_lists);
+    if (n_planes) CUDA_TRY(cudaMemcpyAsync(d_ep, ep.data(), ep.size() * sizeof(EncPlane), cudaMemcpyHostToDevice, st));
+    if (n_chunks) {
+        expand_chunks_kernel<<<(n_chunks + 255) / 256, 256, 0, st>>>(d_ep, n_planes, n_chunks, d_chunks, d_lists);
+        CUDA_TRY(cudaGetLastError());
+    }
+    prof("  work memory, chunk lists");
     int64_t rc;
+    DeviceBuf d_o1list;
     if (!o1sac_chunks.empty()) {  // Order1ScaleAC: counts, rows, then the range coder, one chunk per block / thread
         CUDA_TRY(upload_vec(d_o1list, o1sac_chunks, st));
-        for (uint32_t ci : o1sac_chunks) CUDA_TRY(cudaMemsetAsync(d_tables.as<uint8_t>() + chunks[ci].table_off, 0, O1E_PRESENT, st));
+        for (auto& e : ep) if (e.codec == C_O1SAC && !e.shared && e.n_chunks) CUDA_TRY(cudaMemset2DAsync(d_tables + e.table_off, e.table_bytes, 0, O1E_PRESENT, e.n_chunks, st));
         const uint32_t n_o1 = uint32_t(o1sac_chunks.size());
-        o1sac_count_kernel<<<n_o1, 256, 0, st>>>(d_chunks.as<EncChunk>(), d_o1list.as<uint32_t>(), d_planes.as<uint8_t>(), d_tables.as<uint8_t>());
+        o1sac_count_kernel<<<n_o1, 256, 0, st>>>(d_chunks, d_o1list.as<uint32_t>(), d_planes, d_tables);
         CUDA_TRY(cudaGetLastError());
-        o1sac_fit_kernel<<<n_o1, 288, 0, st>>>(d_chunks.as<EncChunk>(), d_o1list.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
+        o1sac_fit_kernel<<<n_o1, 288, 0, st>>>(d_chunks, d_o1list.as<uint32_t>(), d_tables, d_results);
         CUDA_TRY(cudaGetLastError());
-        o1sac_encode_kernel<<<(n_o1 + 63) / 64, 64, 0, st>>>(d_chunks.as<EncChunk>(), d_o1list.as<uint32_t>(), n_o1, d_planes.as<uint8_t>(), d_tables.as<uint8_t>(),
-                                                             d_slots.as<uint8_t>(), d_results.as<EncResult>());
+        o1sac_encode_kernel<<<(n_o1 + 63) / 64, 64, 0, st>>>(d_chunks, d_o1list.as<uint32_t>(), n_o1, d_planes, d_tables, d_slots, d_results);
         CUDA_TRY(cudaGetLastError());
     }
     DeviceBuf d_o1shared;
@@ -674,68 +730,50 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
                 if (has) put_row(1 + ctx, stt.rows[k++].data());
             }
         }
-        for (size_t k = 0; k < o1shared_chunks.size(); ++k)
-            CUDA_TRY(cudaMemcpyAsync(d_tables.as<uint8_t>() + chunks[o1shared_chunks[k]].table_off + O1E_PRESENT, images[o1shared_state[k]].data(),
-                                     images[o1shared_state[k]].size(), cudaMemcpyHostToDevice, st));
+        size_t k = 0;
+        for (auto& e : ep) if (e.codec == C_O1SAC && e.shared) for (uint32_t j = 0; j < e.n_chunks; ++j, ++k)
+            CUDA_TRY(cudaMemcpyAsync(d_tables + e.table_off + uint64_t(j) * e.table_bytes + O1E_PRESENT, images[o1shared_state[k]].data(), images[o1shared_state[k]].size(), cudaMemcpyHostToDevice, st));
         CUDA_TRY(upload_vec(d_o1shared, o1shared_chunks, st));
         const uint32_t n_sh = uint32_t(o1shared_chunks.size());
-        o1sac_encode_kernel<<<(n_sh + 63) / 64, 64, 0, st>>>(d_chunks.as<EncChunk>(), d_o1shared.as<uint32_t>(), n_sh, d_planes.as<uint8_t>(), d_tables.as<uint8_t>(),
-                                                             d_slots.as<uint8_t>(), d_results.as<EncResult>());
+        o1sac_encode_kernel<<<(n_sh + 63) / 64, 64, 0, st>>>(d_chunks, d_o1shared.as<uint32_t>(), n_sh, d_planes, d_tables, d_slots, d_results);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaStreamSynchronize(st));  // the images are host memory of this scope
     }
     prof("  order1_scale_ac chunks");
+    const uint64_t frame_hdr = chunked ? 5 : 0;  // [state_version][state_len u32] in front of every chunk; an unchunked plane has none
+    std::vector<PlaneSizes> sizes(n_planes);
     if (n_chunks) {
-        table_kernel<<<(n_chunks + 3) / 4, 128, 0, st>>>(d_chunks.as<EncChunk>(), n_chunks, d_codec.as<uint8_t>(), d_hist.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
+        table_kernel<<<(n_chunks + 3) / 4, 128, 0, st>>>(d_ep, d_chunks, n_chunks, d_hist, d_tables, d_results);
         CUDA_TRY(cudaGetLastError());
         prof("  table_kernel");
-        if ((rc = launch_encoders(d_chunks.as<EncChunk>(), lists, d_lists, d_planes.as<uint8_t>(), d_tables.as<uint8_t>(), d_slots.as<uint8_t>(),
-                                  d_results.as<EncResult>(), st)) < 0) return rc;
+        if ((rc = launch_encoders(d_chunks, d_lists, list_sizes, d_planes, d_tables, d_slots, d_results, st)) < 0) return rc;
         prof("  stream encoders");
-        CUDA_TRY(cudaMemcpyAsync(results.data(), d_results.p, results.size() * sizeof(EncResult), cudaMemcpyDeviceToHost, st));
+        layout_kernel<<<n_planes, 256, 0, st>>>(d_ep, d_chunks, d_results, uint32_t(chunked), wb.at<ChunkPlace>(b_places), wb.at<PlaneSizes>(b_sizes));
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(to_host(sizes, wb.at<PlaneSizes>(b_sizes), st));
     }
     CUDA_TRY(cudaStreamSynchronize(st));
-
     prof("tables and streams");
-    // ---- layout: chunk frames, plane payloads, records ------------------------
-    std::vector<uint32_t> chunk_mode(n_chunks);
-    const uint64_t frame_hdr = chunked ? 5 : 0;  // [state_version][state_len u32] in front of every chunk; an unchunked plane has none
-    for (auto& tp : plan) for (auto& pp : tp.planes) {
+    // ---- layout: records around the planes' frames, whose sizes the device has added up ------------------------
+    for (auto& tp : plan) for (size_t p = 0; p < tp.planes.size(); ++p) {
+        PlanePlan& pp = tp.planes[p];
         if (pp.len == 0) {  // an empty plane is one empty chunk (compressor.rs:333-345), or an empty payload / the raw tag alone when unchunked
             // Order1ScaleAC fitted to no symbols: no rows, the smoothed marginal (16 everywhere), and the coder's six flush bytes
             const uint64_t body = pp.codec == C_IDENTITY ? 0 : pp.codec == C_O1SAC ? 6 : 1;
             if (pp.codec == C_O1SAC) pp.state_len = 32 + 512;
-            pp.frame_size.push_back(frame_hdr + pp.state_len + body);
-            pp.payload_len = pp.frame_size[0];
+            pp.payload_len = frame_hdr + pp.state_len + body;
             continue;
         }
-        for (uint32_t k = 0; k < pp.n_chunks; ++k) {
-            uint32_t ci = pp.first_chunk + k;
-            const EncResult& r = results[ci];
-            uint64_t n = chunks[ci].n, size;
-            if (pp.codec == C_IDENTITY) { chunk_mode[ci] = 0; size = frame_hdr + n; }
-            else if (pp.codec == C_O1SAC) {
-                chunk_mode[ci] = pp.shared >= 0 ? (5 | GATHER_BARE) : 5;
-                const uint64_t own_state = pp.shared >= 0 ? 0 : r.stream_len[1];
-                size = frame_hdr + own_state + r.stream_len[0];  // a plane's own state sits in front of the coder's bytes
-                if (!chunked) pp.state_len = own_state;
-            } else {
-                uint64_t blob;
-                if (pp.codec == C_TANS) blob = 3 + 3 * uint64_t(r.hdr_n) + 8 + r.stream_len[0];
-                else {
-                    uint64_t hdr = pp.codec == C_RANS ? 1 + 2 * (uint64_t(r.hdr_n) + 1) : (r.hdr_n <= 127 ? 1 : 2) + (uint64_t(r.hdr_n) + 1) / 2;
-                    blob = hdr + 16 + uint64_t(r.stream_len[0]) + r.stream_len[1] + r.stream_len[2] + r.stream_len[3];
-                }
-                // stored raw when coding does not shrink the chunk (compress.rs NotBeneficial) or the length rule refuses it (length_prefix.rs:29-33)
-                bool coded = r.coded && blob < n && (pp.codec == C_HUFFMAN || n <= (1ull << 30) || n <= blob * 64);
-                chunk_mode[ci] = coded ? (pp.codec == C_RANS ? 2 : pp.codec == C_HUFFMAN ? 3 : 4) : 1;
-                size = coded ? frame_hdr + 1 + 4 + blob : frame_hdr + 1 + n;
-            }
-            if (!chunked) chunk_mode[ci] |= GATHER_NOFRAME;
-            pp.frame_size.push_back(size);
-            pp.payload_len += size;
-        }
+        const PlaneSizes& z = sizes[plane_index(tp, p)];
+        pp.payload_len = z.frames; pp.table_len = z.entries;
+        if (!chunked && pp.codec == C_O1SAC) pp.state_len = z.state_len;
         if (pp.payload_len > 0xFFFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "plane payload exceeds the u32 offset range (compressor.rs:370-372)");
+    }
+    std::vector<uint64_t> hashes(hash_items.size());
+    if (!hashes.empty()) {
+        CUDA_TRY(to_host(hashes, wa.at<uint64_t>(a_hashes), side.s));
+        CUDA_TRY(cudaStreamSynchronize(side.s));
+        prof("hashes");
     }
 
     // Extension Table: chain ops in registry order, then the used codecs in built-in order (container.rs:167-223)
@@ -802,7 +840,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
 
     std::vector<uint8_t> staged = head;
     std::vector<uint64_t> triples = {0, 0, head.size()};
-    std::vector<GatherItem> gathers;
+    std::vector<PlaneDst> dsts(n_planes, PlaneDst{ENC_NOWHERE, ENC_NOWHERE});
     std::vector<uint8_t> index;
     put_varint(index, n_tensors);
     uint64_t pos = head.size();
@@ -820,7 +858,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
         put_varint(b, plan[i].chain_id); put_varint(b, t.dtype_code); b.push_back(2 /* Format.TORCH */); put_varint(b, t.nbytes);
         put_varint(b, t.ndim);
         for (int d = 0; d < t.ndim; ++d) put_varint(b, t.shape[d]);
-        if (opt.emit_payload_hash) put_u64(b, plan[i].hash);
+        if (opt.emit_payload_hash) put_u64(b, hashes[i]);
         put_varint(b, plan[i].planes.size());
         for (size_t p = 0; p < plan[i].planes.size(); ++p) {
             PlanePlan& pp = plan[i].planes[p];
@@ -847,8 +885,8 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
                     continue;
                 }
                 flush(b);
-                gathers.push_back(GatherItem{pos, pp.first_chunk, chunk_mode[pp.first_chunk]});
-                pos += pp.frame_size[0];
+                dsts[plane_index(plan[i], p)].frames = pos;
+                pos += pp.payload_len;
                 continue;
             }
             b.push_back(uint8_t(0x02 | (opt.emit_plane_crc ? 0x01 : 0)));
@@ -856,13 +894,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             put_varint(b, table_index(2, uint16_t(pp.codec)));
             put_varint(b, pp.payload_len);
             if (opt.emit_plane_crc) put_u32(b, pp.crc);
-            put_varint(b, pp.frame_size.size());
-            uint64_t off = 0;
-            for (size_t k = 0; k < pp.frame_size.size(); ++k) {
-                put_varint(b, off);
-                put_varint(b, pp.len ? chunks[pp.first_chunk + k].n : 0);
-                off += pp.frame_size[k];
-            }
+            if (pp.len == 0) { put_varint(b, 1); put_varint(b, 0); put_varint(b, 0); } else put_varint(b, pp.n_chunks);
             if (pp.len == 0) {  // the one empty frame is host data
                 if (pp.codec == C_O1SAC) {
                     b.push_back(1); put_u32(b, 32 + 512);
@@ -877,10 +909,8 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
                 continue;
             }
             flush(b);
-            for (size_t k = 0; k < pp.frame_size.size(); ++k) {
-                gathers.push_back(GatherItem{pos, pp.first_chunk + uint32_t(k), chunk_mode[pp.first_chunk + k]});
-                pos += pp.frame_size[k];
-            }
+            dsts[plane_index(plan[i], p)] = PlaneDst{pos + pp.table_len, pos};  // the gather writes the chunk table, then the frames
+            pos += pp.table_len + pp.payload_len;
         }
         if (!b.empty()) flush(b);
         size_t nl = std::strlen(t.name);
@@ -900,15 +930,16 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     // ---- write the container ----------------------------------------------------
     enc.size = pos; enc.device = device;
     CUDA_TRY(enc.out.alloc(pos, st));
-    DeviceBuf d_staged, d_triples, d_gathers;
-    CUDA_TRY(upload_vec(d_staged, staged, st));
-    CUDA_TRY(upload_vec(d_triples, triples, st));
-    CUDA_TRY(upload_vec(d_gathers, gathers, st));
-    scatter_kernel<<<uint32_t(triples.size() / 3), 128, 0, st>>>(d_staged.as<uint8_t>(), d_triples.as<uint64_t>(), enc.out.as<uint8_t>());
+    Upload rec;
+    const uint64_t r_staged = rec.add(staged), r_triples = rec.add(triples), r_dsts = rec.add(dsts);
+    Arena wr;
+    wr.add(rec.bytes.size());
+    CUDA_TRY(wr.alloc(st));
+    CUDA_TRY(cudaMemcpyAsync(wr.at<uint8_t>(0), rec.bytes.data(), rec.bytes.size(), cudaMemcpyHostToDevice, st));
+    scatter_kernel<<<uint32_t(triples.size() / 3), 128, 0, st>>>(wr.at<uint8_t>(r_staged), wr.at<uint64_t>(r_triples), enc.out.as<uint8_t>());
     CUDA_TRY(cudaGetLastError());
-    if (!gathers.empty()) {
-        gather_kernel<<<uint32_t(gathers.size()), 128, 0, st>>>(d_gathers.as<GatherItem>(), d_chunks.as<EncChunk>(), d_results.as<EncResult>(), d_planes.as<uint8_t>(),
-                                                                d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), enc.out.as<uint8_t>());
+    if (n_chunks) {
+        gather_kernel<<<n_chunks, 128, 0, st>>>(d_chunks, d_results, wb.at<ChunkPlace>(b_places), wr.at<PlaneDst>(r_dsts), d_planes, d_tables, d_slots, enc.out.as<uint8_t>());
         CUDA_TRY(cudaGetLastError());
     }
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -935,10 +966,9 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         return int64_t(n);
     }
     if (n > 0xFFFFFFFFull && codec == C_O1SAC) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
-    DeviceBuf d_chunk, d_codec, d_hist, d_phist, d_tables, d_results, d_slots, d_gather, d_list;
+    DeviceBuf d_chunk, d_tables, d_results, d_slots, d_list, d_job;
     const uint64_t slot_cap = align_up(((n / 4 + 1) * 12 + 7) / 8 + 64, 16);  // a symbol takes at most 12 bits in any of the codecs; slots are written in aligned words
     EncChunk chunk{0, 0, 0, uint32_t(n), uint32_t(slot_cap), 0, 0};
-    const uint8_t codec_byte = uint8_t(codec);
     if (codec == C_O1SAC) {
         // The flat ABI has no way to return a fitted state, so the rows come from the caller (the shared-state form of
         // order1_scale_ac.rs:620-633): [bitmap 32][marginal 512][rows 512 each], one row spanning the plane.
@@ -985,50 +1015,35 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
     }
     uint32_t mode = 1;
     uint64_t size = 1 + uint64_t(n);
-    CUDA_TRY(d_chunk.alloc(sizeof(EncChunk), st, false));
-    CUDA_TRY(d_results.alloc(sizeof(EncResult), st, false));
-    CUDA_TRY(d_tables.alloc(enc_table_bytes(codec), st, false));
+    // one block of device memory: what the kernels find filled in, then the table and the slots
+    struct Job { EncPlane plane; EncChunk chunk; EncResult result; uint32_t list, pad[3]; uint32_t hist[256]; } job{};
+    const uint64_t job_bytes = align_up(sizeof(Job), 256);
     if (n <= 0xFFFFFFFFull) {  // the length prefix is a u32; longer planes stay raw
         if (slot_cap > 0x3FFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
-        CUDA_TRY(d_codec.alloc(1, st, false));
-        CUDA_TRY(d_list.alloc(4, st, false));
-        CUDA_TRY(d_hist.alloc(256 * sizeof(uint32_t), st, false));
-        CUDA_TRY(d_phist.alloc(256 * sizeof(unsigned long long), st, false));
-        CUDA_TRY(d_slots.alloc(4 * slot_cap + ENC_PAD, st, false));
-        CUDA_TRY(cudaMemcpyAsync(d_chunk.p, &chunk, sizeof(chunk), cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(d_codec.p, &codec_byte, 1, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemsetAsync(d_phist.p, 0, 256 * sizeof(unsigned long long), st));
-        hist_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), in, d_hist.as<uint32_t>(), d_phist.as<unsigned long long>());
-        table_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), 1, d_codec.as<uint8_t>(), d_hist.as<uint32_t>(), d_tables.as<uint8_t>(), d_results.as<EncResult>());
-        CUDA_TRY(cudaMemsetAsync(d_list.p, 0, 4, st));  // the list of chunks to code: chunk 0
-        const uint32_t* list = d_list.as<uint32_t>();
-        if (codec == C_RANS) rans_encode_kernel<<<1, 32, renc_smem_bytes(256), st>>>(d_chunk.as<EncChunk>(), list, 1, 256, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
-        else if (codec == C_HUFFMAN) huffman_encode_kernel<<<1, 128, 0, st>>>(d_chunk.as<EncChunk>(), list, 1, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
-        else tans_encode_kernel<<<1, 32, 0, st>>>(d_chunk.as<EncChunk>(), list, 1, in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), d_results.as<EncResult>());
+        job.plane.codec = uint32_t(codec);
+        job.chunk = chunk; job.chunk.slot_off = job_bytes + ENC_HUFF_TABLE_BYTES; job.chunk.table_off = job_bytes;
+        CUDA_TRY(d_job.alloc(job.chunk.slot_off + 4 * slot_cap + ENC_PAD, st, false));
+        CUDA_TRY(cudaMemcpyAsync(d_job.p, &job, sizeof job, cudaMemcpyHostToDevice, st));
+        Job* d = d_job.as<Job>();
+        uint8_t* area = d_job.as<uint8_t>();
+        hist_kernel<<<dim3(1, hist_blocks(n)), 256, 0, st>>>(&d->chunk, in, d->hist);
+        table_kernel<<<1, 128, 0, st>>>(&d->plane, &d->chunk, 1, d->hist, area, &d->result);
+        if (codec == C_RANS) rans_encode_kernel<<<1, 32, renc_smem_bytes(256), st>>>(&d->chunk, &d->list, 1, 256, in, area, area, &d->result);
+        else if (codec == C_HUFFMAN) huffman_encode_kernel<<<1, 128, 0, st>>>(&d->chunk, &d->list, 1, in, area, area, &d->result);
+        else tans_encode_kernel<<<1, 32, 0, st>>>(&d->chunk, &d->list, 1, in, area, area, &d->result);
         CUDA_TRY(cudaGetLastError());
         EncResult r;
-        CUDA_TRY(cudaMemcpyAsync(&r, d_results.p, sizeof(r), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaMemcpyAsync(&r, &d->result, sizeof(r), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
-        uint64_t blob;
-        if (codec == C_TANS) blob = 3 + 3 * uint64_t(r.hdr_n) + 8 + r.stream_len[0];
-        else {
-            const uint64_t hdr = codec == C_RANS ? 1 + 2 * (uint64_t(r.hdr_n) + 1) : (r.hdr_n <= 127 ? 1 : 2) + (uint64_t(r.hdr_n) + 1) / 2;
-            blob = hdr + 16 + uint64_t(r.stream_len[0]) + r.stream_len[1] + r.stream_len[2] + r.stream_len[3];
-        }
-        const bool coded = r.coded && blob < n && (codec == C_HUFFMAN || n <= (1ull << 30) || n <= blob * 64);
-        if (coded) { mode = codec == C_RANS ? 2 : codec == C_HUFFMAN ? 3 : 4; size = 1 + 4 + blob; }
-    } else {
-        CUDA_TRY(d_slots.alloc(16, st, false));
+        size = enc_payload(codec, false, uint32_t(n), r, mode);
     }
     if (need(size) > out_cap) return fail(PTWM_RC_BUFFER_TOO_SMALL, "output buffer too small");
     if (mode == 1 && n > 0xFFFFFFFFull) {  // raw: tag byte, then the plane
         CUDA_TRY(cudaMemsetAsync(out, 0, 1, st));
         CUDA_TRY(cudaMemcpyAsync(out + 1, in, n, cudaMemcpyDeviceToDevice, st));
     } else {
-        const GatherItem g{0, 0, mode | GATHER_BARE};
-        CUDA_TRY(d_gather.alloc(sizeof(g), st, false));
-        CUDA_TRY(cudaMemcpyAsync(d_gather.p, &g, sizeof(g), cudaMemcpyHostToDevice, st));
-        gather_kernel<<<1, 128, 0, st>>>(d_gather.as<GatherItem>(), d_chunk.as<EncChunk>(), d_results.as<EncResult>(), in, d_tables.as<uint8_t>(), d_slots.as<uint8_t>(), out);
+        Job* d = d_job.as<Job>();
+        gather_one_kernel<<<1, 512, 0, st>>>(&d->chunk, &d->result, mode | GATHER_BARE, in, d_job.as<uint8_t>(), d_job.as<uint8_t>(), out);
         CUDA_TRY(cudaGetLastError());
     }
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -1056,7 +1071,7 @@ int64_t ptwm_b200_encode_model(const ptwm_b200_encode_tensor* tensors, size_t n,
     cudaStream_t st = stream ? reinterpret_cast<cudaStream_t>(uintptr_t(stream)) : ds->stream;
     try {
         std::unique_ptr<ptwm_b200_encoded> e(new ptwm_b200_encoded);
-        rc = encode_impl(tensors, n, opt, int(device_ordinal), st, ds->d_tabs, *e);
+        rc = encode_impl(tensors, n, opt, int(device_ordinal), st, *ds, *e);
         if (rc < 0) return rc;
         *out = e.release();
         return 0;
