@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "../../include/ptwm_b200.h"
 #include "kernels.cuh"
@@ -33,6 +34,8 @@ struct DeviceState {
     cudaStream_t stream = nullptr;   // the library's process-persistent stream for the device
     CrcTables* d_tabs = nullptr;     // CRC byte table and x^(2^k) powers
     bool attrs = false;
+    cudaStream_t side[4] = {nullptr, nullptr, nullptr, nullptr};  // independent decoders of one pass run side by side
+    std::vector<uint32_t*> words;    // free words of pinned memory, one for every plan that has run (its status summary)
     void* stage = nullptr;           // pinned host buffer the plan work lists pass through on their way to the device
     size_t stage_cap = 0;
 };

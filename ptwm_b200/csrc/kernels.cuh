@@ -30,6 +30,12 @@ __device__ __forceinline__ uint8_t* wr(const Bases& b, Ref r) {
     return (uint32_t(r >> 62) == SP_SCRATCH ? b.scratch : b.out) + off;
 }
 
+// A failed item: its own status word, and the word before the first one, which is all the host looks at when nothing failed.
+__device__ __forceinline__ void report(uint32_t* status, uint32_t id, uint32_t err) {
+    atomicMax(&status[id], err);
+    atomicMax(status - 1, err);
+}
+
 __device__ __forceinline__ uint32_t ld_u32_unaligned(const uint8_t* p) {
     return uint32_t(p[0]) | uint32_t(p[1]) << 8 | uint32_t(p[2]) << 16 | uint32_t(p[3]) << 24;
 }
@@ -809,7 +815,7 @@ __global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem*
             if (rq > end_q) err = ST_STREAM_UNDERRUN;  // decompress.rs:99-104
         }
     }
-    if (err) atomicMax(&status[it.id], err);
+    if (err) report(status, it.id, err);
 }
 
 // ---- canonical Huffman -----------------------------------------------------
@@ -1101,46 +1107,103 @@ __global__ void __launch_bounds__(32) huffman_decode_kernel(const DecodeItem* __
         }
         if (!err && (c_lo | c_hi) != 0) err = ST_NOT_CONSUMED;
     }
-    if (err) atomicMax(&status[it.id], err);
+    if (err) report(status, it.id, err);
 }
 
 // ---- tANS ------------------------------------------------------------------
 // One serial stream per chunk: a symbol is a table look-up by the state and the
-// next state needs the bits the entry says.  One warp decodes a chunk all the
+// next state needs the bits the entry says.  Many lanes decode a chunk all the
 // same.  The stream's bits are cut into equal runs, one per lane, and every
 // lane decodes its run from the cut in a guessed state.  A decoder that starts
 // wrong falls in with the right one after a while (same bit, same state; about
-// 1,100 symbols on an exponent plane of normal weights, 200 - 700 on flatter
-// planes) and stays with it, so what a lane is left with at the end of its run
-// (bit position and state) is mostly what the serial decoder has there.  That
-// is where the next lane has to start: lanes whose start was something else go
-// again from it, until nobody's start changes.  Every round settles at least
-// one more lane, so the worst case is the serial chain; the usual number of
-// rounds is such that (rounds x run) is four to five times the length above.
-// Then every lane knows where its symbols start and how many it has, the counts
-// are added up, and a last pass decodes again and places the symbols.
+// 1,100 - 1,600 symbols on an exponent plane of normal weights, 200 - 700 on
+// flatter planes) and stays with it, so what a lane is left with at the end of
+// its run (bit position and state) is mostly what the serial decoder has there.
+// That is where the next lane has to start: lanes whose start was something
+// else go again from it, until nobody's start changes.  Every round settles at
+// least one more lane, so the worst case is the serial chain; the usual number
+// of rounds is such that all rounds together are some 8 Ki steps (a stream of
+// 64 Ki symbols: 4.6 rounds of 32 runs, 15 of 128).  Then every lane knows where
+// its symbols start and how many it has, and a last pass decodes once more and
+// places them.  Starting a lane from several guesses side by side saves one
+// round in four and costs more than that.
 //
-// A stream of 64 Ki symbols took 1.75 ms in a lane of its own (52 cycles per
-// symbol); the runs take it to 1/5 of that, and the lanes of a warp share one
-// 8 KiB table, so an SM keeps 640 runs in flight instead of 32 streams.
+// A stream of 64 Ki symbols in a lane of its own took 1.75 ms (52 cycles per
+// symbol), and 32 of them were all an SM held.
 //
 // Table: one word per state, bit count (low five bits: what a funnel shift
-// takes of it) | symbol << 8 | baseline << 16.
-constexpr uint32_t TANS_MIN_RUN = 128;      // symbols per lane at least
+// takes of it) | symbol << 8 | shared-memory address of the baseline's entry <<
+// 16, so that the next entry's address is one multiply-add from the bits.
+constexpr uint32_t TANS_MIN_RUN = 256;        // symbols per lane at least: a short chunk is mostly serial, and every round costs a few hundred cycles beside its symbols
 constexpr uint32_t TANS_GROUP_BITS = 8 * 11;  // a group of eight symbols takes at most this many
+
+// Builds one chunk's table with a full warp (mod.rs:199-211,346-369); false on a bad header.  `work` holds 512 words.
+__device__ __forceinline__ bool tans_build(const uint8_t* src, uint32_t nsym, uint32_t* table, uint32_t* work, uint32_t lane) {
+    const uint32_t base = uint32_t(__cvta_generic_to_shared(table));
+    uint32_t* count = work;  // per symbol; while the states are numbered: the next occurrence's number
+    uint32_t* first = work + 256;
+    for (uint32_t i = lane; i < 256; i += 32) count[i] = 0;
+    __syncwarp();
+    uint32_t sum = 0;
+    bool bad = false;
+    for (uint32_t i = lane; i < nsym; i += 32) {
+        const uint32_t sy = src[3 + 3 * i], fr = uint32_t(src[4 + 3 * i]) | uint32_t(src[5 + 3 * i]) << 8;
+        bad |= fr == 0 || fr > 2048;             // mod.rs:404-411 (above 2048 the sum cannot come out right)
+        bad |= atomicExch(&count[sy], fr) != 0;  // a symbol listed twice
+        sum += fr;
+    }
+    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+    __syncwarp();
+    if (__any_sync(0xFFFFFFFFu, bad) || sum != 2048) return false;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) mine += count[lane * 8 + k];
+    uint32_t run = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, run, d); if (lane >= uint32_t(d)) run += t; }
+    run -= mine;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { first[lane * 8 + k] = run; run += count[lane * 8 + k]; }
+    __syncwarp();
+    // position k of the symbols in order goes to state 1283 k mod 2048; lane l places positions 64 l .. 64 l + 63
+    uint32_t sy = 0;
+    for (uint32_t d = 128; d; d >>= 1) if (sy + d < 256 && first[sy + d] <= 64 * lane) sy += d;
+    for (uint32_t k = 64 * lane; k < 64 * lane + 64; ++k) {
+        while (sy < 255 && first[sy + 1] <= k) ++sy;
+        table[(k * 1283u) & 2047u] = sy;
+    }
+    __syncwarp();
+    for (uint32_t u0 = 0; u0 < 2048; u0 += 32) {  // the states of a symbol are numbered in increasing order, from its frequency on
+        const uint32_t s = table[u0 + lane], same = __match_any_sync(0xFFFFFFFFu, s), before = same & ((1u << lane) - 1u);
+        const uint32_t x = count[s] + __popc(before), nb = 11 - (31 - __clz(x));
+        __syncwarp();
+        table[u0 + lane] = nb | s << 8 | (base + 4 * ((x << nb) - 2048u)) << 16;
+        if (!before) count[s] += __popc(same);
+        __syncwarp();
+    }
+    return true;
+}
+
+template <int THREADS>
 struct TansShared {
     uint32_t table[2048];
-    uint32_t ring[16 * 32];  // while the table is built: counts of the symbols, first spread position of each
+    uint32_t ring[32 * THREADS];  // 64 bytes of stream per lane, kept twice; while the tables are built: 512 words of work space
+    uint64_t words[THREADS];      // what the lanes hand on: the place a run ended at; counts of the warps before
+    uint32_t built;
 };
+template <int THREADS>
+__device__ __forceinline__ void tans_sync() { if (THREADS == 32) __syncwarp(); else __syncthreads(); }
 
-__global__ void __launch_bounds__(32, 20) tans_decode_kernel(const DecodeItem* __restrict__ items, Bases bases, uint32_t* __restrict__ status) {
-    __shared__ TansShared sh;
-    const uint32_t lane = threadIdx.x;
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) tans_decode_kernel(const DecodeItem* __restrict__ items, Bases bases, uint32_t* __restrict__ status) {
+    __shared__ TansShared<THREADS> sh;
+    constexpr uint32_t WORD = THREADS * 4;  // bytes between two words of a lane's ring
+    const uint32_t l = threadIdx.x;
     const DecodeItem it = items[blockIdx.x];
     const uint8_t* src = rd(bases, it.src);
-    const uint32_t* table = sh.table;
+    const uint32_t table = uint32_t(__cvta_generic_to_shared(sh.table));
 
-    // ---- header and table (mod.rs:388-425,199-211,346-369) ----
+    // ---- header (mod.rs:388-425) and table ----
     uint32_t nsym = 0;
     bool bad = it.src_len < 3 || src[0] != 11;
     if (!bad) {
@@ -1153,203 +1216,203 @@ __global__ void __launch_bounds__(32, 20) tans_decode_kernel(const DecodeItem* _
         total_bits = uint64_t(ld_u32_unaligned(bs - 8)) | uint64_t(ld_u32_unaligned(bs - 4)) << 32;
         bad = total_bits > uint64_t(it.src_len - (3 + nsym * 3 + 8)) * 8;
     }
-    if (!bad) {
-        uint32_t* count = sh.ring;         // per symbol; while states are numbered: the next occurrence's number
-        uint32_t* first = sh.ring + 256;
-        for (uint32_t i = lane; i < 256; i += 32) count[i] = 0;
-        __syncwarp();
-        uint32_t sum = 0;
-        for (uint32_t i = lane; i < nsym; i += 32) {
-            const uint32_t sy = src[3 + 3 * i], fr = uint32_t(src[4 + 3 * i]) | uint32_t(src[5 + 3 * i]) << 8;
-            bad |= fr == 0 || fr > 2048;                  // mod.rs:404-411 (above 2048 the sum cannot come out right)
-            bad |= atomicExch(&count[sy], fr) != 0;       // a symbol listed twice
-            sum += fr;
-        }
-        sum = __reduce_add_sync(0xFFFFFFFFu, sum);
-        bad = __any_sync(0xFFFFFFFFu, bad) || sum != 2048;
-        __syncwarp();
-        if (!bad) {
-            uint32_t mine = 0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) mine += count[lane * 8 + k];
-            uint32_t run = mine;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, run, d); if (lane >= uint32_t(d)) run += t; }
-            run -= mine;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) { first[lane * 8 + k] = run; run += count[lane * 8 + k]; }
-            __syncwarp();
-            // position k of the symbols in order goes to state 1283 k mod 2048; lane l places positions 64 l .. 64 l + 63
-            uint32_t sy = 0;
-            for (uint32_t d = 128; d; d >>= 1) if (sy + d < 256 && first[sy + d] <= 64 * lane) sy += d;
-            for (uint32_t k = 64 * lane; k < 64 * lane + 64; ++k) {
-                while (sy < 255 && first[sy + 1] <= k) ++sy;
-                sh.table[(k * 1283u) & 2047u] = sy;
-            }
-            __syncwarp();
-            for (uint32_t u0 = 0; u0 < 2048; u0 += 32) {  // the states of a symbol are numbered in increasing order, from its frequency on
-                const uint32_t s = sh.table[u0 + lane], same = __match_any_sync(0xFFFFFFFFu, s), before = same & ((1u << lane) - 1u);
-                const uint32_t x = count[s] + __popc(before), nb = 11 - (31 - __clz(x));
-                __syncwarp();
-                sh.table[u0 + lane] = nb | s << 8 | ((x << nb) - 2048u) << 16;
-                if (!before) count[s] += __popc(same);
-                __syncwarp();
-            }
-        }
+    if (l < 32) {
+        const bool ok = !bad && tans_build(src, nsym, sh.table, sh.ring, l);
+        if (l == 0) sh.built = ok;
     }
-    if (bad || total_bits < 11) {
-        if (lane == 0) atomicMax(&status[it.id], bad ? uint32_t(ST_BAD_HEADER) : uint32_t(ST_STREAM_UNDERRUN));
-        return;
-    }
+    tans_sync<THREADS>();
+    uint32_t err = bad || !sh.built ? uint32_t(ST_BAD_HEADER) : total_bits < 11 ? uint32_t(ST_STREAM_UNDERRUN) : uint32_t(ST_OK);
+    if (err) { if (l == 0) report(status, it.id, err); return; }
 
     // ---- runs ----
-    // LIFO reader (mod.rs:118-147): the stream is read from its last bit down; `p` bits are left.
-    const uint32_t runs = it.n / TANS_MIN_RUN < 1 ? 1u : it.n / TANS_MIN_RUN > 32 ? 32u : it.n / TANS_MIN_RUN;
+    // LIFO reader (mod.rs:118-147): the stream is read from its last bit down.
+    const uint32_t runs = it.n / TANS_MIN_RUN < 1 ? 1u : it.n / TANS_MIN_RUN > THREADS ? uint32_t(THREADS) : it.n / TANS_MIN_RUN;
     auto cut = [&](uint32_t k) -> uint64_t { return k >= runs ? 0 : total_bits - total_bits * k / runs; };  // bits left at the start of run k
-    const bool live = lane < runs;
-    // Positions of a lane are 32-bit offsets in bits from `org`, a 16-byte aligned address at least 128 bytes below the end of
+    // Positions of a lane are 32-bit offsets in bits from `org`, a 16-byte aligned address at least 112 bytes below the end of
     // its run (the stream may be longer than 2^32 bits, a run is not).
     const uint64_t floor_bit = uint64_t(reinterpret_cast<uintptr_t>(bs)) * 8;  // bit address of the stream's first bit
-    const uint64_t org_bit = ((floor_bit + cut(lane + 1)) & ~uint64_t(127)) - 1024;
+    const uint64_t org_bit = ((floor_bit + cut(l + 1)) & ~uint64_t(127)) - 1024;
     const uintptr_t org = uintptr_t(org_bit >> 3);
-    const uint32_t end_at = uint32_t(floor_bit + cut(lane + 1) - org_bit);
+    const uint32_t start_at = uint32_t(floor_bit + cut(l) - org_bit), end_at = uint32_t(floor_bit + cut(l + 1) - org_bit);
     const uintptr_t lo16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_first) & ~uintptr_t(15);
     const uintptr_t hi16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_end + 15) & ~uintptr_t(15);
-    // A lane's bytes pass through a 64-byte ring in shared memory, filled downward in aligned 16-byte blocks one step ahead of
-    // use; word w of the lane's column holds the stream word at byte offset 4 w (mod 64).  The lanes drain at similar rates:
-    // when any lane of the warp runs low every lane with room takes a block.
-    uint32_t* ring = sh.ring + lane;
-    auto word_at = [&](uint32_t bit) -> uint32_t { return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(ring) + ((bit << 2) & 0x780u)); };
-    uint32_t at = 0, fetched = 0, state = 0;  // bits left (from org), lowest byte offset in the ring
+
+    // The decoder: bits left (from org), address of its state's table entry, and a window on the stream: a 64-byte ring in shared
+    // memory, filled downward in aligned 16-byte blocks one step ahead of use.  Word w of the lane's column holds the stream word
+    // at byte offset 4 w (mod 64) and so does word w + 16, so that the words below any word are at fixed distances.  The lanes
+    // drain at similar rates: when any lane of the warp runs low every one with room takes a block.
+    uint32_t at = 0, entry = table, fetched = 0;
     uint4 pending;
-    auto put_block = [&]() {
-        fetched -= 16;
-        uint32_t* r = ring + ((fetched >> 2) & 15) * 32;
-        r[0] = pending.x; r[32] = pending.y; r[64] = pending.z; r[96] = pending.w;
-        pending = fetch16(org + fetched - 16, lo16, hi16);
+    uint8_t* ring = reinterpret_cast<uint8_t*>(sh.ring) + l * 4;
+    auto park = [&](uint32_t off, const uint4& v) {
+        uint8_t* r = ring + ((off >> 2) & 15u) * WORD;
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            *reinterpret_cast<uint32_t*>(r + k * WORD) = w[k];
+            *reinterpret_cast<uint32_t*>(r + (16 + k) * WORD) = w[k];
+        }
     };
-    auto top_up = [&]() {  // at least sixteen bytes below the word that holds the next bit
-        const uint32_t have = (at >> 3 & ~3u) + 4 - fetched;
-        if (__any_sync(__activemask(), have < 32)) { if (have <= 48) put_block(); }
-    };
-    auto begin = [&](uint32_t bit, uint32_t st) {
-        at = bit; state = st;
+    auto begin = [&](uint32_t bit, uint32_t state) {
+        at = bit; entry = table + 4 * state;
         fetched = (bit >> 3 & ~15u) - 32;
         uint4 b[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) b[k] = fetch16(org + fetched + 16 * k, lo16, hi16);
         pending = fetch16(org + fetched - 16, lo16, hi16);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            uint32_t* r = ring + (((fetched >> 2) + 4 * k) & 15) * 32;
-            r[0] = b[k].x; r[32] = b[k].y; r[64] = b[k].z; r[96] = b[k].w;
+        for (int k = 0; k < 3; ++k) park(fetched + 16 * k, b[k]);
+    };
+    auto refill = [&]() {  // at least sixteen bytes below the word in use
+        const uint32_t have = (at >> 3 & ~3u) + 4 - fetched;
+        if (__any_sync(__activemask(), have < 32)) {
+            if (have <= 48) { fetched -= 16; park(fetched, pending); pending = fetch16(org + fetched - 16, lo16, hi16); }
         }
     };
-    uint32_t c_hi, c_lo;  // the next bits, highest first
+    auto state_now = [&]() -> uint32_t { return (entry - table) >> 2; };
+    auto load_entry = [&]() -> uint32_t { uint32_t e; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(entry)); return e; };
+    uint32_t w;  // the next bits, highest first
     auto step = [&]() -> uint32_t {  // one symbol's entry; takes its bits off the window
-        const uint32_t e = table[state];
-        state = (e >> 16) + __funnelshift_l(c_hi, 0u, e);  // below 2048 whatever the stream holds: the baseline has its low bits clear
-        c_hi = __funnelshift_l(c_lo, c_hi, e);
-        c_lo = __funnelshift_l(0u, c_lo, e);
+        const uint32_t e = load_entry();
+        entry = (e >> 16) + 4 * __funnelshift_l(w, 0u, e);  // inside the table whatever the stream holds: the baseline has its low bits clear
+        w = __funnelshift_l(0u, w, e);
         return e;
     };
-    // Eight symbols: four words (97 bits or more) are read at once, the second half of the group takes its window from them.
+    auto word_below = [&](uint32_t k) -> uint32_t {  // k words below the one that holds the next bit
+        return *reinterpret_cast<const uint32_t*>(ring + (((at >> 5) & 15u) + 16 - k) * WORD);
+    };
+    auto open_window = [&]() { w = __funnelshift_r(word_below(1), word_below(0), at); };
+    // Eight symbols in two halves with a window of 32 bits each; the few groups with a half that takes more are decoded again in
+    // pairs (22 bits at most).
     auto group = [&](uint32_t e[8]) {
-        const uint32_t w3 = word_at(at), w2 = word_at(at - 32), w1 = word_at(at - 64), w0 = word_at(at - 96);
-        const uint32_t h2 = __funnelshift_r(w2, w3, at), h1 = __funnelshift_r(w1, w2, at), h0 = __funnelshift_r(w0, w1, at);
-        c_hi = h2; c_lo = h1;
-        uint32_t used = 0;
+        const uint32_t entry0 = entry, w2 = word_below(0), w1 = word_below(1), w0 = word_below(2);
+        const uint32_t high = __funnelshift_r(w1, w2, at), low = __funnelshift_r(w0, w1, at);
+        uint32_t used = 0, more = 0;
+        w = high;
 #pragma unroll
         for (int j = 0; j < 4; ++j) { e[j] = step(); used += e[j]; }
         used &= 0xFFu;  // 44 at most: the sum of four bit counts stays below the symbols
-        const bool far = used >= 32;
-        const uint32_t m2 = far ? h1 : h2, m1 = far ? h0 : h1, m0 = far ? 0u : h0;  // with 32 bits gone 64 are left: enough for the other 44
-        c_hi = __funnelshift_l(m1, m2, used); c_lo = __funnelshift_l(m0, m1, used);
-        uint32_t more = 0;
+        w = __funnelshift_lc(low, high, used);
 #pragma unroll
         for (int j = 4; j < 8; ++j) { e[j] = step(); more += e[j]; }
-        at -= used + (more & 0xFFu);
+        more &= 0xFFu;
+        if (used > 32 || more > 32) {
+            entry = entry0;
+            used = more = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if ((j & 1) == 0) { at -= used & 0xFFu; used = 0; open_window(); }
+                e[j] = step(); used += e[j];
+            }
+            used &= 0xFFu;
+        }
+        at -= used + more;
+    };
+    auto four = [&]() {  // four symbols of a walk
+        const uint32_t entry0 = entry;
+        open_window();
+        uint32_t used = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) used += step();
+        used &= 0xFFu;
+        if (used > 32) {
+            entry = entry0;
+            used = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if ((j & 1) == 0) { at -= used & 0xFFu; used = 0; open_window(); }
+                used += step();
+            }
+            used &= 0xFFu;
+        }
+        at -= used;
     };
     auto one = [&]() -> uint32_t {  // one symbol on its own
-        c_hi = __funnelshift_r(word_at(at - 32), word_at(at), at); c_lo = 0;
+        open_window();
         const uint32_t e = step();
         at -= e & 31u;
         return e;
     };
-    // symbols from (bit, st) down to the end of the run
-    auto walk = [&](uint32_t bit, uint32_t st) -> uint32_t {
+    // from (bits below the cut << 11 | state) down to the end of the run: the symbols met
+    auto walk = [&](uint32_t start) -> uint32_t {
         uint32_t n = 0;
-        begin(bit, st);
-        while (at >= end_at + TANS_GROUP_BITS && n < it.n) {
+        begin(start_at - (start >> 11), start & 2047u);
+        while (int32_t(at - end_at) >= int32_t(TANS_GROUP_BITS) && n < it.n) {
             uint32_t e[8];
-            top_up();
+            refill();
             group(e);
             n += 8;
         }
+        while (int32_t(at - end_at) >= int32_t(TANS_GROUP_BITS / 2) && n < it.n) {
+            refill();
+            four();
+            n += 4;
+        }
         for (uint32_t k = 0; int32_t(at - end_at) > 0 && n < it.n; ++k) {
-            if ((k & 7) == 0) top_up();
+            if ((k & 7) == 0) refill();
             one();
             ++n;
         }
         return n;
     };
-    // run 0 starts behind the eleven bits of the first state
-    uint64_t p = lane == 0 ? total_bits - 11 : cut(lane);
-    uint32_t from = 0, count = 0;
-    if (lane == 0) {
+    const bool inner = l + 1 < runs;  // the last run's symbols are what is left of the chunk's
+    uint32_t from = 0, mine = 0, end = 0;
+    if (l == 0) {  // run 0 starts behind the eleven bits of the first state
         const uint64_t bit = total_bits - 11;
-        const uint8_t* q = bs + (bit >> 3);
-        const uint64_t three = uint64_t(q[0]) | uint64_t(q[1]) << 8 | ((bit & 7) > 5 ? uint64_t(q[2]) << 16 : 0);
-        from = uint32_t(three >> (bit & 7)) & 2047u;
+        const uint8_t* b = bs + (bit >> 3);
+        const uint32_t three = uint32_t(b[0]) | uint32_t(b[1]) << 8 | ((bit & 7) > 5 ? uint32_t(b[2]) << 16 : 0u);
+        from = 11u << 11 | ((three >> (bit & 7)) & 2047u);
     }
+    for (bool go = inner;;) {
+        if (go) { mine = walk(from); end = (end_at - at) << 11 | state_now(); }
+        uint32_t want;
+        if (THREADS == 32) want = __shfl_up_sync(0xFFFFFFFFu, end, 1);
+        else {
+            sh.words[l] = end;
+            __syncthreads();
+            want = l ? uint32_t(sh.words[l - 1]) : 0u;
+        }
+        const bool moved = l > 0 && l < runs && want != from;
+        if (moved) from = want;
+        go = moved && inner;
+        if (THREADS == 32 ? !__any_sync(0xFFFFFFFFu, go) : !__syncthreads_or(go)) break;
+    }
+    // where the lane's symbols go: the counts of the lanes before it
+    uint64_t before_me, all;
     {
-        uint64_t end_p = 0;
-        uint32_t end_state = 0;
-        bool go = lane + 1 < runs;  // the last run's symbols are what is left of the chunk's
-        for (;;) {
-            if (go) {
-                const uint64_t bit = floor_bit + p - org_bit;
-                count = walk(uint32_t(bit), from);
-                end_p = org_bit + at - floor_bit;  // (wraps below the stream's first bit on a corrupt stream; the last pass notices)
-                end_state = state;
+        uint64_t incl = mine;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) { const uint64_t t = __shfl_up_sync(0xFFFFFFFFu, incl, s); if (l % 32 >= uint32_t(s)) incl += t; }
+        all = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        before_me = incl - mine;
+        if (THREADS > 32) {
+            __syncthreads();
+            if (l % 32 == 0) sh.words[l / 32] = all;
+            __syncthreads();
+            all = 0;
+            for (uint32_t w = 0; w < THREADS / 32; ++w) {
+                if (w < l / 32) before_me += sh.words[w];
+                all += sh.words[w];
             }
-            const uint64_t want_p = __shfl_up_sync(0xFFFFFFFFu, end_p, 1);
-            const uint32_t want = __shfl_up_sync(0xFFFFFFFFu, end_state, 1);
-            const bool moved = live && lane > 0 && (want_p != p || want != from);
-            if (moved) { p = want_p; from = want; }
-            go = moved && lane + 1 < runs;
-            if (!__any_sync(0xFFFFFFFFu, go)) break;
         }
     }
-    uint32_t pos;
-    uint32_t err = ST_OK;
-    {
-        if (lane + 1 >= runs) count = 0;
-        uint64_t incl = count;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) { const uint64_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d); if (lane >= uint32_t(d)) incl += t; }
-        const uint64_t all = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        if (all > it.n) err = ST_NOT_CONSUMED;  // more symbols than the chunk has before its last run
-        pos = uint32_t(incl - count);
-        if (lane + 1 == runs) count = it.n - uint32_t(all);
-    }
-    const uint64_t run_bit = floor_bit + p - org_bit;
-    if (live && p > total_bits) err = ST_STREAM_UNDERRUN;  // below the first bit
-    if (live && !err) {
+    if (all > it.n) err = ST_NOT_CONSUMED;  // more symbols than the chunk has before its last run
+    if (!err && l < runs) {
         // ---- last pass: the symbols to their places ----
         const Epilogue ep = make_epilogue(bases, it);
+        const bool last = l + 1 == runs;
+        uint32_t pos = uint32_t(before_me), remaining = last ? it.n - uint32_t(all) : mine;
         // the last run may not read below the stream's first bit; the others are known to end well above theirs
-        const uint32_t floor_at = lane + 1 == runs ? uint32_t(floor_bit - org_bit) : end_at - 11 - TANS_GROUP_BITS;
-        uint32_t remaining = count;
-        begin(uint32_t(run_bit), from);
+        const uint32_t floor_at = last ? end_at : end_at - 11 - TANS_GROUP_BITS;
+        begin(start_at - (from >> 11), from & 2047u);
+        if (int32_t(at - floor_at) < 0) err = ST_STREAM_UNDERRUN;
         auto one_checked = [&]() -> uint32_t {
             if (err) return 0;
-            const uint32_t nb = table[state] & 31u;
-            if (at - floor_at < nb) { err = ST_STREAM_UNDERRUN; return 0; }
+            if (at - floor_at < (load_entry() & 31u)) { err = ST_STREAM_UNDERRUN; return 0; }
             return one();
         };
         auto dec8 = [&](uint32_t& s_lo, uint32_t& s_hi) {
-            top_up();
+            refill();
             if (at - floor_at >= TANS_GROUP_BITS) {
                 uint32_t e[8];
                 group(e);
@@ -1364,7 +1427,7 @@ __global__ void __launch_bounds__(32, 20) tans_decode_kernel(const DecodeItem* _
         };
         auto short_group = [&](uint32_t g) {
             uint64_t syms = 0;
-            top_up();
+            refill();
             for (uint32_t j = 0; j < g; ++j) syms |= uint64_t((one_checked() >> 8) & 0xFFu) << (8 * j);
             emit(ep, pos, g, syms);
             pos += g; remaining -= g;
@@ -1375,139 +1438,168 @@ __global__ void __launch_bounds__(32, 20) tans_decode_kernel(const DecodeItem* _
         }
         fast_groups(ep, it.n, pos, remaining, dec8);
         while (remaining) short_group(remaining < 8 ? remaining : 8);
-        if (!err && lane + 1 == runs && (at != floor_at || state != 0)) err = ST_NOT_CONSUMED;  // mod.rs:442-449
+        if (!err && last && (at != floor_at || state_now() != 0)) err = ST_NOT_CONSUMED;  // mod.rs:442-449
     }
-    if (err) atomicMax(&status[it.id], err);
+    if (err) report(status, it.id, err);
+}
+inline void tans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, cudaStream_t st) {
+    // Four warps per chunk while an SM has no more than two chunks to itself: 0.56 against 0.62 ms for 256 chunks of 64 Ki symbols.
+    // Beyond that the warps of other chunks fill the gaps and the shorter rounds' overhead counts: 1794 chunks 0.82 ms with one
+    // warp each, 1.34 with four.  (Two chunks per warp, 16 lanes each: 0.91 ms, and 2.39 against 2.15 ms for 7637 chunks.)
+    if (n <= 2 * 148) tans_decode_kernel<128><<<n, 128, 0, st>>>(items, bases, status);
+    else tans_decode_kernel<32><<<n, 32, 0, st>>>(items, bases, status);
+}
+inline cudaError_t tans_prefer_shared() {
+    const cudaError_t e = cudaFuncSetAttribute(tans_decode_kernel<128>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(tans_decode_kernel<32>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
 // ---- Order1ScaleAC ---------------------------------------------------------
-// One range-coder stream per chunk, one warp per chunk.  The warp first turns
-// the chunk's PMFs into cumulative tables (u16, 256 per context: the count
-// below each symbol), then decodes the stream together: every lane carries the
-// same coder state.  The tables live in shared memory when the launch was
-// given room for the chunk's contexts (`smem_tables`, the largest table count
-// of the launch), else in the scratch arena.
-constexpr uint32_t O1_MAX_SMEM_TABLES = 192;  // 96 KiB; launches with more contexts per chunk keep their tables in global memory
-template <bool SMEM, bool LEAN>
-__global__ void __launch_bounds__(32) o1sac_decode_kernel_t(const DecodeItem* __restrict__ items, uint32_t n_items, Bases bases, uint32_t* __restrict__ status,
-                                                            uint32_t smem_tables) {
+// One range-coder stream per chunk, one warp per chunk, every lane carrying the
+// same coder state.  The stream is serial, so what counts is the way from one
+// symbol to the next, and that goes through a search: which symbol's share of
+// the range the code falls into.  The 256 shares of a context are mostly dust
+// (a symbol the plane never showed after this one still has 1 of 4096), so the
+// warp keeps the 32 widest in shared memory, one per lane: cumulative count,
+// width, symbol and where the symbol's own row lies.  A lane tests its share
+// with two multiplies; a maximum over the warp of (hit ? share : 0) is the
+// symbol with everything its step needs, without a second look at a table.  A
+// code that falls into none of the 32 is searched among all 256 from the
+// serialized state.  With the whole cumulative table of the context probed for
+// every symbol (eight counts per lane, three reductions) a symbol took 371
+// cycles and 114 instructions.
+constexpr uint32_t O1_ROW_BYTES = 32 * 8;  // {cumulative count << 20 | width << 8 | symbol, offset of the symbol's row} per lane
+// Context rows of a chunk whose state has `state_len` bytes, the marginal's included (0 when the state is too short to hold any).
+inline uint32_t o1sac_tables(uint64_t state_len) { return state_len >= 32 + 512 ? uint32_t((state_len - 32 - 512) / 512) + 1 : 0; }
+
+__global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __restrict__ items, Bases bases, uint32_t* __restrict__ status, uint32_t smem_rows) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t lane = threadIdx.x;
-    const uint32_t item_idx = blockIdx.x;
-    if (item_idx >= n_items) return;
-    const DecodeItem it = items[item_idx];
+    const DecodeItem it = items[blockIdx.x];
     const uint8_t* st = rd(bases, it.state);
-    uint32_t err = ST_OK;
-    __shared__ uint8_t bitmap[32];
-    __shared__ uint16_t table_of[256];  // which cumulative table a previous byte selects: 0 = marginal, 1 + rank of the context otherwise
-    if (it.state_version != 1 || it.state_len < 32 + 512) err = ST_BAD_STATE;
-    uint32_t pop = 0;
+    __shared__ uint32_t bitmap[8];      // contexts that have a row
+    __shared__ uint16_t row_of[256];    // the row a symbol leads to: 0 = marginal, 1 + rank of the context otherwise
+    uint32_t err = it.state_version != 1 || it.state_len < 32 + 512 ? uint32_t(ST_BAD_STATE) : uint32_t(ST_OK);
+    uint32_t rows = 1;
     if (!err) {
-        bitmap[lane] = st[lane];
+        if (lane < 8) bitmap[lane] = ld_u32_unaligned(st + 4 * lane);
         __syncwarp();
-        for (int i = 0; i < 32; ++i) pop += __popc(uint32_t(bitmap[i]));
-        if (it.state_len != 32 + 512 + pop * 512) err = ST_BAD_STATE;
-        if (SMEM && 1 + pop > smem_tables) err = ST_BAD_STATE;  // the host sized the launch from the same lengths
+        for (int i = 0; i < 8; ++i) rows += __popc(bitmap[i]);
+        // the host sized the launch from the same lengths
+        if (it.state_len != 32 + 512 * rows || rows > smem_rows) err = ST_BAD_STATE;
     }
-    if (err) { if (lane == 0) atomicMax(&status[it.id], err); return; }
-    // rank of every context (order1_scale_ac.rs:95-103)
-    for (uint32_t p = lane; p < 256; p += 32) {
-        uint32_t r = 0;
-        for (uint32_t b = 0; b < (p >> 3); ++b) r += __popc(uint32_t(bitmap[b]));
-        r += __popc(uint32_t(bitmap[p >> 3]) & ((1u << (p & 7)) - 1));
-        table_of[p] = ((bitmap[p >> 3] >> (p & 7)) & 1) ? uint16_t(1 + r) : uint16_t(0);
+    if (err) { if (lane == 0) report(status, it.id, err); return; }
+    for (uint32_t p = lane; p < 256; p += 32) {  // order1_scale_ac.rs:95-103
+        uint32_t r = __popc(bitmap[p >> 5] & ((1u << (p & 31)) - 1));
+        for (uint32_t b = 0; b < (p >> 5); ++b) r += __popc(bitmap[b]);
+        row_of[p] = uint16_t((bitmap[p >> 5] >> (p & 31)) & 1 ? 1 + r : 0);
     }
-    // cumulative tables: table t (0 = marginal, 1+r = row r) = 256 u16 at cum + t*256; the total is 4096 by the check below
-    uint16_t* cum = SMEM ? reinterpret_cast<uint16_t*>(smem) : reinterpret_cast<uint16_t*>(wr(bases, it.work));
-    for (uint32_t t = lane; t < 1 + pop; t += 32) {
-        const uint8_t* pm = st + 32 + t * 512;
-        uint16_t* ct = cum + t * 256;
-        uint32_t acc = 0; bool zero = false;
-        for (uint32_t i = 0; i < 256; ++i) {
-            uint32_t v = uint32_t(pm[2 * i]) | uint32_t(pm[2 * i + 1]) << 8;
-            zero |= v == 0;
-            ct[i] = uint16_t(acc);
-            acc += v;
-        }
-        if (zero || acc != 4096) err = ST_BAD_STATE;  // quantize.rs:53-71
-    }
-    err = __reduce_max_sync(0xFFFFFFFFu, err);
     __syncwarp();
-    __threadfence_block();
-    if (err) { if (lane == 0) atomicMax(&status[it.id], err); return; }
+    // a lane's eight probabilities of a row and the count below the first of them
+    auto load_row = [&](uint32_t row, uint32_t v[8]) -> uint32_t {
+        const uint8_t* q = st + 32 + 512 * row + 16 * lane;
+        const uint64_t a = ld8_unaligned(q), b = ld8_unaligned(q + 8);
+        uint32_t sum = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { v[k] = uint32_t((k < 4 ? a : b) >> (16 * (k & 3))) & 0xFFFFu; sum += v[k]; }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d); if (lane >= uint32_t(d)) incl += t; }
+        return incl - sum;
+    };
+    for (uint32_t row = 0; row < rows; ++row) {
+        uint32_t v[8], cum = load_row(row, v), sum = 0, zero = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { sum += v[k]; zero |= v[k] == 0; }
+        if (__any_sync(0xFFFFFFFFu, zero) || __shfl_sync(0xFFFFFFFFu, cum + sum, 31) != 4096) err = ST_BAD_STATE;  // quantize.rs:53-71
+        if (err) break;
+        // the smallest width that at most 32 symbols exceed
+        auto wider = [&](uint32_t w) -> uint32_t { uint32_t n = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) n += v[k] > w;
+            return __reduce_add_sync(0xFFFFFFFFu, n); };
+        uint32_t dust = 1;
+        if (wider(dust) > 32) {
+            uint32_t hi = 4096;  // more than 32 exceed `dust`, at most 32 exceed `hi`
+            while (hi - dust > 1) { const uint32_t mid = (hi + dust) >> 1; if (wider(mid) > 32) dust = mid; else hi = mid; }
+            dust = hi;
+        }
+        uint32_t mine = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) mine += v[k] > dust;
+        uint32_t at = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, at, d); if (lane >= uint32_t(d)) at += t; }
+        const uint32_t used = __shfl_sync(0xFFFFFFFFu, at, 31);
+        at -= mine;
+        uint2* out = reinterpret_cast<uint2*>(smem + row * O1_ROW_BYTES);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (v[k] > dust) { out[at] = make_uint2(cum << 20 | v[k] << 8 | (lane * 8 + k), uint32_t(row_of[lane * 8 + k]) * O1_ROW_BYTES); ++at; }
+            cum += v[k];
+        }
+        if (lane >= used) out[lane] = make_uint2(0, 0);  // width 0: never hit
+    }
+    if (err) { if (lane == 0) report(status, it.id, err); return; }
+    __syncwarp();
 
-    // The stream is serial, so the warp shares it: one 16-byte load per lane brings the whole table of the context,
-    // every lane counts those of its eight counts that are at or below the target (order1_scale_ac.rs:474-486: the
-    // symbol is the largest index whose count is <= target) and a warp reduction gives the symbol.  Lane 0 places
-    // the symbols.  Two ways to the symbol's count and probability, by the size of the launch: with fewer chunks
-    // than the GPU holds warps a chunk's own chain is what counts, with more the instructions issued are.
     Epilogue ep = make_epilogue(bases, it);
-    const uint8_t* src = rd(bases, it.src);
-    const uint32_t slen = it.src_len;
+    // Stream bytes, big-endian: `hi` and `lo` hold eight of them from an aligned word on, the next byte to use `taken` bits into
+    // them, and `ahead` is on its way.  Zero past the end.
+    const uintptr_t src = reinterpret_cast<uintptr_t>(rd(bases, it.src)), src_end = src + it.src_len;
+    uintptr_t next = src & ~uintptr_t(3);
+    auto fetch = [&]() -> uint32_t {
+        uint32_t w = 0;
+        if (next >= src && next + 4 <= src_end) w = __byte_perm(__ldg(reinterpret_cast<const uint32_t*>(next)), 0, 0x0123);
+        else for (uint32_t k = 0; k < 4; ++k) if (next + k >= src && next + k < src_end) w |= uint32_t(__ldg(reinterpret_cast<const uint8_t*>(next + k))) << (24 - 8 * k);
+        next += 4;
+        return w;
+    };
+    uint32_t hi = fetch(), lo = fetch(), ahead = fetch(), taken = 8 * uint32_t(src & 3);
+    auto advance = [&](uint32_t bits) {
+        taken += bits;
+        if (taken >= 32) { taken -= 32; hi = lo; lo = ahead; ahead = fetch(); }
+    };
     // range_coder.rs:137-155: five bytes start the code register, of which the last four count
-    uint32_t code = 0, rpos = 0;
-    for (; rpos < 5; ++rpos) code = (code << 8) | (rpos < slen ? src[rpos] : 0);
-    uint32_t low = 0, range = 0xFFFFFFFFu;
+    advance(8);
+    uint32_t code = __funnelshift_l(lo, hi, taken);
+    advance(16); advance(16);
+    uint32_t low = 0, range = 0xFFFFFFFFu, row = 0;
     const uint32_t row_len = it.row_len ? it.row_len : (it.n ? it.n : 1);
-    uint32_t row_pos = 0; int prev = -1;
-    uint64_t pos = 0;
-    uint32_t remaining = it.n;
-    uint32_t g = remaining ? first_group(ep, pos, remaining) : 0;
-    // the next stream bytes, four at a time (zero past the end)
-    auto next_bytes = [&](uint32_t at) -> uint32_t {
-        uint32_t v = 0;
-        for (uint32_t k = 0; k < 4; ++k) if (at + k < slen) v |= uint32_t(src[at + k]) << (8 * k);
-        return v;
-    };
-    uint32_t ahead = next_bytes(rpos), ahead_left = 4;
+    uint32_t left_in_row = row_len;
     auto one_symbol = [&]() -> uint32_t {
-        if (row_pos == 0) prev = -1;
-        const uint16_t* ct = cum + (prev >= 0 ? uint32_t(table_of[prev]) * 256u : 0u);
-        const uint4 q = *reinterpret_cast<const uint4*>(ct + lane * 8);  // the lane's eight counts, ascending
-        const uint32_t rpt = range >> 12;  // range / 4096
+        const uint2 mine = *reinterpret_cast<const uint2*>(smem + row + lane * 8);
+        const uint32_t from = row, rpt = range >> 12;  // range / 4096
         const uint32_t offset = code - low;
-        // target = min(offset / rpt, 4095) and "count <= target" is "count * rpt <= offset": no division
-        // (counts are below 4096, rpt < 2^20, so the products fit 32 bits)
-        const uint32_t c[8] = {q.x & 0xFFFFu, q.x >> 16, q.y & 0xFFFFu, q.y >> 16, q.z & 0xFFFFu, q.z >> 16, q.w & 0xFFFFu, q.w >> 16};
-        uint32_t lo, cumv, nextv;
-        if (LEAN) {
-            // few instructions: count, one reduction, then the symbol's count and the next one read back from the table
-            uint32_t fit = 0;
+        // "cumulative count <= offset / rpt < count + width" without the division; the products fit 32 bits
+        const bool hit = offset - (mine.x >> 20) * rpt < ((mine.x >> 8) & 0xFFFu) * rpt;
+        uint32_t share = __reduce_max_sync(0xFFFFFFFFu, hit ? mine.x : 0u);
+        row = __reduce_max_sync(0xFFFFFFFFu, hit ? mine.y : 0u);
+        uint32_t cum = share >> 20, width = (share >> 8) & 0xFFFu, sy = share & 0xFFu;
+        if (share == 0) {
+            // among all 256: the largest index whose count is <= min(offset / rpt, 4095) (order1_scale_ac.rs:474-486)
+            uint32_t v[8], c = load_row(from / O1_ROW_BYTES, v), fit = 0, below = 0, w = 0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) fit += c[i] * rpt <= offset ? 1u : 0u;
-            lo = __reduce_add_sync(0xFFFFFFFFu, fit) - 1;  // >= 0: entry 0 is 0
-            cumv = ct[lo];
-            nextv = lo < 255u ? uint32_t(ct[lo + 1]) : 4096u;
-        } else {
-            // short chain: the symbol's count is the largest that qualifies, the next count the smallest that does not
-            // (4096 when all do); three reductions side by side and no second look at the table
-            uint32_t fit = 0, below = 0, above = 4096;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const bool ok = c[i] * rpt <= offset;
-                fit += ok;
-                below = ok ? max(below, c[i]) : below;
-                above = ok ? above : min(above, c[i]);
+            for (int k = 0; k < 8; ++k) {
+                if (c * rpt <= offset) { ++fit; below = c; w = v[k]; }
+                c += v[k];
             }
-            lo = __reduce_add_sync(0xFFFFFFFFu, fit) - 1;
-            cumv = __reduce_max_sync(0xFFFFFFFFu, below);
-            nextv = __reduce_min_sync(0xFFFFFFFFu, above);
+            sy = __reduce_add_sync(0xFFFFFFFFu, fit) - 1;  // entry 0 counts 0 and always fits
+            cum = __shfl_sync(0xFFFFFFFFu, below, sy >> 3);
+            width = __shfl_sync(0xFFFFFFFFu, w, sy >> 3);
+            row = uint32_t(row_of[sy]) * O1_ROW_BYTES;
         }
-        low += cumv * rpt;
-        range = (nextv - cumv) * rpt;
-        while (range < (1u << 24)) {
-            if (ahead_left == 0) { ahead = next_bytes(rpos); ahead_left = 4; }
-            const uint32_t b = ahead & 0xFFu;
-            ahead >>= 8; --ahead_left;
-            ++rpos;
-            code = (code << 8) | b;
-            low <<= 8;
-            range <<= 8;
-        }
-        prev = int(lo);
-        row_pos = row_pos + 1 == row_len ? 0 : row_pos + 1;
-        return lo;
+        low += cum * rpt;
+        range = width * rpt;
+        const uint32_t bits = range < (1u << 16) ? 16u : range < (1u << 24) ? 8u : 0u;  // rpt >= 2^12: two bytes at most
+        code = __funnelshift_l(__funnelshift_l(lo, hi, taken), code, bits);
+        low <<= bits; range <<= bits;
+        advance(bits);
+        if (--left_in_row == 0) { row = 0; left_in_row = row_len; }  // a row's first symbol has no context
+        return sy;
     };
+    uint64_t pos = 0;
+    uint32_t remaining = it.n, g = remaining ? first_group(ep, pos, remaining) : 0;
     while (remaining) {
         uint32_t s_lo = 0, s_hi = 0;
         if (g == 8) {
@@ -1528,17 +1620,15 @@ __global__ void __launch_bounds__(32) o1sac_decode_kernel_t(const DecodeItem* __
     }
 }
 
-// Tables of a chunk whose state has `state_len` bytes (0 when the state is too short to hold any).
-inline uint32_t o1sac_tables(uint64_t state_len) { return state_len >= 32 + 512 ? uint32_t((state_len - 32 - 512) / 512) + 1 : 0; }
-// `tables` = the largest table count among the items.  A launch that fills the GPU several times over runs the variant
-// with fewer instructions and its tables in shared memory (when they fit); a smaller one the variant with the shorter chain.
-constexpr uint32_t O1_LEAN_FROM_ITEMS = 1024;  // about seven warps per SM: 2016 chunks measured 8.7 ms this way against 10.4 ms the other, 168 chunks 6.9 against 6.3
+// `tables` = the most context rows among the items.
+constexpr uint32_t O1_MAX_ROWS = 257;
 inline void o1sac_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t tables, cudaStream_t st) {
-    if (n >= O1_LEAN_FROM_ITEMS && tables && tables <= O1_MAX_SMEM_TABLES) o1sac_decode_kernel_t<true, true><<<n, 32, tables * 512, st>>>(items, n, bases, status, tables);
-    else o1sac_decode_kernel_t<false, false><<<n, 32, 0, st>>>(items, n, bases, status, 0);
+    const uint32_t rows = tables < O1_MAX_ROWS ? tables : O1_MAX_ROWS;
+    o1sac_decode_kernel<<<n, 32, rows * O1_ROW_BYTES, st>>>(items, bases, status, rows);
 }
-inline cudaError_t o1sac_allow_shared_tables() {
-    return cudaFuncSetAttribute(o1sac_decode_kernel_t<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(O1_MAX_SMEM_TABLES * 512));
+inline cudaError_t o1sac_allow_shared_rows() {
+    const cudaError_t e = cudaFuncSetAttribute(o1sac_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(O1_MAX_ROWS * O1_ROW_BYTES));
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(o1sac_decode_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
 // ---- stand-alone merge / copy ---------------------------------------------

@@ -33,7 +33,7 @@ int64_t noalloc_scratch_for(int device, uint8_t** out) {
         // the decoders need more dynamic shared memory than the default limit; an attribute, not an allocation
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rans_smem_bytes(rans_l_entries(255)))));
         CUDA_TRY(cudaFuncSetAttribute(huffman_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HUF_SMEM));
-        CUDA_TRY(o1sac_allow_shared_tables());
+        CUDA_TRY(o1sac_allow_shared_rows());
         it = g_noalloc_ptr.emplace(device, static_cast<uint8_t*>(p)).first;
     }
     *out = it->second;
@@ -88,7 +88,7 @@ extern "C" int64_t ptwm_b200_decode_plane_noalloc(uint8_t state_format_version, 
         CUDA_TRY(cudaStreamSynchronize(st));
         return int64_t(decoded);
     }
-    // layout of the fixed scratch: [0,4) status, [64, 64+sizeof item) work item, then (Order1ScaleAC) tables and state
+    // layout of the fixed scratch: [0,8) status (summary, item), [64, 64+sizeof item) work item, then (Order1ScaleAC) tables and state
     const size_t tables = codec == C_O1SAC ? (state_len - 32) / 512 : 0;
     const size_t work_off = 256, state_off = work_off + align_up(tables * 514, 256), total = state_off + align_up(codec == C_O1SAC ? state_len : 0, 256);
     if (total > PTWM_B200_NOALLOC_SCRATCH_BYTES)
@@ -97,22 +97,21 @@ extern "C" int64_t ptwm_b200_decode_plane_noalloc(uint8_t state_format_version, 
                                                   std::to_string(PTWM_B200_NOALLOC_SCRATCH_BYTES) + " (use ptwm_hardware_backend_v1_dispatch_decode_cuda)");
     DecodeItem it{};
     it.src = make_ref(SP_BLOB, ch.data_off); it.src_len = uint32_t(ch.data_len); it.n = uint32_t(decoded); it.dst = make_ref(SP_OUT, 0);
-    it.partner[0] = it.partner[1] = it.partner[2] = REF_NONE; it.state = REF_NONE; it.work = REF_NONE; it.id = 0;
+    it.partner[0] = it.partner[1] = it.partner[2] = REF_NONE; it.state = REF_NONE; it.id = 0;
     Bases bases{reinterpret_cast<const uint8_t*>(uintptr_t(in_dev_ptr)), 0, in_len, scratch, reinterpret_cast<uint8_t*>(uintptr_t(out_dev_ptr))};
     if (codec == C_O1SAC) {
         it.state = make_ref(SP_SCRATCH, state_off); it.state_len = uint32_t(state_len); it.state_version = state_format_version; it.row_len = 0;
-        it.work = make_ref(SP_SCRATCH, work_off);
         CUDA_TRY(cudaMemcpyAsync(scratch + state_off, state_ptr, state_len, cudaMemcpyHostToDevice, st));
     }
     // the array keeps what the previous call left: the status word must start at zero
     CUDA_TRY(cudaMemsetAsync(scratch, 0, 256, st));
     CUDA_TRY(cudaMemcpyAsync(scratch + 64, &it, sizeof it, cudaMemcpyHostToDevice, st));
     const DecodeItem* d_it = reinterpret_cast<const DecodeItem*>(scratch + 64);
-    uint32_t* d_status = reinterpret_cast<uint32_t*>(scratch);
+    uint32_t* d_status = reinterpret_cast<uint32_t*>(scratch) + 1;
     switch (codec) {
         case C_RANS: rans_decode_kernel_t<false><<<1, 32, rans_smem_bytes(rans_l_entries(255)), st>>>(d_it, 1, bases, d_status, rans_l_entries(255)); break;
         case C_HUFFMAN: huffman_decode_kernel<<<1, 32, HUF_SMEM, st>>>(d_it, 1, bases, d_status); break;
-        case C_TANS: tans_decode_kernel<<<1, 32, 0, st>>>(d_it, bases, d_status); break;
+        case C_TANS: tans_launch(d_it, 1, bases, d_status, st); break;
         default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), st); break;
     }
     CUDA_TRY(cudaGetLastError());

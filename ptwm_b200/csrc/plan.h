@@ -34,7 +34,6 @@ struct DecodeItem {
     Ref dst;            // plain: where the plane bytes go.  fused: output bytes of this chunk's first element
     Ref partner[3];     // fused: the other planes' bytes for this chunk, in plane order without `slot`
     Ref state;          // Order1ScaleAC: serialized state (bitmap, marginal, rows)
-    Ref work;           // Order1ScaleAC: scratch for the cumulative tables, (1+rows)*514 bytes, 2-byte aligned
     uint32_t state_len;
     uint32_t row_len;   // Order1ScaleAC rows; 0 = one row spanning the chunk
     uint32_t id;        // index into the status array
@@ -97,7 +96,7 @@ struct Bases {
     uint8_t* out;
 };
 
-// Status codes written per item (0 = ok).
+// Status codes written per item (0 = ok); the word before the first item's holds the largest of all.
 enum Status : uint32_t {
     ST_OK = 0,
     ST_BAD_HEADER = 1,      // weights / frequency table / jump table malformed

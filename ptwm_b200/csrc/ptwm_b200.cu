@@ -117,12 +117,27 @@ int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds
     return 0;
 }
 
+// A word of pinned memory for a plan, and back.  They come from pages of 1024 that are kept for the process.
+int64_t take_word(DeviceState& ds, uint32_t** w) {
+    std::lock_guard<std::mutex> g(g_dev_mu);
+    if (ds.words.empty()) {
+        uint32_t* page = nullptr;
+        CUDA_TRY(cudaMallocHost(&page, 4096));
+        for (int i = 1024; i-- > 0;) ds.words.push_back(page + i);
+    }
+    *w = ds.words.back();
+    ds.words.pop_back();
+    return 0;
+}
+void give_word(int dev, uint32_t* w) { std::lock_guard<std::mutex> g(g_dev_mu); g_dev[dev].words.push_back(w); }
+
 const CrcTables& crc_tables() { static CrcTables t = host_crc_tables(); return t; }
 
 int64_t device_state(int dev, DeviceState** out) {
     std::lock_guard<std::mutex> g(g_dev_mu);
     DeviceState& s = g_dev[dev];
     if (!s.stream) CUDA_TRY(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+    for (cudaStream_t& side : s.side) if (!side) CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     if (!s.d_tabs) {
         CUDA_TRY(cudaMalloc(&s.d_tabs, sizeof(CrcTables)));
         CUDA_TRY(cudaMemcpy(s.d_tabs, &crc_tables(), sizeof(CrcTables), cudaMemcpyHostToDevice));
@@ -132,11 +147,11 @@ int64_t device_state(int dev, DeviceState** out) {
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rans_smem_bytes(RANS_NARROW_SYMBOLS + 2, true))));
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         CUDA_TRY(cudaFuncSetAttribute(huffman_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HUF_SMEM));
-        CUDA_TRY(o1sac_allow_shared_tables());
+        CUDA_TRY(o1sac_allow_shared_rows());
         // the decoders are limited by how many chunk tables fit in an SM: ask for the largest shared-memory carve-out
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         CUDA_TRY(cudaFuncSetAttribute(huffman_decode_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-        CUDA_TRY(cudaFuncSetAttribute(tans_decode_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        CUDA_TRY(tans_prefer_shared());
         s.attrs = true;
     }
     *out = &s;
@@ -169,11 +184,15 @@ struct DevicePlan {
     uint32_t* acc = nullptr;
     uint64_t* hash_out = nullptr;
     cudaEvent_t ev[24] = {nullptr};   // begin/end per launch slot, created on first timed run
+    cudaEvent_t order[9] = {nullptr}; // fork, first phase done per codec class, all done per codec class; created on the first run that forks
+    uint32_t* summary = nullptr;      // pinned: the largest status of the last run
     bool timed[12] = {false};
     uint8_t* arena = nullptr;          // everything above lives in this one block
     bool external = false;             // the block belongs to the caller (ptwm_b200_plan_prepare_in)
-    void release() {
+    void release(int dev) {
         for (auto& e : ev) if (e) cudaEventDestroy(e);
+        for (auto& e : order) if (e) cudaEventDestroy(e);
+        if (summary) give_word(dev, summary);
         if (!external) cudaFree(arena);
         *this = DevicePlan{};
     }
@@ -203,22 +222,28 @@ struct ptwm_b200_plan {
     std::vector<uint32_t> item_tensor;  // item id -> tensor index (for error messages)
     uint32_t launches = 0;
     // per launch slot: 0-3 phase-0 decoders (rANS, Huffman, tANS, O1SAC), 4 scratch copies, 5-8 phase-1 decoders, 9 final merge, 10 CRC, 11 XXH64
-    // rANS chunks per phase: the first `rans_narrow` items hold few distinct symbols and go to the kernel with a symbol
-    // list per lane (`rans_rows` rows); the rest go to the general kernel, whose shared list is sized by the most distinct symbols among them.
-    uint32_t rans_wide_distinct[2] = {0, 0}, rans_narrow[2] = {0, 0}, rans_rows[2] = {0, 0};
-    uint32_t o1_tables[2] = {0, 0};  // most cumulative tables among the Order1ScaleAC chunks of a phase
+    // One launch of a decoder: a run of items of a list.  Items of the second phase that read planes the first one puts into
+    // scratch must wait for it, the others need not.  rANS chunks with few distinct symbols go to the kernel with a symbol list
+    // per lane; `size` is its rows there, the most distinct symbols of the run for the general kernel, and the most cumulative
+    // tables of a chunk for Order1ScaleAC.
+    struct Launch { uint32_t first, count, size; bool waits, narrow; };
+    std::vector<Launch> runs[2][4];
+    bool merge_waits = false;  // a final merge reads scratch
+    bool spread = false;       // few chunks: every coded plane to scratch at once, then a merge (see ptwm_b200_plan_create)
     uint64_t slot_bytes[12] = {0};
     uint32_t slot_items[12] = {0};
     std::mutex mu;
     std::map<int, DevicePlan> dev;
     ~ptwm_b200_plan() {
-        for (auto& kv : dev) { DeviceGuard g(kv.first); kv.second.release(); }
+        for (auto& kv : dev) { DeviceGuard g(kv.first); kv.second.release(kv.first); }
     }
 };
 
 namespace {
 
 int codec_class(uint16_t codec) { return codec == C_RANS ? 0 : codec == C_HUFFMAN ? 1 : codec == C_TANS ? 2 : 3; }
+
+constexpr uint64_t SPREAD_CHUNKS = 4 * 148;  // four chunks per SM: every decoder holds at least that many
 
 // Turn one tensor into work items.  See DecodeItem / MergeItem in plan.h.
 void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t out_off) {
@@ -241,17 +266,13 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
     auto decode_item = [&](const PlaneDesc& p, const ChunkDesc& ch) {
         DecodeItem it{};
         it.src = make_ref(SP_BLOB, ch.data_off); it.src_len = uint32_t(ch.data_len); it.n = ch.decoded; it.id = new_id();
-        it.partner[0] = it.partner[1] = it.partner[2] = REF_NONE; it.state = REF_NONE; it.work = REF_NONE;
+        it.partner[0] = it.partner[1] = it.partner[2] = REF_NONE; it.state = REF_NONE;
         span(ch.data_off, ch.data_len);
         it.row_len = uint32_t(ch.max_sym) | uint32_t(ch.distinct) << 16;  // rANS: alphabet bound and distinct symbols, for the planner only (the kernels read row_len for Order1ScaleAC)
         if (p.codec == C_O1SAC) {
             it.state = make_ref(SP_BLOB, ch.state_off); it.state_len = uint32_t(ch.state_len); it.state_version = ch.state_version;
             it.row_len = uint32_t(p.row_len);
             span(ch.state_off, ch.state_len);
-            uint64_t tables = (ch.state_len - 32) / 512;
-            pl.scratch_bytes = align_up(pl.scratch_bytes, 16);
-            it.work = make_ref(SP_SCRATCH, pl.scratch_bytes);
-            pl.scratch_bytes += align_up(tables * 514, 16);
         }
         return it;
     };
@@ -268,12 +289,13 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
             if (!n) continue;
             const uint64_t plane_off = t.planes[0].chunks[k].plane_off;
             const Ref out_ref = make_ref(SP_OUT, out_off + plane_off * uint64_t(eb));
-            int fused_plane = -1;
+            int fused_plane = -1, coded = 0;
             for (int p = 0; p < np; ++p) {
                 const ChunkDesc& ch = t.planes[size_t(p)].chunks[k];
                 uint16_t codec = t.planes[size_t(p)].codec;
-                if (!ch.raw && (codec == C_RANS || codec == C_HUFFMAN || codec == C_TANS)) fused_plane = p;
+                if (!ch.raw && (codec == C_RANS || codec == C_HUFFMAN || codec == C_TANS)) { fused_plane = p; ++coded; }
             }
+            if (pl.spread && coded > 1) fused_plane = -1;
             if (np == 1) {
                 const ChunkDesc& ch = t.planes[0].chunks[k];
                 if (ch.raw) { span(ch.data_off, ch.data_len); pl.merges[1].push_back(MergeItem{{make_ref(SP_BLOB, ch.data_off), REF_NONE, REF_NONE, REF_NONE}, out_ref, n, K_PASS}); }
@@ -341,29 +363,31 @@ void finish_lists(ptwm_b200_plan& pl) {
         for (int cc = 0; cc < 4; ++cc) {
             auto& v = pl.dec[ph][cc];
             auto narrow = [cc](const DecodeItem& a) { return cc == 0 && (a.row_len >> 16) <= RANS_NARROW_SYMBOLS; };
+            auto waits = [ph](const DecodeItem& a) {
+                if (ph == 0) return false;
+                for (Ref r : a.partner) if (r != REF_NONE && (r >> 62) == SP_SCRATCH) return true;
+                return false;
+            };
             std::stable_sort(v.begin(), v.end(), [&](const DecodeItem& a, const DecodeItem& b) {
-                bool na = narrow(a), nb = narrow(b);
-                return na != nb ? na : a.n > b.n;
+                const int ka = 2 * waits(a) + !narrow(a), kb = 2 * waits(b) + !narrow(b);
+                return ka != kb ? ka < kb : a.n > b.n;
             });
-            if (!v.empty()) pl.launches++;
-            int slot = ph * 5 + cc;
+            const int slot = ph * 5 + cc;
             pl.slot_items[slot] = uint32_t(v.size());
-            if (cc == 0) {
-                uint32_t most = 0;
-                for (auto& it : v) {
-                    if (narrow(it)) { pl.rans_narrow[ph]++; most = std::max(most, it.row_len >> 16); }
-                    else pl.rans_wide_distinct[ph] = std::max(pl.rans_wide_distinct[ph], it.row_len >> 16);  // most distinct symbols among the rest
-                }
-                pl.rans_rows[ph] = most + 2;
-                if (pl.rans_narrow[ph] && pl.rans_narrow[ph] < v.size()) pl.launches++;
+            for (size_t k = 0; k < v.size(); ++k) {
+                const bool w = waits(v[k]), nw = narrow(v[k]);
+                auto& runs = pl.runs[ph][cc];
+                if (runs.empty() || runs.back().waits != w || runs.back().narrow != nw) { runs.push_back({uint32_t(k), 0, 0, w, nw}); pl.launches++; }
+                runs.back().count++;
+                runs.back().size = std::max(runs.back().size, cc == 0 ? v[k].row_len >> 16 : cc == 3 ? o1sac_tables(v[k].state_len) : 0u);
             }
-            if (cc == 3) for (auto& it : v) pl.o1_tables[ph] = std::max(pl.o1_tables[ph], o1sac_tables(it.state_len));
             for (auto& it : v) {
                 uint64_t np = it.fused ? uint64_t(kind_planes(it.kind)) : 1, eb = it.fused ? uint64_t(kind_elem_bytes(it.kind)) : 1;
                 pl.slot_bytes[slot] += uint64_t(it.src_len) + it.state_len + uint64_t(it.n) * (np - 1) + uint64_t(it.n) * eb;
             }
         }
         auto& m = pl.merges[ph];
+        if (ph == 1) for (auto& it : m) for (Ref r : it.src) pl.merge_waits |= r != REF_NONE && (r >> 62) == SP_SCRATCH;
         pl.slot_items[ph * 5 + 4] = uint32_t(m.size());
         for (auto& it : m) pl.slot_bytes[ph * 5 + 4] += uint64_t(it.n) * uint64_t(kind_planes(int(it.kind))) + uint64_t(it.n) * uint64_t(kind_elem_bytes(int(it.kind)));
         pl.tiles[ph].clear();
@@ -437,50 +461,50 @@ int64_t device_plan(ptwm_b200_plan& pl, int dev, DeviceState& ds, DevicePlan** o
     std::vector<uint32_t> allt;
     for (int ph = 0; ph < 2; ++ph) { allm.insert(allm.end(), pl.merges[ph].begin(), pl.merges[ph].end()); allt.insert(allt.end(), pl.tiles[ph].begin(), pl.tiles[ph].end()); }
     int64_t rc;
-    if ((rc = upload(d.items, all, ds)) < 0 || (rc = upload(d.merges, allm, ds)) < 0 || (rc = upload(d.tiles, allt, ds)) < 0 || (rc = upload(d.posts, pl.posts, ds)) < 0 ||
+    if ((rc = take_word(ds, &d.summary)) < 0 || (rc = upload(d.items, all, ds)) < 0 || (rc = upload(d.merges, allm, ds)) < 0 || (rc = upload(d.tiles, allt, ds)) < 0 || (rc = upload(d.posts, pl.posts, ds)) < 0 ||
         (rc = upload(d.post_tiles, pl.post_tiles, ds)) < 0 || (rc = upload(d.verify, pl.verify, ds)) < 0 ||
-        (rc = upload(d.hashes, pl.hashes, ds)) < 0) { d.release(); return rc; }
+        (rc = upload(d.hashes, pl.hashes, ds)) < 0) { d.release(dev); return rc; }
     pl.dev[dev] = d;
     *out = &pl.dev[dev];
     return 0;
 }
 
-int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t flags, CrcTables* d_tabs, cudaStream_t st) {
+int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t flags, DeviceState& ds, cudaStream_t st) {
+    CrcTables* d_tabs = ds.d_tabs;
     CUDA_TRY(cudaMemsetAsync(d.status, 0, (pl.item_tensor.size() + 1) * sizeof(uint32_t), st));
     uint32_t* status = d.status + 1;
-    size_t item_base = 0, merge_base = 0, tile_base = 0;
+    size_t merge_base = 0, tile_base = 0;
     const bool timing = flags & PTWM_B200_TIME_KERNELS;
     for (bool& t : d.timed) t = false;
     if (timing) for (auto& e : d.ev) if (!e) CUDA_TRY(cudaEventCreate(&e));
     auto mark = [&](int slot, int end) -> cudaError_t { if (!timing) return cudaSuccess; d.timed[slot] = true; return cudaEventRecord(d.ev[2 * slot + end], st); };
-    auto launch_decodes = [&](int ph) -> int64_t {
-        for (int cc = 0; cc < 4; ++cc) {
-            uint32_t n = uint32_t(pl.dec[ph][cc].size());
-            const DecodeItem* it = d.items + item_base;
-            item_base += n;
-            if (!n) continue;
-            CUDA_TRY(mark(ph * 5 + cc, 0));
-            switch (cc) {
-                case 0: {
-                    const uint32_t nn = pl.rans_narrow[ph], nw = n - nn;
-                    if (nn) {
-                        const uint32_t rows = pl.rans_rows[ph];
-                        rans_decode_kernel_t<true><<<(nn + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, rans_smem_bytes(rows, true), st>>>(it, nn, bases, status, rows);
-                        CUDA_TRY(cudaGetLastError());
-                    }
-                    if (nw) {
-                        const uint32_t le = (pl.rans_wide_distinct[ph] + 2 + 3) & ~3u;
-                        rans_decode_kernel_t<false><<<(nw + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, rans_smem_bytes(le), st>>>(it + nn, nw, bases, status, le);
-                    }
-                    break;
+    const DecodeItem* lists[2][4];
+    {
+        const DecodeItem* at = d.items;
+        for (int ph = 0; ph < 2; ++ph) for (int cc = 0; cc < 4; ++cc) { lists[ph][cc] = at; at += pl.dec[ph][cc].size(); }
+    }
+    auto launch = [&](int ph, int cc, const ptwm_b200_plan::Launch& r, cudaStream_t s) -> int64_t {
+        const DecodeItem* it = lists[ph][cc] + r.first;
+        const uint32_t n = r.count;
+        switch (cc) {
+            case 0:
+                if (r.narrow) {
+                    const uint32_t rows = r.size + 2;
+                    rans_decode_kernel_t<true><<<(n + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, rans_smem_bytes(rows, true), s>>>(it, n, bases, status, rows);
+                } else {
+                    const uint32_t le = (r.size + 2 + 3) & ~3u;
+                    rans_decode_kernel_t<false><<<(n + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, rans_smem_bytes(le), s>>>(it, n, bases, status, le);
                 }
-                case 1: huffman_decode_kernel<<<(n + HUF_WARP_CHUNKS - 1) / HUF_WARP_CHUNKS, 32, HUF_SMEM, st>>>(it, n, bases, status); break;
-                case 2: tans_decode_kernel<<<n, 32, 0, st>>>(it, bases, status); break;
-                default: o1sac_launch(it, n, bases, status, pl.o1_tables[ph], st); break;
-            }
-            CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(mark(ph * 5 + cc, 1));
+                break;
+            case 1: huffman_decode_kernel<<<(n + HUF_WARP_CHUNKS - 1) / HUF_WARP_CHUNKS, 32, HUF_SMEM, s>>>(it, n, bases, status); break;
+            case 2: tans_launch(it, n, bases, status, s); break;
+            default: o1sac_launch(it, n, bases, status, r.size, s); break;
         }
+        CUDA_TRY(cudaGetLastError());
+        return 0;
+    };
+    auto launch_class = [&](int ph, int cc, bool waiting, cudaStream_t s) -> int64_t {
+        for (auto& r : pl.runs[ph][cc]) if (r.waits == waiting) { const int64_t rc = launch(ph, cc, r, s); if (rc < 0) return rc; }
         return 0;
     };
     auto launch_merges = [&](int ph) -> int64_t {
@@ -515,7 +539,54 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         return 0;
     };
     int64_t rc;
-    if ((rc = launch_decodes(0)) < 0 || (rc = launch_merges(0)) < 0 || (rc = launch_posts()) < 0 || (rc = launch_decodes(1)) < 0 || (rc = launch_merges(1)) < 0) return rc;
+    int classes = 0;
+    for (int cc = 0; cc < 4; ++cc) classes += !pl.runs[0][cc].empty() || !pl.runs[1][cc].empty();
+    if (timing || classes < 2) {  // one after the other
+        for (int ph = 0; ph < 2; ++ph) {
+            for (int cc = 0; cc < 4; ++cc) {
+                if (pl.runs[ph][cc].empty()) continue;
+                CUDA_TRY(mark(ph * 5 + cc, 0));
+                if ((rc = launch_class(ph, cc, false, st)) < 0 || (rc = launch_class(ph, cc, true, st)) < 0) return rc;
+                CUDA_TRY(mark(ph * 5 + cc, 1));
+            }
+            if (ph == 0 && ((rc = launch_merges(0)) < 0 || (rc = launch_posts()) < 0)) return rc;
+        }
+        if ((rc = launch_merges(1)) < 0) return rc;
+    } else {
+        // The codecs' decoders do not depend on one another, except where a plane is decoded to scratch for another one's lanes to
+        // merge: every codec has a stream of its own, the ones with the longest serial chains first.  One after the other the four
+        // kernels of a microscaling layer took 9.5 ms, 6.4 of them an Order1ScaleAC launch that leaves the GPU nearly idle.
+        for (auto& e : d.order) if (!e) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        bool first = false, waiting = pl.merge_waits || !pl.posts.empty();
+        for (int cc = 0; cc < 4; ++cc) { first |= !pl.runs[0][cc].empty(); for (auto& r : pl.runs[1][cc]) waiting |= r.waits; }
+        CUDA_TRY(cudaEventRecord(d.order[0], st));
+        for (int cc = 3; cc >= 0; --cc) {
+            if (pl.runs[0][cc].empty() && pl.runs[1][cc].empty()) continue;
+            cudaStream_t s = ds.side[cc];
+            CUDA_TRY(cudaStreamWaitEvent(s, d.order[0], 0));
+            if ((rc = launch_class(0, cc, false, s)) < 0) return rc;
+            if (waiting && !pl.runs[0][cc].empty()) { CUDA_TRY(cudaEventRecord(d.order[1 + cc], s)); CUDA_TRY(cudaStreamWaitEvent(st, d.order[1 + cc], 0)); }
+            if ((rc = launch_class(1, cc, false, s)) < 0) return rc;
+        }
+        if ((rc = launch_merges(0)) < 0 || (rc = launch_posts()) < 0) return rc;
+        if (waiting) {  // st has waited for everything that goes to scratch
+            CUDA_TRY(cudaEventRecord(d.order[0], st));
+            for (int cc = 3; cc >= 0; --cc) {
+                bool any = false;
+                for (auto& r : pl.runs[1][cc]) any |= r.waits;
+                if (!any) continue;
+                CUDA_TRY(cudaStreamWaitEvent(ds.side[cc], d.order[0], 0));
+                if ((rc = launch_class(1, cc, true, ds.side[cc])) < 0) return rc;
+            }
+        }
+        if ((rc = launch_merges(1)) < 0) return rc;
+        for (int cc = 0; cc < 4; ++cc) {
+            if (pl.runs[0][cc].empty() && pl.runs[1][cc].empty()) continue;
+            CUDA_TRY(cudaEventRecord(d.order[5 + cc], ds.side[cc]));
+            CUDA_TRY(cudaStreamWaitEvent(st, d.order[5 + cc], 0));
+        }
+    }
+    CUDA_TRY(cudaMemcpyAsync(d.summary, d.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     if ((flags & PTWM_B200_VERIFY_CRC) && !pl.verify.empty()) {
         CUDA_TRY(cudaMemsetAsync(d.acc, 0, (pl.n_acc + 1) * sizeof(uint32_t), st));
         uint64_t blocks = (pl.n_runs + 127) / 128;
@@ -546,11 +617,11 @@ const char* status_text(uint32_t s) {
 
 int64_t evaluate(ptwm_b200_plan& pl, DevicePlan& d, uint32_t flags, cudaStream_t st) {
     CUDA_TRY(cudaStreamSynchronize(st));
-    // decode status: items write their own slot; scan on the host
-    std::vector<uint32_t> status(pl.item_tensor.size() + 1);
-    CUDA_TRY(cudaMemcpy(status.data(), d.status, status.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    for (size_t i = 1; i < status.size(); ++i)
-        if (status[i]) return fail(PTWM_RC_CORRUPT, "tensor '" + pl.c->file.tensors[pl.item_tensor[i - 1]].name + "': " + status_text(status[i]));
+    if (*d.summary) {  // some item failed: which one
+        std::vector<uint32_t> status(pl.item_tensor.size() + 1);
+        CUDA_TRY(cudaMemcpy(status.data(), d.status, status.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+        for (size_t i = 1; i < status.size(); ++i) if (status[i]) return fail(PTWM_RC_CORRUPT, "tensor '" + pl.c->file.tensors[pl.item_tensor[i - 1]].name + "': " + status_text(status[i]));
+    }
     if ((flags & PTWM_B200_VERIFY_CRC) && !pl.crc_expect.empty()) {
         std::vector<uint32_t> acc(pl.n_acc);
         CUDA_TRY(cudaMemcpy(acc.data(), d.acc, acc.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
@@ -631,27 +702,25 @@ int64_t decode_plane_cuda(uint8_t sfv, const uint8_t* state, size_t state_len, c
     }
     DecodeItem it{};
     it.src = make_ref(SP_BLOB, ch.data_off); it.src_len = uint32_t(ch.data_len); it.n = uint32_t(decoded); it.dst = make_ref(SP_OUT, 0);
-    it.partner[0] = it.partner[1] = it.partner[2] = REF_NONE; it.state = REF_NONE; it.work = REF_NONE; it.id = 0;
-    // device scratch for the item, the status word and (O1SAC) the state and its tables
-    size_t tables = codec == C_O1SAC ? (state_len - 32) / 512 : 0;
-    size_t work_off = 256, state_off = work_off + align_up(tables * 514, 256), total = state_off + align_up(state_len, 256);
+    it.partner[0] = it.partner[1] = it.partner[2] = REF_NONE; it.state = REF_NONE; it.id = 0;
+    // device scratch for the item, the status words and (O1SAC) the state
+    const size_t state_off = 256, total = state_off + align_up(state_len, 256);
     uint8_t* scratch = nullptr;
     CUDA_TRY(cudaMalloc(&scratch, total));
     struct Free { uint8_t* p; ~Free() { cudaFree(p); } } freer{scratch};
     bases.scratch = scratch;
     if (codec == C_O1SAC) {
         it.state = make_ref(SP_SCRATCH, state_off); it.state_len = uint32_t(state_len); it.state_version = sfv; it.row_len = 0;
-        it.work = make_ref(SP_SCRATCH, work_off);
         CUDA_TRY(cudaMemcpyAsync(scratch + state_off, state, state_len, cudaMemcpyHostToDevice, st));
     }
     CUDA_TRY(cudaMemsetAsync(scratch, 0, 256, st));
     CUDA_TRY(cudaMemcpyAsync(scratch + 64, &it, sizeof it, cudaMemcpyHostToDevice, st));
     const DecodeItem* d_it = reinterpret_cast<const DecodeItem*>(scratch + 64);
-    uint32_t* d_status = reinterpret_cast<uint32_t*>(scratch);
+    uint32_t* d_status = reinterpret_cast<uint32_t*>(scratch) + 1;  // the summary word in front
     switch (codec) {
         case C_RANS: rans_decode_kernel_t<false><<<1, 32, rans_smem_bytes(rans_l_entries(255)), st>>>(d_it, 1, bases, d_status, rans_l_entries(255)); break;
         case C_HUFFMAN: huffman_decode_kernel<<<1, 32, HUF_SMEM, st>>>(d_it, 1, bases, d_status); break;
-        case C_TANS: tans_decode_kernel<<<1, 32, 0, st>>>(d_it, bases, d_status); break;
+        case C_TANS: tans_launch(d_it, 1, bases, d_status, st); break;
         default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), st); break;
     }
     CUDA_TRY(cudaGetLastError());
@@ -799,6 +868,15 @@ int64_t ptwm_b200_plan_create(const ptwm_b200_container* c, const uint32_t* indi
         if (!indices) { n = c->file.tensors.size(); for (size_t i = 0; i < n; ++i) pl->tensors.push_back(uint32_t(i)); }
         else pl->tensors.assign(indices, indices + n);
         pl->blob_lo = UINT64_MAX;
+        {
+            // A tensor with two coded planes decodes the second in lanes that merge it with the first, so one waits for the other.
+            // While all chunks of the plan run at once anyway that only adds up their latencies: with few chunks every coded plane
+            // goes to scratch and one more launch merges them (a 4096-element norm vector: 0.48 -> 0.3 ms).
+            uint64_t coded = 0;
+            for (uint32_t ti : pl->tensors) if (ti < c->file.tensors.size())
+                for (const PlaneDesc& p : c->file.tensors[ti].planes) for (const ChunkDesc& ch : p.chunks) coded += !ch.raw;
+            pl->spread = coded <= SPREAD_CHUNKS;
+        }
         for (uint32_t ti : pl->tensors) {
             if (ti >= c->file.tensors.size()) return fail(PTWM_RC_INVALID_INPUT, "tensor index out of range");
             const TensorDesc& t = c->file.tensors[ti];
@@ -866,7 +944,7 @@ int64_t ptwm_b200_plan_run(ptwm_b200_plan* p, uint64_t blob_dev_ptr, uint64_t bl
     // Refs hold file offsets; the kernels clamp their 16-byte fetches to the resident span
     Bases launch{reinterpret_cast<const uint8_t*>(uintptr_t(blob_dev_ptr)), blob_first, blob_first + blob_len, reinterpret_cast<uint8_t*>(uintptr_t(scratch_dev_ptr)),
                  reinterpret_cast<uint8_t*>(uintptr_t(out_dev_ptr))};
-    if ((rc = enqueue(*p, *d, launch, flags, ds->d_tabs, st)) < 0) return rc;
+    if ((rc = enqueue(*p, *d, launch, flags, *ds, st)) < 0) return rc;
     if (flags & PTWM_B200_NO_SYNC) return 0;
     return evaluate(*p, *d, flags, st);
 }
