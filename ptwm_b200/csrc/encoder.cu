@@ -421,7 +421,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
             CUDA_TRY(cudaStreamWaitEvent(side.s, side.ready, 0));
         }
         Bases b{nullptr, 0, 0, nullptr, nullptr};
-        xxh64_kernel<<<uint32_t(hash_items.size()), 32, 0, side.s>>>(wa.at<HashItem>(a_up + u_hitems), uint32_t(hash_items.size()), b, wa.at<uint64_t>(a_hashes));
+        xxh64_kernel<<<uint32_t(hash_items.size()), XXH_THREADS, 0, side.s>>>(wa.at<HashItem>(a_up + u_hitems), uint32_t(hash_items.size()), b, wa.at<uint64_t>(a_hashes));
         CUDA_TRY(cudaGetLastError());
     }
     CUDA_TRY(cudaMemsetAsync(d_plane_hist, 0, (a_hashes - a_plane_hist) + (n_planes ? 0 : 1), st));  // plane counts, OR words, CRC accumulators

@@ -1996,67 +1996,88 @@ __global__ void __launch_bounds__(128) crc_planes_kernel(const VerifyTensor* __r
     for (int p = 0; p < np; ++p) atomicXor(&acc[t.acc_base + p], gf2_mulmod(shift, c[p]));
 }
 
-// XXH64 (seed 0) of each tensor, one warp per tensor.  The hash is sequential by design: four accumulators, each
-// fed one 8-byte word of every 32-byte stripe through add, rotate and a 64-bit multiply, so four lanes carry the
-// state and a tensor cannot go faster than that dependent chain allows (add, rotate, one 64-bit multiply per 32
-// bytes).  What the rest of the warp does is keep the chain short and fed: all 32 lanes fetch the next 4 KiB of the
-// tensor with 128-bit loads and multiply the current block's words by the second prime, while lanes 0-3 work through
-// the 128 stripes of the current block out of shared memory, so neither DRAM latency nor that multiply shows.  Tensors hash
-// concurrently, one per block, and the host lists the largest first: the longest tensor is the critical path.
+// XXH64 (seed 0) of each tensor.  The hash is sequential by design: four accumulators, each fed one 8-byte word of every
+// 32-byte stripe through add, rotate and a 64-bit multiply, so four lanes carry the state and a tensor cannot go faster
+// than that dependent chain allows.  Tensors hash concurrently, one per block, and the host lists the largest first: the
+// longest tensor is the critical path.  Two warps per block: lanes 0-3 of the first work through the stripes of one block of
+// words in shared memory and do nothing else; the second warp meanwhile brings the next block from memory and multiplies its
+// words by the second prime.  A step adds the next word's product inside the widening multiply of the low halves, the cross
+// products run beside that one, and a three-way add joins the high half: 24 cycles per stripe instead of 27 with the add in
+// front of the rotation.  59 MB, the largest tensor of a fp32 model: 28.2 ms with one warp that did all of it, 22.4 now.
 __device__ __forceinline__ uint64_t rotl64(uint64_t x, int r) { return (x << r) | (x >> (64 - r)); }
 __device__ __forceinline__ uint64_t ld_u64_unaligned(const uint8_t* p) { return uint64_t(ld_u32_unaligned(p)) | uint64_t(ld_u32_unaligned(p + 4)) << 32; }
-constexpr uint32_t XXH_BLOCK = 4096;
+constexpr uint32_t XXH_BLOCK = 8192, XXH_THREADS = 64;
+// rotl64(s, 31) * P1 + k
+__device__ __forceinline__ uint64_t xxh_step(uint64_t s, uint64_t k) {
+    constexpr uint64_t P1 = 11400714785074694791ull;
+    const uint32_t a = uint32_t(s), b = uint32_t(s >> 32);
+    const uint32_t lo = __funnelshift_l(b, a, 31), hi = __funnelshift_l(a, b, 31);
+    const uint64_t t = uint64_t(lo) * uint32_t(P1) + k;
+    return uint64_t(uint32_t(t >> 32) + lo * uint32_t(P1 >> 32) + hi * uint32_t(P1)) << 32 | uint32_t(t);
+}
 
-__global__ void __launch_bounds__(32) xxh64_kernel(const HashItem* __restrict__ items, uint32_t n_items, Bases bases, uint64_t* __restrict__ out) {
+__global__ void __launch_bounds__(XXH_THREADS) xxh64_kernel(const HashItem* __restrict__ items, uint32_t n_items, Bases bases, uint64_t* __restrict__ out) {
     const uint64_t P1 = 11400714785074694791ull, P2 = 14029467366897019727ull, P3 = 1609587929392839161ull, P4 = 9650029242287828579ull,
                    P5 = 2870177450012600261ull;
-    __shared__ __align__(16) uint8_t stage[XXH_BLOCK];
-    const uint32_t lane = threadIdx.x, idx = blockIdx.x;
+    __shared__ __align__(16) uint64_t stage[2][XXH_BLOCK / 8];
+    const uint32_t lane = threadIdx.x & 31, idx = blockIdx.x;
+    const bool feeds = threadIdx.x >= 32;
     if (idx >= n_items) return;
     const HashItem it = items[idx];
     const uint8_t* p = rd(bases, it.data);
     const uint64_t len = it.len, stripes = len / 32;
+    const uint64_t blocks = (stripes * 32 + XXH_BLOCK - 1) / XXH_BLOCK;
+    const bool aligned = (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+    constexpr int PAIRS = XXH_BLOCK / 16 / 32;  // pairs of words per lane and block
+    uint4 nxt[PAIRS];
+    auto fetch = [&](uint64_t b) {  // block b; zero behind the last whole stripe
+        const uint64_t first = b * (XXH_BLOCK / 16) + lane, end = stripes * 2;
+#pragma unroll
+        for (int k = 0; k < PAIRS; ++k) {
+            const uint64_t at = first + 32 * k;
+            nxt[k] = make_uint4(0, 0, 0, 0);
+            if (at >= end) continue;
+            if (aligned) nxt[k] = __ldg(reinterpret_cast<const uint4*>(p) + at);
+            else {
+                const uint64_t x = ld8_unaligned(p + 16 * at), y = ld8_unaligned(p + 16 * at + 8);
+                nxt[k] = make_uint4(uint32_t(x), uint32_t(x >> 32), uint32_t(y), uint32_t(y >> 32));
+            }
+        }
+    };
+    auto store = [&](uint64_t b) {
+        uint64_t* w = stage[b & 1];
+#pragma unroll
+        for (int k = 0; k < PAIRS; ++k) {
+            const uint4 v = nxt[k];
+            const uint64_t x = (uint64_t(v.y) << 32 | v.x) * P2, y = (uint64_t(v.w) << 32 | v.z) * P2;
+            reinterpret_cast<uint4*>(w)[k * 32 + lane] = make_uint4(uint32_t(x), uint32_t(x >> 32), uint32_t(y), uint32_t(y >> 32));
+        }
+    };
     uint64_t v = lane == 0 ? P1 + P2 : lane == 1 ? P2 : lane == 2 ? 0 : 0 - P1;
-    uint64_t done = 0;  // stripes consumed
-    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        const uint64_t blocks = len / XXH_BLOCK;
-        uint4 nxt[8];
-        if (blocks) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) nxt[k] = __ldg(reinterpret_cast<const uint4*>(p) + k * 32 + lane);
-        }
-        for (uint64_t b = 0; b < blocks; ++b) {
-            __syncwarp();  // the previous block has been read
-#pragma unroll
-            for (int k = 0; k < 8; ++k) reinterpret_cast<uint4*>(stage)[k * 32 + lane] = nxt[k];
-            if (b + 1 < blocks) {
-                const uint4* q = reinterpret_cast<const uint4*>(p + (b + 1) * XXH_BLOCK);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) nxt[k] = __ldg(q + k * 32 + lane);
-            }
-            __syncwarp();
-            {   // the products word * P2 do not depend on the accumulators: all lanes take them off the serial chain
-                uint64_t* w = reinterpret_cast<uint64_t*>(stage);
-#pragma unroll
-                for (int k = 0; k < int(XXH_BLOCK / 8 / 32); ++k) w[k * 32 + lane] *= P2;
-            }
-            __syncwarp();
-            if (lane < 4) {
-                const uint64_t* w = reinterpret_cast<const uint64_t*>(stage) + lane;
+    if (feeds && blocks) {
+        fetch(0);
+        store(0);
+        if (blocks > 1) fetch(1);
+    }
+    for (uint64_t b = 0; b < blocks; ++b) {
+        __syncthreads();  // block b is in place, and nobody reads the other buffer any more
+        if (feeds) {
+            if (b + 1 < blocks) store(b + 1);
+            if (b + 2 < blocks) fetch(b + 2);
+        } else if (lane < 4) {
+            const uint64_t* w = stage[b & 1] + lane;
+            const uint64_t left = stripes - b * (XXH_BLOCK / 32);
+            v += w[0];
+            if (left >= XXH_BLOCK / 32) {
 #pragma unroll 16
-                for (int st = 0; st < int(XXH_BLOCK / 32); ++st) { v += w[4 * st]; v = rotl64(v, 31); v *= P1; }
+                for (int st = 1; st < int(XXH_BLOCK / 32); ++st) v = xxh_step(v, w[4 * st]);
+            } else {
+                for (uint32_t st = 1; st < uint32_t(left); ++st) v = xxh_step(v, w[4 * st]);
             }
-        }
-        done = blocks * (XXH_BLOCK / 32);
-    }
-    if (lane < 4) {  // what is left of the stripes (all of them for a source that is not 16-byte aligned)
-        const bool aligned = (reinterpret_cast<uintptr_t>(p) & 7) == 0;
-        for (uint64_t st = done; st < stripes; ++st) {
-            const uint8_t* q = p + st * 32 + lane * 8;
-            const uint64_t in = aligned ? *reinterpret_cast<const uint64_t*>(q) : ld_u64_unaligned(q);
-            v += in * P2; v = rotl64(v, 31); v *= P1;
+            v = xxh_step(v, 0);
         }
     }
+    if (feeds) return;
     const uint64_t v1 = __shfl_sync(0xFFFFFFFFu, v, 0), v2 = __shfl_sync(0xFFFFFFFFu, v, 1), v3 = __shfl_sync(0xFFFFFFFFu, v, 2), v4 = __shfl_sync(0xFFFFFFFFu, v, 3);
     if (lane != 0) return;
     auto round = [&](uint64_t acc, uint64_t in) { acc += in * P2; acc = rotl64(acc, 31); return acc * P1; };

@@ -598,7 +598,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
     if ((flags & PTWM_B200_VERIFY_HASH) && !pl.hashes.empty()) {
         uint32_t n = uint32_t(pl.hashes.size());
         CUDA_TRY(mark(11, 0));
-        xxh64_kernel<<<n, 32, 0, st>>>(d.hashes, n, bases, d.hash_out);
+        xxh64_kernel<<<n, XXH_THREADS, 0, st>>>(d.hashes, n, bases, d.hash_out);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(mark(11, 1));
     }
