@@ -555,6 +555,14 @@ __host__ __device__ inline uint32_t rans_smem_bytes(uint32_t l_entries, bool per
     return RANS_WARP_CHUNKS * RANS_RANK_BYTES + (per_lane ? 128 * l_entries : RANS_WARP_CHUNKS * 4 * l_entries) + RING_SMEM;
 }
 
+// Chunks of a launch up to which the kernel with a table entry per slot is the faster one: what the GPU holds of it at once (six
+// blocks of four chunks per SM).  Chunks of 32 Ki symbols of a bf16 model, table per slot against rank tables: 1 chunk 447 / 736 us,
+// 592 chunks 455 / 771, 2368 506 / 783, 3552 609 / 786, and beyond that a second wave (4736: 1050 / 789).  fp32: 491 / 826, 621 /
+// 863, 650 / 867, 834 / 872.
+constexpr uint32_t RANS_DIRECT_CHUNKS = 6 * 4 * 148;
+constexpr uint32_t RANS_DIRECT_BYTES = 2048 * 4;  // per chunk
+__host__ __device__ inline uint32_t rans_direct_smem(uint32_t warp_chunks) { return warp_chunks * RANS_DIRECT_BYTES + RING_SMEM; }
+
 // Ring addressing: byte q of a lane's ring lives in word (q >> 2) & 15 of the
 // [word][lane] array, `rw` points at the lane's column.
 __device__ __forceinline__ uint32_t ring_byte(const uint32_t* rw, uint32_t q) {
@@ -649,22 +657,77 @@ __device__ __forceinline__ void rans_group8(const uint32_t* tab, const uint32_t*
     }
 }
 
+// The same on a table with an entry per slot: frequency << 20 | slot's distance from the symbol's first << 8 | symbol.  From
+// one state to the next it is a mask, one shared-memory read, a shift and a multiply-add; renormalising picks among the state
+// shifted by none, one or two bytes, which are there by the time the comparisons are.  A state that has been normalised once
+// never needs more than two bytes (an update leaves at least 2^12), so eight bytes of stream last for four symbols and nothing
+// is decoded twice.  A stream whose stored initial state is not normalised goes byte by byte.
+__device__ __forceinline__ uint32_t rans_direct_lookup(const uint32_t* tab, uint32_t& x) {
+    const uint32_t e = tab[x & 2047u];
+    x = (e >> 20) * (x >> 11) + ((e >> 8) & 0xFFFu);
+    return e;
+}
+// The ring's words are kept with their first byte on top here.
+__device__ __forceinline__ void rans_direct_short(const uint32_t* tab, const uint32_t* rw, uint32_t& x, uint32_t& rq, uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
+    s_lo = 0; s_hi = 0;
+    for (uint32_t j = 0; j < g; ++j) {
+        const uint32_t sym = rans_direct_lookup(tab, x) & 0xFFu;
+        if (j < 4) s_lo |= sym << (8 * j); else s_hi |= sym << (8 * (j - 4));
+        for (int k = 0; k < 3 && x < RANS_L; ++k) { x = (x << 8) | ring_byte(rw, rq ^ 3u); ++rq; }
+    }
+}
+__device__ __forceinline__ void rans_direct_words(const uint32_t* rw, uint32_t rq, uint32_t v[5]) {  // five ring words from the one that holds byte rq on
+#pragma unroll
+    for (uint32_t k = 0; k < 5; ++k) v[k] = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(rw) + (((rq << 5) + 0x80u * k) & 0x780u));
+}
+// Four symbols.  `v` are five ring words read before the last four symbols were decoded, `skip` the bits of them that are used
+// up by now (88 at most).  The five words for the next four are requested here.
+__device__ __forceinline__ uint32_t rans_direct_four(const uint32_t* tab, const uint32_t* rw, uint32_t& x, uint32_t& rq, uint32_t v[5], uint32_t& skip) {
+    const bool one_off = skip >= 32, two_off = skip >= 64;
+    const uint32_t a = two_off ? v[2] : one_off ? v[1] : v[0], b = two_off ? v[3] : one_off ? v[2] : v[1], c = two_off ? v[4] : one_off ? v[3] : v[2];
+    uint32_t wh = __funnelshift_l(b, a, skip), wl = __funnelshift_l(c, b, skip), used = 0, sy = 0;  // a funnel shift takes the amount mod 32
+    rans_direct_words(rw, rq, v);
+    skip = (rq & 3u) * 8;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t e = rans_direct_lookup(tab, x);
+        sy = __byte_perm(sy, e, (0x3210u & ~(0xFu << (4 * j))) | (4u << (4 * j)));
+        const uint32_t one = __byte_perm(x, wh, 0x2107), two = __byte_perm(x, wh, 0x1076);
+        const bool some = x < RANS_L, more = x < (RANS_L >> 8);
+        const uint32_t y = more ? two : one, sh = more ? 16u : 8u;
+        x = some ? y : x;
+        const uint32_t bits = some ? sh : 0u;
+        wh = __funnelshift_l(wl, wh, bits);
+        wl <<= bits;
+        used += bits;
+    }
+    skip += used;
+    rq += used >> 3;
+    return sy;
+}
+
 // 20 blocks per SM lets the compiler use 96 registers (21 blocks), which the 32-bit rounds need to stay out of local
 // memory; shared memory allows 22, and more blocks than that gave nothing (the load/store pipe, the integer pipe and the
 // issue slots are each about 55-60 % busy there).
-template <bool PER_LANE>
-__global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem* __restrict__ items, uint32_t n_items, Bases bases, uint32_t* __restrict__ status,
+//
+// DIRECT (chunks per warp, 0 = the rank tables above): a table entry per slot, 8 KiB per chunk, for launches that do not fill
+// the GPU, where the time from one symbol to the next is all that counts (rans_direct_four).
+template <bool PER_LANE, int DIRECT = 0>
+__global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(const DecodeItem* __restrict__ items, uint32_t n_items, Bases bases, uint32_t* __restrict__ status,
                                                            uint32_t l_entries) {
     constexpr int LS = PER_LANE ? 32 : 1;
+    constexpr uint32_t CHUNKS = DIRECT ? DIRECT : RANS_WARP_CHUNKS;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t lane = threadIdx.x, c = lane >> 2, s = lane & 3;
-    uint32_t* ranktab = reinterpret_cast<uint32_t*>(smem);                                       // [8][128]
-    uint32_t* symlist = reinterpret_cast<uint32_t*>(smem + RANS_WARP_CHUNKS * RANS_RANK_BYTES);  // entry 0 of every list is a pad
-    const uint32_t list_bytes = PER_LANE ? 128 * l_entries : RANS_WARP_CHUNKS * 4 * l_entries;
-    Ring ring{reinterpret_cast<uint32_t*>(smem + RANS_WARP_CHUNKS * RANS_RANK_BYTES + list_bytes) + lane};
+    // DIRECT: the rings come first, and in their place, while the tables are built, one chunk's rank table and symbol list
+    uint32_t* slots = reinterpret_cast<uint32_t*>(smem + RING_SMEM);                                  // DIRECT: [chunk][2048]
+    uint32_t* ranktab = reinterpret_cast<uint32_t*>(smem);                                            // [8][128]
+    uint32_t* symlist = reinterpret_cast<uint32_t*>(smem + (DIRECT ? 1 : CHUNKS) * RANS_RANK_BYTES);  // entry 0 of every list is a pad
+    const uint32_t list_bytes = PER_LANE ? 128 * l_entries : CHUNKS * 4 * l_entries;
+    Ring ring{reinterpret_cast<uint32_t*>(DIRECT ? smem : smem + CHUNKS * RANS_RANK_BYTES + list_bytes) + lane};
 
-    const uint32_t item_idx = blockIdx.x * RANS_WARP_CHUNKS + c;
-    const bool valid = item_idx < n_items;
+    const uint32_t item_idx = blockIdx.x * CHUNKS + c;
+    const bool valid = c < CHUNKS && item_idx < n_items;
     DecodeItem it;
     if (valid) it = items[item_idx];
     const uint8_t* src = valid ? rd(bases, it.src) : nullptr;
@@ -693,7 +756,7 @@ __global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem*
 
     // tables: the whole warp builds one chunk's tables at a time
     bool dense = false;  // this lane's chunk is close to incompressible (see rans_group8)
-    for (uint32_t c2 = 0; c2 < RANS_WARP_CHUNKS; ++c2) {
+    for (uint32_t c2 = 0; c2 < CHUNKS; ++c2) {
         const uint32_t leader = c2 * 4;
         uintptr_t psrc = __shfl_sync(0xFFFFFFFFu, reinterpret_cast<uintptr_t>(src), leader);
         uint32_t pms = __shfl_sync(0xFFFFFFFFu, max_sym, leader);
@@ -721,8 +784,8 @@ __global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem*
         if (distinct + 2 > l_entries) bad = true;  // the host sizes the list from the planned bytes; a blob that differs from them may not fit
         if (bad) { if (c == c2) err = ST_BAD_HEADER; continue; }
         uint32_t start = incl - sum, rank = rincl - present;
-        uint32_t* tab = ranktab + c2 * 128;
-        uint32_t* lst = PER_LANE ? symlist + c2 * 4 : symlist + c2 * l_entries;
+        uint32_t* tab = DIRECT ? ranktab : ranktab + c2 * 128;
+        uint32_t* lst = DIRECT ? symlist : PER_LANE ? symlist + c2 * 4 : symlist + c2 * l_entries;
         if (lane == 0) {
             if (PER_LANE) *reinterpret_cast<uint4*>(lst) = make_uint4(0, 0, 0, 0); else lst[0] = 0;
         }
@@ -753,6 +816,15 @@ __global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem*
         bm.z |= before << 16; before += p2;
         bm.w |= before << 16;
         *reinterpret_cast<uint4*>(tab + 4 * lane) = bm;
+        if (DIRECT) {
+            __syncwarp();
+#pragma unroll 8
+            for (uint32_t u = lane; u < 2048; u += 32) {
+                const uint32_t w = tab[u >> 4], e = lst[(w >> 16) + __popc(w << ((~u & 15u) | 16u))];
+                slots[c2 * 2048 + u] = ((e >> 8) & 0xFFFu) << 20 | (u - (e >> 20)) << 8 | (e & 0xFFu);
+            }
+            __syncwarp();
+        }
     }
     __syncwarp();
 
@@ -761,13 +833,13 @@ __global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem*
     if (valid && !err && seg_len > 0) {
         if (my_len < 4) err = ST_STREAM_UNDERRUN;  // decompress.rs:82-86
         else {
-            const uint32_t* tab = ranktab + c * 128;
+            const uint32_t* tab = DIRECT ? slots + c * 2048 : ranktab + c * 128;
             const uint32_t* lst = PER_LANE ? symlist + lane : symlist + c * l_entries;
             const uint32_t* rw = ring.base;
             Epilogue ep = make_epilogue(bases, it);
             const uint8_t* st = src + my_off;
             uint32_t x = ld_u32_unaligned(st);
-            const bool slow = x >> 31;  // see rans_group8
+            const bool slow = x >> 31 || (DIRECT && x < RANS_L);  // see rans_group8, rans_direct_four
             // ring cursor as a 32-bit offset from the 16-byte aligned block that holds the first renorm byte
             const uintptr_t g0 = (reinterpret_cast<uintptr_t>(st) + 4) & ~uintptr_t(15);
             uint32_t rq = uint32_t(reinterpret_cast<uintptr_t>(st) + 4 - g0);
@@ -775,40 +847,65 @@ __global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem*
             const uintptr_t lo16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_first) & ~uintptr_t(15);
             const uintptr_t hi16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_end + 15) & ~uintptr_t(15);
             uint32_t fq = 0;
-            ring.put(fq, fetch16(g0 + fq, lo16, hi16)); fq += 16;
-            ring.put(fq, fetch16(g0 + fq, lo16, hi16)); fq += 16;
-            ring.put(fq, fetch16(g0 + fq, lo16, hi16)); fq += 16;
+            auto park = [&](uint4 v) {
+                if (DIRECT) v = make_uint4(__byte_perm(v.x, 0, 0x0123), __byte_perm(v.y, 0, 0x0123), __byte_perm(v.z, 0, 0x0123), __byte_perm(v.w, 0, 0x0123));
+                ring.put(fq, v);
+                fq += 16;
+            };
+            for (int k = 0; k < 3; ++k) park(fetch16(g0 + fq, lo16, hi16));
             uint4 pending = fetch16(g0 + fq, lo16, hi16);
             // A group consumes at most 24 bytes; 32 valid bytes at its start always suffice.
             // The lanes of a warp drain their rings at similar rates: when any active lane runs low,
             // every lane with room for a block takes one, so the refill code runs once per several groups.
-            auto top_up = [&]() {
-                if (__any_sync(__activemask(), fq - rq < 32)) {
-                    if (fq - rq <= 48) { ring.put(fq, pending); fq += 16; pending = fetch16(g0 + fq, lo16, hi16); }
+            auto top_up_at = [&](uint32_t q, uint32_t low) {
+                if (__any_sync(__activemask(), fq - q < low)) {
+                    if (fq - q <= 48) { park(pending); pending = fetch16(g0 + fq, lo16, hi16); }
                 }
             };
+            auto top_up = [&]() { top_up_at(rq, 32); };
 
             uint32_t pos = seg_start, remaining = seg_len;
+            auto short_group = [&](uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
+                if (DIRECT) rans_direct_short(tab, rw, x, rq, g, s_lo, s_hi);
+                else rans_short_group<LS>(tab, lst, rw, x, rq, g, s_lo, s_hi);
+            };
             // head: a short group up to the next 8-element boundary of the destination
             {
                 uint32_t g = first_group(ep, pos, remaining);
                 if (g < 8 || remaining < 16) {
                     uint32_t s_lo, s_hi;
                     top_up();
-                    rans_short_group<LS>(tab, lst, rw, x, rq, g, s_lo, s_hi);
+                    short_group(g, s_lo, s_hi);
                     emit(ep, pos, g, uint64_t(s_lo) | uint64_t(s_hi) << 32);
                     pos += g; remaining -= g;
                 }
             }
-            fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {
+            if (DIRECT && !slow) {
+                // A read of the ring takes as long as half a symbol, so words are read four symbols before they are used, and the
+                // ring is topped up by where the group began: that position has been known for long, and no wait hangs on it.
+                // Four symbols take eight bytes at most and words are read for eight: from a group's beginning on 24 bytes are
+                // there, and 40 after the top-up, which is 24 behind a group's end.
+                uint32_t v[5], skip = (rq & 3u) * 8;
                 top_up();
-                rans_group8<LS, !PER_LANE>(tab, lst, rw, x, rq, s_lo, s_hi, dense, slow);
-            });
+                rans_direct_words(rw, rq, v);
+                fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {
+                    const uint32_t began = rq;
+                    s_lo = rans_direct_four(tab, rw, x, rq, v, skip);
+                    top_up_at(began, 40);
+                    s_hi = rans_direct_four(tab, rw, x, rq, v, skip);
+                });
+            } else {
+                fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {
+                    top_up();
+                    if (DIRECT) rans_direct_short(tab, rw, x, rq, 8, s_lo, s_hi);
+                    else rans_group8<LS, !PER_LANE>(tab, lst, rw, x, rq, s_lo, s_hi, dense, slow);
+                });
+            }
             // tail: whatever the fast loops left
             while (remaining) {
                 uint32_t g = remaining < 8 ? remaining : 8, s_lo, s_hi;
                 top_up();
-                rans_short_group<LS>(tab, lst, rw, x, rq, g, s_lo, s_hi);
+                short_group(g, s_lo, s_hi);
                 emit(ep, pos, g, uint64_t(s_lo) | uint64_t(s_hi) << 32);
                 pos += g; remaining -= g;
             }
@@ -816,6 +913,23 @@ __global__ void __launch_bounds__(32, 20) rans_decode_kernel_t(const DecodeItem*
         }
     }
     if (err) report(status, it.id, err);
+}
+
+// `direct`: the launch takes the kernel with a table entry per slot.  Else `size` is the rows of the symbol lists (`narrow`) or the
+// most distinct symbols of a chunk.
+inline void rans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, bool direct, bool narrow, uint32_t size, cudaStream_t st) {
+    auto blocks = [n](uint32_t per) { return (n + per - 1) / per; };
+    if (direct && n <= 4 * 148) rans_decode_kernel_t<false, 1><<<n, 32, rans_direct_smem(1), st>>>(items, n, bases, status, rans_l_entries(255));
+    else if (direct) rans_decode_kernel_t<false, 4><<<blocks(4), 32, rans_direct_smem(4), st>>>(items, n, bases, status, rans_l_entries(255));
+    else if (narrow) rans_decode_kernel_t<true><<<blocks(RANS_WARP_CHUNKS), 32, rans_smem_bytes(size + 2, true), st>>>(items, n, bases, status, size + 2);
+    else {
+        const uint32_t le = (size + 2 + 3) & ~3u;
+        rans_decode_kernel_t<false><<<blocks(RANS_WARP_CHUNKS), 32, rans_smem_bytes(le), st>>>(items, n, bases, status, le);
+    }
+}
+inline cudaError_t rans_direct_allow_shared() {
+    const cudaError_t e = cudaFuncSetAttribute(rans_decode_kernel_t<false, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(rans_decode_kernel_t<false, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
 // ---- canonical Huffman -----------------------------------------------------

@@ -147,6 +147,7 @@ int64_t device_state(int dev, DeviceState** out) {
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rans_smem_bytes(RANS_NARROW_SYMBOLS + 2, true))));
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         CUDA_TRY(cudaFuncSetAttribute(huffman_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HUF_SMEM));
+        CUDA_TRY(rans_direct_allow_shared());
         CUDA_TRY(o1sac_allow_shared_rows());
         // the decoders are limited by how many chunk tables fit in an SM: ask for the largest shared-memory carve-out
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
@@ -362,20 +363,27 @@ void finish_lists(ptwm_b200_plan& pl) {
     for (int ph = 0; ph < 2; ++ph) {
         for (int cc = 0; cc < 4; ++cc) {
             auto& v = pl.dec[ph][cc];
-            auto narrow = [cc](const DecodeItem& a) { return cc == 0 && (a.row_len >> 16) <= RANS_NARROW_SYMBOLS; };
+            const bool direct = v.size() <= RANS_DIRECT_CHUNKS;  // one kernel for any alphabet
+            auto narrow = [cc, direct](const DecodeItem& a) { return cc == 0 && !direct && (a.row_len >> 16) <= RANS_NARROW_SYMBOLS; };
             auto waits = [ph](const DecodeItem& a) {
                 if (ph == 0) return false;
                 for (Ref r : a.partner) if (r != REF_NONE && (r >> 62) == SP_SCRATCH) return true;
                 return false;
             };
-            std::stable_sort(v.begin(), v.end(), [&](const DecodeItem& a, const DecodeItem& b) {
-                const int ka = 2 * waits(a) + !narrow(a), kb = 2 * waits(b) + !narrow(b);
-                return ka != kb ? ka < kb : a.n > b.n;
-            });
+            // by launch (waiting or not, narrow or not), the longest chunks first; most lists are in that order already
+            std::vector<std::pair<uint64_t, uint32_t>> order(v.size());
+            for (size_t k = 0; k < v.size(); ++k) order[k] = {uint64_t(2 * waits(v[k]) + !narrow(v[k])) << 32 | (0xFFFFFFFFu - v[k].n), uint32_t(k)};
+            if (!std::is_sorted(order.begin(), order.end())) {
+                std::sort(order.begin(), order.end());  // equal keys by place in the list
+                std::vector<DecodeItem> sorted;
+                sorted.reserve(v.size());
+                for (auto& o : order) sorted.push_back(v[o.second]);
+                v.swap(sorted);
+            }
             const int slot = ph * 5 + cc;
             pl.slot_items[slot] = uint32_t(v.size());
             for (size_t k = 0; k < v.size(); ++k) {
-                const bool w = waits(v[k]), nw = narrow(v[k]);
+                const bool w = order[k].first >> 33, nw = !(order[k].first >> 32 & 1);
                 auto& runs = pl.runs[ph][cc];
                 if (runs.empty() || runs.back().waits != w || runs.back().narrow != nw) { runs.push_back({uint32_t(k), 0, 0, w, nw}); pl.launches++; }
                 runs.back().count++;
@@ -488,13 +496,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         const uint32_t n = r.count;
         switch (cc) {
             case 0:
-                if (r.narrow) {
-                    const uint32_t rows = r.size + 2;
-                    rans_decode_kernel_t<true><<<(n + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, rans_smem_bytes(rows, true), s>>>(it, n, bases, status, rows);
-                } else {
-                    const uint32_t le = (r.size + 2 + 3) & ~3u;
-                    rans_decode_kernel_t<false><<<(n + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, rans_smem_bytes(le), s>>>(it, n, bases, status, le);
-                }
+                rans_launch(it, n, bases, status, pl.dec[ph][0].size() <= RANS_DIRECT_CHUNKS, r.narrow, r.size, s);
                 break;
             case 1: huffman_decode_kernel<<<(n + HUF_WARP_CHUNKS - 1) / HUF_WARP_CHUNKS, 32, HUF_SMEM, s>>>(it, n, bases, status); break;
             case 2: tans_launch(it, n, bases, status, s); break;
@@ -718,7 +720,7 @@ int64_t decode_plane_cuda(uint8_t sfv, const uint8_t* state, size_t state_len, c
     const DecodeItem* d_it = reinterpret_cast<const DecodeItem*>(scratch + 64);
     uint32_t* d_status = reinterpret_cast<uint32_t*>(scratch) + 1;  // the summary word in front
     switch (codec) {
-        case C_RANS: rans_decode_kernel_t<false><<<1, 32, rans_smem_bytes(rans_l_entries(255)), st>>>(d_it, 1, bases, d_status, rans_l_entries(255)); break;
+        case C_RANS: rans_launch(d_it, 1, bases, d_status, true, false, 0, st); break;
         case C_HUFFMAN: huffman_decode_kernel<<<1, 32, HUF_SMEM, st>>>(d_it, 1, bases, d_status); break;
         case C_TANS: tans_launch(d_it, 1, bases, d_status, st); break;
         default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), st); break;
@@ -874,7 +876,10 @@ int64_t ptwm_b200_plan_create(const ptwm_b200_container* c, const uint32_t* indi
             // goes to scratch and one more launch merges them (a 4096-element norm vector: 0.48 -> 0.3 ms).
             uint64_t coded = 0;
             for (uint32_t ti : pl->tensors) if (ti < c->file.tensors.size())
-                for (const PlaneDesc& p : c->file.tensors[ti].planes) for (const ChunkDesc& ch : p.chunks) coded += !ch.raw;
+                for (const PlaneDesc& p : c->file.tensors[ti].planes) {
+                    if (coded > SPREAD_CHUNKS) break;
+                    for (const ChunkDesc& ch : p.chunks) coded += !ch.raw;
+                }
             pl->spread = coded <= SPREAD_CHUNKS;
         }
         for (uint32_t ti : pl->tensors) {
