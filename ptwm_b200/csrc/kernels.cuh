@@ -1575,14 +1575,21 @@ inline cudaError_t tans_prefer_shared() {
 // the range the code falls into.  The 256 shares of a context are mostly dust
 // (a symbol the plane never showed after this one still has 1 of 4096), so the
 // warp keeps the 32 widest in shared memory, one per lane: cumulative count,
-// width, symbol and where the symbol's own row lies.  A lane tests its share
-// with two multiplies; a maximum over the warp of (hit ? share : 0) is the
-// symbol with everything its step needs, without a second look at a table.  A
-// code that falls into none of the 32 is searched among all 256 from the
-// serialized state.  With the whole cumulative table of the context probed for
-// every symbol (eight counts per lane, three reductions) a symbol took 371
-// cycles and 114 instructions.
-constexpr uint32_t O1_ROW_BYTES = 32 * 8;  // {cumulative count << 20 | width << 8 | symbol, offset of the symbol's row} per lane
+// width, symbol and where the symbol's own row lies.  Every lane goes on as if
+// its share were the one: new offset and range, renormalised.  One of them is
+// right, and three maxima over the warp hand its state to all.  From row to row
+// that is a shared-memory read, a multiply-add, a comparison and a maximum (20
+// cycles; a vote, its first set bit and a shuffle are 80).  A code that falls into none of the 32 shares is searched among all
+// 256 from the serialized state.  Only the code's distance from the low end of
+// the range matters (both lose the same bits to renormalisation), so that is
+// what is carried.
+// Branches are left out of that way as well.  A code outside the 32 shares leaves a range of zero, which no share of any row
+// can win again, so one look per eight symbols finds it and the eight are decoded again one by one; the end of a row is looked
+// for once per eight symbols too, and the stream's words for eight symbols are read at once, from a buffer in shared memory
+// that the warp fills 256 bytes at a time.  280 chunks of 32 Ki scales: 4.12 ms (247 cycles per symbol) with two maxima over
+// packed shares and everything else behind them, 4.00 with the lanes' own next states, 2.19 (131 cycles) without the branches.
+constexpr uint32_t O1_ROW_BYTES = 32 * 12;  // per lane {minus the cumulative count, width}, then per lane the offset of the symbol's row << 8 | symbol
+constexpr uint32_t O1_HALF = 64;            // words in half of the stream buffer
 // Context rows of a chunk whose state has `state_len` bytes, the marginal's included (0 when the state is too short to hold any).
 inline uint32_t o1sac_tables(uint64_t state_len) { return state_len >= 32 + 512 ? uint32_t((state_len - 32 - 512) / 512) + 1 : 0; }
 
@@ -1592,6 +1599,7 @@ __global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __re
     const DecodeItem it = items[blockIdx.x];
     const uint8_t* st = rd(bases, it.state);
     __shared__ uint32_t bitmap[8];      // contexts that have a row
+    __shared__ uint32_t words[2 * O1_HALF];  // the stream
     __shared__ uint16_t row_of[256];    // the row a symbol leads to: 0 = marginal, 1 + rank of the context otherwise
     uint32_t err = it.state_version != 1 || it.state_len < 32 + 512 ? uint32_t(ST_BAD_STATE) : uint32_t(ST_OK);
     uint32_t rows = 1;
@@ -1647,67 +1655,89 @@ __global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __re
         const uint32_t used = __shfl_sync(0xFFFFFFFFu, at, 31);
         at -= mine;
         uint2* out = reinterpret_cast<uint2*>(smem + row * O1_ROW_BYTES);
+        uint32_t* leads = reinterpret_cast<uint32_t*>(out + 32);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            if (v[k] > dust) { out[at] = make_uint2(cum << 20 | v[k] << 8 | (lane * 8 + k), uint32_t(row_of[lane * 8 + k]) * O1_ROW_BYTES); ++at; }
+            if (v[k] > dust) {
+                out[at] = make_uint2(0u - cum, v[k]);
+                leads[at] = uint32_t(row_of[lane * 8 + k]) * O1_ROW_BYTES << 8 | (lane * 8 + k);
+                ++at;
+            }
             cum += v[k];
         }
-        if (lane >= used) out[lane] = make_uint2(0, 0);  // width 0: never hit
+        if (lane >= used) { out[lane] = make_uint2(0, 0); leads[lane] = 0; }  // width 0: never hit
     }
     if (err) { if (lane == 0) report(status, it.id, err); return; }
     __syncwarp();
 
     Epilogue ep = make_epilogue(bases, it);
-    // Stream bytes, big-endian: `hi` and `lo` hold eight of them from an aligned word on, the next byte to use `taken` bits into
-    // them, and `ahead` is on its way.  Zero past the end.
-    const uintptr_t src = reinterpret_cast<uintptr_t>(rd(bases, it.src)), src_end = src + it.src_len;
-    uintptr_t next = src & ~uintptr_t(3);
-    auto fetch = [&]() -> uint32_t {
+    // Stream words, first byte on top, from the aligned word on that holds the first byte; zero past the end.  Word i lies in
+    // words[i mod 128]; the half that holds the current word and the next half are there, the one after that is on its way.
+    const uintptr_t src = reinterpret_cast<uintptr_t>(rd(bases, it.src)), src_end = src + it.src_len, src_word = src & ~uintptr_t(3);
+    auto fetch = [&](uint64_t i) -> uint32_t {
+        const uintptr_t q = src_word + 4 * i;
+        if (q >= src && q + 4 <= src_end) return __byte_perm(__ldg(reinterpret_cast<const uint32_t*>(q)), 0, 0x0123);
         uint32_t w = 0;
-        if (next >= src && next + 4 <= src_end) w = __byte_perm(__ldg(reinterpret_cast<const uint32_t*>(next)), 0, 0x0123);
-        else for (uint32_t k = 0; k < 4; ++k) if (next + k >= src && next + k < src_end) w |= uint32_t(__ldg(reinterpret_cast<const uint8_t*>(next + k))) << (24 - 8 * k);
-        next += 4;
+        for (uint32_t k = 0; k < 4; ++k) if (q + k >= src && q + k < src_end) w |= uint32_t(__ldg(reinterpret_cast<const uint8_t*>(q + k))) << (24 - 8 * k);
         return w;
     };
-    uint32_t hi = fetch(), lo = fetch(), ahead = fetch(), taken = 8 * uint32_t(src & 3);
-    auto advance = [&](uint32_t bits) {
-        taken += bits;
-        if (taken >= 32) { taken -= 32; hi = lo; lo = ahead; ahead = fetch(); }
+    for (uint32_t i = lane; i < 2 * O1_HALF; i += 32) words[i] = fetch(i);
+    uint32_t coming[2] = {fetch(2 * O1_HALF + lane), fetch(2 * O1_HALF + 32 + lane)};
+    __syncwarp();
+    uint64_t bit = 8 * (src & 3) + 8;  // range_coder.rs:137-155: five bytes start the code register, of which the last four count
+    auto word = [&](uint32_t k) { return words[(uint32_t(bit >> 5) + k) & (2 * O1_HALF - 1)]; };
+    auto advance = [&](uint32_t bits) {  // at most 128
+        const uint64_t half = bit / (32 * O1_HALF);
+        bit += bits;
+        if (bit / (32 * O1_HALF) != half) {
+            __syncwarp();
+            words[(half & 1) * O1_HALF + lane] = coming[0];
+            words[(half & 1) * O1_HALF + 32 + lane] = coming[1];
+            __syncwarp();
+            coming[0] = fetch((half + 3) * O1_HALF + lane);
+            coming[1] = fetch((half + 3) * O1_HALF + 32 + lane);
+        }
     };
-    // range_coder.rs:137-155: five bytes start the code register, of which the last four count
-    advance(8);
-    uint32_t code = __funnelshift_l(lo, hi, taken);
-    advance(16); advance(16);
-    uint32_t low = 0, range = 0xFFFFFFFFu, row = 0;
+    uint32_t offset = __funnelshift_l(word(1), word(0), uint32_t(bit));  // code - low
+    advance(32);
+    uint32_t rpt = 0xFFFFFFFFu >> 12, row = 0;  // range / 4096; the context's row, in bytes
     const uint32_t row_len = it.row_len ? it.row_len : (it.n ? it.n : 1);
     uint32_t left_in_row = row_len;
-    auto one_symbol = [&]() -> uint32_t {
+    // One symbol, by the 32 shares; rpt is 0 if none of them has it (and stays 0 if it was).  Returns the symbol, the bits taken and
+    // the next row: row << 8 | symbol, bits.
+    auto by_share = [&](uint32_t window, uint32_t& bits) -> uint32_t {
         const uint2 mine = *reinterpret_cast<const uint2*>(smem + row + lane * 8);
-        const uint32_t from = row, rpt = range >> 12;  // range / 4096
-        const uint32_t offset = code - low;
+        const uint32_t lead = *reinterpret_cast<const uint32_t*>(smem + row + 256 + lane * 4);
         // "cumulative count <= offset / rpt < count + width" without the division; the products fit 32 bits
-        const bool hit = offset - (mine.x >> 20) * rpt < ((mine.x >> 8) & 0xFFFu) * rpt;
-        uint32_t share = __reduce_max_sync(0xFFFFFFFFu, hit ? mine.x : 0u);
-        row = __reduce_max_sync(0xFFFFFFFFu, hit ? mine.y : 0u);
-        uint32_t cum = share >> 20, width = (share >> 8) & 0xFFFu, sy = share & 0xFFu;
-        if (share == 0) {
+        const uint32_t rest = offset + mine.x * rpt, range = mine.y * rpt;
+        const bool won = rest < range;
+        const uint32_t got = __reduce_max_sync(0xFFFFFFFFu, won ? lead : 0u);
+        const uint32_t b = range < (1u << 16) ? 16u : range < (1u << 24) ? 8u : 0u;  // rpt >= 2^12: two bytes at most
+        const uint32_t next = __reduce_max_sync(0xFFFFFFFFu, won ? (range << b) >> 12 | b << 24 : 0u);
+        offset = __reduce_max_sync(0xFFFFFFFFu, won ? __funnelshift_l(window, rest, b) : 0u);
+        rpt = next & 0xFFFFFFu;
+        bits = next >> 24;
+        row = got >> 8;
+        return got & 0xFFu;
+    };
+    auto one_symbol = [&]() -> uint32_t {
+        const uint32_t was = offset, per = rpt, from = row, window = __funnelshift_l(word(1), word(0), uint32_t(bit));
+        uint32_t bits, sy = by_share(window, bits);
+        if (rpt == 0) {
             // among all 256: the largest index whose count is <= min(offset / rpt, 4095) (order1_scale_ac.rs:474-486)
             uint32_t v[8], c = load_row(from / O1_ROW_BYTES, v), fit = 0, below = 0, w = 0;
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                if (c * rpt <= offset) { ++fit; below = c; w = v[k]; }
+                if (c * per <= was) { ++fit; below = c; w = v[k]; }
                 c += v[k];
             }
             sy = __reduce_add_sync(0xFFFFFFFFu, fit) - 1;  // entry 0 counts 0 and always fits
-            cum = __shfl_sync(0xFFFFFFFFu, below, sy >> 3);
-            width = __shfl_sync(0xFFFFFFFFu, w, sy >> 3);
+            const uint32_t range = __shfl_sync(0xFFFFFFFFu, w, sy >> 3) * per;
+            bits = range < (1u << 16) ? 16u : range < (1u << 24) ? 8u : 0u;
+            offset = __funnelshift_l(window, was - __shfl_sync(0xFFFFFFFFu, below, sy >> 3) * per, bits);
+            rpt = (range << bits) >> 12;
             row = uint32_t(row_of[sy]) * O1_ROW_BYTES;
         }
-        low += cum * rpt;
-        range = width * rpt;
-        const uint32_t bits = range < (1u << 16) ? 16u : range < (1u << 24) ? 8u : 0u;  // rpt >= 2^12: two bytes at most
-        code = __funnelshift_l(__funnelshift_l(lo, hi, taken), code, bits);
-        low <<= bits; range <<= bits;
         advance(bits);
         if (--left_in_row == 0) { row = 0; left_in_row = row_len; }  // a row's first symbol has no context
         return sy;
@@ -1716,13 +1746,26 @@ __global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __re
     uint32_t remaining = it.n, g = remaining ? first_group(ep, pos, remaining) : 0;
     while (remaining) {
         uint32_t s_lo = 0, s_hi = 0;
-        if (g == 8) {
+        bool done = false;
+        if (g == 8 && left_in_row > 8) {
+            const uint32_t offset0 = offset, rpt0 = rpt, row0 = row;
+            uint32_t w0 = word(0), w1 = word(1), w2 = word(2), w3 = word(3), w4 = word(4), at = uint32_t(bit) & 31, used = 0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const uint32_t sy = one_symbol();
+                uint32_t bits;
+                const uint32_t sy = by_share(__funnelshift_l(w1, w0, at), bits);
                 if (j < 4) s_lo |= sy << (8 * j); else s_hi |= sy << (8 * (j - 4));
+                at += bits; used += bits;
+                const bool over = at >= 32;
+                w0 = over ? w1 : w0; w1 = over ? w2 : w1; w2 = over ? w3 : w2; w3 = over ? w4 : w3;
+                at &= 31;
             }
-        } else {
+            done = rpt != 0;
+            if (done) { advance(used); left_in_row -= 8; }
+            else { offset = offset0; rpt = rpt0; row = row0; s_lo = s_hi = 0; }
+        }
+        if (!done) {
+#pragma unroll 1
             for (uint32_t j = 0; j < g; ++j) {
                 const uint32_t sy = one_symbol();
                 if (j < 4) s_lo |= sy << (8 * j); else s_hi |= sy << (8 * (j - 4));
