@@ -1,0 +1,120 @@
+"""The decoders and encoders at the sizes where their work splits: remainders of lanes, warps, runs and blocks, launches on
+either side of a choice of kernel, and planes that leave the usual alphabet.  Everything is exact: decoded bytes against the
+source, written containers against the oracle's."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import ptwm_b200
+from ptwm_b200.compressor import CompressionConfig, HUFFMAN, IDENTITY, RANS, TANS, compress_model
+from _data import mixed_model, weights
+
+pytestmark = pytest.mark.gpu
+
+
+def plane(kind: str, n: int, seed: int = 0) -> bytes:
+    rng = np.random.default_rng((n, seed))
+    if kind == "exponent":
+        w = weights(1, n, seed + n, False).to(torch.bfloat16).view(torch.int16).numpy().reshape(-1)
+        return ((w.astype(np.uint16) >> 7) & 0xFF).astype(np.uint8).tobytes()
+    if kind == "rare":  # one symbol with nearly all of the table
+        return np.where(rng.random(n) < 1 / 3000, 7, 200).astype(np.uint8).tobytes()
+    if kind == "nibble":
+        return rng.integers(0, 16, n, dtype=np.uint8).tobytes()
+    return np.minimum(rng.geometric(0.03, n), 255).astype(np.uint8).tobytes()  # "wide": an alphabet of 200 and more
+
+
+def check(specs, **kw):
+    blob = oracle.write_container(specs, **kw)
+    got = ptwm_b200.ContainerHandle(blob, device=0, verify=True).decode_model()
+    for (name, t), s in zip(got, specs):
+        assert t.contiguous().view(torch.uint8).cpu().numpy().tobytes() == s.raw, name
+
+
+def u8(name, raw, cols=None):
+    return oracle.TensorSpec(name, oracle.DT_U8, [len(raw)] if cols is None else [len(raw) // cols, cols], raw, usage="standard" if cols is None else "scale")
+
+
+@pytest.mark.parametrize("kind", ["exponent", "rare", "nibble", "wide"])
+@pytest.mark.parametrize("codec", [HUFFMAN, RANS, TANS])
+def test_decode_chunk_lengths(kind, codec):
+    # lanes with nothing to do, groups of eight and their remainders, runs of 256 symbols: 1, 31, 32, 127, 128 and more than that
+    lengths = (1, 2, 3, 5, 31, 33, 63, 64, 65, 255, 256, 257, 511, 513, 1029, 8191, 8193, 127 * 256 + 9, 128 * 256, 128 * 256 + 1, 70001)
+    check([u8(f"p{n}", plane(kind, n)) for n in lengths], chunk_size=1 << 20, forced_codec=codec, emit_crc=True)
+
+
+@pytest.mark.parametrize("codec,chunks", [(RANS, 1), (RANS, 591), (RANS, 592), (RANS, 593), (RANS, 595), (RANS, 3552), (RANS, 3553),
+                                          (TANS, 295), (TANS, 296), (TANS, 297), (HUFFMAN, 593)])
+@pytest.mark.parametrize("dtype", ["u8", "bf16", "fp32"])
+def test_decode_launch_sizes(codec, chunks, dtype):
+    n = 67 * (chunks - 1) + 5  # a last chunk of five
+    if dtype == "u8":
+        specs = [u8("p", plane("exponent", n))]
+    else:
+        t = weights(1, n, chunks, False).to(torch.bfloat16 if dtype == "bf16" else torch.float32)
+        specs = [oracle.TensorSpec("p", oracle.DT_BF16 if dtype == "bf16" else oracle.DT_F32, [n], t.view(torch.uint8).numpy().tobytes())]
+    check(specs, chunk_size=67, forced_codec=codec)
+
+
+@pytest.mark.parametrize("alphabet", [2, 31, 33, 64, 256])
+@pytest.mark.parametrize("cols", [1, 5, 8, 9, 37, 0])
+def test_order1_scale_ac_shares_and_rows(alphabet, cols):
+    # more than 32 symbols after one another leave the shares that are searched first; rows end inside and between groups of eight
+    rng = np.random.default_rng(alphabet)
+    specs = []
+    for k, n in enumerate((37 * 8, 37 * 80, 37 * 400)):
+        raw = ((np.cumsum(rng.integers(0, 2, n)) * 7 + rng.integers(0, alphabet, n)) % alphabet).astype(np.uint8).tobytes()
+        raw = raw[:n // cols * cols] if cols else raw
+        specs.append(u8(f"s{k}", raw, cols or None))
+    check(specs, chunk_size=None if cols else 1500, forced_codec=oracle.O1SAC)
+
+
+def test_decode_two_coded_planes_in_many_chunks():
+    # more chunks than are spread over scratch: the second plane's lanes merge with the first one, every codec on its own stream
+    for menu in ((oracle.HUFFMAN, oracle.RANS, oracle.O1SAC), (oracle.TANS, oracle.O1SAC), (oracle.IDENTITY, oracle.HUFFMAN, oracle.RANS, oracle.TANS, oracle.O1SAC)):
+        check(mixed_model(2), chunk_size=501, menu=menu, emit_crc=True, emit_hash=True)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 8])
+def test_payload_hash_blocks_and_alignment(shift):
+    lengths = (0, 1, 31, 32, 33, 8191, 8192, 8193, 8192 + 32, 2 * 8192, 3 * 8192 + 45)
+    specs, tensors = [], {}
+    for n in lengths:
+        raw = np.random.default_rng(n).integers(0, 256, n + shift, dtype=np.uint8)
+        tensors[f"t{n}"] = torch.from_numpy(raw).cuda()[shift:]
+        specs.append(u8(f"t{n}", raw[shift:].tobytes()))
+    enc = compress_model(tensors, CompressionConfig(streaming_chunk=4096, forced_codec=IDENTITY, emit_payload_hash=True))
+    assert enc.to_bytes() == oracle.write_container(specs, chunk_size=4096, forced_codec=IDENTITY, emit_hash=True)
+    check(specs, chunk_size=4096, forced_codec=IDENTITY, emit_hash=True)
+
+
+@pytest.mark.parametrize("kind", ["exponent", "rare", "nibble", "wide"])
+@pytest.mark.parametrize("codec", [HUFFMAN, RANS, TANS])
+def test_encode_chunk_lengths(kind, codec):
+    lengths = (1, 2, 3, 4, 5, 7, 31, 32, 33, 255, 257, 511, 512, 513, 1023, 1025, 4099, 16385, 40000)
+    specs = [u8(f"p{n}", plane(kind, n)) for n in lengths]
+    tensors = {s.name: torch.frombuffer(bytearray(s.raw), dtype=torch.uint8).cuda() for s in specs}
+    for chunk in (None, 1021):
+        got = compress_model(tensors, CompressionConfig(streaming_chunk=chunk, forced_codec=codec)).to_bytes()
+        assert got == oracle.write_container(specs, chunk_size=chunk, forced_codec=codec), chunk
+
+
+def test_plan_run_in_a_captured_graph():
+    specs = mixed_model()
+    handle = ptwm_b200.ContainerHandle(oracle.write_container(specs, chunk_size=1000, menu=(oracle.HUFFMAN, oracle.RANS, oracle.O1SAC)), device=0)
+    plan, blob = handle.plan(None), handle.blob_on_device()
+    out = torch.zeros(plan.out_bytes, dtype=torch.uint8, device="cuda")
+    scratch = torch.empty(max(plan.scratch_bytes, 1), dtype=torch.uint8, device="cuda")
+    plan.run(blob, out, scratch)
+    want = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.run(blob, out, scratch, flags=ptwm_b200.NO_SYNC)
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        for k, s in enumerate(specs):
+            a = plan.out_offsets[k]
+            assert torch.equal(out[a:a + len(s.raw)], want[a:a + len(s.raw)]), s.name
