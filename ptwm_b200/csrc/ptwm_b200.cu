@@ -193,8 +193,8 @@ struct DevicePlan {
     void release(int dev) {
         for (auto& e : ev) if (e) cudaEventDestroy(e);
         for (auto& e : order) if (e) cudaEventDestroy(e);
+        if (!external) cudaFree(arena);  // waits for the plan's runs; the caller's memory outlives them by contract, and so must the word
         if (summary) give_word(dev, summary);
-        if (!external) cudaFree(arena);
         *this = DevicePlan{};
     }
 };
@@ -543,7 +543,10 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
     int64_t rc;
     int classes = 0;
     for (int cc = 0; cc < 4; ++cc) classes += !pl.runs[0][cc].empty() || !pl.runs[1][cc].empty();
-    if (timing || classes < 2) {  // one after the other
+    // A stream that is being captured gets its launches in a row too: the side streams belong to every thread of the device.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (classes >= 2) CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+    if (timing || classes < 2 || capture != cudaStreamCaptureStatusNone) {  // one after the other
         for (int ph = 0; ph < 2; ++ph) {
             for (int cc = 0; cc < 4; ++cc) {
                 if (pl.runs[ph][cc].empty()) continue;
@@ -561,6 +564,12 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         for (auto& e : d.order) if (!e) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         bool first = false, waiting = pl.merge_waits || !pl.posts.empty();
         for (int cc = 0; cc < 4; ++cc) { first |= !pl.runs[0][cc].empty(); for (auto& r : pl.runs[1][cc]) waiting |= r.waits; }
+        // whatever ends this early, nothing on a side stream outlives the call unseen by st
+        struct Join {
+            DeviceState& ds;
+            bool joined;
+            ~Join() { if (!joined) for (cudaStream_t s : ds.side) cudaStreamSynchronize(s); }
+        } join{ds, false};
         CUDA_TRY(cudaEventRecord(d.order[0], st));
         for (int cc = 3; cc >= 0; --cc) {
             if (pl.runs[0][cc].empty() && pl.runs[1][cc].empty()) continue;
@@ -587,6 +596,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
             CUDA_TRY(cudaEventRecord(d.order[5 + cc], ds.side[cc]));
             CUDA_TRY(cudaStreamWaitEvent(st, d.order[5 + cc], 0));
         }
+        join.joined = true;
     }
     CUDA_TRY(cudaMemcpyAsync(d.summary, d.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     if ((flags & PTWM_B200_VERIFY_CRC) && !pl.verify.empty()) {
