@@ -319,6 +319,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     uint64_t planes_bytes = 0, slots_bytes = 0, n_chunks64 = 0, tiles64 = 0;
     uint32_t n_or_words = 0;
     int most_planes = 1;
+    bool given_ops = false;  // some tensor brings a per-plane op of its own
     auto new_plane = [&](PlanePlan& pp, uint32_t row_len) {
         const uint64_t n = (pp.len + chunk_size - 1) / chunk_size;
         pp.buf_off = planes_bytes; pp.first_chunk = uint32_t(n_chunks64); pp.n_chunks = uint32_t(n);
@@ -362,6 +363,7 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
         if (opt.emit_payload_hash) hash_items.push_back(HashItem{make_ref(SP_BLOB, t.dev_ptr), t.nbytes});
         const bool split_kind = (kind == K_M16 || kind == K_M32) && plane_len;
         plan[i].post_op = t.post_op; plan[i].post_k = t.post_k;
+        given_ops |= t.post_op != 0;
         plan[i].has_delta = split_kind && (t.post_op == 1 || (!t.post_op && (opt.candidates & PTWM_B200_TRY_INTDELTA)));
         if (split_kind && (t.post_op == 2 || (!t.post_op && (opt.candidates & PTWM_B200_TRY_MZS)))) plan[i].try_mzs = ++n_or_words;
     }
@@ -391,7 +393,8 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
 
     prof("plan (host)");
     // ---- device pipeline: split, histograms ---------------------------------
-    const bool counted = opt.forced_codec != C_IDENTITY || opt.candidates;  // an Identity container needs no counts
+    // An Identity container needs no counts, unless an op on a plane is tried or given: those kernels count the new bytes, or move the counts.
+    const bool counted = opt.forced_codec != C_IDENTITY || opt.candidates || given_ops;
     Arena wa;
     const uint64_t a_planes = wa.add(planes_bytes + ENC_PAD), a_hist = wa.add(counted ? uint64_t(n_chunks) * 1024 : 0), a_plane_hist = wa.add(uint64_t(n_planes) * 256 * 8),
                    a_or = wa.add(uint64_t(n_or_words) * 4), a_acc = wa.add(uint64_t(n_planes) * 4), a_hashes = wa.add(hash_items.size() * 8),

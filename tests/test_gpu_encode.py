@@ -267,7 +267,7 @@ def _specs_of(tensors, post):
 
 
 @pytest.mark.parametrize("chunk", [8192, None])
-@pytest.mark.parametrize("codec", [None, RANS, TANS])
+@pytest.mark.parametrize("codec", [None, IDENTITY, RANS, TANS])
 def test_given_chains_bytes_equal_oracle(chunk, codec):
     host = _chain_model()
     given = {"smooth.bf16": ("intdelta",), "smooth.f32": ("intdelta",), "coarse.bf16": ("mzs", 4), "coarse.f16": ("mzs", 2), "coarse.f32": ("mzs", 6)}
