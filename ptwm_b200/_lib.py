@@ -13,7 +13,7 @@ import subprocess
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("PTWM_B200_LIB") or os.path.join(_HERE, "libptwm_b200.so")  # PTWM_B200_LIB: load another build of the same library
 _SOURCES = [os.path.join(_HERE, "csrc", f) for f in ("unity.cu", "ptwm_b200.cu", "encoder.cu", "kernels.cuh", "encode.cuh", "encode_tables.cuh", "noalloc.cu",
-                                                      "format.hpp", "host_common.hpp", "plan.h")] + [
+                                                      "format.hpp", "host_common.hpp", "slice_copy.hpp", "plan.h")] + [
     os.path.join(_HERE, "..", "include", "ptwm_b200.h")]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-pthread", "-shared"]

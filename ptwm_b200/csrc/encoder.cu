@@ -1134,11 +1134,13 @@ int64_t ptwm_b200_encoded_copy(const ptwm_b200_encoded* e, uint8_t* host_dst, si
     if (!e || !host_dst) return fail(PTWM_RC_INVALID_INPUT, "null argument");
     if (cap < e->size) return fail(PTWM_RC_BUFFER_TOO_SMALL, "host buffer smaller than the container");
     DeviceGuard guard{e->device};
-    DeviceState* ds;
-    int64_t rc = device_state(e->device, &ds);
-    if (rc < 0) return rc;
-    if ((rc = copy_to_host(host_dst, e->out.as<uint8_t>(), e->size, *ds)) < 0) return rc;
-    return int64_t(e->size);
+    try {
+        DeviceState* ds;
+        int64_t rc = device_state(e->device, &ds);
+        if (rc < 0) return rc;
+        if ((rc = copy_to_host(host_dst, e->out.as<uint8_t>(), e->size, *ds)) < 0) return rc;
+        return int64_t(e->size);
+    } catch (const std::exception& ex) { return fail(PTWM_RC_INTERNAL, ex.what()); }
 }
 int64_t ptwm_b200_encoded_copy_to_device(const ptwm_b200_encoded* e, uint64_t dst_dev_ptr, uint64_t cap, uint64_t stream) {
     if (!e || !dst_dev_ptr) return fail(PTWM_RC_INVALID_INPUT, "null argument");

@@ -4,17 +4,17 @@
 #include <sys/mman.h>
 
 #include <algorithm>
-#include <condition_variable>
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "format.hpp"
 #include "host_common.hpp"
+#include "slice_copy.hpp"
 
 using namespace ptwm;
 
@@ -71,49 +71,23 @@ int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds
         ~Events() { for (auto e : ev) if (e) cudaEventDestroy(e); }
     } events;
     for (auto& e : events.ev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    const size_t slices = (n + SLICE - 1) / SLICE;
     uint8_t* stage = static_cast<uint8_t*>(ds.stage);
-    std::mutex mu;
-    std::condition_variable cv;
-    size_t sent = 0;                       // slices handed to the copy engine
-    std::vector<char> moved(slices, 0);    // slices that have left the staging buffer
-    cudaError_t failed = cudaSuccess;
+    std::atomic<cudaError_t> failed{cudaSuccess};
+    auto ok = [&](cudaError_t e) { if (e != cudaSuccess) failed = e; return e == cudaSuccess; };
     int device = 0;
     CUDA_TRY(cudaGetDevice(&device));
-    auto worker = [&](size_t first, size_t step) {
-        cudaSetDevice(device);
-        for (size_t k = first; k < slices; k += step) {
-            {
-                std::unique_lock<std::mutex> l(mu);
-                cv.wait(l, [&] { return sent > k || failed != cudaSuccess; });
-                if (failed != cudaSuccess) return;
-            }
-            const cudaError_t e = cudaEventSynchronize(events.ev[k % RING]);
-            if (e == cudaSuccess) std::memcpy(dst + k * SLICE, stage + (k % RING) * SLICE, std::min(SLICE, n - k * SLICE));
-            std::lock_guard<std::mutex> l(mu);
-            if (e != cudaSuccess) failed = e;
-            moved[k] = 1;
-            cv.notify_all();
-        }
-    };
-    const size_t n_threads = std::min<size_t>(slices, 4);
-    std::vector<std::thread> threads;
-    for (size_t t = 0; t < n_threads; ++t) threads.emplace_back(worker, t, n_threads);
-    for (size_t k = 0; k < slices; ++k) {
-        if (k >= RING) {
-            std::unique_lock<std::mutex> l(mu);
-            cv.wait(l, [&] { return moved[k - RING] || failed != cudaSuccess; });
-        }
-        cudaError_t e = cudaMemcpyAsync(stage + (k % RING) * SLICE, src + k * SLICE, std::min(SLICE, n - k * SLICE), cudaMemcpyDeviceToHost, ds.stream);
-        if (e == cudaSuccess) e = cudaEventRecord(events.ev[k % RING], ds.stream);
-        std::lock_guard<std::mutex> l(mu);
-        if (e != cudaSuccess) failed = e;
-        sent = k + 1;
-        cv.notify_all();
-        if (failed != cudaSuccess) break;
+    const Moved m = move_slices(
+        dst, stage, n, SLICE, RING, 4,
+        [&](size_t k) {
+            return ok(cudaMemcpyAsync(stage + (k % RING) * SLICE, src + k * SLICE, std::min(SLICE, n - k * SLICE), cudaMemcpyDeviceToHost, ds.stream)) &&
+                   ok(cudaEventRecord(events.ev[k % RING], ds.stream));
+        },
+        [&](size_t k) { return ok(cudaSetDevice(device)) && ok(cudaEventSynchronize(events.ev[k % RING])); });
+    if (m == Moved::no_threads) {  // the driver's own copy then
+        CUDA_TRY(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, ds.stream));
+        CUDA_TRY(cudaStreamSynchronize(ds.stream));
     }
-    for (auto& t : threads) t.join();
-    CUDA_TRY(failed);
+    CUDA_TRY(failed.load());
     return 0;
 }
 
