@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -38,13 +39,16 @@ struct DeviceState {
     std::vector<uint32_t*> words;    // free words of pinned memory, one for every plan that has run (its status summary)
     void* stage = nullptr;           // pinned host buffer the plan work lists pass through on their way to the device
     size_t stage_cap = 0;
+    std::mutex copy_mu;              // for the two below: containers on their way to host memory (copy_to_host)
+    uint8_t* copy_stage = nullptr;
+    cudaStream_t copy_stream = nullptr;
 };
 
 // Caller holds a DeviceGuard for `dev`.
 int64_t device_state(int dev, DeviceState** out);
 const CrcTables& crc_tables();
 
-// Device bytes into ordinary host memory (`src` complete, or ordered before ds.stream).
+// Device bytes into ordinary host memory; what writes them has completed.
 int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds);
 
 inline uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }

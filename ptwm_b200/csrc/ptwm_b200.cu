@@ -37,41 +37,36 @@ CrcTables host_crc_tables() {
     for (int k = 0; k < 64; ++k) { t.x2n[k] = p; p = gf2_mulmod(p, p); }
     return t;
 }
-std::mutex g_stage_mu;  // one staging buffer per device, used under this lock
-// Caller holds the lock.
-int64_t stage_reserve(DeviceState& ds, size_t bytes) {
-    if (ds.stage_cap >= bytes) return 0;
-    // grows only on the first large plan of a process: pinning synchronises with the device
-    if (ds.stage) CUDA_TRY(cudaFreeHost(ds.stage));
-    ds.stage = nullptr; ds.stage_cap = 0;
-    const size_t cap = std::max<size_t>(bytes + bytes / 2, size_t(32) << 20);
-    CUDA_TRY(cudaMallocHost(&ds.stage, cap));
-    ds.stage_cap = cap;
-    return 0;
-}
 }  // namespace
 
-// Through the pinned staging buffer in slices: the copy engine fills slice k + 4 while host threads move slice k on.  A copy
+// Through a pinned staging buffer in slices: the copy engine fills slice k + 4 while host threads move slice k on.  A copy
 // into pageable memory by the driver runs at 5 - 10 GB/s, and memory nobody has touched yet costs a page fault per 4 KiB on
-// top of that, so the slices are taken by four threads, on huge pages where the system grants them.
+// top of that, so the slices are taken by four threads, on huge pages where the system grants them.  Buffer, stream and lock are
+// this function's own (16 MiB per device, kept for the process): a container of some GB is on its way for a tenth of a second,
+// and no plan that another thread sends to the device waits for that.
 int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds) {
     constexpr size_t SLICE = size_t(2) << 20, RING = 8;
-    if (n < SLICE) {
+    auto by_driver = [&]() -> int64_t {
         CUDA_TRY(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, ds.stream));
         CUDA_TRY(cudaStreamSynchronize(ds.stream));
         return 0;
-    }
+    };
+    if (n < SLICE) return by_driver();
     const uintptr_t page = uintptr_t(1) << 21, lo = (reinterpret_cast<uintptr_t>(dst) + page - 1) & ~(page - 1), hi = (reinterpret_cast<uintptr_t>(dst) + n) & ~(page - 1);
     if (hi > lo) madvise(reinterpret_cast<void*>(lo), hi - lo, MADV_HUGEPAGE);  // a hint; refused is fine
-    std::lock_guard<std::mutex> g(g_stage_mu);
-    int64_t rc = stage_reserve(ds, SLICE * RING);
-    if (rc < 0) return rc;
+    std::lock_guard<std::mutex> g(ds.copy_mu);
+    if (!ds.copy_stream) CUDA_TRY(cudaStreamCreateWithFlags(&ds.copy_stream, cudaStreamNonBlocking));
+    if (!ds.copy_stage && cudaMallocHost(&ds.copy_stage, SLICE * RING) != cudaSuccess) {
+        ds.copy_stage = nullptr;
+        cudaGetLastError();  // answered here: not the next launch's
+        return by_driver();
+    }
+    uint8_t* stage = ds.copy_stage;
     struct Events {
         cudaEvent_t ev[RING] = {nullptr};
         ~Events() { for (auto e : ev) if (e) cudaEventDestroy(e); }
     } events;
     for (auto& e : events.ev) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    uint8_t* stage = static_cast<uint8_t*>(ds.stage);
     std::atomic<cudaError_t> failed{cudaSuccess};
     auto ok = [&](cudaError_t e) { if (e != cudaSuccess) failed = e; return e == cudaSuccess; };
     int device = 0;
@@ -79,14 +74,12 @@ int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds
     const Moved m = move_slices(
         dst, stage, n, SLICE, RING, 4,
         [&](size_t k) {
-            return ok(cudaMemcpyAsync(stage + (k % RING) * SLICE, src + k * SLICE, std::min(SLICE, n - k * SLICE), cudaMemcpyDeviceToHost, ds.stream)) &&
-                   ok(cudaEventRecord(events.ev[k % RING], ds.stream));
+            return ok(cudaMemcpyAsync(stage + (k % RING) * SLICE, src + k * SLICE, std::min(SLICE, n - k * SLICE), cudaMemcpyDeviceToHost, ds.copy_stream)) &&
+                   ok(cudaEventRecord(events.ev[k % RING], ds.copy_stream));
         },
         [&](size_t k) { return ok(cudaSetDevice(device)) && ok(cudaEventSynchronize(events.ev[k % RING])); });
-    if (m == Moved::no_threads) {  // the driver's own copy then
-        CUDA_TRY(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, ds.stream));
-        CUDA_TRY(cudaStreamSynchronize(ds.stream));
-    }
+    if (m == Moved::no_threads) return by_driver();
+    if (m == Moved::failed) cudaStreamSynchronize(ds.copy_stream);  // the next call fills the same slots
     CUDA_TRY(failed.load());
     return 0;
 }
@@ -390,13 +383,19 @@ void finish_lists(ptwm_b200_plan& pl) {
 // host-to-device copy: a caller that streams a container to the GPU has tens of large copies queued on the copy
 // engine, and a small copy issued now would only run after all of them (the plan of the first piece would be ready
 // when the last byte of the container has arrived).  The kernel runs on the library's stream beside those copies.
+std::mutex g_stage_mu;  // one staging buffer per device, used under this lock
 template <class T>
 int64_t upload(T* dst, const std::vector<T>& v, DeviceState& ds) {
     if (v.empty()) return 0;
     const size_t bytes = v.size() * sizeof(T), padded = (bytes + 15) & ~size_t(15);
     std::lock_guard<std::mutex> g(g_stage_mu);
-    const int64_t rc = stage_reserve(ds, padded);
-    if (rc < 0) return rc;
+    if (ds.stage_cap < padded) {  // grows only on the first large plan of a process: pinning synchronises with the device
+        if (ds.stage) CUDA_TRY(cudaFreeHost(ds.stage));
+        ds.stage = nullptr; ds.stage_cap = 0;
+        const size_t cap = std::max<size_t>(padded + padded / 2, size_t(32) << 20);
+        CUDA_TRY(cudaMallocHost(&ds.stage, cap));
+        ds.stage_cap = cap;
+    }
     std::memcpy(ds.stage, v.data(), bytes);
     const size_t n16 = padded / 16;
     stage_in_kernel<<<unsigned(std::min<size_t>((n16 + 255) / 256, 1184)), 256, 0, ds.stream>>>(static_cast<const uint4*>(ds.stage), reinterpret_cast<uint4*>(dst), n16);

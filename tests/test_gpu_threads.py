@@ -1,0 +1,41 @@
+"""Calls from several threads of one process: no call waits for another's copy, and every one gets its own bytes."""
+import threading
+import time
+
+import pytest
+import torch
+
+import oracle
+import ptwm_b200
+from ptwm_b200.compressor import CompressionConfig, IDENTITY, compress_model
+from _data import mixed_model
+
+pytestmark = pytest.mark.gpu
+
+
+def test_plans_reach_the_device_while_a_container_is_copied_to_the_host():
+    big = torch.randint(0, 256, (768 << 20,), dtype=torch.uint8, device="cuda")
+    enc = compress_model({"w": big}, CompressionConfig(streaming_chunk=None, forced_codec=IDENTITY))
+    enc.to_bytes()  # staging memory and threads are there
+    handle = ptwm_b200.ContainerHandle(oracle.write_container(mixed_model(), chunk_size=4096), device=0)
+    ptwm_b200.DecodePlan(handle).prepare(0)
+    data, span = [], []
+
+    def copy():
+        span.append(time.perf_counter())
+        data.append(enc.to_bytes())
+        span.append(time.perf_counter())
+
+    done = []
+    t = threading.Thread(target=copy)
+    t.start()
+    while t.is_alive():
+        began = time.perf_counter()
+        ptwm_b200.DecodePlan(handle).prepare(0)
+        done.append((began, time.perf_counter()))
+    t.join()
+    # a plan takes well under a millisecond, the copy some fifty
+    assert sum(span[0] <= a and b <= span[1] for a, b in done) >= 10
+    assert torch.equal(torch.frombuffer(bytearray(data[0]), dtype=torch.uint8)[-(1 << 20):], enc.to_tensor()[-(1 << 20):].cpu())
+    raw = ptwm_b200.ContainerHandle(data[0], device=0).decode("w")
+    assert torch.equal(raw, big)
