@@ -157,11 +157,16 @@ struct DevicePlan {
     bool timed[12] = {false};
     uint8_t* arena = nullptr;          // everything above lives in this one block
     bool external = false;             // the block belongs to the caller (ptwm_b200_plan_prepare_in)
+    cudaEvent_t written = nullptr;     // external: the last run has written the summary
+    bool captured = false;             // external: a graph holds a run, which may write the summary at any time
     void release(int dev) {
         for (auto& e : ev) if (e) cudaEventDestroy(e);
         for (auto& e : order) if (e) cudaEventDestroy(e);
-        if (!external) cudaFree(arena);  // waits for the plan's runs; the caller's memory outlives them by contract, and so must the word
-        if (summary) give_word(dev, summary);
+        // The word goes to another plan: nothing of this one's may write to it any more.  cudaFree waits for the plan's runs; the
+        // caller's memory outlives them by contract, so they are waited for here, and a word in a graph is never given back.
+        if (!external) cudaFree(arena);
+        if (written) { cudaEventSynchronize(written); cudaEventDestroy(written); }
+        if (summary && !captured) give_word(dev, summary);
         *this = DevicePlan{};
     }
 };
@@ -572,6 +577,14 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         join.joined = true;
     }
     CUDA_TRY(cudaMemcpyAsync(d.summary, d.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    if (d.external) {
+        CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+        if (capture != cudaStreamCaptureStatusNone) d.captured = true;
+        else {
+            if (!d.written) CUDA_TRY(cudaEventCreateWithFlags(&d.written, cudaEventDisableTiming));
+            CUDA_TRY(cudaEventRecord(d.written, st));
+        }
+    }
     if ((flags & PTWM_B200_VERIFY_CRC) && !pl.verify.empty()) {
         CUDA_TRY(cudaMemsetAsync(d.acc, 0, (pl.n_acc + 1) * sizeof(uint32_t), st));
         uint64_t blocks = (pl.n_runs + 127) / 128;

@@ -1,4 +1,5 @@
-"""Calls from several threads of one process: no call waits for another's copy, and every one gets its own bytes."""
+"""Calls from several threads and on several streams of one process: no call waits for another's copy, and every one gets its
+own bytes and its own verdict."""
 import threading
 import time
 
@@ -39,3 +40,30 @@ def test_plans_reach_the_device_while_a_container_is_copied_to_the_host():
     assert torch.equal(torch.frombuffer(bytearray(data[0]), dtype=torch.uint8)[-(1 << 20):], enc.to_tensor()[-(1 << 20):].cpu())
     raw = ptwm_b200.ContainerHandle(data[0], device=0).decode("w")
     assert torch.equal(raw, big)
+
+
+def test_a_plan_dropped_in_flight_does_not_answer_for_the_next_one():
+    blob = oracle.write_container(mixed_model(), chunk_size=4096, forced_codec=oracle.RANS)
+    handle = ptwm_b200.ContainerHandle(blob, device=0)
+    handle.decode_model()  # every kernel is loaded: a load waits for the device
+    resident = handle.blob_on_device()
+    damaged = torch.zeros_like(resident)  # no valid header in it
+    first, second = ptwm_b200.DecodePlan(handle), ptwm_b200.DecodePlan(handle)
+    out, out2 = (torch.empty(first.out_bytes, dtype=torch.uint8, device="cuda") for _ in range(2))
+    scratch, scratch2 = (torch.empty(max(first.scratch_bytes, 1), dtype=torch.uint8, device="cuda") for _ in range(2))
+    first.prepare(0)
+    memory = first._dev_mem  # of the runs, kept until they are over
+    slow, fast = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(slow):
+        torch.cuda._sleep(1_000_000_000)  # half a second
+        first.run(resident, out, scratch, flags=ptwm_b200.NO_SYNC)
+    del first
+    second.prepare(0)
+    with torch.cuda.stream(fast):
+        second.run(damaged, out2, scratch2, flags=ptwm_b200.NO_SYNC)
+    slow.synchronize()
+    with torch.cuda.stream(fast), pytest.raises(ptwm_b200.PtwmError):
+        second.finish(0)
+    del memory
