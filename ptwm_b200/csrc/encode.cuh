@@ -776,7 +776,6 @@ __global__ void __launch_bounds__(128) huffman_encode_kernel(const EncChunk* __r
 // the state the serial coder has there.  The state a lane leaves in is where the lane below must start: lanes whose start
 // was not that go again until nobody's changes.  Each round settles at least one more lane, so the worst case is the serial
 // chain.  A last pass writes the bits at the places the runs' bit counts give.
-constexpr uint32_t TENC_MIN_RUN = 256;  // shorter runs would hardly ever end in the right state
 __global__ void __launch_bounds__(32) tans_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
                                                          const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
                                                          EncResult* __restrict__ results) {
@@ -823,8 +822,7 @@ __global__ void __launch_bounds__(32) tans_encode_kernel(const EncChunk* __restr
         }
     }
     const uintptr_t base = reinterpret_cast<uintptr_t>(planes + c.plane_off);
-    uint32_t per = (c.n + 31) / 32;
-    if (per < TENC_MIN_RUN) per = TENC_MIN_RUN;
+    const uint32_t per = tans_encode_run(c.n);
     const uint64_t first = uint64_t(lane) * per;
     const uint32_t r_lo = first < c.n ? uint32_t(first) : c.n, r_hi = first + per < c.n ? uint32_t(first + per) : c.n;
     auto entry = [&](uint32_t b) { return sym[b]; };

@@ -138,4 +138,11 @@ inline int huffman_lengths(const unsigned long long* raw, uint8_t* lengths) {
     return last + 1;
 }
 
+// tANS: symbols per lane when a warp codes a chunk of n.  Any 32-bit n: the lanes' runs cover it.
+constexpr uint32_t TENC_MIN_RUN = 256;  // shorter runs would hardly ever end in the right state
+__host__ __device__ inline uint32_t tans_encode_run(uint32_t n) {
+    const uint32_t per = n / 32 + (n % 32 != 0);
+    return per < TENC_MIN_RUN ? TENC_MIN_RUN : per;
+}
+
 }  // namespace ptwm
