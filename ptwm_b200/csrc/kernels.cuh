@@ -1335,7 +1335,10 @@ __global__ void __launch_bounds__(THREADS) tans_decode_kernel(const DecodeItem* 
         if (l == 0) sh.built = ok;
     }
     tans_sync<THREADS>();
-    uint32_t err = bad || !sh.built ? uint32_t(ST_BAD_HEADER) : total_bits < 11 ? uint32_t(ST_STREAM_UNDERRUN) : uint32_t(ST_OK);
+    // A symbol takes at most eleven bits, and so does the first state: what is longer cannot be used up.  (Lane positions are 32-bit
+    // offsets: without this a stream of more than 2^32 bits for few symbols would come out right modulo 2^32.)
+    uint32_t err = bad || !sh.built ? uint32_t(ST_BAD_HEADER) : total_bits < 11 ? uint32_t(ST_STREAM_UNDERRUN)
+                 : total_bits > 11 * (uint64_t(it.n) + 1) ? uint32_t(ST_NOT_CONSUMED) : uint32_t(ST_OK);
     if (err) { if (l == 0) report(status, it.id, err); return; }
 
     // ---- runs ----

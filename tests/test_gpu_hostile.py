@@ -8,6 +8,7 @@ import torch
 
 import oracle
 import ptwm_b200
+from ptwm_b200 import _lib
 from _data import spec_bf16, specs_fp8
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +50,26 @@ def test_truncated_container_is_refused():
     for cut in (10, len(blob) // 2, len(blob) - 1):
         with pytest.raises((ptwm_b200.PtwmError, ValueError)):
             ptwm_b200.ContainerHandle(blob[:cut], device=0)
+
+
+def test_tans_stream_of_more_than_2_32_bits_for_few_symbols_is_refused():
+    # as the right stream modulo 2^32 bits: its symbols at the bottom, the first state at the top, 512 MiB of nothing between them
+    plane = bytes(7 if i % 9 == 0 else 200 for i in range(400))
+    _, _, payload = oracle.plane_encode(oracle.TANS, plane)
+    assert payload[0] == 1 and payload[5] == 11
+    at = 5 + 3 + 3 * int.from_bytes(payload[6:8], "little")
+    bits = int.from_bytes(payload[at:at + 8], "little")
+    stream = int.from_bytes(payload[at + 8:], "little")
+    state, top = stream >> (bits - 11), 2**32 + bits - 11
+    src = torch.zeros(at + 8 + (2**32 + bits + 7) // 8, dtype=torch.uint8, device="cuda")
+    put = lambda pos, raw: src[pos:pos + len(raw)].copy_(torch.frombuffer(bytearray(raw), dtype=torch.uint8))
+    put(0, payload[:at] + (2**32 + bits).to_bytes(8, "little"))
+    low = stream & ((1 << (bits - 11)) - 1)
+    put(at + 8, low.to_bytes((bits + 7) // 8, "little"))
+    high = (state << (top % 8)).to_bytes(3, "little")
+    put(at + 8 + top // 8, high[:src.numel() - at - 8 - top // 8])
+    out = torch.zeros(len(plane), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    rc = _lib.lib().ptwm_hardware_backend_v1_dispatch_decode_cuda(0, None, 0, bytes.fromhex("e4868545e7b22282695972441494e70569ab27595d19349114e852125d96daa4"), 32,
+                                                                  src.data_ptr(), src.numel(), out.data_ptr(), out.numel(), 0)
+    assert rc == -8, rc
