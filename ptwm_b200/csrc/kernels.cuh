@@ -1473,25 +1473,47 @@ __global__ void __launch_bounds__(THREADS) tans_decode_kernel(const DecodeItem* 
         return n;
     };
     const bool inner = l + 1 < runs;  // the last run's symbols are what is left of the chunk's
-    uint32_t from = 0, mine = 0, end = 0;
+    uint32_t from = 0, end = 0;
+    uint64_t mine = 0;
     if (l == 0) {  // run 0 starts behind the eleven bits of the first state
         const uint64_t bit = total_bits - 11;
         const uint8_t* b = bs + (bit >> 3);
         const uint32_t three = uint32_t(b[0]) | uint32_t(b[1]) << 8 | ((bit & 7) > 5 ? uint32_t(b[2]) << 16 : 0u);
         from = 11u << 11 | ((three >> (bit & 7)) & 2047u);
     }
-    for (bool go = inner;;) {
-        if (go) { mine = walk(from); end = (end_at - at) << 11 | state_now(); }
+    // In round r the start of lane r is the right one at the latest.  A damaged or very uneven stream can hold the whole chunk's symbols, or
+    // more, in any run: a warp walks as many steps as the chunk has symbols from starts that may still change, and from then on a
+    // lane waits for its right one; and once the runs with right starts hold more symbols than the chunk, it is refused.  All
+    // of that together is at most a few times the chunk's symbols.
+    uint32_t spent = 0;
+    uint64_t settled = 0;
+    bool too_many = false;
+    bool go = inner;
+    for (uint32_t round = 0;; ++round) {
+        uint32_t met = 0;
+        if (go && (l <= round || spent < it.n)) {
+            met = walk(from);
+            mine = uint64_t(met) + (int32_t(at - end_at) > 0);  // still above the run's end: the bits of more symbols than the chunk has
+            end = (end_at - at) << 11 | state_now();
+            go = false;
+        }
+        met = __reduce_max_sync(0xFFFFFFFFu, met);
+        spent = met > it.n - spent ? it.n : spent + met;
+        const uint32_t sure = round < runs ? round : runs - 1;
         uint32_t want;
-        if (THREADS == 32) want = __shfl_up_sync(0xFFFFFFFFu, end, 1);
-        else {
-            sh.words[l] = end;
+        if (THREADS == 32) {
+            want = __shfl_up_sync(0xFFFFFFFFu, end, 1);
+            if (round < runs) settled += __shfl_sync(0xFFFFFFFFu, mine, sure);
+        } else {
+            sh.words[l] = mine << 32 | end;
             __syncthreads();
             want = l ? uint32_t(sh.words[l - 1]) : 0u;
+            if (round < runs) settled += sh.words[sure] >> 32;
         }
+        too_many = settled > it.n;
         const bool moved = l > 0 && l < runs && want != from;
         if (moved) from = want;
-        go = moved && inner;
+        go = (go || moved) && inner && !too_many;
         if (THREADS == 32 ? !__any_sync(0xFFFFFFFFu, go) : !__syncthreads_or(go)) break;
     }
     // where the lane's symbols go: the counts of the lanes before it
@@ -1513,12 +1535,12 @@ __global__ void __launch_bounds__(THREADS) tans_decode_kernel(const DecodeItem* 
             }
         }
     }
-    if (all > it.n) err = ST_NOT_CONSUMED;  // more symbols than the chunk has before its last run
+    if (too_many || all > it.n) err = ST_NOT_CONSUMED;  // more symbols than the chunk has before its last run
     if (!err && l < runs) {
         // ---- last pass: the symbols to their places ----
         const Epilogue ep = make_epilogue(bases, it);
         const bool last = l + 1 == runs;
-        uint32_t pos = uint32_t(before_me), remaining = last ? it.n - uint32_t(all) : mine;
+        uint32_t pos = uint32_t(before_me), remaining = last ? it.n - uint32_t(all) : uint32_t(mine);
         // the last run may not read below the stream's first bit; the others are known to end well above theirs
         const uint32_t floor_at = last ? end_at : end_at - 11 - TANS_GROUP_BITS;
         begin(start_at - (from >> 11), from & 2047u);

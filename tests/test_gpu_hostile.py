@@ -2,6 +2,8 @@
 fault: every decode loop is bounded by the symbol count and every read is
 clamped to the resident blob.  Mirrors the reference's accepted outcomes
 (tests/ptwm/core/test_decompressor_errors.py:35-77)."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -68,8 +70,26 @@ def test_tans_stream_of_more_than_2_32_bits_for_few_symbols_is_refused():
     put(at + 8, low.to_bytes((bits + 7) // 8, "little"))
     high = (state << (top % 8)).to_bytes(3, "little")
     put(at + 8 + top // 8, high[:src.numel() - at - 8 - top // 8])
-    out = torch.zeros(len(plane), dtype=torch.uint8, device="cuda")
+    assert _plane_decode_tans(src, len(plane)) == -8
+
+
+def _plane_decode_tans(src, n):
+    out = torch.zeros(n, dtype=torch.uint8, device="cuda")
     torch.cuda.synchronize()
-    rc = _lib.lib().ptwm_hardware_backend_v1_dispatch_decode_cuda(0, None, 0, bytes.fromhex("e4868545e7b22282695972441494e70569ab27595d19349114e852125d96daa4"), 32,
-                                                                  src.data_ptr(), src.numel(), out.data_ptr(), out.numel(), 0)
-    assert rc == -8, rc
+    return _lib.lib().ptwm_hardware_backend_v1_dispatch_decode_cuda(0, None, 0, bytes.fromhex("e4868545e7b22282695972441494e70569ab27595d19349114e852125d96daa4"), 32,
+                                                                    src.data_ptr(), src.numel(), out.data_ptr(), n, 0)
+
+
+def test_tans_stream_with_far_more_symbols_than_declared_is_refused_in_the_time_of_a_few_chunks():
+    # a stream of ones under this table: runs of some 56,000 symbols each that never fall in with one another; one lane walks 64 Ki
+    # symbols in 3 ms at most
+    n, bits = 1 << 16, 312557
+    table = b"".join(bytes([sym]) + freq.to_bytes(2, "little") for sym, freq in enumerate((2039, 3, 2, 4)))
+    blob = bytes([11]) + (4).to_bytes(2, "little") + table + bits.to_bytes(8, "little") + b"\xff" * ((bits + 7) // 8)
+    src = torch.frombuffer(bytearray(b"\x01" + n.to_bytes(4, "little") + blob), dtype=torch.uint8).cuda()
+    took = []
+    for _ in range(3):
+        began = time.perf_counter()
+        assert _plane_decode_tans(src, n) == -8
+        took.append(time.perf_counter() - began)
+    assert min(took) < 0.03, took
