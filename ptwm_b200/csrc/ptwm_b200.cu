@@ -201,6 +201,9 @@ struct ptwm_b200_plan {
     // tables of a chunk for Order1ScaleAC.
     struct Launch { uint32_t first, count, size; bool waits, narrow; };
     std::vector<Launch> runs[2][4];
+    // The same lists for launches in a row on one stream, where the items that wait have nothing to be kept apart from: a few of
+    // them in a launch of their own are one more serial chain that the whole pass waits for.
+    std::vector<Launch> in_row[2][4];
     bool merge_waits = false;  // a final merge reads scratch
     bool spread = false;       // few chunks: every coded plane to scratch at once, then a merge (see ptwm_b200_plan_create)
     uint64_t slot_bytes[12] = {0};
@@ -331,20 +334,27 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
     }
 }
 
+int codec_classes(const ptwm_b200_plan& pl) {
+    int n = 0;
+    for (int cc = 0; cc < 4; ++cc) n += !pl.dec[0][cc].empty() || !pl.dec[1][cc].empty();
+    return n;
+}
+
 void finish_lists(ptwm_b200_plan& pl) {
+    const bool side_by_side = codec_classes(pl) >= 2;
     for (int ph = 0; ph < 2; ++ph) {
         for (int cc = 0; cc < 4; ++cc) {
             auto& v = pl.dec[ph][cc];
             const bool direct = v.size() <= RANS_DIRECT_CHUNKS;  // one kernel for any alphabet
             auto narrow = [cc, direct](const DecodeItem& a) { return cc == 0 && !direct && (a.row_len >> 16) <= RANS_NARROW_SYMBOLS; };
-            auto waits = [ph](const DecodeItem& a) {
-                if (ph == 0) return false;
+            auto waits = [ph, side_by_side](const DecodeItem& a) {
+                if (ph == 0 || !side_by_side) return false;
                 for (Ref r : a.partner) if (r != REF_NONE && (r >> 62) == SP_SCRATCH) return true;
                 return false;
             };
-            // by launch (waiting or not, narrow or not), the longest chunks first; most lists are in that order already
+            // by launch (narrow or not, waiting or not), the longest chunks first; most lists are in that order already
             std::vector<std::pair<uint64_t, uint32_t>> order(v.size());
-            for (size_t k = 0; k < v.size(); ++k) order[k] = {uint64_t(2 * waits(v[k]) + !narrow(v[k])) << 32 | (0xFFFFFFFFu - v[k].n), uint32_t(k)};
+            for (size_t k = 0; k < v.size(); ++k) order[k] = {uint64_t(2 * !narrow(v[k]) + waits(v[k])) << 32 | (0xFFFFFFFFu - v[k].n), uint32_t(k)};
             if (!std::is_sorted(order.begin(), order.end())) {
                 std::sort(order.begin(), order.end());  // equal keys by place in the list
                 std::vector<DecodeItem> sorted;
@@ -355,12 +365,17 @@ void finish_lists(ptwm_b200_plan& pl) {
             const int slot = ph * 5 + cc;
             pl.slot_items[slot] = uint32_t(v.size());
             for (size_t k = 0; k < v.size(); ++k) {
-                const bool w = order[k].first >> 33, nw = !(order[k].first >> 32 & 1);
-                auto& runs = pl.runs[ph][cc];
-                if (runs.empty() || runs.back().waits != w || runs.back().narrow != nw) { runs.push_back({uint32_t(k), 0, 0, w, nw}); pl.launches++; }
-                runs.back().count++;
-                runs.back().size = std::max(runs.back().size, cc == 0 ? v[k].row_len >> 16 : cc == 3 ? o1sac_tables(v[k].state_len) : 0u);
+                const bool nw = !(order[k].first >> 33), w = order[k].first >> 32 & 1;
+                const uint32_t size = cc == 0 ? v[k].row_len >> 16 : cc == 3 ? o1sac_tables(v[k].state_len) : 0u;
+                auto add = [&](std::vector<ptwm_b200_plan::Launch>& to, bool cut) {
+                    if (to.empty() || to.back().narrow != nw || (cut && to.back().waits != w)) to.push_back({uint32_t(k), 0, 0, w, nw});
+                    to.back().count++;
+                    to.back().size = std::max(to.back().size, size);
+                };
+                add(pl.runs[ph][cc], true);
+                add(pl.in_row[ph][cc], false);
             }
+            pl.launches += uint32_t((side_by_side ? pl.runs : pl.in_row)[ph][cc].size());
             for (auto& it : v) {
                 uint64_t np = it.fused ? uint64_t(kind_planes(it.kind)) : 1, eb = it.fused ? uint64_t(kind_elem_bytes(it.kind)) : 1;
                 pl.slot_bytes[slot] += uint64_t(it.src_len) + it.state_len + uint64_t(it.n) * (np - 1) + uint64_t(it.n) * eb;
@@ -483,6 +498,10 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         CUDA_TRY(cudaGetLastError());
         return 0;
     };
+    auto launch_all = [&](int ph, int cc) -> int64_t {
+        for (auto& r : pl.in_row[ph][cc]) { const int64_t rc = launch(ph, cc, r, st); if (rc < 0) return rc; }
+        return 0;
+    };
     auto launch_class = [&](int ph, int cc, bool waiting, cudaStream_t s) -> int64_t {
         for (auto& r : pl.runs[ph][cc]) if (r.waits == waiting) { const int64_t rc = launch(ph, cc, r, s); if (rc < 0) return rc; }
         return 0;
@@ -519,8 +538,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         return 0;
     };
     int64_t rc;
-    int classes = 0;
-    for (int cc = 0; cc < 4; ++cc) classes += !pl.runs[0][cc].empty() || !pl.runs[1][cc].empty();
+    const int classes = codec_classes(pl);
     // A stream that is being captured gets its launches in a row too: the side streams belong to every thread of the device.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (classes >= 2) CUDA_TRY(cudaStreamIsCapturing(st, &capture));
@@ -529,7 +547,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
             for (int cc = 0; cc < 4; ++cc) {
                 if (pl.runs[ph][cc].empty()) continue;
                 CUDA_TRY(mark(ph * 5 + cc, 0));
-                if ((rc = launch_class(ph, cc, false, st)) < 0 || (rc = launch_class(ph, cc, true, st)) < 0) return rc;
+                if ((rc = launch_all(ph, cc)) < 0) return rc;
                 CUDA_TRY(mark(ph * 5 + cc, 1));
             }
             if (ph == 0 && ((rc = launch_merges(0)) < 0 || (rc = launch_posts()) < 0)) return rc;
@@ -540,8 +558,8 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         // merge: every codec has a stream of its own, the ones with the longest serial chains first.  One after the other the four
         // kernels of a microscaling layer took 9.5 ms, 6.4 of them an Order1ScaleAC launch that leaves the GPU nearly idle.
         for (auto& e : d.order) if (!e) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        bool first = false, waiting = pl.merge_waits || !pl.posts.empty();
-        for (int cc = 0; cc < 4; ++cc) { first |= !pl.runs[0][cc].empty(); for (auto& r : pl.runs[1][cc]) waiting |= r.waits; }
+        bool waiting = pl.merge_waits || !pl.posts.empty();
+        for (int cc = 0; cc < 4; ++cc) for (auto& r : pl.runs[1][cc]) waiting |= r.waits;
         // whatever ends this early, nothing on a side stream outlives the call unseen by st
         struct Join {
             DeviceState& ds;

@@ -14,6 +14,7 @@ import oracle
 import ptwm_b200
 from ptwm_b200 import _lib
 from ptwm_b200.sharding import contiguous_shards, shard_for_rank
+from _data import spec_bf16, spec_norm
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 GOLD = os.path.join(ROOT, "tests", "golden")
@@ -335,3 +336,25 @@ def test_shared_state_fit_on_the_host(L):
     assert states[0] == oracle.plane_encode(oracle.O1SAC, planes[0] + planes[2] + planes[4], 256)[0]
     assert states[1] == oracle.plane_encode(oracle.O1SAC, planes[1] + planes[3] + planes[5], 256)[0]
     assert _lib.fit_shared_states_host([], []) == []
+
+
+@pytest.mark.parametrize("codec,chunk", [(oracle.RANS, 1024), (oracle.HUFFMAN, 512), (oracle.TANS, 64)])
+def test_plans_of_one_codec_have_one_launch_per_phase(L, codec, chunk):
+    """A norm vector's second coded plane rides in the launch of the weights: nothing runs beside a launch of its own."""
+    def launches(specs):
+        blob = oracle.write_container(specs, chunk_size=chunk, forced_codec=codec)
+        buf = (C.c_char * len(blob)).from_buffer_copy(blob)
+        h, p, n = C.c_void_p(), C.c_void_p(), C.c_uint32()
+        assert L.ptwm_b200_open(C.addressof(buf), len(blob), C.byref(h)) == 0
+        assert L.ptwm_b200_plan_create(h, None, 0, C.byref(p)) == 0
+        L.ptwm_b200_plan_stats(p, C.byref(C.c_uint64()), C.byref(C.c_uint64()), C.byref(n))
+        scratch = L.ptwm_b200_plan_scratch_bytes(p)
+        L.ptwm_b200_plan_destroy(p)
+        L.ptwm_b200_close(h)
+        return n.value, scratch
+
+    rows = 700 * chunk // 512
+    weights_only, none = launches([spec_bf16("w", rows, 512, 1)])
+    both, scratch = launches([spec_bf16("w", rows, 512, 1), spec_norm("n", 8 * chunk, 5)])
+    assert none == 0 and scratch > 0  # the norm vector decodes its first plane to scratch
+    assert both == weights_only + 1   # in a launch of the first phase
