@@ -94,7 +94,7 @@ struct ChunkDesc {
     uint8_t state_version;
     uint32_t decoded;
     uint64_t plane_off;   // first plane byte of this chunk
-    // filled by classify_chunk:
+    // filled by classify_chunk (the last two by look_at_table):
     bool raw;             // bytes stored verbatim at data_off
     uint64_t data_off, data_len;  // raw bytes, or the codec blob after TAG and length prefix
     uint8_t max_sym;      // rANS coded chunks: alphabet bound from the first blob byte (sizes the decoder's tables)
@@ -330,6 +330,7 @@ inline std::vector<TableEntry> read_table(const uint8_t* base, size_t begin, siz
 
 // Frame header, tag byte and length prefix of one chunk (compressor.rs:316-321;
 // codecs/{huffman,rans,tans}.rs decode; codecs/length_prefix.rs:29-33).
+// Reads no more of the payload than the tag and the length prefix.
 inline void classify_chunk(const uint8_t* base, uint16_t codec, ChunkDesc& ch) {
     ch.raw = false; ch.data_off = ch.body_off; ch.data_len = ch.body_len; ch.max_sym = 255; ch.distinct = 256;
     if (codec == C_IDENTITY) {
@@ -353,6 +354,11 @@ inline void classify_chunk(const uint8_t* base, uint16_t codec, ChunkDesc& ch) {
     if (!ok) throw FormatError("implausible orig_len for the encoded bytes");
     if (orig != ch.decoded) throw FormatError("decoded length differs from the length the chunk declares");
     ch.data_off = ch.body_off + 5; ch.data_len = enc;
+}
+// What the planner wants to know of a coded chunk's table.  The whole payload is at `base` here.
+inline void look_at_table(const uint8_t* base, uint16_t codec, ChunkDesc& ch) {
+    if (ch.raw) return;
+    const uint64_t enc = ch.data_len;
     ch.max_sym = (codec == C_RANS && enc) ? base[ch.data_off] : 255;
     if (codec == C_RANS && enc >= 1 + 2 * (uint64_t(ch.max_sym) + 1)) {
         // frequency table: u16 per symbol after the alphabet bound (rans/decompress.rs:36-47)
@@ -409,6 +415,7 @@ class FileReader {
                 ch.body_off = ch.state_off + sl; ch.body_len = end - start - 5 - sl; ch.decoded = entries[i].second; ch.plane_off = total;
                 total += ch.decoded;
                 detail::classify_chunk(b_, p.codec, ch);
+                detail::look_at_table(b_, p.codec, ch);
                 p.chunks.push_back(ch);
             }
             if (total != p.decoded_len) throw FormatError("chunk table does not decode to the plane's length");  // container.rs:1982-1994
@@ -430,6 +437,7 @@ class FileReader {
                 ch.state_off = e->off; ch.state_len = e->len; ch.state_version = e->version;
             } else if (p.state_source == 3) throw FormatError("External state not supported");
             detail::classify_chunk(b_, p.codec, ch);
+            detail::look_at_table(b_, p.codec, ch);
             p.chunks.push_back(ch);
         }
         if (p.codec == C_O1SAC)
