@@ -98,7 +98,8 @@ struct ChunkDesc {
     bool raw;             // bytes stored verbatim at data_off
     uint64_t data_off, data_len;  // raw bytes, or the codec blob after TAG and length prefix
     uint8_t max_sym;      // rANS coded chunks: alphabet bound from the first blob byte (sizes the decoder's tables)
-    uint16_t distinct;    // rANS coded chunks: symbols with a non-zero frequency (picks the decoder variant); 256 when unknown
+    uint16_t distinct;    // picks the decoder variant.  rANS coded chunks: symbols with a non-zero frequency; 256 when unknown.  tANS: of 2048 symbols,
+                          // those that take more than eight bits (a frequency of 6 or less)
 };
 
 struct PlaneDesc {
@@ -365,6 +366,15 @@ inline void look_at_table(const uint8_t* base, uint16_t codec, ChunkDesc& ch) {
         const uint8_t* f = base + ch.data_off + 1;
         uint32_t d = 0;
         for (uint32_t k = 0; k <= ch.max_sym; ++k) d += (f[2 * k] | f[2 * k + 1]) != 0;
+        ch.distinct = uint16_t(d);
+    }
+    if (codec == C_TANS && enc >= 3) {
+        // [11][symbols u16][symbol, frequency u16 each] (tans/mod.rs:388-411)
+        const uint8_t* f = base + ch.data_off + 1;
+        const uint32_t n = f[0] | f[1] << 8;
+        uint32_t d = 0;
+        if (n <= 256 && enc >= 3 + 3 * uint64_t(n))
+            for (uint32_t k = 0; k < n; ++k) { const uint32_t fr = f[3 + 3 * k] | f[4 + 3 * k] << 8; d += fr <= 6 ? fr : 0; }
         ch.distinct = uint16_t(d);
     }
 }

@@ -46,6 +46,24 @@ def test_mutated_payload_bytes(codec):
     assert _raw(dict(base.decode_model())["w"]) == specs[0].raw
 
 
+def test_mutated_payload_bytes_with_a_lane_per_stream():
+    # 4300 tANS chunks: the kernel with 32 chunks per block
+    raw = np.minimum(np.random.default_rng(8).geometric(0.4, 1029 * 4300), 40).astype(np.uint8).tobytes()
+    blob = oracle.write_container([oracle.TensorSpec("p", oracle.DT_U8, [len(raw)], raw)], forced_codec=oracle.TANS, chunk_size=1029)
+    base = ptwm_b200.ContainerHandle(blob, device=0, verify=False)
+    info = base.tensor_infos()[0]
+    rng = np.random.default_rng(9)
+    for trial in range(8):
+        m = bytearray(blob)
+        for pos in rng.integers(info["first_byte"] + (info["end_byte"] - info["first_byte"]) // 50, info["end_byte"], 1 << trial):
+            m[pos] ^= int(rng.integers(1, 256))
+        try:
+            assert _raw(ptwm_b200.ContainerHandle(bytes(m), device=0, verify=False).decode("p")) != raw
+        except (ptwm_b200.PtwmError, ValueError):
+            pass
+    assert _raw(base.decode("p")) == raw
+
+
 def test_truncated_container_is_refused():
     specs = [spec_bf16("w", 32, 256, 6)]
     blob = oracle.write_container(specs, chunk_size=2048)

@@ -70,6 +70,22 @@ def test_order1_scale_ac_shares_and_rows(alphabet, cols):
     check(specs, chunk_size=None if cols else 1500, forced_codec=oracle.O1SAC)
 
 
+@pytest.mark.parametrize("chunks", [1, 31, 33, 4735, 4736, 4737])
+@pytest.mark.parametrize("dtype", ["u8", "bf16", "fp32", "fp8"])
+def test_tans_decode_with_a_lane_per_stream(dtype, chunks):
+    # chunks of 1029 symbols: from some 4000 on they go to the kernel with 32 chunks per block, and one more than fills the GPU goes back
+    n = 1029 * (chunks - 1) + 7 if chunks > 4000 else 1029 * 4200 + 1029 * (chunks - 1) + 515  # a last chunk of 7, or blocks with 1, 31 and 1 chunks
+    if dtype == "u8":
+        specs = [u8("p", plane("exponent", n))]
+    elif dtype == "fp8":
+        t = weights(1, n, chunks, False).mul(40).to(torch.float8_e4m3fn)
+        specs = [oracle.TensorSpec("p", oracle.DT_E4M3, [n], t.view(torch.uint8).numpy().tobytes())]
+    else:
+        t = weights(1, n, chunks, False).to(torch.bfloat16 if dtype == "bf16" else torch.float32)
+        specs = [oracle.TensorSpec("p", oracle.DT_BF16 if dtype == "bf16" else oracle.DT_F32, [n], t.view(torch.uint8).numpy().tobytes())]
+    check(specs, chunk_size=1029, forced_codec=TANS)
+
+
 def test_decode_two_coded_planes_in_many_chunks():
     # more chunks than are spread over scratch: the second plane's lanes merge with the first one, every codec on its own stream
     for menu in ((oracle.HUFFMAN, oracle.RANS, oracle.O1SAC), (oracle.TANS, oracle.O1SAC), (oracle.IDENTITY, oracle.HUFFMAN, oracle.RANS, oracle.TANS, oracle.O1SAC)):
