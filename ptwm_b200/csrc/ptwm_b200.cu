@@ -220,6 +220,7 @@ namespace {
 int codec_class(uint16_t codec) { return codec == C_RANS ? 0 : codec == C_HUFFMAN ? 1 : codec == C_TANS ? 2 : 3; }
 
 constexpr uint64_t SPREAD_CHUNKS = 4 * 148;  // four chunks per SM: every decoder holds at least that many
+constexpr uint64_t SPREAD_BYTES = 256u << 20;  // of scratch: whole planes of any length count as one chunk, and their scratch is as much again as the tensors
 
 // Turn one tensor into work items.  See DecodeItem / MergeItem in plan.h.
 void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t out_off) {
@@ -917,13 +918,13 @@ int64_t ptwm_b200_plan_create(const ptwm_b200_container* c, const uint32_t* indi
             // A tensor with two coded planes decodes the second in lanes that merge it with the first, so one waits for the other.
             // While all chunks of the plan run at once anyway that only adds up their latencies: with few chunks every coded plane
             // goes to scratch and one more launch merges them (a 4096-element norm vector: 0.48 -> 0.3 ms).
-            uint64_t coded = 0;
+            uint64_t coded = 0, bytes = 0;
             for (uint32_t ti : pl->tensors) if (ti < c->file.tensors.size())
                 for (const PlaneDesc& p : c->file.tensors[ti].planes) {
                     if (coded > SPREAD_CHUNKS) break;
-                    for (const ChunkDesc& ch : p.chunks) coded += !ch.raw;
+                    for (const ChunkDesc& ch : p.chunks) if (!ch.raw) { ++coded; bytes += ch.decoded; }
                 }
-            pl->spread = coded <= SPREAD_CHUNKS;
+            pl->spread = coded <= SPREAD_CHUNKS && bytes <= SPREAD_BYTES;
         }
         for (uint32_t ti : pl->tensors) {
             if (ti >= c->file.tensors.size()) return fail(PTWM_RC_INVALID_INPUT, "tensor index out of range");

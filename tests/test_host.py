@@ -338,23 +338,36 @@ def test_shared_state_fit_on_the_host(L):
     assert _lib.fit_shared_states_host([], []) == []
 
 
+def _plan_sizes(L, blob):
+    """(launches, scratch bytes) of the plan of all tensors"""
+    buf = (C.c_char * len(blob)).from_buffer_copy(blob)
+    h, p, n = C.c_void_p(), C.c_void_p(), C.c_uint32()
+    assert L.ptwm_b200_open(C.addressof(buf), len(blob), C.byref(h)) == 0
+    assert L.ptwm_b200_plan_create(h, None, 0, C.byref(p)) == 0
+    L.ptwm_b200_plan_stats(p, C.byref(C.c_uint64()), C.byref(C.c_uint64()), C.byref(n))
+    scratch = L.ptwm_b200_plan_scratch_bytes(p)
+    L.ptwm_b200_plan_destroy(p)
+    L.ptwm_b200_close(h)
+    return n.value, scratch
+
+
 @pytest.mark.parametrize("codec,chunk", [(oracle.RANS, 1024), (oracle.HUFFMAN, 512), (oracle.TANS, 64)])
 def test_plans_of_one_codec_have_one_launch_per_phase(L, codec, chunk):
     """A norm vector's second coded plane rides in the launch of the weights: nothing runs beside a launch of its own."""
     def launches(specs):
-        blob = oracle.write_container(specs, chunk_size=chunk, forced_codec=codec)
-        buf = (C.c_char * len(blob)).from_buffer_copy(blob)
-        h, p, n = C.c_void_p(), C.c_void_p(), C.c_uint32()
-        assert L.ptwm_b200_open(C.addressof(buf), len(blob), C.byref(h)) == 0
-        assert L.ptwm_b200_plan_create(h, None, 0, C.byref(p)) == 0
-        L.ptwm_b200_plan_stats(p, C.byref(C.c_uint64()), C.byref(C.c_uint64()), C.byref(n))
-        scratch = L.ptwm_b200_plan_scratch_bytes(p)
-        L.ptwm_b200_plan_destroy(p)
-        L.ptwm_b200_close(h)
-        return n.value, scratch
+        return _plan_sizes(L, oracle.write_container(specs, chunk_size=chunk, forced_codec=codec))
 
     rows = 700 * chunk // 512
     weights_only, none = launches([spec_bf16("w", rows, 512, 1)])
     both, scratch = launches([spec_bf16("w", rows, 512, 1), spec_norm("n", 8 * chunk, 5)])
     assert none == 0 and scratch > 0  # the norm vector decodes its first plane to scratch
     assert both == weights_only + 1   # in a launch of the first phase
+
+
+def test_planes_of_any_length_do_not_double_the_scratch(L):
+    """Two coded planes: both decode to scratch at once while that is little memory, else one of them does."""
+    def scratch(n):
+        return _plan_sizes(L, oracle.write_container([oracle.TensorSpec("w", oracle.DT_BF16, [n], b"\x80\x3f" * n)], chunk_size=None, forced_codec=oracle.RANS))[1]
+
+    assert scratch(1 << 20) == 2 << 20
+    assert scratch((128 << 20) + 256) == (128 << 20) + 256
