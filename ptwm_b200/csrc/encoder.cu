@@ -410,19 +410,23 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
     EncChunk* d_chunks = wa.at<EncChunk>(a_chunks);
     EncPlane* d_ep = wa.at<EncPlane>(a_up + u_ep);
     CUDA_TRY(cudaMemcpyAsync(wa.at<uint8_t>(a_up), up.bytes.data(), up.bytes.size(), cudaMemcpyHostToDevice, st));
-    // The payload hashes only need the tensors; each is a serial chain, so they run beside everything else.
+    // The payload hashes only need the tensors; each is a serial chain, so they run beside everything else, on a stream of this call's
+    // own: the chain of a large tensor takes tenths of a second, which nothing else should wait for.
     struct Side {
+        DeviceState& ds;
         cudaStream_t s = nullptr;
         cudaEvent_t ready = nullptr;
-        ~Side() { if (s) cudaStreamSynchronize(s); if (ready) cudaEventDestroy(ready); }  // nothing of it may outlive the work memory
-    } side;
-    if (!hash_items.empty()) {
-        side.s = ds.stream;
-        if (side.s != st) {
-            CUDA_TRY(cudaEventCreateWithFlags(&side.ready, cudaEventDisableTiming));
-            CUDA_TRY(cudaEventRecord(side.ready, st));
-            CUDA_TRY(cudaStreamWaitEvent(side.s, side.ready, 0));
+        ~Side() {  // nothing of it may outlive the work memory
+            if (s) { cudaStreamSynchronize(s); give_stream(ds, s); }
+            if (ready) cudaEventDestroy(ready);
         }
+    } side{ds};
+    if (!hash_items.empty()) {
+        const int64_t got = take_stream(ds, &side.s);
+        if (got < 0) return got;
+        CUDA_TRY(cudaEventCreateWithFlags(&side.ready, cudaEventDisableTiming));
+        CUDA_TRY(cudaEventRecord(side.ready, st));
+        CUDA_TRY(cudaStreamWaitEvent(side.s, side.ready, 0));
         Bases b{nullptr, 0, 0, nullptr, nullptr};
         xxh64_kernel<<<uint32_t(hash_items.size()), XXH_THREADS, 0, side.s>>>(wa.at<HashItem>(a_up + u_hitems), uint32_t(hash_items.size()), b, wa.at<uint64_t>(a_hashes));
         CUDA_TRY(cudaGetLastError());

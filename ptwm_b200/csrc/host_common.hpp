@@ -36,6 +36,7 @@ struct DeviceState {
     CrcTables* d_tabs = nullptr;     // CRC byte table and x^(2^k) powers
     bool attrs = false;
     cudaStream_t side[4] = {nullptr, nullptr, nullptr, nullptr};  // independent decoders of one pass run side by side
+    std::vector<cudaStream_t> spare; // streams of encodes that have ended (their payload hashes ran there)
     std::vector<uint32_t*> words;    // free words of pinned memory, one for every plan that has run (its status summary)
     void* stage = nullptr;           // pinned host buffer the plan work lists pass through on their way to the device
     size_t stage_cap = 0;
@@ -47,6 +48,10 @@ struct DeviceState {
 // Caller holds a DeviceGuard for `dev`.
 int64_t device_state(int dev, DeviceState** out);
 const CrcTables& crc_tables();
+
+// A stream that nobody else uses until it is given back, idle by then.
+int64_t take_stream(DeviceState& ds, cudaStream_t* s);
+void give_stream(DeviceState& ds, cudaStream_t s);
 
 // Device bytes into ordinary host memory; what writes them has completed.
 int64_t copy_to_host(uint8_t* dst, const uint8_t* src, size_t n, DeviceState& ds);

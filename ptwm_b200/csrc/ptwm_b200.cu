@@ -98,6 +98,19 @@ int64_t take_word(DeviceState& ds, uint32_t** w) {
 }
 void give_word(int dev, uint32_t* w) { std::lock_guard<std::mutex> g(g_dev_mu); g_dev[dev].words.push_back(w); }
 
+int64_t take_stream(DeviceState& ds, cudaStream_t* s) {
+    std::lock_guard<std::mutex> g(g_dev_mu);
+    if (ds.spare.empty()) {
+        ds.spare.reserve(ds.spare.capacity() + 1);  // giving it back allocates nothing
+        CUDA_TRY(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+    } else {
+        *s = ds.spare.back();
+        ds.spare.pop_back();
+    }
+    return 0;
+}
+void give_stream(DeviceState& ds, cudaStream_t s) { std::lock_guard<std::mutex> g(g_dev_mu); ds.spare.push_back(s); }
+
 const CrcTables& crc_tables() { static CrcTables t = host_crc_tables(); return t; }
 
 int64_t device_state(int dev, DeviceState** out) {

@@ -42,6 +42,34 @@ def test_plans_reach_the_device_while_a_container_is_copied_to_the_host():
     assert torch.equal(raw, big)
 
 
+def test_plans_reach_the_device_while_another_thread_hashes():
+    # the hash of one tensor is a serial chain, here of some 100 ms
+    big = torch.randint(0, 256, (256 << 20,), dtype=torch.uint8, device="cuda")
+    config = CompressionConfig(streaming_chunk=None, forced_codec=IDENTITY, emit_payload_hash=True)
+    compress_model({"w": big[:4096]}, config)
+    handle = ptwm_b200.ContainerHandle(oracle.write_container(mixed_model(), chunk_size=4096), device=0)
+    ptwm_b200.DecodePlan(handle).prepare(0)
+    torch.cuda.synchronize()
+    span, blob = [], []
+
+    def encode():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            span.append(time.perf_counter())
+            blob.append(compress_model({"w": big}, config))
+            span.append(time.perf_counter())
+
+    done = []
+    t = threading.Thread(target=encode)
+    t.start()
+    while t.is_alive():
+        began = time.perf_counter()
+        ptwm_b200.DecodePlan(handle).prepare(0)
+        done.append((began, time.perf_counter()))
+    t.join()
+    assert sum(span[0] + 0.02 <= a and b <= span[1] for a, b in done) >= 10
+    assert torch.equal(ptwm_b200.ContainerHandle(blob[0].to_tensor(), verify=True).decode("w"), big)
+
+
 def test_a_plan_dropped_in_flight_does_not_answer_for_the_next_one():
     blob = oracle.write_container(mixed_model(), chunk_size=4096, forced_codec=oracle.RANS)
     handle = ptwm_b200.ContainerHandle(blob, device=0)
