@@ -46,17 +46,16 @@ def test_plans_reach_the_device_while_another_thread_hashes():
     # the hash of one tensor is a serial chain, here of some 100 ms
     big = torch.randint(0, 256, (256 << 20,), dtype=torch.uint8, device="cuda")
     config = CompressionConfig(streaming_chunk=None, forced_codec=IDENTITY, emit_payload_hash=True)
-    compress_model({"w": big[:4096]}, config)
+    compress_model({"w": big}, config)  # its memory is in the pool
     handle = ptwm_b200.ContainerHandle(oracle.write_container(mixed_model(), chunk_size=4096), device=0)
     ptwm_b200.DecodePlan(handle).prepare(0)
     torch.cuda.synchronize()
     span, blob = [], []
 
     def encode():
-        with torch.cuda.stream(torch.cuda.Stream()):
-            span.append(time.perf_counter())
-            blob.append(compress_model({"w": big}, config))
-            span.append(time.perf_counter())
+        span.append(time.perf_counter())
+        blob.append(compress_model({"w": big}, config))
+        span.append(time.perf_counter())
 
     done = []
     t = threading.Thread(target=encode)
@@ -66,7 +65,7 @@ def test_plans_reach_the_device_while_another_thread_hashes():
         ptwm_b200.DecodePlan(handle).prepare(0)
         done.append((began, time.perf_counter()))
     t.join()
-    assert sum(span[0] + 0.02 <= a and b <= span[1] for a, b in done) >= 10
+    assert max(b - a for a, b in done) < (span[1] - span[0]) / 2, (span[1] - span[0], max(b - a for a, b in done))
     assert torch.equal(ptwm_b200.ContainerHandle(blob[0].to_tensor(), verify=True).decode("w"), big)
 
 
