@@ -247,6 +247,8 @@ int64_t ptwm_b200_set_allocator(ptwm_b200_alloc_fn alloc, ptwm_b200_free_fn free
 int64_t ptwm_b200_encode_model(const ptwm_b200_encode_tensor* tensors, size_t n, const ptwm_b200_encode_options* options, uint32_t device_ordinal,
                                uint64_t stream, ptwm_b200_encoded** out);
 uint64_t ptwm_b200_encoded_size(const ptwm_b200_encoded* e);
+/* Where the container lies, until ptwm_b200_encoded_free: which then waits for the device, so that work enqueued on any stream
+ * may read it. */
 uint64_t ptwm_b200_encoded_device_ptr(const ptwm_b200_encoded* e);
 /* Copy the container bytes to host memory. */
 int64_t ptwm_b200_encoded_copy(const ptwm_b200_encoded* e, uint8_t* host_dst, size_t cap);

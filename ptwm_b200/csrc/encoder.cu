@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -235,7 +236,13 @@ struct ptwm_b200_encoded {
     DeviceBuf out;
     uint64_t size = 0;
     int device = 0;
+    mutable std::atomic<bool> shown{false};  // the caller has the address
     std::vector<std::vector<int>> plane_codecs;
+    ~ptwm_b200_encoded() {
+        // What the caller enqueued on streams of its own may still read the container.  cudaFree waits for all of the device; an
+        // allocator that recycles memory in the order of one stream does not.
+        if (shown && out.p && out.from.free) { DeviceGuard g{device}; cudaDeviceSynchronize(); }
+    }
 };
 
 namespace {
@@ -1133,7 +1140,11 @@ int64_t ptwm_b200_fit_shared_states_host(const uint8_t* const* planes, const uin
     } catch (const std::exception& ex) { return fail(PTWM_RC_INTERNAL, ex.what()); }
 }
 uint64_t ptwm_b200_encoded_size(const ptwm_b200_encoded* e) { return e ? e->size : 0; }
-uint64_t ptwm_b200_encoded_device_ptr(const ptwm_b200_encoded* e) { return e ? uint64_t(reinterpret_cast<uintptr_t>(e->out.p)) : 0; }
+uint64_t ptwm_b200_encoded_device_ptr(const ptwm_b200_encoded* e) {
+    if (!e) return 0;
+    e->shown = true;
+    return uint64_t(reinterpret_cast<uintptr_t>(e->out.p));
+}
 int64_t ptwm_b200_encoded_copy(const ptwm_b200_encoded* e, uint8_t* host_dst, size_t cap) {
     if (!e || !host_dst) return fail(PTWM_RC_INVALID_INPUT, "null argument");
     if (cap < e->size) return fail(PTWM_RC_BUFFER_TOO_SMALL, "host buffer smaller than the container");

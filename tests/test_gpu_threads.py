@@ -8,6 +8,7 @@ import torch
 
 import oracle
 import ptwm_b200
+from ptwm_b200 import _lib
 from ptwm_b200.compressor import CompressionConfig, IDENTITY, compress_model
 from _data import mixed_model
 
@@ -94,3 +95,24 @@ def test_a_plan_dropped_in_flight_does_not_answer_for_the_next_one():
     with torch.cuda.stream(fast), pytest.raises(ptwm_b200.PtwmError):
         second.finish(0)
     del memory
+
+
+def test_a_container_whose_address_was_taken_outlives_the_work_that_reads_it():
+    tensors = {"w": torch.randint(0, 256, (1 << 20,), dtype=torch.uint8, device="cuda")}
+    enc = compress_model(tensors, CompressionConfig(streaming_chunk=65536, forced_codec=IDENTITY))
+    size = enc.size
+    plan = ptwm_b200.DecodePlan(ptwm_b200.ContainerHandle(enc.to_bytes(), device=0))
+    out = torch.empty(plan.out_bytes, dtype=torch.uint8, device="cuda")
+    slow, L = torch.cuda.Stream(), _lib.lib()
+    plan.prepare(0)
+    where = L.ptwm_b200_encoded_device_ptr(enc._e)
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(slow):
+        torch.cuda._sleep(500_000_000)
+        assert L.ptwm_b200_plan_run(plan._p, where, 0, size, out.data_ptr(), out.numel(), 0, 0, ptwm_b200.NO_SYNC, 0, slow.cuda_stream) == 0
+    del enc
+    recycled = [torch.full((size,), 255, dtype=torch.uint8, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    assert torch.equal(out[:1 << 20], tensors["w"])
+    del recycled
