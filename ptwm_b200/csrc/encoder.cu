@@ -194,44 +194,6 @@ struct Piece { uint64_t dst; std::vector<uint8_t> bytes; };
 
 }  // namespace
 
-namespace {
-
-// Device memory comes from the allocator the program registered (ptwm_b200_set_allocator), else from cudaMalloc.  An encode
-// takes work memory several times the size of the tensors; handed out and taken back by the driver that was 55 of the 64 ms
-// of a 1.7 GB model.  The blocks belong to the stream the encode runs on, which is all an allocator that recycles memory in
-// stream order has to know.
-struct Allocator { ptwm_b200_alloc_fn alloc = nullptr; ptwm_b200_free_fn free = nullptr; };
-std::mutex g_alloc_mu;
-Allocator g_alloc;
-Allocator current_allocator() { std::lock_guard<std::mutex> g(g_alloc_mu); return g_alloc; }
-
-struct DeviceBuf {
-    void* p = nullptr;
-    Allocator from;
-    int device = 0;
-    cudaStream_t stream = nullptr;
-    DeviceBuf() = default;
-    DeviceBuf(const DeviceBuf&) = delete;
-    DeviceBuf& operator=(const DeviceBuf&) = delete;
-    ~DeviceBuf() {
-        if (!p) return;
-        if (from.free) from.free(uint64_t(reinterpret_cast<uintptr_t>(p)), uint32_t(device), uint64_t(reinterpret_cast<uintptr_t>(stream)));
-        else { DeviceGuard g{device}; cudaFree(p); }
-    }
-    template <class T> T* as() const { return static_cast<T*>(p); }
-    cudaError_t alloc(size_t n, cudaStream_t st, bool registered = true) {
-        stream = st;
-        cudaError_t e = cudaGetDevice(&device);
-        if (e != cudaSuccess) return e;
-        from = registered ? current_allocator() : Allocator{};
-        if (!from.alloc) return cudaMalloc(&p, n ? n : 1);
-        p = reinterpret_cast<void*>(uintptr_t(from.alloc(n ? n : 1, uint32_t(device), uint64_t(reinterpret_cast<uintptr_t>(st)))));
-        return p ? cudaSuccess : cudaErrorMemoryAllocation;
-    }
-};
-
-}  // namespace
-
 struct ptwm_b200_encoded {
     DeviceBuf out;
     uint64_t size = 0;
@@ -1068,8 +1030,7 @@ extern "C" {
 
 int64_t ptwm_b200_set_allocator(ptwm_b200_alloc_fn alloc, ptwm_b200_free_fn free) {
     if ((alloc == nullptr) != (free == nullptr)) return fail(PTWM_RC_INVALID_INPUT, "an allocator is a pair of functions");
-    std::lock_guard<std::mutex> g(g_alloc_mu);
-    g_alloc = Allocator{alloc, free};
+    set_allocator(Allocator{alloc, free});
     return 0;
 }
 int64_t ptwm_b200_encode_model(const ptwm_b200_encode_tensor* tensors, size_t n, const ptwm_b200_encode_options* options, uint32_t device_ordinal, uint64_t stream,

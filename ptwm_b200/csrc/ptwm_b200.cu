@@ -39,6 +39,13 @@ CrcTables host_crc_tables() {
 }
 }  // namespace
 
+namespace {
+std::mutex g_alloc_mu;
+Allocator g_alloc;
+}  // namespace
+Allocator current_allocator() { std::lock_guard<std::mutex> g(g_alloc_mu); return g_alloc; }
+void set_allocator(Allocator a) { std::lock_guard<std::mutex> g(g_alloc_mu); g_alloc = a; }
+
 // Through a pinned staging buffer in slices: the copy engine fills slice k + 4 while host threads move slice k on.  A copy
 // into pageable memory by the driver runs at 5 - 10 GB/s, and memory nobody has touched yet costs a page fault per 4 KiB on
 // top of that, so the slices are taken by four threads, on huge pages where the system grants them.  Buffer, stream and lock are
@@ -169,15 +176,18 @@ struct DevicePlan {
     uint32_t* summary = nullptr;      // pinned: the largest status of the last run
     bool timed[12] = {false};
     uint8_t* arena = nullptr;          // everything above lives in this one block
+    std::shared_ptr<DeviceBuf> own;    // the block, unless it is the caller's
     bool external = false;             // the block belongs to the caller (ptwm_b200_plan_prepare_in)
     cudaEvent_t written = nullptr;     // external: the last run has written the summary
     bool captured = false;             // external: a graph holds a run, which may write the summary at any time
     void release(int dev) {
         for (auto& e : ev) if (e) cudaEventDestroy(e);
         for (auto& e : order) if (e) cudaEventDestroy(e);
-        // The word goes to another plan: nothing of this one's may write to it any more.  cudaFree waits for the plan's runs; the
-        // caller's memory outlives them by contract, so they are waited for here, and a word in a graph is never given back.
-        if (!external) cudaFree(arena);
+        // The word goes to another plan: nothing of this one's may write to it any more.  cudaFree waits for the plan's runs, the
+        // program's allocator does not; the caller's memory outlives them by contract, so they are waited for here, and a word in a
+        // graph is never given back.
+        if (own && own->from.free) cudaDeviceSynchronize();
+        own.reset();
         if (written) { cudaEventSynchronize(written); cudaEventDestroy(written); }
         if (summary && !captured) give_word(dev, summary);
         *this = DevicePlan{};
@@ -492,7 +502,9 @@ int64_t device_plan(ptwm_b200_plan& pl, int dev, DeviceState& ds, DevicePlan** o
         if (cap < L.total || (reinterpret_cast<uintptr_t>(mem) & 255)) return fail(PTWM_RC_BUFFER_TOO_SMALL, "plan memory smaller than ptwm_b200_plan_device_bytes or not 256-byte aligned");
         d.arena = mem; d.external = true;
     } else {
-        CUDA_TRY(cudaMalloc(&d.arena, L.total));
+        d.own = std::make_shared<DeviceBuf>();
+        CUDA_TRY(d.own->alloc(L.total, ds.stream, false));
+        d.arena = d.own->as<uint8_t>();
     }
     d.items = reinterpret_cast<DecodeItem*>(d.arena + L.off[0]); d.merges = reinterpret_cast<MergeItem*>(d.arena + L.off[1]);
     d.tiles = reinterpret_cast<uint32_t*>(d.arena + L.off[2]); d.posts = reinterpret_cast<PostItem*>(d.arena + L.off[3]);
@@ -764,9 +776,9 @@ int64_t decode_plane_cuda(uint8_t sfv, const uint8_t* state, size_t state_len, c
     it.partner[0] = it.partner[1] = it.partner[2] = REF_NONE; it.state = REF_NONE; it.id = 0;
     // device scratch for the item, the status words and (O1SAC) the state
     const size_t state_off = 256, total = state_off + align_up(state_len, 256);
-    uint8_t* scratch = nullptr;
-    CUDA_TRY(cudaMalloc(&scratch, total));
-    struct Free { uint8_t* p; ~Free() { cudaFree(p); } } freer{scratch};
+    DeviceBuf mem;
+    CUDA_TRY(mem.alloc(total, st, false));
+    uint8_t* scratch = mem.as<uint8_t>();
     bases.scratch = scratch;
     if (codec == C_O1SAC) {
         it.state = make_ref(SP_SCRATCH, state_off); it.state_len = uint32_t(state_len); it.state_version = sfv; it.row_len = 0;
@@ -841,11 +853,10 @@ int64_t ptwm_plane_codec_v1_encode(const uint8_t* in, size_t in_len, uint8_t* ou
     int64_t rc = device_state(0, &ds);
     if (rc < 0) return rc;
     const size_t cap = in_len + 16;
-    uint8_t *d_in = nullptr, *d_out = nullptr;
-    CUDA_TRY(cudaMalloc(&d_in, in_len ? in_len : 1));
-    struct Free { uint8_t* p; ~Free() { cudaFree(p); } } f1{d_in};
-    CUDA_TRY(cudaMalloc(&d_out, cap));
-    Free f2{d_out};
+    DeviceBuf in_mem, out_mem;
+    CUDA_TRY(in_mem.alloc(in_len, ds->stream, false));
+    CUDA_TRY(out_mem.alloc(cap, ds->stream, false));
+    uint8_t *d_in = in_mem.as<uint8_t>(), *d_out = out_mem.as<uint8_t>();
     CUDA_TRY(cudaMemcpy(d_in, in, in_len, cudaMemcpyHostToDevice));
     uint64_t needed = 0;
     int64_t n = encode_plane_cuda(C_RANS, nullptr, 0, 0, uint64_t(reinterpret_cast<uintptr_t>(d_in)), in_len, uint64_t(reinterpret_cast<uintptr_t>(d_out)), cap, &needed, ds->stream);
@@ -859,11 +870,13 @@ int64_t ptwm_plane_codec_v1_decode_stateful(uint8_t sv, const uint8_t* state, si
     if ((in_len && !in) || (out_cap && !out)) return fail(PTWM_RC_INVALID_INPUT, "null buffer");
     DeviceGuard guard{0};
     if (guard.err != cudaSuccess) return fail(PTWM_RC_MISSING_CAPABILITY, "no CUDA device");
-    uint8_t *d_in = nullptr, *d_out = nullptr;
-    CUDA_TRY(cudaMalloc(&d_in, in_len ? in_len : 1));
-    struct Free { uint8_t* p; ~Free() { cudaFree(p); } } f1{d_in};
-    CUDA_TRY(cudaMalloc(&d_out, out_cap ? out_cap : 1));
-    Free f2{d_out};
+    DeviceState* ds;
+    const int64_t rc = device_state(0, &ds);
+    if (rc < 0) return rc;
+    DeviceBuf in_mem, out_mem;
+    CUDA_TRY(in_mem.alloc(in_len, ds->stream, false));
+    CUDA_TRY(out_mem.alloc(out_cap, ds->stream, false));
+    uint8_t *d_in = in_mem.as<uint8_t>(), *d_out = out_mem.as<uint8_t>();
     CUDA_TRY(cudaMemcpy(d_in, in, in_len, cudaMemcpyHostToDevice));
     int64_t n = decode_plane_cuda(sv, state, state_len, kBuiltins[2].id, 32, uint64_t(reinterpret_cast<uintptr_t>(d_in)), in_len,
                                   uint64_t(reinterpret_cast<uintptr_t>(d_out)), out_cap, 0);
