@@ -594,10 +594,15 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
     };
     int64_t rc;
     const int classes = codec_classes(pl);
-    // A stream that is being captured gets its launches in a row too: the side streams belong to every thread of the device.
+    // A stream that is being captured gets its launches in a row too: the side streams belong to every thread of the device.  And so
+    // does one of another priority than theirs, which its decoders are to have.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (classes >= 2) CUDA_TRY(cudaStreamIsCapturing(st, &capture));
-    if (timing || classes < 2 || capture != cudaStreamCaptureStatusNone) {  // one after the other
+    int priority = 0;
+    if (classes >= 2) {
+        CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+        if (capture == cudaStreamCaptureStatusNone) CUDA_TRY(cudaStreamGetPriority(st, &priority));
+    }
+    if (timing || classes < 2 || capture != cudaStreamCaptureStatusNone || priority != 0) {  // one after the other
         for (int ph = 0; ph < 2; ++ph) {
             for (int cc = 0; cc < 4; ++cc) {
                 if (pl.runs[ph][cc].empty()) continue;

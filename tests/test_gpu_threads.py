@@ -116,3 +116,26 @@ def test_a_container_whose_address_was_taken_outlives_the_work_that_reads_it():
     torch.cuda.synchronize()
     assert torch.equal(out[:1 << 20], tensors["w"])
     del recycled
+
+
+@pytest.mark.parametrize("priority", [0, -1])
+def test_threads_decode_plans_of_several_codecs_at_once(priority):
+    specs = mixed_model(2)
+    blobs = [oracle.write_container(specs, chunk_size=chunk, menu=(oracle.HUFFMAN, oracle.RANS, oracle.TANS, oracle.O1SAC)) for chunk in (501, 4096, 65536)]
+    wrong, raised = [], []
+
+    def decode(blob):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream(priority=priority)):
+                handle = ptwm_b200.ContainerHandle(blob, device=0)
+                for _ in range(8):
+                    wrong.extend(s.name for (name, t), s in zip(handle.decode_model(), specs) if t.contiguous().view(torch.uint8).cpu().numpy().tobytes() != s.raw)
+        except Exception as e:
+            raised.append(e)
+
+    threads = [threading.Thread(target=decode, args=(blob,)) for blob in blobs + blobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not raised and not wrong
