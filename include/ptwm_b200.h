@@ -272,7 +272,7 @@ void ptwm_b200_encoded_free(ptwm_b200_encoded* e);
  * `stream` must be given (1 = the legacy default stream).
  *
  * - Limit: identity / huffman / rans / tans payloads of any size fit; an
- *   Order1ScaleAC state fits up to 62 context rows, a larger one is refused with
+ *   Order1ScaleAC state fits up to 126 context rows, a larger one is refused with
  *   PTWM_RC_BUFFER_TOO_SMALL and a message naming the limit.
  * - The first call on a device looks the array's address up
  *   (cudaGetSymbolAddress) and raises the kernels' shared-memory limit; make that

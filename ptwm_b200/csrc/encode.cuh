@@ -759,7 +759,6 @@ __global__ void __launch_bounds__(128) huffman_encode_kernel(const EncChunk* __r
         for (uint32_t i = lane; i < full; i += 32) out[i] = words[i];
         __syncwarp();
         for (uint32_t i = lane; i <= full; i += 32) words[i] = i == 0 ? rest : 0u;
-        if (lane == 0 && full == 0) words[0] = rest;
         out += full;
         __syncwarp();
     }

@@ -2,7 +2,7 @@
 // memory.  It decodes a single plane payload like
 // ptwm_hardware_backend_v1_dispatch_decode_cuda, but everything the kernel
 // needs besides the caller's input and output (the work item, the status
-// word, and for Order1ScaleAC the state bytes and their cumulative tables)
+// words, and for Order1ScaleAC the state bytes)
 // lives in one fixed array in device memory that is part of this library's
 // image.  Every GPU that loads the library carries that array until the
 // process exits.
@@ -11,8 +11,8 @@
 using namespace ptwm;
 
 // Scratch of the no-allocation entry point.  64 KiB: 256 bytes for the status
-// word and the work item, the rest for an Order1ScaleAC state plus its tables
-// (up to 62 context rows).  The name below is only a host-side handle for the
+// words and the work item, the rest for an Order1ScaleAC state (up to 126
+// context rows).  The name below is only a host-side handle for the
 // symbol; the device address comes from cudaGetSymbolAddress.
 #define PTWM_B200_NOALLOC_SCRATCH_BYTES 65536
 static __device__ __align__(256) uint8_t g_noalloc_scratch[PTWM_B200_NOALLOC_SCRATCH_BYTES];
@@ -88,11 +88,10 @@ extern "C" int64_t ptwm_b200_decode_plane_noalloc(uint8_t state_format_version, 
         CUDA_TRY(cudaStreamSynchronize(st));
         return int64_t(decoded);
     }
-    // layout of the fixed scratch: [0,8) status (summary, item), [64, 64+sizeof item) work item, then (Order1ScaleAC) tables and state
-    const size_t tables = codec == C_O1SAC ? (state_len - 32) / 512 : 0;
-    const size_t work_off = 256, state_off = work_off + align_up(tables * 514, 256), total = state_off + align_up(codec == C_O1SAC ? state_len : 0, 256);
+    // layout of the fixed scratch: [0,8) status (summary, item), [64, 64+sizeof item) work item, then (Order1ScaleAC) the state
+    const size_t state_off = 256, total = state_off + align_up(codec == C_O1SAC ? state_len : 0, 256);
     if (total > PTWM_B200_NOALLOC_SCRATCH_BYTES)
-        return fail(PTWM_RC_BUFFER_TOO_SMALL, "Order1ScaleAC state with " + std::to_string(tables - 1) + " context rows needs " + std::to_string(total) +
+        return fail(PTWM_RC_BUFFER_TOO_SMALL, "Order1ScaleAC state with " + std::to_string(o1sac_tables(state_len) - 1) + " context rows needs " + std::to_string(total) +
                                                   " bytes of scratch; the built-in scratch of ptwm_b200_decode_plane_noalloc holds " +
                                                   std::to_string(PTWM_B200_NOALLOC_SCRATCH_BYTES) + " (use ptwm_hardware_backend_v1_dispatch_decode_cuda)");
     DecodeItem it{};

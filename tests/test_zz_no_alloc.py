@@ -10,7 +10,7 @@ device image.  This test drives it through the C ABI, twice in a row per case
 (the array keeps the previous call's contents, so the second call proves the
 entry point clears what it must), and requires byte-identical output to
 ptwm_hardware_backend_v1_dispatch_decode_cuda.  It also checks the documented
-limit: an Order1ScaleAC state with more than 62 context rows is refused with a
+limit: an Order1ScaleAC state with more than 126 context rows is refused with a
 clear message.  The file sorts last so a run that stops at the first failure
 has already finished every other test.
 """
@@ -77,7 +77,7 @@ def test_noalloc_refuses_a_state_beyond_its_scratch():
     rng = np.random.default_rng(22)
     plane = rng.integers(0, 256, (200, 256), dtype=np.uint8).tobytes()  # every byte value is a context: 256 rows
     st, sv, payload = oracle.plane_encode(oracle.O1SAC, plane, 0)
-    assert (len(st) - 32) // 512 - 1 > 62
+    assert (len(st) - 32) // 512 - 1 > 126
     rc, _ = _decode("ptwm_b200_decode_plane_noalloc", oracle.O1SAC, payload, len(plane), st, sv, stream=1)
     assert rc == -2 and "holds 65536" in _lib.last_error()
     rc_ref, ref = _decode("ptwm_hardware_backend_v1_dispatch_decode_cuda", oracle.O1SAC, payload, len(plane), st, sv)
@@ -86,6 +86,15 @@ def test_noalloc_refuses_a_state_beyond_its_scratch():
     _, _, p2 = oracle.plane_encode(oracle.RANS, plane[:4096] * 4)
     rc, got = _decode("ptwm_b200_decode_plane_noalloc", oracle.RANS, p2, 16384, stream=1)
     assert rc == 16384 and got[:16384] == plane[:4096] * 4
+
+
+@pytest.mark.parametrize("rows,fits", [(62, True), (63, True), (126, True), (127, False)])
+def test_noalloc_state_sizes(rows, fits):
+    plane = np.random.default_rng(rows).integers(0, rows, (200, 256)).astype(np.uint8).tobytes()
+    st, sv, payload = oracle.plane_encode(oracle.O1SAC, plane, 0)
+    assert (len(st) - 32) // 512 - 1 == rows
+    rc, got = _decode("ptwm_b200_decode_plane_noalloc", oracle.O1SAC, payload, len(plane), st, sv, stream=1)
+    assert (rc == len(plane) and got[:rc] == plane) if fits else rc == -2
 
 
 def test_noalloc_needs_a_stream():
