@@ -138,6 +138,12 @@ inline int huffman_lengths(const unsigned long long* raw, uint8_t* lengths) {
     return last + 1;
 }
 
+// A single plane of n bytes through the plane call: bytes of one of its four stream slots (a symbol takes at most 12 bits in any of the
+// codecs; slots start on 16-byte boundaries and are written in aligned words), and whether the call takes planes that long.
+__host__ __device__ inline uint64_t plane_slot_bytes(uint64_t n) { return ((n / 4 + 1) * 12 + 7) / 8 + 64; }
+__host__ __device__ inline uint64_t plane_slot_cap(uint64_t n) { return (plane_slot_bytes(n) + 15) / 16 * 16; }
+__host__ __device__ inline bool plane_codable(uint64_t n) { return plane_slot_bytes(n) <= 0x3FFFFFFFull; }
+
 // tANS: symbols per lane when a warp codes a chunk of n.  Any 32-bit n: the lanes' runs cover it.
 constexpr uint32_t TENC_MIN_RUN = 256;  // shorter runs would hardly ever end in the right state
 __host__ __device__ inline uint32_t tans_encode_run(uint32_t n) {

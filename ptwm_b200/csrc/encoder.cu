@@ -943,14 +943,14 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
     }
     if (n > 0xFFFFFFFFull && codec == C_O1SAC) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
     DeviceBuf d_chunk, d_tables, d_results, d_slots, d_list, d_job;
-    const uint64_t slot_cap = align_up(((n / 4 + 1) * 12 + 7) / 8 + 64, 16);  // a symbol takes at most 12 bits in any of the codecs; slots are written in aligned words
+    const uint64_t slot_cap = plane_slot_cap(n);
     EncChunk chunk{0, 0, 0, uint32_t(n), uint32_t(slot_cap), 0, 0};
     if (codec == C_O1SAC) {
         // The flat ABI has no way to return a fitted state, so the rows come from the caller (the shared-state form of
         // order1_scale_ac.rs:620-633): [bitmap 32][marginal 512][rows 512 each], one row spanning the plane.
         if (!state_len) return fail(PTWM_RC_UNSUPPORTED, "order1_scale_ac through the plane-codec ABI needs the state to encode with (state_ptr, state_len)");
         try { check_o1sac(state, state_len, state_version, 5, 0, 0); } catch (const FormatError& e) { return fail(PTWM_RC_INVALID_INPUT, e.what()); }
-        if (slot_cap > 0x3FFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
+        if (!plane_codable(n)) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
         std::vector<uint8_t> tab(ENC_O1SAC_TABLE_BYTES, 0);
         uint16_t* pmf = reinterpret_cast<uint16_t*>(tab.data() + O1E_PMF);
         uint16_t* cum = reinterpret_cast<uint16_t*>(tab.data() + O1E_CUM);
@@ -995,7 +995,7 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
     struct Job { EncPlane plane; EncChunk chunk; EncResult result; uint32_t list, pad[3]; uint32_t hist[256]; } job{};
     const uint64_t job_bytes = align_up(sizeof(Job), 256);
     if (n <= 0xFFFFFFFFull) {  // the length prefix is a u32; longer planes stay raw
-        if (slot_cap > 0x3FFFFFFFull) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
+        if (!plane_codable(n)) return fail(PTWM_RC_UNSUPPORTED, "plane too long for the device encoder");
         job.plane.codec = uint32_t(codec);
         job.chunk = chunk; job.chunk.slot_off = job_bytes + ENC_HUFF_TABLE_BYTES; job.chunk.table_off = job_bytes;
         CUDA_TRY(d_job.alloc(job.chunk.slot_off + 4 * slot_cap + ENC_PAD, st, false));
