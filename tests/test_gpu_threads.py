@@ -66,7 +66,7 @@ def test_plans_reach_the_device_while_another_thread_hashes():
         ptwm_b200.DecodePlan(handle).prepare(0)
         done.append((began, time.perf_counter()))
     t.join()
-    assert max(b - a for a, b in done) < (span[1] - span[0]) / 2, (span[1] - span[0], max(b - a for a, b in done))
+    assert sum(a >= span[0] + 0.3 * (span[1] - span[0]) and b <= span[1] for a, b in done) >= 3  # begun and done in the midst of the hash
     assert torch.equal(ptwm_b200.ContainerHandle(blob[0].to_tensor(), verify=True).decode("w"), big)
 
 
