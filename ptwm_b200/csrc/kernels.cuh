@@ -414,6 +414,45 @@ __device__ __forceinline__ void extract16(const uint4& cur, const uint4& nxt, ui
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[i] = __byte_perm(c[i], c[i + 1], sel);
 }
+// ---- sixteen elements of a merge --------------------------------------------
+// Sixteen elements to `out`, which lies on a boundary of their size, from 16 bytes of every plane.
+__device__ __forceinline__ void merge_store16(int kind, uint8_t* out, const uint32_t pw[4][4]) {
+    switch (kind) {
+        case K_PASS: *reinterpret_cast<uint4*>(out) = make_uint4(pw[0][0], pw[0][1], pw[0][2], pw[0][3]); break;
+        case K_E4M3:
+        case K_E5M2: {
+            const bool e4m3 = kind == K_E4M3;
+            *reinterpret_cast<uint4*>(out) = make_uint4(compose_fp8x4(pw[0][0], pw[1][0], e4m3), compose_fp8x4(pw[0][1], pw[1][1], e4m3),
+                                                        compose_fp8x4(pw[0][2], pw[1][2], e4m3), compose_fp8x4(pw[0][3], pw[1][3], e4m3));
+            break;
+        }
+        case K_M16: {
+            uint4 v[2];
+            compose16x4(pw[0][0], pw[1][0], v[0].x, v[0].y); compose16x4(pw[0][1], pw[1][1], v[0].z, v[0].w);
+            compose16x4(pw[0][2], pw[1][2], v[1].x, v[1].y); compose16x4(pw[0][3], pw[1][3], v[1].z, v[1].w);
+            stg256(out, v[0], v[1]);
+            break;
+        }
+        default: {  // K_M32 (transforms/fusion.rs:287-292)
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {
+                uint32_t w[8];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t t0 = __byte_perm(pw[0][k + h], pw[1][k + h], 0x5140), t1 = __byte_perm(pw[2][k + h], pw[3][k + h], 0x5140);
+                    const uint32_t t2 = __byte_perm(pw[0][k + h], pw[1][k + h], 0x7362), t3 = __byte_perm(pw[2][k + h], pw[3][k + h], 0x7362);
+                    w[4 * h + 0] = revert32(__byte_perm(t0, t1, 0x5410));
+                    w[4 * h + 1] = revert32(__byte_perm(t0, t1, 0x7632));
+                    w[4 * h + 2] = revert32(__byte_perm(t2, t3, 0x5410));
+                    w[4 * h + 3] = revert32(__byte_perm(t2, t3, 0x7632));
+                }
+                stg256(out + 16 * k, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
+            }
+            break;
+        }
+    }
+}
+
 template <class Dec8>
 __device__ __forceinline__ void fused32_rounds(const Epilogue& ep, uint32_t chunk_n, uint32_t& pos, uint32_t& remaining, Dec8&& dec8) {
     uint8_t* out = ep.dst + size_t(pos) * 4;
@@ -1228,94 +1267,226 @@ __global__ void __launch_bounds__(32) huffman_decode_kernel(const DecodeItem* __
 // One serial stream per chunk: a symbol is a table look-up by the state and the
 // next state needs the bits the entry says.  Many lanes decode a chunk all the
 // same.  The stream's bits are cut into equal runs, one per lane, and every
-// lane decodes its run from the cut in a guessed state.  A decoder that starts
-// wrong falls in with the right one after a while (same bit, same state; about
-// 1,100 - 1,600 symbols on an exponent plane of normal weights, 200 - 700 on
-// flatter planes) and stays with it, so what a lane is left with at the end of
-// its run (bit position and state) is mostly what the serial decoder has there.
-// That is where the next lane has to start: lanes whose start was something
-// else go again from it, until nobody's start changes.  Every round settles at
-// least one more lane, so the worst case is the serial chain; the usual number
-// of rounds is such that all rounds together are some 8 Ki steps (a stream of
-// 64 Ki symbols: 4.6 rounds of 32 runs, 15 of 128).  Then every lane knows where
-// its symbols start and how many it has, and a last pass decodes once more and
-// places them.  Starting a lane from several guesses side by side saves one
-// round in four and costs more than that.
+// lane decodes from its cut on in a guessed state.  Two decoders of one stream
+// fall in with one another after a while (same bit, same state; about 1,400
+// symbols on an exponent plane of normal weights, 200 - 700 on flatter planes)
+// and stay together, so it is enough to know where each of them meets a path
+// that another lane walks anyway:
 //
-// A stream of 64 Ki symbols in a lane of its own took 1.75 ms (52 cycles per
-// symbol), and 32 of them were all an SM held.
+// * The stream has nodes at fixed bits, TansShape::SEGS to a run.  A lane that
+//   comes past one enters (bit, state) of its first symbol boundary there, with
+//   the symbols it has met so far.  A lane that finds its own pair entered
+//   already stops: from here on its path is the other lane's.  Lanes do not stop
+//   at the end of their run but when they have met another path, or at the
+//   start of the last run.
+// * Nobody waits for anybody while this goes on; which of two lanes enters a
+//   pair first does not change what is decoded from it.
+// * Lane 0 starts in the right state.  Its path, then that of the lane it met,
+//   and so on is the right one; along it the state at every cut and the number
+//   of symbols before it are known.
+// * A last pass decodes every run from its right start and puts the symbols to
+//   their places.
+//
+// A path may meet any other that passes the same node, so with short runs they
+// meet sooner: 64 Ki symbols, steps until the last of all lanes has met one:
+// 6900 with 32 lanes, 5500 with 64, 4500 with 128, 3400 with 256 (8200 with 128
+// lanes that each walked its run again from its neighbour's end until no start
+// changed).  Walks that have ended leave their lanes idle, so the ones that go
+// on are gathered into fewer warps.  What bounds it: in launches of few chunks
+// the latency of a step (54 cycles: the table read, two shifts, an add) times
+// those steps; in large ones shared memory (a look-up of 32 lanes takes 3.4
+// passes) and the issue slots, 2.7 to 4.3 look-ups per symbol.  A 4096 x 4096
+// bf16 tensor in 256 chunks: 646 -> 287 us.
 //
 // Table: one word per state, bit count (low five bits: what a funnel shift
-// takes of it) | symbol << 8 | shared-memory address of the baseline's entry <<
-// 16, so that the next entry's address is one multiply-add from the bits.
-constexpr uint32_t TANS_MIN_RUN = 256;        // symbols per lane at least: a short chunk is mostly serial, and every round costs a few hundred cycles beside its symbols
+// takes of it) | symbol << 8 | byte offset of the baseline's entry << 16.
+constexpr uint32_t TANS_MIN_RUN = 64, TANS_SHORT = 3000, TANS_SHORT_RUN = 256;  // symbols per lane at least; in chunks shorter than TANS_SHORT, which are mostly serial
+constexpr uint32_t TANS_GATHER = 512;          // symbols between two looks at how many walks are left
 constexpr uint32_t TANS_GROUP_BITS = 8 * 11;  // a group of eight symbols takes at most this many
 
-// Builds one chunk's table with a full warp (mod.rs:199-211,346-369); false on a bad header.  `work` holds 512 words.
-__device__ __forceinline__ bool tans_build(const uint8_t* src, uint32_t nsym, uint32_t* table, uint32_t* work, uint32_t lane) {
-    const uint32_t base = uint32_t(__cvta_generic_to_shared(table));
-    uint32_t* count = work;  // per symbol; while the states are numbered: the next occurrence's number
-    uint32_t* first = work + 256;
-    for (uint32_t i = lane; i < 256; i += 32) count[i] = 0;
-    __syncwarp();
-    uint32_t sum = 0;
-    bool bad = false;
-    for (uint32_t i = lane; i < nsym; i += 32) {
-        const uint32_t sy = src[3 + 3 * i], fr = uint32_t(src[4 + 3 * i]) | uint32_t(src[5 + 3 * i]) << 8;
-        bad |= fr == 0 || fr > 2048;             // mod.rs:404-411 (above 2048 the sum cannot come out right)
-        bad |= atomicExch(&count[sy], fr) != 0;  // a symbol listed twice
-        sum += fr;
+// SEGS: nodes per run; SLOTS: paths a node can hold when every lane has a run (a power of two; what finds no room is met later);
+// BLOCKS: per SM.
+template <int LANES> struct TansShape;
+template <> struct TansShape<32> { static constexpr uint32_t SEGS = 2, SLOTS = 2, BLOCKS = 16; };
+template <> struct TansShape<64> { static constexpr uint32_t SEGS = 1, SLOTS = 4, BLOCKS = 12; };
+template <> struct TansShape<128> { static constexpr uint32_t SEGS = 1, SLOTS = 8, BLOCKS = 6; };
+template <> struct TansShape<256> { static constexpr uint32_t SEGS = 1, SLOTS = 8, BLOCKS = 4; };
+
+template <int LANES>
+struct TansShared {
+    static constexpr uint32_t NODES = LANES * TansShape<LANES>::SEGS, SLOTS = TansShape<LANES>::SLOTS;
+    uint32_t table[2048];
+    uint32_t ring[20 * LANES];      // 64 bytes of stream per lane, the last 16 twice; while the table is built: work space
+    uint32_t key[NODES * SLOTS];   // 0 or 1 << 31 | lane << 16 | bits below the node << 11 | state
+    uint32_t count[NODES * SLOTS]; // symbols of that lane so far
+    uint32_t link[LANES];          // the entry the lane met, or a TANS_ value
+    uint32_t met[LANES];           // its symbols up to there
+    uint32_t from[LANES];          // node from which its path is the right one
+    uint32_t base[LANES];          // symbols of the chunk minus symbols of the lane, on its right part
+    uint32_t start[LANES];         // bits below the cut << 11 | state: the right start of the run
+    uint32_t at[LANES];            // symbols before it
+    uint32_t tally[LANES / 32];    // walks of each warp
+};
+constexpr uint32_t TANS_PAUSED = 0xFFFFFFFFu, TANS_FINISHED = 0xFFFFFFFEu, TANS_DEAD = 0xFFFFFFFDu, TANS_NONE = 0xFFFFFFFFu;
+
+// All lanes of a chunk.
+template <int LANES>
+__device__ __forceinline__ void tans_sync() {
+    if (LANES == 32) __syncwarp();
+    else __syncthreads();
+}
+
+// Builds one chunk's table (mod.rs:199-211,346-369); false on a bad header.  `work` holds 384 words and 128 for every warp.
+template <int LANES>
+__device__ __forceinline__ bool tans_build(const uint8_t* src, uint32_t nsym, uint32_t* table, uint32_t* work) {
+    constexpr uint32_t WARPS = LANES / 32, ROWS = 64 / WARPS;  // rows of 32 states to a warp
+    const uint32_t l = threadIdx.x, lane = l % 32, warp = l / 32;
+    uint32_t* count = work;  // per symbol
+    uint16_t* first = reinterpret_cast<uint16_t*>(work + 256);  // its place among the symbols in order
+    uint16_t* next = reinterpret_cast<uint16_t*>(work + 384) + 256 * warp;  // the number of its next occurrence in the warp's rows
+    for (uint32_t i = l; i < 256; i += LANES) count[i] = 0;
+    tans_sync<LANES>();
+    if (warp == 0) {
+        uint32_t sum = 0;
+        bool bad = false;
+        for (uint32_t i = lane; i < nsym; i += 32) {
+            const uint32_t sy = src[3 + 3 * i], fr = uint32_t(src[4 + 3 * i]) | uint32_t(src[5 + 3 * i]) << 8;
+            bad |= fr == 0 || fr > 2048;             // mod.rs:404-411 (above 2048 the sum cannot come out right)
+            bad |= atomicExch(&count[sy], fr) != 0;  // a symbol listed twice
+            sum += fr;
+        }
+        sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+        if (__any_sync(0xFFFFFFFFu, bad) || sum != 2048) { if (lane == 0) count[0] = ~0u; }
+        __syncwarp();
+        uint32_t mine = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) mine += count[lane * 8 + k];
+        uint32_t run = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, run, d); if (lane >= uint32_t(d)) run += t; }
+        run -= mine;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { first[lane * 8 + k] = uint16_t(run); run += count[lane * 8 + k]; }
     }
-    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
-    __syncwarp();
-    if (__any_sync(0xFFFFFFFFu, bad) || sum != 2048) return false;
-    uint32_t mine = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) mine += count[lane * 8 + k];
-    uint32_t run = mine;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, run, d); if (lane >= uint32_t(d)) run += t; }
-    run -= mine;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { first[lane * 8 + k] = run; run += count[lane * 8 + k]; }
-    __syncwarp();
-    // position k of the symbols in order goes to state 1283 k mod 2048; lane l places positions 64 l .. 64 l + 63
+    tans_sync<LANES>();
+    if (count[0] == ~0u) return false;
+    // position k of the symbols in order goes to state 1283 k mod 2048
+    constexpr uint32_t EACH = 2048 / LANES;
     uint32_t sy = 0;
-    for (uint32_t d = 128; d; d >>= 1) if (sy + d < 256 && first[sy + d] <= 64 * lane) sy += d;
-    for (uint32_t k = 64 * lane; k < 64 * lane + 64; ++k) {
+    for (uint32_t d = 128; d; d >>= 1) if (sy + d < 256 && first[sy + d] <= EACH * l) sy += d;
+    for (uint32_t k = EACH * l; k < EACH * l + EACH; ++k) {
         while (sy < 255 && first[sy + 1] <= k) ++sy;
         table[(k * 1283u) & 2047u] = sy;
     }
-    __syncwarp();
-    for (uint32_t u0 = 0; u0 < 2048; u0 += 32) {  // the states of a symbol are numbered in increasing order, from its frequency on
-        const uint32_t s = table[u0 + lane], same = __match_any_sync(0xFFFFFFFFu, s), before = same & ((1u << lane) - 1u);
-        const uint32_t x = count[s] + __popc(before), nb = 11 - (31 - __clz(x));
+    tans_sync<LANES>();
+    // The states of a symbol are numbered in increasing order, from its frequency on: every warp counts the symbols of its rows,
+    // the counts are summed over the warps before it, and the rows are gone through once more.
+    uint32_t* rows = table + warp * ROWS * 32 + lane;
+    if (WARPS > 1) {
+        for (uint32_t i = lane; i < 128; i += 32) reinterpret_cast<uint32_t*>(next)[i] = 0;
         __syncwarp();
-        table[u0 + lane] = nb | s << 8 | (base + 4 * ((x << nb) - 2048u)) << 16;
-        if (!before) count[s] += __popc(same);
-        __syncwarp();
+#pragma unroll 4
+        for (uint32_t r = 0; r < ROWS; ++r) {
+            const uint32_t s = rows[32 * r], same = __match_any_sync(0xFFFFFFFFu, s);
+            if ((same & ((1u << lane) - 1u)) == 0) next[s] += uint16_t(__popc(same));
+            __syncwarp();
+        }
+        tans_sync<LANES>();
     }
+    for (uint32_t s = l; s < 256; s += LANES) {
+        uint32_t run = count[s];
+        uint16_t* q = reinterpret_cast<uint16_t*>(work + 384) + s;
+        for (uint32_t w = 0; w < WARPS; ++w, q += 256) { const uint32_t t = *q; *q = uint16_t(run); run += t; }
+    }
+    tans_sync<LANES>();
+    constexpr uint32_t UNROLL = ROWS < 8 ? ROWS : 8;
+    for (uint32_t r0 = 0; r0 < ROWS; r0 += UNROLL) {
+        uint32_t s[UNROLL], same[UNROLL];
+#pragma unroll
+        for (uint32_t k = 0; k < UNROLL; ++k) s[k] = rows[32 * (r0 + k)];
+#pragma unroll
+        for (uint32_t k = 0; k < UNROLL; ++k) same[k] = __match_any_sync(0xFFFFFFFFu, s[k]);
+#pragma unroll
+        for (uint32_t k = 0; k < UNROLL; ++k) {
+            const uint32_t before = same[k] & ((1u << lane) - 1u);
+            const uint32_t x = next[s[k]] + __popc(before), nb = 11 - (31 - __clz(x));
+            __syncwarp();
+            rows[32 * (r0 + k)] = nb | s[k] << 8 | ((x << nb) - 2048u) << 18;
+            if (!before) next[s[k]] = uint16_t(x + __popc(same[k]));
+            __syncwarp();
+        }
+    }
+    tans_sync<LANES>();
     return true;
 }
 
-template <int THREADS>
-struct TansShared {
-    uint32_t table[2048];
-    uint32_t ring[32 * THREADS];  // 64 bytes of stream per lane, kept twice; while the tables are built: 512 words of work space
-    uint64_t words[THREADS];      // what the lanes hand on: the place a run ended at; counts of the warps before
-    uint32_t built;
-};
-template <int THREADS>
-__device__ __forceinline__ void tans_sync() { if (THREADS == 32) __syncwarp(); else __syncthreads(); }
+// Merges a chunk in the block that decoded one of its planes: that plane's bytes lie at `stage`, the end of the chunk's own output
+// [dst, dst + n * element size).  Elements go to their places in tiles of ascending position, each read whole before any of it is
+// written: a tile's elements end at or below the bytes of the next one's symbols.
+template <int LANES, int NP>
+__device__ __forceinline__ void merge_in_place(const Bases& bases, const DecodeItem& it, uint8_t* dst, const uint8_t* stage) {
+    constexpr int U = NP == 2 ? 2 : 1;  // groups of sixteen elements per thread and tile, all their loads in flight together
+    const int kind = it.kind;
+    const uint32_t eb = uint32_t(kind_elem_bytes(kind)), n = it.n;
+    const uint8_t* src[NP];
+    int j = 0;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) src[p] = p == it.slot ? stage : rd(bases, it.partner[j++]);
+    auto slow = [&](uint32_t begin, uint32_t end) {
+        for (; begin < end; begin += 8 * LANES) {
+            const uint32_t pos = begin + 8 * threadIdx.x, count = pos >= end ? 0 : end - pos < 8 ? end - pos : 8;
+            uint64_t b[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int p = 0; p < NP; ++p) b[p] = ld_bytes(src[p] + pos, count);
+            tans_sync<LANES>();
+            if (count) compose_store(kind, dst, pos, count, b);
+        }
+    };
+    // the groups whose aligned blocks lie inside the planes whatever their alignment: not the first and not the last two
+    uint32_t head = uint32_t((16 - ((reinterpret_cast<uintptr_t>(dst) / eb) & 15)) & 15) + 16;
+    if (head > n) head = n;
+    const uint32_t full = n - head < 48 ? 0 : (n - head - 32) >> 4;
+    slow(0, head);
+    for (uint32_t g0 = 0; g0 < full; g0 += LANES * U) {
+        uint4 cur[U][NP], nxt[U][NP];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t g = g0 + u * LANES + threadIdx.x;
+            if (g < full) {
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const uintptr_t at = reinterpret_cast<uintptr_t>(src[p]) + head + g * 16;
+                    const uint4* q = reinterpret_cast<const uint4*>(at & ~uintptr_t(15));
+                    cur[u][p] = *q;
+                    if (at & 15) nxt[u][p] = q[1];
+                }
+            }
+        }
+        tans_sync<LANES>();
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t g = g0 + u * LANES + threadIdx.x;
+            if (g < full) {
+                uint32_t pw[4][4];
+#pragma unroll
+                for (int p = 0; p < NP; ++p) extract16(cur[u][p], nxt[u][p], uint32_t(reinterpret_cast<uintptr_t>(src[p]) + head) & 15u, pw[p]);
+                merge_store16(kind, dst + size_t(head + g * 16) * eb, pw);
+            }
+        }
+    }
+    slow(head + full * 16, n);
+}
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) tans_decode_kernel(const DecodeItem* __restrict__ items, Bases bases, uint32_t* __restrict__ status) {
-    __shared__ TansShared<THREADS> sh;
-    constexpr uint32_t WORD = THREADS * 4;  // bytes between two words of a lane's ring
+template <int LANES>
+__global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_kernel(const DecodeItem* __restrict__ items, Bases bases, uint32_t* __restrict__ status) {
+    extern __shared__ __align__(16) uint8_t tans_smem[];
+    typedef TansShared<LANES> Shared;
+    constexpr uint32_t SEGS = TansShape<LANES>::SEGS, SLOTS = TansShape<LANES>::SLOTS;
+    constexpr uint32_t WORD = LANES * 4;  // bytes between two words of a lane's ring
+    Shared& sh = *reinterpret_cast<Shared*>(tans_smem);
     const uint32_t l = threadIdx.x;
     const DecodeItem it = items[blockIdx.x];
     const uint8_t* src = rd(bases, it.src);
-    const uint32_t table = uint32_t(__cvta_generic_to_shared(sh.table));
 
     // ---- header (mod.rs:388-425) and table ----
     uint32_t nsym = 0;
@@ -1330,49 +1501,60 @@ __global__ void __launch_bounds__(THREADS) tans_decode_kernel(const DecodeItem* 
         total_bits = uint64_t(ld_u32_unaligned(bs - 8)) | uint64_t(ld_u32_unaligned(bs - 4)) << 32;
         bad = total_bits > uint64_t(it.src_len - (3 + nsym * 3 + 8)) * 8;
     }
-    if (l < 32) {
-        const bool ok = !bad && tans_build(src, nsym, sh.table, sh.ring, l);
-        if (l == 0) sh.built = ok;
-    }
-    tans_sync<THREADS>();
-    // A symbol takes at most eleven bits, and so does the first state: what is longer cannot be used up.  (Lane positions are 32-bit
-    // offsets: without this a stream of more than 2^32 bits for few symbols would come out right modulo 2^32.)
-    uint32_t err = bad || !sh.built ? uint32_t(ST_BAD_HEADER) : total_bits < 11 ? uint32_t(ST_STREAM_UNDERRUN)
+    for (uint32_t i = l; i < Shared::NODES * SLOTS; i += LANES) sh.key[i] = 0;
+    sh.link[l] = TANS_PAUSED;
+    bad = bad || !tans_build<LANES>(src, nsym, sh.table, sh.ring);
+    // A symbol takes at most eleven bits, and so does the first state: what is longer cannot be used up.
+    uint32_t err = bad ? uint32_t(ST_BAD_HEADER) : total_bits < 11 ? uint32_t(ST_STREAM_UNDERRUN)
                  : total_bits > 11 * (uint64_t(it.n) + 1) ? uint32_t(ST_NOT_CONSUMED) : uint32_t(ST_OK);
     if (err) { if (l == 0) report(status, it.id, err); return; }
 
     // ---- runs ----
     // LIFO reader (mod.rs:118-147): the stream is read from its last bit down.
-    const uint32_t runs = it.n / TANS_MIN_RUN < 1 ? 1u : it.n / TANS_MIN_RUN > THREADS ? uint32_t(THREADS) : it.n / TANS_MIN_RUN;
-    auto cut = [&](uint32_t k) -> uint64_t { return k >= runs ? 0 : total_bits - total_bits * k / runs; };  // bits left at the start of run k
-    // Positions of a lane are 32-bit offsets in bits from `org`, a 16-byte aligned address at least 112 bytes below the end of
-    // its run (the stream may be longer than 2^32 bits, a run is not).
+    uint32_t runs = it.n / (it.n < TANS_SHORT ? TANS_SHORT_RUN : TANS_MIN_RUN);
+    if (runs > LANES) runs = LANES;
+    if (uint64_t(runs) * (32 * SEGS) > total_bits) runs = uint32_t(total_bits) / (32 * SEGS);  // nodes at least 32 bits apart
+    if (runs < 1) runs = 1;
+    const uint64_t apart = total_bits / (runs * SEGS);
+    uint32_t slots = SLOTS;  // short runs leave more paths to a node, and fewer nodes
+    while (slots < 32 && slots * 2 * runs <= SLOTS * LANES) slots *= 2;
+    const uint32_t last_node = (runs - 1) * SEGS;  // start of the last run, whose symbols are what is left of the chunk's
     const uint64_t floor_bit = uint64_t(reinterpret_cast<uintptr_t>(bs)) * 8;  // bit address of the stream's first bit
-    const uint64_t org_bit = ((floor_bit + cut(l + 1)) & ~uint64_t(127)) - 1024;
-    const uintptr_t org = uintptr_t(org_bit >> 3);
-    const uint32_t start_at = uint32_t(floor_bit + cut(l) - org_bit), end_at = uint32_t(floor_bit + cut(l + 1) - org_bit);
+    const uint64_t top_bit = floor_bit + total_bits;
     const uintptr_t lo16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_first) & ~uintptr_t(15);
     const uintptr_t hi16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_end + 15) & ~uintptr_t(15);
 
-    // The decoder: bits left (from org), address of its state's table entry, and a window on the stream: a 64-byte ring in shared
-    // memory, filled downward in aligned 16-byte blocks one step ahead of use.  Word w of the lane's column holds the stream word
-    // at byte offset 4 w (mod 64) and so does word w + 16, so that the words below any word are at fixed distances.  The lanes
-    // drain at similar rates: when any lane of the warp runs low every one with room takes a block.
-    uint32_t at = 0, entry = table, fetched = 0;
+    // The decoder: bits left (32-bit offset from `org`), byte offset of its state's table entry, and a window on the stream: a 64-byte
+    // ring in shared memory, filled downward in aligned 16-byte blocks one step ahead of use.  Word w of the lane's column is row
+    // 4 + w; rows 0 to 3 repeat the last four, so that the words below any word are at fixed distances.  The lanes drain at
+    // similar rates: when any lane of the warp runs low every one with room takes a block.  `org` lies on a 64-byte boundary, at
+    // least 128 bytes below what the lane is on its way to, and moves along (the stream may be longer than 2^32 bits).
+    uintptr_t org = 0;
+    uint32_t at = 0, entry = 0, fetched = 0;
     uint4 pending;
     uint8_t* ring = reinterpret_cast<uint8_t*>(sh.ring) + l * 4;
     auto park = [&](uint32_t off, const uint4& v) {
-        uint8_t* r = ring + ((off >> 2) & 15u) * WORD;
+        const uint32_t row = (off >> 2) & 12u;
+        uint8_t* r = ring + (row + 4) * WORD;
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            *reinterpret_cast<uint32_t*>(r + k * WORD) = w[k];
-            *reinterpret_cast<uint32_t*>(r + (16 + k) * WORD) = w[k];
+        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint32_t*>(r + k * WORD) = w[k];
+        if (row == 12) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) *reinterpret_cast<uint32_t*>(ring + k * WORD) = w[k];
         }
     };
-    auto begin = [&](uint32_t bit, uint32_t state) {
-        at = bit; entry = table + 4 * state;
-        fetched = (bit >> 3 & ~15u) - 32;
+    auto head_for = [&](uint64_t bit) -> uint32_t {  // moves `org` to suit a walk down to this bit address; its offset
+        const uintptr_t to = uintptr_t(bit >> 9 << 6) - 128;
+        const uint32_t down = uint32_t(org - to);
+        at += down * 8; fetched += down;
+        org = to;
+        return uint32_t(bit - uint64_t(to) * 8);
+    };
+    auto begin = [&](uint64_t bit, uint32_t state, uint64_t down_to) {
+        org = uintptr_t(down_to >> 9 << 6) - 128;
+        at = uint32_t(bit - uint64_t(org) * 8); entry = 4 * state;
+        fetched = (at >> 3 & ~15u) - 32;
         uint4 b[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) b[k] = fetch16(org + fetched + 16 * k, lo16, hi16);
@@ -1380,206 +1562,286 @@ __global__ void __launch_bounds__(THREADS) tans_decode_kernel(const DecodeItem* 
 #pragma unroll
         for (int k = 0; k < 3; ++k) park(fetched + 16 * k, b[k]);
     };
-    auto refill = [&]() {  // at least sixteen bytes below the word in use
-        const uint32_t have = (at >> 3 & ~3u) + 4 - fetched;
-        if (__any_sync(__activemask(), have < 32)) {
+    auto refill = [&]() {  // at least 28 bytes below the word in use: two groups and the window
+        for (;;) {
+            const uint32_t have = (at >> 3 & ~3u) + 4 - fetched;
+            if (!__any_sync(__activemask(), have < 32)) break;
             if (have <= 48) { fetched -= 16; park(fetched, pending); pending = fetch16(org + fetched - 16, lo16, hi16); }
         }
     };
-    auto state_now = [&]() -> uint32_t { return (entry - table) >> 2; };
-    auto load_entry = [&]() -> uint32_t { uint32_t e; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(entry)); return e; };
+    const uint8_t* table = reinterpret_cast<const uint8_t*>(sh.table);
     uint32_t w;  // the next bits, highest first
     auto step = [&]() -> uint32_t {  // one symbol's entry; takes its bits off the window
-        const uint32_t e = load_entry();
+        const uint32_t e = *reinterpret_cast<const uint32_t*>(table + entry);
         entry = (e >> 16) + 4 * __funnelshift_l(w, 0u, e);  // inside the table whatever the stream holds: the baseline has its low bits clear
         w = __funnelshift_l(0u, w, e);
         return e;
     };
-    auto word_below = [&](uint32_t k) -> uint32_t {  // k words below the one that holds the next bit
-        return *reinterpret_cast<const uint32_t*>(ring + (((at >> 5) & 15u) + 16 - k) * WORD);
+    // The next 96 bits in three words.
+    auto window = [&](uint32_t& h0, uint32_t& h1, uint32_t& h2) {
+        const uint8_t* r = ring + (((at >> 5) & 15u) + 4) * WORD;
+        const uint32_t w3 = *reinterpret_cast<const uint32_t*>(r), w2 = *reinterpret_cast<const uint32_t*>(r - WORD), w1 = *reinterpret_cast<const uint32_t*>(r - 2 * WORD),
+                       w0 = *reinterpret_cast<const uint32_t*>(r - 3 * WORD);
+        h0 = __funnelshift_r(w2, w3, at); h1 = __funnelshift_r(w1, w2, at); h2 = __funnelshift_r(w0, w1, at);
     };
-    auto open_window = [&]() { w = __funnelshift_r(word_below(1), word_below(0), at); };
-    // Eight symbols in two halves with a window of 32 bits each; the few groups with a half that takes more are decoded again in
-    // pairs (22 bits at most).
-    auto group = [&](uint32_t e[8]) {
-        const uint32_t entry0 = entry, w2 = word_below(0), w1 = word_below(1), w0 = word_below(2);
-        const uint32_t high = __funnelshift_r(w1, w2, at), low = __funnelshift_r(w0, w1, at);
-        uint32_t used = 0, more = 0;
-        w = high;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { e[j] = step(); used += e[j]; }
-        used &= 0xFFu;  // 44 at most: the sum of four bit counts stays below the symbols
-        w = __funnelshift_lc(low, high, used);
-#pragma unroll
-        for (int j = 4; j < 8; ++j) { e[j] = step(); more += e[j]; }
-        more &= 0xFFu;
-        if (used > 32 || more > 32) {
-            entry = entry0;
-            used = more = 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if ((j & 1) == 0) { at -= used & 0xFFu; used = 0; open_window(); }
-                e[j] = step(); used += e[j];
-            }
-            used &= 0xFFu;
-        }
-        at -= used + more;
+    // Eight symbols.  Two take at most 22 bits and four 44, so that 32 fresh bits for every two need no check.  `each` gets the
+    // number and the bits of every symbol.
+    auto group = [&](auto&& each) {
+        uint32_t h0, h1, h2;
+        window(h0, h1, h2);
+        w = h0;
+        uint32_t e0 = step(); each(0, e0);
+        uint32_t e1 = step(); each(1, e1);
+        uint32_t two = (e0 + e1) & 31u;  // the low five bits of the sum: 22 at most
+        w = __funnelshift_l(h1, h0, two);
+        e0 = step(); each(2, e0);
+        e1 = step(); each(3, e1);
+        uint32_t used = two + ((e0 + e1) & 31u);
+        const bool far = used >= 32;
+        const uint32_t g0 = __funnelshift_l(far ? h2 : h1, far ? h1 : h0, used), g1 = __funnelshift_l(far ? 0u : h2, far ? h2 : h1, used);
+        w = g0;
+        e0 = step(); each(4, e0);
+        e1 = step(); each(5, e1);
+        two = (e0 + e1) & 31u;
+        w = __funnelshift_l(g1, g0, two);
+        e0 = step(); each(6, e0);
+        e1 = step(); each(7, e1);
+        used += two + ((e0 + e1) & 31u);
+        return used;
     };
-    auto four = [&]() {  // four symbols of a walk
-        const uint32_t entry0 = entry;
-        open_window();
-        uint32_t used = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) used += step();
-        used &= 0xFFu;
-        if (used > 32) {
-            entry = entry0;
-            used = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if ((j & 1) == 0) { at -= used & 0xFFu; used = 0; open_window(); }
-                used += step();
-            }
-            used &= 0xFFu;
-        }
-        at -= used;
-    };
-    auto one = [&]() -> uint32_t {  // one symbol on its own
-        open_window();
-        const uint32_t e = step();
-        at -= e & 31u;
-        return e;
-    };
-    // from (bits below the cut << 11 | state) down to the end of the run: the symbols met
-    auto walk = [&](uint32_t start) -> uint32_t {
-        uint32_t n = 0;
-        begin(start_at - (start >> 11), start & 2047u);
-        while (int32_t(at - end_at) >= int32_t(TANS_GROUP_BITS) && n < it.n) {
-            uint32_t e[8];
+    // ---- walks ----
+    uint32_t who = l, node = l * SEGS, n = 0;  // the walk the lane is on, the node behind it, symbols since its start
+    bool alive = l + 1 < runs;
+    auto segment = [&]() -> uint32_t {  // on to the next node: the symbols met
+        const uint32_t n0 = n;
+        ++node;
+        const uint32_t stop = head_for(top_bit - node * apart);
+        while (int32_t(at - stop) >= int32_t(2 * TANS_GROUP_BITS) && n < it.n) {
             refill();
-            group(e);
-            n += 8;
+            at -= group([](int, uint32_t) {});
+            at -= group([](int, uint32_t) {});
+            n += 16;
         }
-        while (int32_t(at - end_at) >= int32_t(TANS_GROUP_BITS / 2) && n < it.n) {
+        while (int32_t(at - stop) > 0 && n < it.n) {  // up to the first boundary at or below the node
             refill();
-            four();
-            n += 4;
+            const uint32_t need = at - stop;
+            uint32_t bits = 0, taken = 0, there = 0, symbols = 0;
+            group([&](int, uint32_t e) {
+                const bool above = bits < need;
+                bits += e & 31u;
+                if (above) { taken = bits; there = entry; ++symbols; }
+            });
+            at -= taken; entry = there; n += symbols;
         }
-        for (uint32_t k = 0; int32_t(at - end_at) > 0 && n < it.n; ++k) {
-            if ((k & 7) == 0) refill();
-            one();
-            ++n;
+        if (int32_t(at - stop) > 0) {  // more symbols than the chunk has
+            alive = false;
+            sh.link[who] = TANS_DEAD;
+            return n - n0;
         }
-        return n;
+        const uint32_t pair = (stop - at) << 11 | entry >> 2, mine = 1u << 31 | who << 16 | pair;
+        for (uint32_t k = 0; k < slots; ++k) {
+            const uint32_t slot = node * slots + ((pair + k) & (slots - 1));
+            const uint32_t old = atomicCAS(&sh.key[slot], 0u, mine);
+            if (old == 0) { sh.count[slot] = n; break; }
+            if (((old ^ pair) & 0x7FFFu) == 0) {
+                alive = false;
+                sh.link[who] = slot; sh.met[who] = n;
+                break;
+            }
+        }
+        if (alive && node == last_node) { alive = false; sh.link[who] = TANS_FINISHED; sh.met[who] = n; }
+        return n - n0;
     };
-    const bool inner = l + 1 < runs;  // the last run's symbols are what is left of the chunk's
-    uint32_t from = 0, end = 0;
-    uint64_t mine = 0;
+    uint32_t start0 = 0;
     if (l == 0) {  // run 0 starts behind the eleven bits of the first state
         const uint64_t bit = total_bits - 11;
         const uint8_t* b = bs + (bit >> 3);
         const uint32_t three = uint32_t(b[0]) | uint32_t(b[1]) << 8 | ((bit & 7) > 5 ? uint32_t(b[2]) << 16 : 0u);
-        from = 11u << 11 | ((three >> (bit & 7)) & 2047u);
+        start0 = 11u << 11 | ((three >> (bit & 7)) & 2047u);
+        if (!alive) { sh.link[0] = TANS_FINISHED; sh.met[0] = 0; }
     }
-    // In round r the start of lane r is the right one at the latest.  A damaged or very uneven stream can hold the whole chunk's symbols, or
-    // more, in any run: a warp walks as many steps as the chunk has symbols from starts that may still change, and from then on a
-    // lane waits for its right one; and once the runs with right starts hold more symbols than the chunk, it is refused.  All
-    // of that together is at most a few times the chunk's symbols.
-    uint32_t spent = 0;
-    uint64_t settled = 0;
+    if (alive) begin(top_bit - node * apart - (start0 >> 11), start0 & 2047u, top_bit - (node + 1) * apart);
+    // A damaged or very uneven stream can hold the whole chunk's symbols, or more, between any two nodes: once a warp has walked three
+    // times the chunk's symbols the lanes only finish their runs, and the one with the right path goes on alone.  (So it is in
+    // streams of more than 2^31 bits, where a run whose right start found no room at its node must not become part of the one before.)
+    const uint64_t budget = total_bits >> 31 ? 0 : 3 * uint64_t(it.n);
+    uint64_t spent = 0;
+    // As walks end, the others move together into as few warps as hold them, every TANS_GATHER symbols or so.
+    uint32_t warps = LANES / 32, looks = 0;
+    const uint32_t every = uint32_t(uint64_t(TANS_GATHER) * runs * SEGS / it.n) + 1;
+    enum { ALL, OWN_RUN, ALONE } walks = ALL;
+    // The right path is followed from lane 0's on, once nothing moves any more.
+    uint32_t lane = 0;
+    int64_t base = 0;
     bool too_many = false;
-    bool go = inner;
-    for (uint32_t round = 0;; ++round) {
-        uint32_t met = 0;
-        if (go && (l <= round || spent < it.n)) {
-            met = walk(from);
-            mine = uint64_t(met) + (int32_t(at - end_at) > 0);  // still above the run's end: the bits of more symbols than the chunk has
-            end = (end_at - at) << 11 | state_now();
-            go = false;
+    for (;;) {
+        const bool go = alive && (walks == ALL ? spent < budget && (warps == 1 || looks < every) : walks == OWN_RUN ? node < (who + 1) * SEGS : who == lane);
+        if (__any_sync(0xFFFFFFFFu, go)) {
+            uint32_t met = 0;
+            if (go) met = segment();
+            spent += __reduce_max_sync(0xFFFFFFFFu, met);
+            ++looks;
+            continue;
         }
-        met = __reduce_max_sync(0xFFFFFFFFu, met);
-        spent = met > it.n - spent ? it.n : spent + met;
-        const uint32_t sure = round < runs ? round : runs - 1;
-        uint32_t want;
-        if (THREADS == 32) {
-            want = __shfl_up_sync(0xFFFFFFFFu, end, 1);
-            if (round < runs) settled += __shfl_sync(0xFFFFFFFFu, mine, sure);
-        } else {
-            sh.words[l] = mine << 32 | end;
-            __syncthreads();
-            want = l ? uint32_t(sh.words[l - 1]) : 0u;
-            if (round < runs) settled += sh.words[sure] >> 32;
-        }
-        too_many = settled > it.n;
-        const bool moved = l > 0 && l < runs && want != from;
-        if (moved) from = want;
-        go = (go || moved) && inner && !too_many;
-        if (THREADS == 32 ? !__any_sync(0xFFFFFFFFu, go) : !__syncthreads_or(go)) break;
-    }
-    // where the lane's symbols go: the counts of the lanes before it
-    uint64_t before_me, all;
-    {
-        uint64_t incl = mine;
+        if (walks == ALL) {
+            looks = 0;
+            if (LANES == 32) { walks = OWN_RUN; continue; }
+            const uint32_t votes = __ballot_sync(0xFFFFFFFFu, alive);
+            if (l % 32 == 0) sh.tally[l / 32] = __popc(votes);
+            if (__syncthreads_or(spent >= budget)) { walks = OWN_RUN; continue; }
+            uint32_t before = 0, total = 0;
 #pragma unroll
-        for (int s = 1; s < 32; s <<= 1) { const uint64_t t = __shfl_up_sync(0xFFFFFFFFu, incl, s); if (l % 32 >= uint32_t(s)) incl += t; }
-        all = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        before_me = incl - mine;
-        if (THREADS > 32) {
+            for (uint32_t v = 0; v < LANES / 32; ++v) { if (v < l / 32) before += sh.tally[v]; total += sh.tally[v]; }
+            const bool gather = (total + 31) / 32 < warps;
+            if (gather && alive) {  // every walk stands at a node
+                const uint32_t place = before + __popc(votes & ((1u << (l % 32)) - 1u));
+                const uint64_t bit = top_bit - node * apart;
+                sh.from[place] = who << 16 | node; sh.base[place] = n; sh.start[place] = uint32_t(bit - (uint64_t(org) * 8 + at)) << 11 | entry >> 2;
+            }
             __syncthreads();
-            if (l % 32 == 0) sh.words[l / 32] = all;
-            __syncthreads();
-            all = 0;
-            for (uint32_t w = 0; w < THREADS / 32; ++w) {
-                if (w < l / 32) before_me += sh.words[w];
-                all += sh.words[w];
+            if (gather) {
+                warps = (total + 31) / 32;
+                alive = l < total;
+                if (alive) {
+                    who = sh.from[l] >> 16; node = sh.from[l] & 0xFFFFu; n = sh.base[l];
+                    const uint32_t pair = sh.start[l];
+                    begin(top_bit - node * apart - (pair >> 11), pair & 2047u, top_bit - (node + 1) * apart);
+                }
+                __syncthreads();
+            }
+            if (total == 0) walks = OWN_RUN;
+            continue;
+        }
+        if (walks == OWN_RUN) {
+            sh.from[l] = TANS_NONE; sh.start[l] = TANS_NONE;
+            if (l == 0) { sh.start[0] = start0; sh.at[0] = 0; sh.from[0] = 0; sh.base[0] = 0; }
+            walks = ALONE;
+        }
+        tans_sync<LANES>();
+        uint32_t link;
+        while ((link = sh.link[lane]) < TANS_DEAD && !too_many) {
+            base += sh.met[lane];
+            too_many = base > int64_t(it.n);
+            base -= sh.count[link];
+            lane = (sh.key[link] >> 16) & 0x3FFu;
+            if (l == 0) { sh.from[lane] = link / slots; sh.base[lane] = uint32_t(base); }
+        }
+        if (too_many || link != TANS_PAUSED) {
+            too_many = too_many || link == TANS_DEAD || base + int64_t(sh.met[lane]) > int64_t(it.n);
+            break;
+        }
+        tans_sync<LANES>();
+    }
+    if (too_many) { if (l == 0) report(status, it.id, ST_NOT_CONSUMED); return; }  // more symbols than the chunk has
+    tans_sync<LANES>();
+    if (sh.from[l] != TANS_NONE) {  // the lane's path is right between these nodes: where it enters the runs
+        const uint32_t link = sh.link[l], base = sh.base[l], end = link < TANS_DEAD ? link / slots : last_node + 1;
+        for (uint32_t k = l == 0 ? 1 : (sh.from[l] + SEGS - 1) / SEGS; k * SEGS < end; ++k) {
+            for (uint32_t slot = k * SEGS * slots; slot < (k * SEGS + 1) * slots; ++slot) {
+                const uint32_t key = sh.key[slot];
+                if (key >> 16 == (0x8000u | l)) { sh.start[k] = key & 0x7FFFu; sh.at[k] = base + sh.count[slot]; }
             }
         }
     }
-    if (too_many || all > it.n) err = ST_NOT_CONSUMED;  // more symbols than the chunk has before its last run
-    if (!err && l < runs) {
-        // ---- last pass: the symbols to their places ----
-        const Epilogue ep = make_epilogue(bases, it);
-        const bool last = l + 1 == runs;
-        uint32_t pos = uint32_t(before_me), remaining = last ? it.n - uint32_t(all) : uint32_t(mine);
+    tans_sync<LANES>();
+    // ---- last pass: the symbols to their places ----
+    // With several warps the symbols of a plane that is merged go to the end of the chunk's own output and the block merges them from there,
+    // with coalesced accesses; a lone warp merges them as it decodes.
+    const bool staged = LANES > 32 && it.fused;
+    uint8_t* dst = wr(bases, it.dst);
+    uint8_t* stage = staged ? dst + size_t(it.n) * (uint32_t(kind_elem_bytes(it.kind)) - 1) : dst;
+    const uint32_t mine = l < runs ? sh.start[l] : TANS_NONE;
+    if (mine != TANS_NONE) {
+        uint32_t next = l + 1;
+        while (next < runs && sh.start[next] == TANS_NONE) ++next;  // no room for the right start at that cut
+        const bool last = next >= runs;
+        uint32_t pos = sh.at[l], remaining = (last ? it.n : sh.at[next]) - pos;
+        const uint64_t end_bit = last ? floor_bit : top_bit - next * SEGS * apart;
+        begin(top_bit - l * SEGS * apart - (mine >> 11), mine & 2047u, end_bit);
         // the last run may not read below the stream's first bit; the others are known to end well above theirs
-        const uint32_t floor_at = last ? end_at : end_at - 11 - TANS_GROUP_BITS;
-        begin(start_at - (from >> 11), from & 2047u);
+        const uint32_t floor_at = uint32_t(end_bit - uint64_t(org) * 8) - (last ? 0u : 11 + TANS_GROUP_BITS);
         if (int32_t(at - floor_at) < 0) err = ST_STREAM_UNDERRUN;
         auto one_checked = [&]() -> uint32_t {
             if (err) return 0;
-            if (at - floor_at < (load_entry() & 31u)) { err = ST_STREAM_UNDERRUN; return 0; }
-            return one();
+            if (at - floor_at < (*reinterpret_cast<const uint32_t*>(table + entry) & 31u)) { err = ST_STREAM_UNDERRUN; return 0; }
+            uint32_t h1, h2;
+            window(w, h1, h2);
+            const uint32_t e = step();
+            at -= e & 31u;
+            return (e >> 8) & 0xFFu;
         };
-        auto dec8 = [&](uint32_t& s_lo, uint32_t& s_hi) {
-            refill();
-            if (at - floor_at >= TANS_GROUP_BITS) {
-                uint32_t e[8];
-                group(e);
-                s_lo = __byte_perm(__byte_perm(e[0], e[1], 0x0051), __byte_perm(e[2], e[3], 0x0051), 0x5410);
-                s_hi = __byte_perm(__byte_perm(e[4], e[5], 0x0051), __byte_perm(e[6], e[7], 0x0051), 0x5410);
-            } else {
-                uint64_t syms = 0;
-#pragma unroll 1
-                for (int j = 0; j < 8; ++j) syms |= uint64_t((one_checked() >> 8) & 0xFFu) << (8 * j);
-                s_lo = uint32_t(syms); s_hi = uint32_t(syms >> 32);
-            }
-        };
-        auto short_group = [&](uint32_t g) {
+        // Symbols are decoded eight at a time from the start of the run and handed out eight at a time from the first boundary of the
+        // output on; `kept` holds the `keep` between the two.  `todo` more belong to the run: a run that another one follows may go on
+        // past its end, the last one may not.
+        uint64_t kept = 0;
+        uint32_t keep = 0, todo = remaining;
+        auto more = [&]() -> uint64_t {
             uint64_t syms = 0;
             refill();
-            for (uint32_t j = 0; j < g; ++j) syms |= uint64_t((one_checked() >> 8) & 0xFFu) << (8 * j);
-            emit(ep, pos, g, syms);
-            pos += g; remaining -= g;
+            if (at - floor_at >= TANS_GROUP_BITS && (todo >= 8 || !last)) {
+                uint32_t s[8];
+                at -= group([&](int j, uint32_t e) { s[j] = e; });
+                syms = uint64_t(__byte_perm(__byte_perm(s[4], s[5], 0x0051), __byte_perm(s[6], s[7], 0x0051), 0x5410)) << 32 |
+                       __byte_perm(__byte_perm(s[0], s[1], 0x0051), __byte_perm(s[2], s[3], 0x0051), 0x5410);
+                todo = todo > 8 ? todo - 8 : 0;
+            } else {
+#pragma unroll 1
+                for (int j = 0; j < 8 && todo; ++j, --todo) syms |= uint64_t(one_checked()) << (8 * j);
+            }
+            return syms;
         };
-        if (remaining) {
-            const uint32_t g = first_group(ep, pos, remaining);
-            if (g < 8 || remaining < 16) short_group(g);
+        if (LANES > 32) {
+            uint32_t g = uint32_t(8 - (reinterpret_cast<uintptr_t>(stage + pos) & 7));
+            while (remaining) {
+                if (g > remaining) g = remaining;
+                uint64_t syms = kept;
+                if (g > keep) {
+                    const uint64_t next = more();
+                    syms |= next << (8 * keep);
+                    kept = keep + 8 - g ? next >> (8 * (g - keep)) : 0;
+                    keep = keep + 8 - g;
+                } else { kept >>= 8 * g; keep -= g; }
+                uint8_t* to = stage + pos;
+                if (g == 8) *reinterpret_cast<uint64_t*>(to) = syms;
+                else for (uint32_t k = 0; k < g; ++k) to[k] = uint8_t(syms >> (8 * k));
+                pos += g; remaining -= g;
+                g = 8;
+            }
+        } else {
+            const Epilogue ep = make_epilogue(bases, it);
+            auto dec8 = [&](uint32_t& s_lo, uint32_t& s_hi) {
+                const uint64_t next = more(), out = kept | next << (8 * keep);
+                if (keep) kept = next >> (64 - 8 * keep);
+                s_lo = uint32_t(out); s_hi = uint32_t(out >> 32);
+            };
+            uint32_t g = remaining ? first_group(ep, pos, remaining) : 8;
+            if (g < 8) {
+                const uint64_t next = more();
+                emit(ep, pos, g, next);
+                kept = next >> (8 * g); keep = 8 - g;
+                pos += g; remaining -= g;
+            }
+            fast_groups(ep, it.n, pos, remaining, dec8);
+            while (remaining) {
+                g = remaining < 8 ? remaining : 8;
+                uint64_t syms = kept;
+                if (g > keep) {
+                    const uint64_t next = more();
+                    syms |= next << (8 * keep);
+                    if (keep) kept = next >> (64 - 8 * keep);
+                }
+                emit(ep, pos, g, syms);
+                pos += g; remaining -= g;
+            }
         }
-        fast_groups(ep, it.n, pos, remaining, dec8);
-        while (remaining) short_group(remaining < 8 ? remaining : 8);
-        if (!err && last && (at != floor_at || state_now() != 0)) err = ST_NOT_CONSUMED;  // mod.rs:442-449
+        if (!err && last && (at != floor_at || entry != 0)) err = ST_NOT_CONSUMED;  // mod.rs:442-449
     }
     if (err) report(status, it.id, err);
+    if (staged) {
+        tans_sync<LANES>();
+        if (it.kind == K_M32) merge_in_place<LANES, 4>(bases, it, dst, stage);
+        else merge_in_place<LANES, 2>(bases, it, dst, stage);
+    }
 }
 
 // The other kernel: a lane per stream, 32 chunks per block, for launches whose chunks fill the GPU that way (tans_lanes_win).
@@ -2062,22 +2324,46 @@ __global__ void __launch_bounds__(TANS_LANES_THREADS, 1) tans_lanes_decode_kerne
     if (!err && (cnt != 0 || rp != start || state != 0)) err = ST_NOT_CONSUMED;  // mod.rs:442-449
     if (err && live) report(status, it.id, err);
 }
-// `lanes`: the kernel with a lane per stream.
-inline void tans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, bool lanes, cudaStream_t st) {
-    // Four warps per chunk while an SM has no more than two chunks to itself: 0.56 against 0.62 ms for 256 chunks of 64 Ki symbols.
-    // Beyond that the warps of other chunks fill the gaps and the shorter rounds' overhead counts: 1794 chunks 0.82 ms with one
-    // warp each, 1.34 with four.  (Two chunks per warp, 16 lanes each: 0.91 ms, and 2.39 against 2.15 ms for 7637 chunks.)
-    if (lanes) tans_lanes_decode_kernel<<<(n + TANS_CTA_CHUNKS - 1) / TANS_CTA_CHUNKS, TANS_LANES_THREADS, TANS_LANES_SMEM, st>>>(items, n, bases, status);
-    else if (n <= 2 * 148) tans_decode_kernel<128><<<n, 128, 0, st>>>(items, bases, status);
-    else tans_decode_kernel<32><<<n, 32, 0, st>>>(items, bases, status);
+template <int LANES>
+inline void tans_launch_t(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, cudaStream_t st) {
+    tans_decode_kernel<LANES><<<n, LANES, sizeof(TansShared<LANES>), st>>>(items, bases, status);
+}
+// Lanes per chunk: many shorten a chunk's latency and cost more walks per symbol, so as many as the GPU has room for.  us with
+// 256 / 128 / 64 / 32 lanes, bf16: 64 Ki symbols, 148 chunks 256 / 257 / 364 / 498, 592: 351 / 340 / 438 / 589, 1184: 607 / 585 / 576 / 686,
+// 2368: 1120 / 909 / 928 / 907; 16 Ki, 296: 231 / 187 / 267 / 489, 1184: 452 / 355 / 351 / 659, 2368: 796 / 525 / 511 / 626; 8 Ki, 1776:
+// 479 / 378 / 417 / 561.  Runs that are long against the way to a meeting (`apart`, in symbols of 1,400) need fewer walks: 128 Ki, 3552 chunks
+// 2344 / 2050 / 2052 / 1881; fp8, 64 Ki, 2368: 2011 / 1667 / 1565 / 1396; fp16, 8 Ki, 2368: 398 / 321 / 298 / 248.  In chunks that are mostly
+// serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 176, 32: 113.
+inline uint32_t tans_lanes(uint32_t chunks, uint32_t longest, double apart) {
+    if (longest < TANS_SHORT) return chunks <= 4 * 148 ? 128 : 32;
+    if (chunks <= (longest <= 4096 ? 148 : 2 * 148)) return 256;
+    if (chunks <= 6 * 148) return 128;
+    if (chunks > 12 * 148 && longest > 65536 * apart) return 32;
+    return longest <= 8192 ? 128 : 64;
+}
+// `lanes` per chunk; 1: the kernel with a lane per stream.
+inline void tans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t lanes, cudaStream_t st) {
+    switch (lanes) {
+        case 256: tans_launch_t<256>(items, n, bases, status, st); break;
+        case 128: tans_launch_t<128>(items, n, bases, status, st); break;
+        case 64: tans_launch_t<64>(items, n, bases, status, st); break;
+        case 32: tans_launch_t<32>(items, n, bases, status, st); break;
+        default: tans_lanes_decode_kernel<<<(n + TANS_CTA_CHUNKS - 1) / TANS_CTA_CHUNKS, TANS_LANES_THREADS, TANS_LANES_SMEM, st>>>(items, n, bases, status);
+    }
+}
+template <int LANES>
+inline cudaError_t tans_allow_shared_t() {
+    const cudaError_t e = cudaFuncSetAttribute(tans_decode_kernel<LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TansShared<LANES>)));
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(tans_decode_kernel<LANES>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 inline cudaError_t tans_allow_shared() {
     cudaError_t e = cudaFuncSetAttribute(tans_lanes_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TANS_LANES_SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(tans_lanes_decode_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(tans_decode_kernel<128>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(tans_decode_kernel<32>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if ((e = tans_allow_shared_t<256>()) != cudaSuccess || (e = tans_allow_shared_t<128>()) != cudaSuccess ||
+        (e = tans_allow_shared_t<64>()) != cudaSuccess) return e;
+    return tans_allow_shared_t<32>();
 }
 
 // ---- Order1ScaleAC ---------------------------------------------------------
@@ -2346,41 +2632,7 @@ __global__ void __launch_bounds__(256) merge_kernel(const MergeItem* __restrict_
             if (off) { const uint4 nxt = load_block16_guarded(q + 16, p_lo[p], p_hi[p]); extract16(cur, nxt, off, pw[p]); }
             else { pw[p][0] = cur.x; pw[p][1] = cur.y; pw[p][2] = cur.z; pw[p][3] = cur.w; }
         }
-        uint8_t* out = dst + size_t(pos) * eb;
-        switch (int(it.kind)) {
-            case K_PASS: *reinterpret_cast<uint4*>(out) = make_uint4(pw[0][0], pw[0][1], pw[0][2], pw[0][3]); break;
-            case K_E4M3:
-            case K_E5M2: {
-                const bool e4m3 = it.kind == K_E4M3;
-                *reinterpret_cast<uint4*>(out) = make_uint4(compose_fp8x4(pw[0][0], pw[1][0], e4m3), compose_fp8x4(pw[0][1], pw[1][1], e4m3),
-                                                            compose_fp8x4(pw[0][2], pw[1][2], e4m3), compose_fp8x4(pw[0][3], pw[1][3], e4m3));
-                break;
-            }
-            case K_M16: {
-                uint4 v[2];
-                compose16x4(pw[0][0], pw[1][0], v[0].x, v[0].y); compose16x4(pw[0][1], pw[1][1], v[0].z, v[0].w);
-                compose16x4(pw[0][2], pw[1][2], v[1].x, v[1].y); compose16x4(pw[0][3], pw[1][3], v[1].z, v[1].w);
-                stg256(out, v[0], v[1]);
-                break;
-            }
-            default: {  // K_M32 (transforms/fusion.rs:287-292)
-#pragma unroll
-                for (int k = 0; k < 4; k += 2) {
-                    uint32_t w[8];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t t0 = __byte_perm(pw[0][k + h], pw[1][k + h], 0x5140), t1 = __byte_perm(pw[2][k + h], pw[3][k + h], 0x5140);
-                        const uint32_t t2 = __byte_perm(pw[0][k + h], pw[1][k + h], 0x7362), t3 = __byte_perm(pw[2][k + h], pw[3][k + h], 0x7362);
-                        w[4 * h + 0] = revert32(__byte_perm(t0, t1, 0x5410));
-                        w[4 * h + 1] = revert32(__byte_perm(t0, t1, 0x7632));
-                        w[4 * h + 2] = revert32(__byte_perm(t2, t3, 0x5410));
-                        w[4 * h + 3] = revert32(__byte_perm(t2, t3, 0x7632));
-                    }
-                    stg256(out + 16 * k, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
-                }
-                break;
-            }
-        }
+        merge_store16(int(it.kind), dst + size_t(pos) * eb, pw);
     }
 }
 

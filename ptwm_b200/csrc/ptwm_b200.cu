@@ -221,7 +221,7 @@ struct ptwm_b200_plan {
     // One launch of a decoder: a run of items of a list.  Items of the second phase that read planes the first one puts into
     // scratch must wait for it, the others need not.  rANS chunks with few distinct symbols go to the kernel with a symbol list
     // per lane; `size` is its rows there, the most distinct symbols of the run for the general kernel, the most cumulative
-    // tables of a chunk for Order1ScaleAC, and for tANS whether the kernel with a lane per stream takes it.
+    // tables of a chunk for Order1ScaleAC, and for tANS the kernel (tans_kernel).
     struct Launch { uint32_t first, count, size; bool waits, narrow; };
     std::vector<Launch> runs[2][4];
     // The same lists for launches in a row on one stream, where the items that wait have nothing to be kept apart from: a few of
@@ -358,32 +358,33 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
     }
 }
 
-// tANS chunks of one launch, longest first: is the kernel with a lane per stream the faster one?  It takes 148 us and 27 ns per symbol
-// of the longest chunk for every 4736 chunks (148 SMs x 32), and up to 3.3 times that per symbol where some lane in most rounds of 32 symbols
-// has four in a row that take more than 32 bits (8 groups, 32 lanes) and all of them go back.  With a warp per chunk a
-// launch takes about the latency of a chunk (30 us, and 25 ns per symbol of the first 12 Ki) and then its work: per chunk 16 to 28 ns,
-// 10 ps per symbol of the first 8 Ki (the runs falling in), and what placing a symbol costs, for 32-bit elements more the longer the
-// chunk.  Planes above four bits per symbol fall in sooner.  Fitted to 300 to 30,000 chunks of 256 to 131,072 symbols: the kernel it
-// picks is within 8 % of the faster one in nearly all of 314 launches measured.
-// us, lane per stream / warp per chunk: fp32, 16 Ki: 1200 chunks 599 / 518, 2400 599 / 700, 4736 601 / 1034, 14000 1775 / 2321;
-// bf16, 32 Ki: 2400 1023 / 756, 4736 1029 / 1262, 5500 2041 / 1331; bf16, 64 Ki: 4736 1897 / 1485; fp16, 16 Ki: 4736 634 / 534; bytes, 8 Ki:
-// 4736 357 / 674; bf16, half of it zeros, 16 Ki: 4736 2606 / 1435.
-bool tans_lanes_win(const DecodeItem* items, size_t n) {
+// tANS chunks of one launch, longest first: the kernel they go to, as tans_launch takes it.
+// The kernel with a lane per stream takes 148 us and 27 ns per symbol of the longest chunk for every 4736 chunks (148 SMs x 32), and up to
+// 3.3 times that per symbol where some lane in most rounds of 32 symbols has four in a row that take more than 32 bits (8 groups, 32
+// lanes) and all of them go back.  With several lanes per chunk a launch takes some 150 us and then its work: per chunk 16 to 28 ns,
+// 10 ps per symbol of the first 8 Ki (paths meeting), and what placing a symbol costs.  Planes above four bits per symbol meet sooner,
+// and so do nibbles.  Chunks below TANS_SHORT are next to serial.
+// us, lane per stream / several lanes: bf16, 4 Ki: 1184 chunks 259 / 236, 1776 258 / 320; 8 Ki: 1184 363 / 327, 2368 365 / 513; 16 Ki: 2368
+// 590 / 511, 3552 592 / 741; 32 Ki: 3552 1034 / 864, 4736 1031 / 1021; 64 Ki: 4736 1902 / 1481; fp32, 32 Ki: 2368 1041 / 674, 4736 1038 / 1122;
+// fp16, 32 Ki, 4736 1078 / 765; fp8, 8 Ki, 2368 694 / 793; bf16, half of it zeros, 16 Ki: 4736 2606 / 1435.
+uint32_t tans_kernel(const DecodeItem* items, size_t n) {
     constexpr size_t WAVE = 148 * TANS_CTA_CHUNKS;
-    double by_lanes = 0, wave = 0, latency = 0, work = 0;
-    for (size_t k = 0; k < n; ++k) {
+    double by_lanes = 0, wave = 0, work = n && items[0].n < TANS_SHORT ? 40 + 0.03 * items[0].n : 150, apart = 1;
+    bool placed = true;
+    for (size_t k = 0; k < n && placed; ++k) {
         const DecodeItem& it = items[k];
         const uint32_t eb = it.fused ? uint32_t(kind_elem_bytes(it.kind)) : 1u;
-        if (eb == 4 && it.slot != 3) return false;  // placed by its decoding warp alone there
+        placed = eb != 4 || it.slot == 3;  // otherwise its decoding warp alone places the elements there
         const double len = it.n, bits = 8.0 * (it.src_len > 200 ? it.src_len - 100 : it.src_len) / std::max(len, 1.0);  // a header is some 100 bytes
         const double q = double(it.row_len >> 16) / 2048, back = std::min(1.0, 256 * q * q * q * q), f = 4.2 / std::max(bits, 4.2), fall = f * f * f * f;
         if (k % WAVE == 0) { by_lanes += wave; wave = 0; }
         wave = std::max(wave, 148 + 0.0267 * len * (1 + 3.3 * back));
-        latency = std::max(latency, 30 + 0.025 * std::min(len, 12288 * fall));
-        const double place = eb == 1 ? 2e-6 : eb == 2 ? 2.2e-6 : len <= 16384 ? 2.4e-6 : len <= 32768 ? 4.2e-6 : len <= 65536 ? 5.5e-6 : 7.5e-6;
-        work += 0.016 + 1.2e-5 * std::min(len, 1024.0) + 1e-5 * std::min(len, 8192 * fall) + len * place;
+        if (k == 0) apart = fall * fall * (it.fused && eb == 1 ? 0.25 : 1);
+        work += it.n < TANS_SHORT ? 0.012 + 1.2e-5 * len
+                                  : 0.016 + 1.2e-5 * std::min(len, 1024.0) + 1e-5 * std::min(len, 8192 * fall) + len * (eb == 1 ? 2e-6 : eb == 2 ? 2.2e-6 : 2.6e-6);
     }
-    return by_lanes + wave < 0.95 * (latency + work);
+    if (placed && by_lanes + wave < work) return 1;
+    return tans_lanes(uint32_t(n), items[0].n, apart);
 }
 
 int codec_classes(const ptwm_b200_plan& pl) {
@@ -427,7 +428,7 @@ void finish_lists(ptwm_b200_plan& pl) {
                 add(pl.runs[ph][cc], true);
                 add(pl.in_row[ph][cc], false);
             }
-            if (cc == 2) for (auto* l : {&pl.runs[ph][cc], &pl.in_row[ph][cc]}) for (auto& r : *l) r.size = tans_lanes_win(&v[r.first], r.count);
+            if (cc == 2) for (auto* l : {&pl.runs[ph][cc], &pl.in_row[ph][cc]}) for (auto& r : *l) r.size = tans_kernel(&v[r.first], r.count);
             pl.launches += uint32_t((side_by_side ? pl.runs : pl.in_row)[ph][cc].size());
             for (auto& it : v) {
                 uint64_t np = it.fused ? uint64_t(kind_planes(it.kind)) : 1, eb = it.fused ? uint64_t(kind_elem_bytes(it.kind)) : 1;
@@ -547,7 +548,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
                 rans_launch(it, n, bases, status, pl.dec[ph][0].size() <= RANS_DIRECT_CHUNKS, r.narrow, r.size, s);
                 break;
             case 1: huffman_decode_kernel<<<(n + HUF_WARP_CHUNKS - 1) / HUF_WARP_CHUNKS, 32, HUF_SMEM, s>>>(it, n, bases, status); break;
-            case 2: tans_launch(it, n, bases, status, r.size != 0, s); break;
+            case 2: tans_launch(it, n, bases, status, r.size, s); break;
             default: o1sac_launch(it, n, bases, status, r.size, s); break;
         }
         CUDA_TRY(cudaGetLastError());
@@ -796,7 +797,7 @@ int64_t decode_plane_cuda(uint8_t sfv, const uint8_t* state, size_t state_len, c
     switch (codec) {
         case C_RANS: rans_launch(d_it, 1, bases, d_status, true, false, 0, st); break;
         case C_HUFFMAN: huffman_decode_kernel<<<1, 32, HUF_SMEM, st>>>(d_it, 1, bases, d_status); break;
-        case C_TANS: tans_launch(d_it, 1, bases, d_status, false, st); break;
+        case C_TANS: tans_launch(d_it, 1, bases, d_status, tans_lanes(1, uint32_t(decoded), 1), st); break;
         default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), st); break;
     }
     CUDA_TRY(cudaGetLastError());

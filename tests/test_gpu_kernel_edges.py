@@ -86,6 +86,36 @@ def test_tans_decode_with_a_lane_per_stream(dtype, chunks):
     check(specs, chunk_size=1029, forced_codec=TANS)
 
 
+@pytest.mark.parametrize("dtype", ["u8", "bf16", "fp32", "fp8"])
+@pytest.mark.parametrize("chunk, chunks", [(63, 3), (255, 3), (257, 3), (513, 600), (2999, 3), (3000, 297), (4097, 149), (16385, 2), (70001, 2), (3001, 889), (8193, 889), (3001, 1777)])
+def test_tans_decode_with_many_lanes_per_chunk(dtype, chunk, chunks):
+    # every number of lanes, with runs that fill them, fewer runs than lanes and a single one, odd lengths, and a short last chunk
+    n = chunk * chunks - chunk // 3
+    specs = [u8("p", plane("exponent", n))]
+    if dtype == "fp8":
+        t = weights(1, n, chunks, False).mul(40).to(torch.float8_e4m3fn)
+        specs = [oracle.TensorSpec("p", oracle.DT_E4M3, [n], t.view(torch.uint8).numpy().tobytes())]
+    elif dtype != "u8":
+        t = weights(1, n, chunks, False).to(torch.bfloat16 if dtype == "bf16" else torch.float32)
+        specs = [oracle.TensorSpec("p", oracle.DT_BF16 if dtype == "bf16" else oracle.DT_F32, [n], t.view(torch.uint8).numpy().tobytes())]
+    check(specs, chunk_size=chunk, forced_codec=TANS)
+
+
+@pytest.mark.parametrize("chunks", [1, 400, 1200])
+def test_tans_decode_of_uneven_streams(chunks):
+    # nearly all of the symbols in a small part of the bits: walks that meet late or never, and paths that are followed by one lane alone
+    rng = np.random.default_rng(chunks)
+    specs = []
+    for k, n in enumerate((3500, 20000, 65536) if chunks == 1 else (3500,)):
+        zeros = np.zeros(n * chunks, dtype=np.uint8)
+        half = zeros.copy(); half[::2 * n] = 1
+        for at in range(0, n * chunks, n): half[at + n // 2:at + n // 2 + n // 4] = rng.integers(0, 200, n // 4)
+        rare = (rng.random(n * chunks) < 0.001).astype(np.uint8)
+        period = np.resize(np.array([0, 0, 1, 0, 2], dtype=np.uint8), n * chunks)
+        specs += [u8(f"half{k}", half.tobytes()), u8(f"rare{k}", rare.tobytes()), u8(f"period{k}", period.tobytes())]
+    check(specs, chunk_size=len(specs[-1].raw) // chunks if chunks > 1 else None, forced_codec=TANS)
+
+
 def test_decode_two_coded_planes_in_many_chunks():
     # more chunks than are spread over scratch: the second plane's lanes merge with the first one, every codec on its own stream
     for menu in ((oracle.HUFFMAN, oracle.RANS, oracle.O1SAC), (oracle.TANS, oracle.O1SAC), (oracle.IDENTITY, oracle.HUFFMAN, oracle.RANS, oracle.TANS, oracle.O1SAC)):
