@@ -696,15 +696,16 @@ __device__ __forceinline__ void rans_group8(const uint32_t* tab, const uint32_t*
     }
 }
 
-// The same on a table with an entry per slot: frequency << 20 | slot's distance from the symbol's first << 8 | symbol.  From
-// one state to the next it is a mask, one shared-memory read, a shift and a multiply-add; renormalising picks among the state
-// shifted by none, one or two bytes, which are there by the time the comparisons are.  A state that has been normalised once
+// The same on a table with an entry per slot: slot's distance from the symbol's first << 20 | symbol << 12 | frequency, so that
+// both factors of the update are one step away.  From one state to the next it is a mask, one shared-memory read, a shift and a
+// multiply-add; renormalising moves the state shifted by one or two bytes over the state, two moves that hang on the comparisons
+// alone (a chunk of 64 Ki symbols in a call of its own 778 -> 751 us).  A state that has been normalised once
 // never needs more than two bytes (an update leaves at least 2^12), so eight bytes of stream last for four symbols and nothing
 // is decoded twice.  A stream whose stored initial state is not normalised goes byte by byte.
 __device__ __forceinline__ uint32_t rans_direct_lookup(const uint32_t* tab, uint32_t& x) {
     const uint32_t e = tab[x & 2047u];
-    x = (e >> 20) * (x >> 11) + ((e >> 8) & 0xFFFu);
-    return e;
+    x = (e & 0xFFFu) * (x >> 11) + (e >> 20);
+    return e >> 12;
 }
 // The ring's words are kept with their first byte on top here.
 __device__ __forceinline__ void rans_direct_short(const uint32_t* tab, const uint32_t* rw, uint32_t& x, uint32_t& rq, uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
@@ -731,11 +732,14 @@ __device__ __forceinline__ uint32_t rans_direct_four(const uint32_t* tab, const 
     for (int j = 0; j < 4; ++j) {
         const uint32_t e = rans_direct_lookup(tab, x);
         sy = __byte_perm(sy, e, (0x3210u & ~(0xFu << (4 * j))) | (4u << (4 * j)));
-        const uint32_t one = __byte_perm(x, wh, 0x2107), two = __byte_perm(x, wh, 0x1076);
-        const bool some = x < RANS_L, more = x < (RANS_L >> 8);
-        const uint32_t y = more ? two : one, sh = more ? 16u : 8u;
-        x = some ? y : x;
-        const uint32_t bits = some ? sh : 0u;
+        uint32_t bits;
+        asm("{\n\t.reg .pred some, more;\n\t.reg .u32 y;\n\t"
+            "setp.lt.u32 some, %0, 0x800000;\n\tsetp.lt.u32 more, %0, 0x8000;\n\t"
+            "mov.u32 y, %0;\n\tmov.u32 %1, 0;\n\t"
+            "@some prmt.b32 y, %0, %2, 0x2107;\n\t@some mov.u32 %1, 8;\n\t"
+            "@more prmt.b32 y, %0, %2, 0x1076;\n\t@more mov.u32 %1, 16;\n\t"
+            "mov.u32 %0, y;\n\t}"
+            : "+r"(x), "=&r"(bits) : "r"(wh));
         wh = __funnelshift_l(wl, wh, bits);
         wl <<= bits;
         used += bits;
@@ -860,7 +864,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
 #pragma unroll 8
             for (uint32_t u = lane; u < 2048; u += 32) {
                 const uint32_t w = tab[u >> 4], e = lst[(w >> 16) + __popc(w << ((~u & 15u) | 16u))];
-                slots[c2 * 2048 + u] = ((e >> 8) & 0xFFFu) << 20 | (u - (e >> 20)) << 8 | (e & 0xFFu);
+                slots[c2 * 2048 + u] = (u - (e >> 20)) << 20 | (e & 0xFFu) << 12 | ((e >> 8) & 0xFFFu);
             }
             __syncwarp();
         }
@@ -872,7 +876,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
     if (valid && !err && seg_len > 0) {
         if (my_len < 4) err = ST_STREAM_UNDERRUN;  // decompress.rs:82-86
         else {
-            const uint32_t* tab = DIRECT ? slots + c * 2048 : ranktab + c * 128;
+            const uint32_t* tab = DIRECT == 1 ? slots : DIRECT ? slots + c * 2048 : ranktab + c * 128;
             const uint32_t* lst = PER_LANE ? symlist + lane : symlist + c * l_entries;
             const uint32_t* rw = ring.base;
             Epilogue ep = make_epilogue(bases, it);
