@@ -696,18 +696,26 @@ __global__ void __launch_bounds__(32) rans_encode_kernel(const EncChunk* __restr
 // Huffman: the place of a symbol's bits follows from the lengths before it, so a warp codes a stream 512 symbols at a time:
 // every lane strings its sixteen codes together, a prefix sum over the lanes gives the bit each string starts at, and the
 // strings are put together in shared memory.  (One thread per stream took 107 ns per symbol.)
-constexpr uint32_t HENC_LANE = 16, HENC_WORDS = (32 * HENC_LANE * 11 + 31) / 32 + 2;
-__global__ void __launch_bounds__(128) huffman_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
-                                                             const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
-                                                             EncResult* __restrict__ results) {
-    __shared__ uint32_t codes[256];
-    __shared__ uint32_t words_all[4][HENC_WORDS];
-    const uint32_t ci = list[blockIdx.x], lane = threadIdx.x & 31, s = threadIdx.x >> 5;
+// WARPS > 1, for launches that do not fill the GPU: that many warps to a stream, each with a share of its rounds.  They first
+// count the bits of their shares; a word that two shares meet in is kept by both and put together at the end.
+constexpr uint32_t HENC_LANE = 16, HENC_WORDS = (32 * HENC_LANE * 11 + 31) / 32 + 2, HENC_ROUND = 32 * HENC_LANE;
+template <int WARPS>
+__global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
+                                                                     const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
+                                                                     EncResult* __restrict__ results) {
+    struct Shared {
+        uint32_t codes[256];
+        uint32_t words[4 * WARPS][HENC_WORDS];
+        uint64_t bits[4][WARPS];
+        uint32_t head_at[4][WARPS], head[4][WARPS], tail_at[4][WARPS], tail[4][WARPS];  // the words a share meets its neighbours in
+    };
+    __shared__ Shared sh;
+    const uint32_t ci = list[blockIdx.x], lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = warp / WARPS, part = warp % WARPS;
     const EncChunk c = chunks[ci];
     if (!c.n || !results[ci].coded) return;
     const uint32_t* g_codes = reinterpret_cast<const uint32_t*>(tables + c.table_off + 256);
-    for (uint32_t i = threadIdx.x; i < 256; i += 128) codes[i] = g_codes[i];
-    uint32_t* words = words_all[s];
+    for (uint32_t i = threadIdx.x; i < 256; i += 128 * WARPS) sh.codes[i] = g_codes[i];
+    uint32_t* words = sh.words[warp];
     for (uint32_t i = lane; i < HENC_WORDS; i += 32) words[i] = 0;
     __syncthreads();
     uint32_t start, len;
@@ -715,24 +723,45 @@ __global__ void __launch_bounds__(128) huffman_encode_kernel(const EncChunk* __r
     const uint8_t* src = planes + c.plane_off + start;
     uint8_t* slot = slots + c.slot_off + uint64_t(s) * c.slot_cap;
     uint32_t* out = reinterpret_cast<uint32_t*>(slot);
-    uint32_t have = 0;  // bits of the word that is not full yet, which stays in words[0]
+    const uint32_t rounds = (len + HENC_ROUND - 1) / HENC_ROUND;
+    const uint32_t from = uint32_t(uint64_t(rounds) * part / WARPS) * HENC_ROUND, to = part + 1 == WARPS ? len : uint32_t(uint64_t(rounds) * (part + 1) / WARPS) * HENC_ROUND;
     auto fetch = [&](uint32_t at, uint32_t n, uint64_t& a, uint64_t& b) {  // up to sixteen bytes from src + at
         a = b = 0;
         if (n == HENC_LANE) { a = ld8_unaligned(src + at); b = ld8_unaligned(src + at + 8); }
         else { a = ld_bytes(src + at, n < 8 ? n : 8); if (n > 8) b = ld_bytes(src + at + 8, n - 8); }
     };
-    auto count_at = [&](uint32_t base) -> uint32_t { const uint32_t at = base + lane * HENC_LANE; return at >= len ? 0u : len - at < HENC_LANE ? len - at : HENC_LANE; };
-    uint64_t na, nb;
-    fetch(lane * HENC_LANE, count_at(0), na, nb);
-    for (uint32_t base = 0; base < len; base += 32 * HENC_LANE) {
+    auto count_at = [&](uint32_t base) -> uint32_t { const uint32_t at = base + lane * HENC_LANE; return at >= to ? 0u : to - at < HENC_LANE ? to - at : HENC_LANE; };
+    auto code_of = [&](uint64_t a, uint64_t b, uint32_t k) { return sh.codes[uint32_t((k < 8 ? a : b) >> (8 * (k & 7))) & 0xFFu]; };
+    uint64_t na, nb, before_us = 0;
+    if (WARPS > 1) {
+        uint64_t mine = 0;
+        fetch(from + lane * HENC_LANE, count_at(from), na, nb);
+        for (uint32_t base = from; base < to; base += HENC_ROUND) {
+            const uint32_t n = count_at(base);
+            const uint64_t ca = na, cb = nb;
+            if (base + HENC_ROUND < to) fetch(base + HENC_ROUND + lane * HENC_LANE, count_at(base + HENC_ROUND), na, nb);
+#pragma unroll
+            for (uint32_t k = 0; k < HENC_LANE; ++k) mine += k < n ? code_of(ca, cb, k) >> 16 : 0u;
+        }
+#pragma unroll
+        for (int d = 16; d; d >>= 1) mine += __shfl_xor_sync(0xFFFFFFFFu, mine, d);
+        if (lane == 0) sh.bits[s][part] = mine;
+        __syncthreads();
+        for (uint32_t w = 0; w < part; ++w) before_us += sh.bits[s][w];
+    }
+    uint32_t have = uint32_t(before_us) & 31;  // bits of the word that is not full yet, which stays in words[0]
+    out += before_us >> 5;
+    bool meets = have != 0;  // words[0] is the last one of the share before
+    if (WARPS > 1 && lane == 0) sh.head_at[s][part] = sh.tail_at[s][part] = 0xFFFFFFFFu;
+    fetch(from + lane * HENC_LANE, count_at(from), na, nb);
+    for (uint32_t base = from; base < to; base += HENC_ROUND) {
         const uint32_t n = count_at(base);
         const uint64_t ca = na, cb = nb;
-        if (base + 32 * HENC_LANE < len) fetch(base + (32 + lane) * HENC_LANE, count_at(base + 32 * HENC_LANE), na, nb);  // the next round's symbols
+        if (base + HENC_ROUND < to) fetch(base + HENC_ROUND + lane * HENC_LANE, count_at(base + HENC_ROUND), na, nb);  // the next round's symbols
         uint32_t e[HENC_LANE], bits = 0;
 #pragma unroll
         for (uint32_t k = 0; k < HENC_LANE; ++k) {
-            const uint32_t sy = uint32_t((k < 8 ? ca : cb) >> (8 * (k & 7))) & 0xFFu;
-            e[k] = k < n ? codes[sy] : 0u;
+            e[k] = k < n ? code_of(ca, cb, k) : 0u;
             bits += e[k] >> 16;
         }
         const uint32_t before = warp_prefix(bits, lane), total = __shfl_sync(0xFFFFFFFFu, before + bits, 31);
@@ -756,16 +785,49 @@ __global__ void __launch_bounds__(128) huffman_encode_kernel(const EncChunk* __r
         const uint32_t full = (have + total) >> 5;
         have = (have + total) & 31;
         const uint32_t rest = words[full];
-        for (uint32_t i = lane; i < full; i += 32) out[i] = words[i];
+        if (WARPS > 1 && meets && full) {
+            if (lane == 0) { sh.head_at[s][part] = uint32_t(out - reinterpret_cast<uint32_t*>(slot)); sh.head[s][part] = words[0]; }
+            for (uint32_t i = lane; i < full; i += 32) if (i) out[i] = words[i];
+            meets = false;
+        } else {
+            for (uint32_t i = lane; i < full; i += 32) out[i] = words[i];
+        }
         __syncwarp();
         for (uint32_t i = lane; i <= full; i += 32) words[i] = i == 0 ? rest : 0u;
         out += full;
         __syncwarp();
     }
-    if (lane == 0) {
-        if (have) *out = words[0];
-        results[ci].stream_len[s] = uint32_t(reinterpret_cast<uint8_t*>(out) - slot) + (have + 7) / 8;
+    if (WARPS == 1) {
+        if (lane == 0) {
+            if (have) *out = words[0];
+            results[ci].stream_len[s] = uint32_t(reinterpret_cast<uint8_t*>(out) - slot) + (have + 7) / 8;
+        }
+        return;
     }
+    if (lane == 0 && have) { sh.tail_at[s][part] = uint32_t(out - reinterpret_cast<uint32_t*>(slot)); sh.tail[s][part] = words[0]; }
+    __syncthreads();
+    if (part == 0 && lane == 0) {
+        uint64_t all = 0;
+        uint32_t at = 0xFFFFFFFFu, v = 0;
+        auto word = [&](uint32_t a, uint32_t x) {  // in ascending order; the same word more than once
+            if (a == 0xFFFFFFFFu) return;
+            if (at == a) { v |= x; return; }
+            if (at != 0xFFFFFFFFu) reinterpret_cast<uint32_t*>(slot)[at] = v;
+            at = a; v = x;
+        };
+        for (uint32_t w = 0; w < WARPS; ++w) { all += sh.bits[s][w]; word(sh.head_at[s][w], sh.head[s][w]); word(sh.tail_at[s][w], sh.tail[s][w]); }
+        if (at != 0xFFFFFFFFu) reinterpret_cast<uint32_t*>(slot)[at] = v;
+        results[ci].stream_len[s] = uint32_t((all + 7) / 8);
+    }
+}
+// Chunks of a launch up to which eight warps take a stream.  us of a whole compress_model with one / eight warps: 64 Ki symbols, 1 chunk 194 /
+// 165, 148: 198 / 162, 592: 246 / 253; 16 Ki, 148: 158 / 146, 592: 174 / 185; 4 Ki, 148: 147 / 149, 296: 147 / 161.  A plane of 200,003 in a call of its
+// own: 243 -> 122.
+constexpr uint32_t HENC_WIDE_CHUNKS = 148;
+inline void huffman_encode_launch(const EncChunk* chunks, const uint32_t* list, uint32_t n, const uint8_t* planes, const uint8_t* tables, uint8_t* slots, EncResult* results,
+                                  cudaStream_t st) {
+    if (n <= HENC_WIDE_CHUNKS) huffman_encode_kernel<8><<<n, 1024, 0, st>>>(chunks, list, n, planes, tables, slots, results);
+    else huffman_encode_kernel<1><<<n, 128, 0, st>>>(chunks, list, n, planes, tables, slots, results);
 }
 
 // tANS (entropy/tans/mod.rs:268-318): one serial stream per chunk, its symbols walked last to first, its bits going upward.

@@ -229,7 +229,7 @@ int64_t launch_encoders(const EncChunk* chunks, const uint32_t* lists, const uin
         if (k < LIST_HUFFMAN) {
             const uint32_t span = rans_list_span(k);
             rans_encode_kernel<<<(n[k] + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, renc_smem_bytes(span), st>>>(chunks, lists, n[k], span, planes, tables, slots, results);
-        } else if (k == LIST_HUFFMAN) huffman_encode_kernel<<<n[k], 128, 0, st>>>(chunks, lists, n[k], planes, tables, slots, results);
+        } else if (k == LIST_HUFFMAN) huffman_encode_launch(chunks, lists, n[k], planes, tables, slots, results, st);
         else tans_encode_kernel<<<n[k], 32, 0, st>>>(chunks, lists, n[k], planes, tables, slots, results);
         CUDA_TRY(cudaGetLastError());
         lists += n[k];
@@ -1005,7 +1005,7 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         hist_kernel<<<dim3(1, hist_blocks(n)), 256, 0, st>>>(&d->chunk, in, d->hist);
         table_kernel<<<1, 128, 0, st>>>(&d->plane, &d->chunk, 1, d->hist, area, &d->result);
         if (codec == C_RANS) rans_encode_kernel<<<1, 32, renc_smem_bytes(256), st>>>(&d->chunk, &d->list, 1, 256, in, area, area, &d->result);
-        else if (codec == C_HUFFMAN) huffman_encode_kernel<<<1, 128, 0, st>>>(&d->chunk, &d->list, 1, in, area, area, &d->result);
+        else if (codec == C_HUFFMAN) huffman_encode_launch(&d->chunk, &d->list, 1, in, area, area, &d->result, st);
         else tans_encode_kernel<<<1, 32, 0, st>>>(&d->chunk, &d->list, 1, in, area, area, &d->result);
         CUDA_TRY(cudaGetLastError());
         EncResult r;

@@ -146,6 +146,20 @@ def test_encode_chunk_lengths(kind, codec):
         assert got == oracle.write_container(specs, chunk_size=chunk, forced_codec=codec), chunk
 
 
+def encode_check(planes, chunk, codec):
+    specs = [u8(f"p{k}", raw) for k, raw in enumerate(planes)]
+    tensors = {s.name: torch.frombuffer(bytearray(s.raw), dtype=torch.uint8).cuda() for s in specs}
+    assert compress_model(tensors, CompressionConfig(streaming_chunk=chunk, forced_codec=codec)).to_bytes() == oracle.write_container(specs, chunk_size=chunk, forced_codec=codec)
+
+
+@pytest.mark.parametrize("kind", ["exponent", "rare", "nibble", "wide"])
+def test_huffman_encode_shares_of_a_stream(kind):
+    # eight warps to a stream: shares without a round, of one, with words that two or more shares meet in; more chunks than take them
+    lengths = [4 * 512 * k + d for k in (1, 7, 8, 9, 17) for d in (-5, 0, 1, 6)]
+    encode_check([plane(kind, n) for n in lengths], None, HUFFMAN)
+    encode_check([plane(kind, 600 * 149)], 600, HUFFMAN)
+
+
 def test_plan_run_in_a_captured_graph():
     specs = mixed_model()
     handle = ptwm_b200.ContainerHandle(oracle.write_container(specs, chunk_size=1000, menu=(oracle.HUFFMAN, oracle.RANS, oracle.O1SAC)), device=0)
