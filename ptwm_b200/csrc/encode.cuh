@@ -590,43 +590,51 @@ __device__ __forceinline__ void walk_down(uintptr_t lo, uintptr_t hi, Byte&& byt
 // integer pipe is what bounds a launch that fills the GPU: the bytes that leave are shifted into a register pair from above,
 // and every two symbols the oldest word of the pair is put into a ring in shared memory whether it is full or not (only the
 // write position moves on a full word), from where sixteen bytes at a time go out.  A branch with a store per full word was
-// taken by some lane in nearly every step.  The rows cover `range` symbols from the chunk's first one on: the host knows the
-// span of a plane's alphabet and sends planes of similar span together, so that exponent planes (some 40 values) keep 22
-// blocks on an SM.  With 16-byte entries in global memory and a loop per byte a symbol took 330 ns.
+// taken by some lane in nearly every step.  The rows cover `range` symbols: the chunk's lowest one first, whatever its distance (an
+// exact zero lies far below the other exponents), then all values from its second lowest on.  The host knows the span of a
+// plane's alphabet and sends planes of similar span together, so that exponent planes (some 30 values) keep 24 blocks on an SM.
+// 26,640 chunks of 32 Ki symbols, with and without zeros in them: 1170 + 335 us in one launch of 12 and one of 20 blocks per SM,
+// 1190 in one of 24, 1121 with a row's entries of the eight chunks side by side, where a quarter of a warp reads eight chunks' entries
+// from banks of their own.  That is 12 cycles per warp and symbol with the integer pipe 73 % busy.  With 16-byte entries in global
+// memory and a loop per byte a symbol took 330 ns.
 // x' = x + bias + floor(x / f) * (2048 - f) with the quotient from a rounded-up reciprocal: exact for every state below 2^31,
 // i.e. identical to (x / f) * 2048 + x % f + start (entropy/rans/compress.rs:140-185).
 constexpr uint32_t RENC_RING = 16;  // words per lane: up to 3 waiting, up to 8 more in sixteen symbols, one being filled
-__host__ __device__ inline uint32_t renc_smem_bytes(uint32_t range) { return RANS_WARP_CHUNKS * (range + 1) * 16 + RENC_RING * 32 * 4; }  // a row is one entry longer: rows shifted in the banks
+__host__ __device__ inline uint32_t renc_smem_bytes(uint32_t range) { return RANS_WARP_CHUNKS * range * 16 + RENC_RING * 32 * 4; }
 __global__ void __launch_bounds__(32) rans_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list, uint32_t range,
                                                          const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables, uint8_t* __restrict__ slots,
                                                          EncResult* __restrict__ results) {
     extern __shared__ __align__(16) uint8_t renc_smem[];
     uint4* entries = reinterpret_cast<uint4*>(renc_smem);
-    uint32_t* ring_all = reinterpret_cast<uint32_t*>(renc_smem + RANS_WARP_CHUNKS * (range + 1) * 16);
-    const uint32_t lane = threadIdx.x, c8 = lane >> 2, s = lane & 3, li = blockIdx.x * RANS_WARP_CHUNKS + c8;
+    uint32_t* ring_all = reinterpret_cast<uint32_t*>(renc_smem + RANS_WARP_CHUNKS * range * 16);
+    const uint32_t lane = threadIdx.x, c8 = lane & 7, s = lane >> 3, li = blockIdx.x * RANS_WARP_CHUNKS + c8;
     const uint32_t ci = li < n_list ? list[li] : 0xFFFFFFFFu;
     EncChunk c{};
     if (li < n_list) c = chunks[ci];
     const bool live = li < n_list && c.n && results[ci].coded;
     uint32_t first_sym = 0;
     for (uint32_t k = 0; k < RANS_WARP_CHUNKS; ++k) {  // entry: reciprocal, bias << 8 | reciprocal shift, 2048 - frequency, frequency << 20
-        if (!__shfl_sync(0xFFFFFFFFu, uint32_t(live), 4 * k)) continue;
-        uint32_t f[8], sum = 0, lowest = 0xFFFFFFFFu;
-        warp_load_freqs(tables + __shfl_sync(0xFFFFFFFFu, c.table_off, 4 * k), lane, f);
+        if (!__shfl_sync(0xFFFFFFFFu, uint32_t(live), k)) continue;
+        uint32_t f[8], sum = 0, lowest = 0xFFFFFFFFu, second = 0xFFFFFFFFu;
+        warp_load_freqs(tables + __shfl_sync(0xFFFFFFFFu, c.table_off, k), lane, f);
 #pragma unroll
         for (int j = 7; j >= 0; --j) { sum += f[j]; if (f[j]) lowest = lane * 8 + j; }
         lowest = __reduce_min_sync(0xFFFFFFFFu, lowest);
-        if (c8 == k) first_sym = lowest;
+#pragma unroll
+        for (int j = 7; j >= 0; --j) if (f[j] && lane * 8 + j > lowest) second = lane * 8 + j;
+        second = __reduce_min_sync(0xFFFFFFFFu, second);
+        const uint32_t base = second == 0xFFFFFFFFu ? lowest : second - 1;  // the value of the first row
+        if (c8 == k) first_sym = base;
         uint32_t start = warp_prefix(sum, lane);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const uint32_t at = lane * 8 + j - lowest;  // (wraps for the symbols below the first)
+            const uint32_t sym = lane * 8 + j, at = sym == lowest ? 0u : sym - base;  // (wraps for symbols below the second, which have no count)
             uint4 e = make_uint4(0xFFFFFFFFu, (start + 2047u) << 8, 2047u, 1u << 20);  // f = 1: the quotient comes out one short of x
             if (f[j] > 1) {
                 const uint32_t shift = 32 - __clz(f[j] - 1);  // smallest with f <= 2^shift
                 e = make_uint4(uint32_t(((1ull << (shift + 31)) + f[j] - 1) / f[j]), start << 8 | (shift - 1), 2048u - f[j], f[j] << 20);
             }
-            if (f[j] && at < range) entries[k * (range + 1) + at] = e;
+            if (f[j] && at < range) entries[at * RANS_WARP_CHUNKS + k] = e;
             start += f[j];
         }
     }
@@ -635,7 +643,8 @@ __global__ void __launch_bounds__(32) rans_encode_kernel(const EncChunk* __restr
     uint32_t start, len;
     split_four_dev(c.n, s, start, len);
     uint8_t* slot = slots + c.slot_off + uint64_t(s) * c.slot_cap;
-    const uint4* row = entries + c8 * (range + 1) - first_sym;
+    const uint4* rows = entries + c8 - first_sym * RANS_WARP_CHUNKS;
+    auto row = [&](uint32_t sym) -> const uint4& { return rows[(sym > first_sym ? sym : first_sym) * RANS_WARP_CHUNKS]; };
     uint32_t* ring = ring_all + lane;
     uint32_t x = 1u << 23;
     uint32_t b_lo = 0, b_hi = 0, have = 0;  // the youngest `have` bits wait at the top of b_hi:b_lo; below 32 between pairs of symbols
@@ -667,14 +676,14 @@ __global__ void __launch_bounds__(32) rans_encode_kernel(const EncChunk* __restr
         }
     };
     const uintptr_t lo = reinterpret_cast<uintptr_t>(planes + c.plane_off) + start;
-    walk_down(lo, lo + len, [&](uint32_t b) { step(row[b]); settle(); drain(); },
+    walk_down(lo, lo + len, [&](uint32_t b) { step(row(b)); settle(); drain(); },
               [&](const uint4& v) {
                   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                   for (int h = 3; h >= 0; --h) {
                       uint4 e[4];
 #pragma unroll
-                      for (int k = 0; k < 4; ++k) e[k] = row[(w[h] >> (8 * k)) & 0xFFu];
+                      for (int k = 0; k < 4; ++k) e[k] = row((w[h] >> (8 * k)) & 0xFFu);
                       step(e[3]); step(e[2]); settle();
                       step(e[1]); step(e[0]); settle();
                   }

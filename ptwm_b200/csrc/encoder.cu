@@ -217,10 +217,10 @@ cudaError_t upload_vec(DeviceBuf& b, const std::vector<T>& v, cudaStream_t st) {
 }
 
 // Chunks by the codec of their plane, for the kernels that code them; rANS chunks also by the span of their plane's alphabet,
-// which sizes the shared memory of a block: 64 symbols for exponent planes, 128 and 256 for the others.
-enum { LIST_RANS = 0 /* and 1, 2 */, LIST_HUFFMAN = 3, LIST_TANS = 4, LIST_KINDS = 5 };
-int rans_list(uint32_t span) { return span <= 64 ? 0 : span <= 128 ? 1 : 2; }
-uint32_t rans_list_span(int k) { return 64u << k; }
+// which sizes the shared memory of a block: 48 symbols for exponent planes, 64, 128 and 256 for the others.
+enum { LIST_RANS = 0 /* to 3 */, LIST_HUFFMAN = 4, LIST_TANS = 5, LIST_KINDS = 6 };
+int rans_list(uint32_t span) { return span <= 48 ? 0 : span <= 64 ? 1 : span <= 128 ? 2 : 3; }
+uint32_t rans_list_span(int k) { return k == 0 ? 48u : 32u << k; }
 // The stream encoders over chunks whose tables are built; `lists` holds the chunks of all kinds, one kind after the other.
 int64_t launch_encoders(const EncChunk* chunks, const uint32_t* lists, const uint32_t n[LIST_KINDS], const uint8_t* planes, const uint8_t* tables, uint8_t* slots,
                         EncResult* results, cudaStream_t st) {
@@ -619,11 +619,12 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
                     if (pp.shared >= 0) o1shared_state.insert(o1shared_state.end(), pp.n_chunks, uint32_t(pp.shared));
                 } else if (pp.codec == C_RANS) {
                     const unsigned long long* h = &plane_hist[size_t(pi) * 256];
-                    int lo = 0, hi = 255;
+                    int lo = 0, hi = 255;  // the second lowest symbol (rans_encode_kernel) and the highest
                     while (lo < 255 && !h[lo]) ++lo;
                     while (hi > lo && !h[hi]) --hi;
+                    if (lo < hi) for (++lo; !h[lo];) ++lo;
                     if (tp.post_op == 2 && p == 0) { lo >>= tp.post_k; hi >>= tp.post_k; }  // counted before the shift
-                    list_kind[pi] = rans_list(uint32_t(hi - lo + 1));
+                    list_kind[pi] = rans_list(uint32_t(hi - lo + 2));
                 } else list_kind[pi] = pp.codec == C_HUFFMAN ? int(LIST_HUFFMAN) : int(LIST_TANS);
                 if (list_kind[pi] >= 0) list_sizes[list_kind[pi]] += pp.n_chunks;
             }
@@ -654,6 +655,15 @@ int64_t encode_impl(const ptwm_b200_encode_tensor* tensors, size_t n_tensors, co
 
     prof("codec and chain choice (host)");
     // ---- tables and streams ---------------------------------------------------
+    // A launch takes a stream's time (41 ns a symbol) however few chunks it has: a list that is small against one with longer rows joins it.
+    for (int k = LIST_RANS; k < LIST_HUFFMAN; ++k) {
+        int to = k + 1;
+        while (to < LIST_HUFFMAN && list_sizes[to] / 8 < list_sizes[k]) ++to;
+        if (!list_sizes[k] || to >= LIST_HUFFMAN) continue;
+        for (int& kind : list_kind) if (kind == k) kind = to;
+        list_sizes[to] += list_sizes[k];
+        list_sizes[k] = 0;
+    }
     uint32_t n_listed = 0, list_at[LIST_KINDS];
     for (int k = 0; k < LIST_KINDS; ++k) { list_at[k] = n_listed; n_listed += list_sizes[k]; }
     for (uint32_t p = 0; p < n_planes; ++p) if (list_kind[p] >= 0) { ep[p].list_off = list_at[list_kind[p]]; list_at[list_kind[p]] += ep[p].n_chunks; }

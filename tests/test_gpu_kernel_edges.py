@@ -160,6 +160,17 @@ def test_huffman_encode_shares_of_a_stream(kind):
     encode_check([plane(kind, 600 * 149)], 600, HUFFMAN)
 
 
+@pytest.mark.parametrize("span", [1, 2, 46, 47, 48, 63, 64, 127, 128, 200])
+@pytest.mark.parametrize("far", [False, True])
+def test_rans_encode_rows_of_an_alphabet(span, far):
+    # symbols 50 .. 50 + span - 1 on either side of a list's rows, with and without one that lies far below, which some chunks do not hold
+    rng = np.random.default_rng(span)
+    p = (50 + np.minimum(rng.geometric(0.08, 40000) - 1, span - 1)).astype(np.uint8)
+    p[7], p[20000] = 50 + span - 1, 50
+    if far: p[rng.integers(0, 20000, 3)] = 3
+    encode_check([p.tobytes(), plane("exponent", 9001), plane("wide", 3000)], 1500, RANS)
+
+
 def test_plan_run_in_a_captured_graph():
     specs = mixed_model()
     handle = ptwm_b200.ContainerHandle(oracle.write_container(specs, chunk_size=1000, menu=(oracle.HUFFMAN, oracle.RANS, oracle.O1SAC)), device=0)
