@@ -229,6 +229,8 @@ struct ptwm_b200_plan {
     std::vector<Launch> in_row[2][4];
     bool merge_waits = false;  // a final merge reads scratch
     bool spread = false;       // few chunks: every coded plane to scratch at once, then a merge (see ptwm_b200_plan_create)
+    bool join_small = false;   // the coded planes of small tensors go to scratch in the launch of the others, and a merge follows
+    uint64_t joined_bytes = 0;
     uint64_t slot_bytes[12] = {0};
     uint32_t slot_items[12] = {0};
     std::mutex mu;
@@ -243,6 +245,9 @@ namespace {
 int codec_class(uint16_t codec) { return codec == C_RANS ? 0 : codec == C_HUFFMAN ? 1 : codec == C_TANS ? 2 : 3; }
 
 constexpr uint64_t SPREAD_CHUNKS = 4 * 148;  // four chunks per SM: every decoder holds at least that many
+// Length and chunks of a plane and bytes of a tensor whose planes join the launch of the others, and bytes of all of them together.  (A
+// launch of chunks below 1024 symbols is over in 50 to 70 us; it is left as it is.)
+constexpr uint64_t JOIN_LENGTH = 1024, JOIN_CHUNKS = 16, JOIN_BYTES = 128u << 10, JOIN_ALL_BYTES = 64u << 20;
 constexpr uint64_t SPREAD_BYTES = 256u << 20;  // of scratch: whole planes of any length count as one chunk, and their scratch is as much again as the tensors
 
 // Turn one tensor into work items.  See DecodeItem / MergeItem in plan.h.
@@ -283,6 +288,7 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
     }
     bool has_post = false;
     for (const PlaneDesc& pd : t.planes) has_post |= pd.post != POST_NONE;
+    const bool join = pl.join_small && np > 1 && t.planes[0].decoded_len >= JOIN_LENGTH && t.planes[0].chunks.size() <= JOIN_CHUNKS && t.orig_size <= JOIN_BYTES && pl.joined_bytes + t.orig_size <= JOIN_ALL_BYTES;
     if (aligned && !has_post) {
         for (size_t k = 0; k < t.planes[0].chunks.size(); ++k) {
             const uint32_t n = t.planes[0].chunks[k].decoded;
@@ -295,7 +301,9 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
                 uint16_t codec = t.planes[size_t(p)].codec;
                 if (!ch.raw && (codec == C_RANS || codec == C_HUFFMAN || codec == C_TANS)) { fused_plane = p; ++coded; }
             }
-            if (pl.spread && coded > 1) fused_plane = -1;
+            const bool joins = join && coded > 1;
+            if (joins || (pl.spread && coded > 1)) fused_plane = -1;
+            if (joins) pl.joined_bytes += uint64_t(n) * uint64_t(np);
             if (np == 1) {
                 const ChunkDesc& ch = t.planes[0].chunks[k];
                 if (ch.raw) { span(ch.data_off, ch.data_len); pl.merges[1].push_back(MergeItem{{make_ref(SP_BLOB, ch.data_off), REF_NONE, REF_NONE, REF_NONE}, out_ref, n, K_PASS}); }
@@ -311,7 +319,7 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
                     DecodeItem it = decode_item(pd, ch);
                     it.dst = make_ref(SP_SCRATCH, scratch_of(p) + ch.plane_off);
                     srcs[p] = it.dst;
-                    pl.dec[0][codec_class(pd.codec)].push_back(it);
+                    pl.dec[joins][codec_class(pd.codec)].push_back(it);
                 }
             }
             if (fused_plane >= 0) {
@@ -951,12 +959,19 @@ int64_t ptwm_b200_plan_create(const ptwm_b200_container* c, const uint32_t* indi
             // While all chunks of the plan run at once anyway that only adds up their latencies: with few chunks every coded plane
             // goes to scratch and one more launch merges them (a 4096-element norm vector: 0.48 -> 0.3 ms).
             uint64_t coded = 0, bytes = 0;
+            uint32_t classes = 0;
             for (uint32_t ti : pl->tensors) if (ti < c->file.tensors.size())
                 for (const PlaneDesc& p : c->file.tensors[ti].planes) {
-                    if (coded > SPREAD_CHUNKS) break;
+                    if (p.codec != C_IDENTITY) classes |= 1u << codec_class(p.codec);
+                    if (coded > SPREAD_CHUNKS) continue;
                     for (const ChunkDesc& ch : p.chunks) if (!ch.raw) { ++coded; bytes += ch.decoded; }
                 }
             pl->spread = coded <= SPREAD_CHUNKS && bytes <= SPREAD_BYTES;
+            // In a larger plan the first planes of small tensors (norm vectors) would be a launch of their own before everything else, which
+            // leaves the GPU idle: 126 of 1630 us with tANS (the whole pass 1571 -> 1450), 70 with Huffman.  They join the large launch, and a merge follows.  rANS
+            // chunks stay apart: what is small there goes to the kernel with a table entry per slot (57 us; as part of the
+            // large launch its rarer alphabets would need one more kernel), and so do plans of several codecs, whose launches overlap.
+            pl->join_small = !pl->spread && (classes == 1u << 1 || classes == 1u << 2);
         }
         for (uint32_t ti : pl->tensors) {
             if (ti >= c->file.tensors.size()) return fail(PTWM_RC_INVALID_INPUT, "tensor index out of range");

@@ -122,6 +122,17 @@ def test_decode_two_coded_planes_in_many_chunks():
         check(mixed_model(2), chunk_size=501, menu=menu, emit_crc=True, emit_hash=True)
 
 
+@pytest.mark.parametrize("codec", [HUFFMAN, TANS, RANS])
+def test_decode_small_tensors_beside_a_large_one(codec):
+    # more chunks than are spread over scratch: small tensors with two and more coded planes join the launch of the large one (not with rANS)
+    specs = []
+    for k, n in enumerate((501 * 620 + 7, 1, 37, 500, 501, 502, 1500, 30000, 70000)):
+        for name, dt, code in (("b", torch.bfloat16, oracle.DT_BF16), ("f", torch.float32, oracle.DT_F32), ("e", torch.float8_e4m3fn, oracle.DT_E4M3)):
+            t = (1 + 0.01 * weights(1, n, k, False)) if dt == torch.bfloat16 else weights(1, n, k, False).mul(8)
+            specs.append(oracle.TensorSpec(f"{name}{k}", code, [n], t.to(dt).view(torch.uint8).numpy().tobytes()))
+    check(specs, chunk_size=501, forced_codec=codec, emit_crc=True)
+
+
 @pytest.mark.parametrize("shift", [0, 1, 2, 8])
 def test_payload_hash_blocks_and_alignment(shift):
     lengths = (0, 1, 31, 32, 33, 8191, 8192, 8193, 8192 + 32, 2 * 8192, 3 * 8192 + 45)
