@@ -371,3 +371,17 @@ def test_planes_of_any_length_do_not_double_the_scratch(L):
 
     assert scratch(1 << 20) == 2 << 20
     assert scratch((128 << 20) + 256) == (128 << 20) + 256
+
+
+@pytest.mark.parametrize("at", [0, 256, 8, 1])
+def test_views_of_a_plan_are_the_views_of_its_tensors(at):
+    # one view of the arena per dtype against a slice, a view and a reshape of every tensor; an arena that cannot be viewed whole
+    import torch
+    from _data import mixed_model
+    specs = mixed_model() + [oracle.TensorSpec("none", oracle.DT_F32, [3, 0, 5], b""), oracle.TensorSpec("scalar", oracle.DT_F32, [], b"\0\0\x80\x3f")]
+    handle = ptwm_b200.ContainerHandle(oracle.write_container(specs, chunk_size=4096), device=0)
+    plan = handle.plan(None)
+    arena = torch.randint(0, 256, (plan.out_bytes + 512,), dtype=torch.uint8)[at:at + plan.out_bytes]
+    for i, off, got in zip(plan.indices, plan.out_offsets, plan.views(arena)):
+        want = handle._view(i, arena, off)
+        assert (got.dtype, got.shape, got.stride(), got.data_ptr()) == (want.dtype, want.shape, want.stride(), want.data_ptr())
