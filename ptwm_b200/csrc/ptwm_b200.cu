@@ -968,7 +968,7 @@ int64_t ptwm_b200_plan_create(const ptwm_b200_container* c, const uint32_t* indi
                 }
             pl->spread = coded <= SPREAD_CHUNKS && bytes <= SPREAD_BYTES;
             // In a larger plan the first planes of small tensors (norm vectors) would be a launch of their own before everything else, which
-            // leaves the GPU idle: 126 of 1630 us with tANS (the whole pass 1571 -> 1450), 70 with Huffman.  They join the large launch, and a merge follows.  rANS
+            // leaves the GPU idle: 126 of 1630 us with tANS, 70 with Huffman.  They join the large launch, and a merge follows.  rANS
             // chunks stay apart: what is small there goes to the kernel with a table entry per slot (57 us; as part of the
             // large launch its rarer alphabets would need one more kernel), and so do plans of several codecs, whose launches overlap.
             pl->join_small = !pl->spread && (classes == 1u << 1 || classes == 1u << 2);
