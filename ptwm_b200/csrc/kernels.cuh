@@ -1848,7 +1848,7 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
     }
 }
 
-// The other kernel: a lane per stream, 32 chunks per block, for launches whose chunks fill the GPU that way (tans_lanes_win).
+// The other kernel: a lane per stream, 32 chunks per block, for launches whose chunks fill the GPU that way (tans_kernel).
 // One stream per lane and an entry per state: the spread symbols (u8 per state) and (baseline << 5 | bit count) (u16 per
 // state), 6 KiB per chunk, so an SM holds 32 chunks whatever the kernel does.  Both tables are laid out [state][lane]: the
 // address of an entry is one multiply-add from the state and a lane only touches its own columns.
