@@ -1288,6 +1288,11 @@ __global__ void __launch_bounds__(32) huffman_decode_kernel(const DecodeItem* __
 // * Lane 0 starts in the right state.  Its path, then that of the lane it met,
 //   and so on is the right one; along it the state at every cut and the number
 //   of symbols before it are known.
+// * Before it falls in, a lane can take many more symbols out of the same bits
+//   than the right path does (codes of rare symbols read out of step are mostly
+//   the frequent one).  So a lane that has met as many symbols as the chunk
+//   holds is only set aside; where the right path has come to it, one lane
+//   takes it up with the number of symbols the right path has left.
 // * A last pass decodes every run from its right start and puts the symbols to
 //   their places.
 //
@@ -1324,11 +1329,11 @@ struct TansShared {
     uint32_t key[NODES * SLOTS];   // 0 or 1 << 31 | lane << 16 | bits below the node << 11 | state
     uint32_t count[NODES * SLOTS]; // symbols of that lane so far
     uint32_t link[LANES];          // the entry the lane met, or a TANS_ value
-    uint32_t met[LANES];           // its symbols up to there
+    uint32_t met[LANES];           // its symbols up to there, or up to where it was set aside
     uint32_t from[LANES];          // node from which its path is the right one
     uint32_t base[LANES];          // symbols of the chunk minus symbols of the lane, on its right part
     uint32_t start[LANES];         // bits below the cut << 11 | state: the right start of the run
-    uint32_t at[LANES];            // symbols before it
+    uint32_t at[LANES];            // symbols before it; during the walks, node << 16 | bits below it << 11 | state of a walk set aside
     uint32_t tally[LANES / 32];    // walks of each warp
 };
 constexpr uint32_t TANS_PAUSED = 0xFFFFFFFFu, TANS_FINISHED = 0xFFFFFFFEu, TANS_DEAD = 0xFFFFFFFDu, TANS_NONE = 0xFFFFFFFFu;
@@ -1614,19 +1619,23 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
         return used;
     };
     // ---- walks ----
-    uint32_t who = l, node = l * SEGS, n = 0;  // the walk the lane is on, the node behind it, symbols since its start
+    uint32_t who = l, node = l * SEGS, stand = 0;  // the walk the lane is on, the node behind it, where it stood there: bits below the node << 11 | state
+    uint32_t n = 0, most = it.n;                   // symbols since its start (modulo 2^32), and where it is set aside
     bool alive = l + 1 < runs;
+    enum { ALL, OWN_RUN, ALONE } walks = ALL;
+    auto take_up = [&]() { begin(top_bit - node * apart - (stand >> 11), stand & 2047u, top_bit - (node + 1) * apart); };
+    auto set_aside = [&](uint32_t at_node, uint32_t symbols) { alive = false; sh.at[who] = at_node << 16 | stand; sh.met[who] = symbols; };
     auto segment = [&]() -> uint32_t {  // on to the next node: the symbols met
         const uint32_t n0 = n;
         ++node;
         const uint32_t stop = head_for(top_bit - node * apart);
-        while (int32_t(at - stop) >= int32_t(2 * TANS_GROUP_BITS) && n < it.n) {
+        while (int32_t(at - stop) >= int32_t(2 * TANS_GROUP_BITS) && most - n >= 16) {
             refill();
             at -= group([](int, uint32_t) {});
             at -= group([](int, uint32_t) {});
             n += 16;
         }
-        while (int32_t(at - stop) > 0 && n < it.n) {  // up to the first boundary at or below the node
+        while (int32_t(at - stop) > 0) {  // up to the first boundary at or below the node
             refill();
             const uint32_t need = at - stop;
             uint32_t bits = 0, taken = 0, there = 0, symbols = 0;
@@ -1635,19 +1644,20 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
                 bits += e & 31u;
                 if (above) { taken = bits; there = entry; ++symbols; }
             });
+            if (symbols > most - n) {
+                set_aside(node - 1, n0);
+                if (walks == ALONE) sh.link[who] = TANS_DEAD;  // the right path: more symbols than the chunk has
+                return n - n0;
+            }
             at -= taken; entry = there; n += symbols;
         }
-        if (int32_t(at - stop) > 0) {  // more symbols than the chunk has
-            alive = false;
-            sh.link[who] = TANS_DEAD;
-            return n - n0;
-        }
-        const uint32_t pair = (stop - at) << 11 | entry >> 2, mine = 1u << 31 | who << 16 | pair;
+        stand = (stop - at) << 11 | entry >> 2;
+        const uint32_t mine = 1u << 31 | who << 16 | stand;
         for (uint32_t k = 0; k < slots; ++k) {
-            const uint32_t slot = node * slots + ((pair + k) & (slots - 1));
+            const uint32_t slot = node * slots + ((stand + k) & (slots - 1));
             const uint32_t old = atomicCAS(&sh.key[slot], 0u, mine);
             if (old == 0) { sh.count[slot] = n; break; }
-            if (((old ^ pair) & 0x7FFFu) == 0) {
+            if (((old ^ mine) & 0x7FFFu) == 0) {
                 alive = false;
                 sh.link[who] = slot; sh.met[who] = n;
                 break;
@@ -1661,10 +1671,10 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
         const uint64_t bit = total_bits - 11;
         const uint8_t* b = bs + (bit >> 3);
         const uint32_t three = uint32_t(b[0]) | uint32_t(b[1]) << 8 | ((bit & 7) > 5 ? uint32_t(b[2]) << 16 : 0u);
-        start0 = 11u << 11 | ((three >> (bit & 7)) & 2047u);
+        start0 = stand = 11u << 11 | ((three >> (bit & 7)) & 2047u);
         if (!alive) { sh.link[0] = TANS_FINISHED; sh.met[0] = 0; }
     }
-    if (alive) begin(top_bit - node * apart - (start0 >> 11), start0 & 2047u, top_bit - (node + 1) * apart);
+    if (alive) take_up();
     // A damaged or very uneven stream can hold the whole chunk's symbols, or more, between any two nodes: once a warp has walked three
     // times the chunk's symbols the lanes only finish their runs, and the one with the right path goes on alone.  (So it is in
     // streams of more than 2^31 bits, where a run whose right start found no room at its node must not become part of the one before.)
@@ -1673,13 +1683,12 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
     // As walks end, the others move together into as few warps as hold them, every TANS_GATHER symbols or so.
     uint32_t warps = LANES / 32, looks = 0;
     const uint32_t every = uint32_t(uint64_t(TANS_GATHER) * runs * SEGS / it.n) + 1;
-    enum { ALL, OWN_RUN, ALONE } walks = ALL;
-    // The right path is followed from lane 0's on, once nothing moves any more.
+    // The right path is followed from lane 0's on, once nothing moves any more; walks set aside on it are taken up by lane 0.
     uint32_t lane = 0;
-    int64_t base = 0;
+    int64_t base = 0;  // below zero on a lane that had more symbols before it fell in
     bool too_many = false;
     for (;;) {
-        const bool go = alive && (walks == ALL ? spent < budget && (warps == 1 || looks < every) : walks == OWN_RUN ? node < (who + 1) * SEGS : who == lane);
+        const bool go = alive && (walks == ALL ? spent < budget && (warps == 1 || looks < every) : walks == ALONE || node < (who + 1) * SEGS);
         if (__any_sync(0xFFFFFFFFu, go)) {
             uint32_t met = 0;
             if (go) met = segment();
@@ -1699,17 +1708,15 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
             const bool gather = (total + 31) / 32 < warps;
             if (gather && alive) {  // every walk stands at a node
                 const uint32_t place = before + __popc(votes & ((1u << (l % 32)) - 1u));
-                const uint64_t bit = top_bit - node * apart;
-                sh.from[place] = who << 16 | node; sh.base[place] = n; sh.start[place] = uint32_t(bit - (uint64_t(org) * 8 + at)) << 11 | entry >> 2;
+                sh.from[place] = who << 16 | node; sh.base[place] = n; sh.start[place] = stand;
             }
             __syncthreads();
             if (gather) {
                 warps = (total + 31) / 32;
                 alive = l < total;
                 if (alive) {
-                    who = sh.from[l] >> 16; node = sh.from[l] & 0xFFFFu; n = sh.base[l];
-                    const uint32_t pair = sh.start[l];
-                    begin(top_bit - node * apart - (pair >> 11), pair & 2047u, top_bit - (node + 1) * apart);
+                    who = sh.from[l] >> 16; node = sh.from[l] & 0xFFFFu; n = sh.base[l]; stand = sh.start[l];
+                    take_up();
                 }
                 __syncthreads();
             }
@@ -1717,27 +1724,35 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
             continue;
         }
         if (walks == OWN_RUN) {
+            if (alive) set_aside(node, n);
             sh.from[l] = TANS_NONE; sh.start[l] = TANS_NONE;
-            if (l == 0) { sh.start[0] = start0; sh.at[0] = 0; sh.from[0] = 0; sh.base[0] = 0; }
+            if (l == 0) { sh.start[0] = start0; sh.from[0] = 0; sh.base[0] = 0; }
             walks = ALONE;
         }
         tans_sync<LANES>();
         uint32_t link;
         while ((link = sh.link[lane]) < TANS_DEAD && !too_many) {
             base += sh.met[lane];
+            if (base < 0) base += int64_t(1) << 32;  // (a walk taken up whose count went past 2^32)
             too_many = base > int64_t(it.n);
             base -= sh.count[link];
             lane = (sh.key[link] >> 16) & 0x3FFu;
             if (l == 0) { sh.from[lane] = link / slots; sh.base[lane] = uint32_t(base); }
         }
-        if (too_many || link != TANS_PAUSED) {
-            too_many = too_many || link == TANS_DEAD || base + int64_t(sh.met[lane]) > int64_t(it.n);
-            break;
-        }
+        const int64_t before = base + sh.met[lane];
+        too_many = too_many || link == TANS_DEAD || before > int64_t(it.n);
+        if (too_many || link == TANS_FINISHED) break;
         tans_sync<LANES>();
+        if (l == 0) {
+            who = lane; node = sh.at[lane] >> 16; stand = sh.at[lane] & 0xFFFFu;
+            n = sh.met[lane]; most = n + uint32_t(int64_t(it.n) - before);
+            alive = true;
+            take_up();
+        }
     }
     if (too_many) { if (l == 0) report(status, it.id, ST_NOT_CONSUMED); return; }  // more symbols than the chunk has
     tans_sync<LANES>();
+    if (l == 0) sh.at[0] = 0;
     if (sh.from[l] != TANS_NONE) {  // the lane's path is right between these nodes: where it enters the runs
         const uint32_t link = sh.link[l], base = sh.base[l], end = link < TANS_DEAD ? link / slots : last_node + 1;
         for (uint32_t k = l == 0 ? 1 : (sh.from[l] + SEGS - 1) / SEGS; k * SEGS < end; ++k) {

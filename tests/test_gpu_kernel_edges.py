@@ -116,6 +116,44 @@ def test_tans_decode_of_uneven_streams(chunks):
     check(specs, chunk_size=len(specs[-1].raw) // chunks if chunks > 1 else None, forced_codec=TANS)
 
 
+def uneven(kind: str, n: int, rng) -> np.ndarray:
+    """A chunk whose rarer symbols lie together or far apart: a walk that starts wrong meets more symbols than the chunk holds."""
+    p = np.zeros(n, dtype=np.uint8)
+    k = max(2, int(n * rng.uniform(0.002, 0.05)))
+    if kind == "sparse":
+        return (rng.random(n) < rng.uniform(0.005, 0.05)).astype(np.uint8)
+    if kind == "front":  # followed by two symbols in turn
+        p[:k], p[k + 1::2] = rng.integers(1, 6, k), 250
+    else:  # exponents of normal weights, or bytes of any value, at both ends
+        e = rng.normal(0, 0.02, 2 * k).astype(np.float32).view(np.uint32) >> 23 & 0xFF if kind == "ends" else rng.integers(1, 256, 2 * k)
+        p[:k], p[n - k:] = e[:k], e[k:]
+    return p
+
+
+@pytest.mark.parametrize("kind", ["sparse", "front", "ends", "noise"])
+@pytest.mark.parametrize("chunk, chunks", [(1225, 1), (2000, 400), (2000, 1800), (3000, 120), (3000, 400), (4096, 200), (9000, 1000), (16384, 100), (70001, 4)])
+def test_tans_decode_where_wrong_starts_meet_more_symbols(kind, chunk, chunks):
+    rng = np.random.default_rng(chunk + chunks)
+    raw = np.concatenate([uneven(kind, chunk, rng) for _ in range(chunks)])
+    wide = raw.astype(np.uint16) << 7  # bf16 with these exponents
+    check([u8("p", raw.tobytes())], chunk_size=chunk, forced_codec=TANS)
+    check([oracle.TensorSpec("p", oracle.DT_BF16, [len(raw)], wide.tobytes())], chunk_size=chunk, forced_codec=TANS)
+
+
+def test_decode_of_mostly_zero_weights():
+    # nonzero at both ends of a vector, or in the first and last row of a matrix: tANS has the smallest payload
+    specs = []
+    for k in range(40):
+        v, m = torch.zeros(4096), torch.zeros(64 << k % 2, 64 << k % 2)
+        v[:20], v[-20:] = weights(1, 20, k, False), weights(1, 20, k + 99, False)
+        m[0], m[-1] = weights(1, m.shape[1], k, False), weights(1, m.shape[1], k + 99, False)
+        for name, t in (("v", v), ("m", m)):
+            specs.append(oracle.TensorSpec(f"{name}{k}", oracle.DT_BF16, list(t.shape), t.to(torch.bfloat16).view(torch.uint8).numpy().tobytes()))
+    for chunk in (4096, 65536):
+        check(specs, chunk_size=chunk, menu=(oracle.IDENTITY, oracle.HUFFMAN, oracle.RANS, oracle.TANS, oracle.O1SAC), emit_crc=True)
+        check(specs, chunk_size=chunk, forced_codec=TANS)
+
+
 def test_decode_two_coded_planes_in_many_chunks():
     # more chunks than are spread over scratch: the second plane's lanes merge with the first one, every codec on its own stream
     for menu in ((oracle.HUFFMAN, oracle.RANS, oracle.O1SAC), (oracle.TANS, oracle.O1SAC), (oracle.IDENTITY, oracle.HUFFMAN, oracle.RANS, oracle.TANS, oracle.O1SAC)):
