@@ -33,6 +33,7 @@ int64_t noalloc_scratch_for(int device, uint8_t** out) {
         // the decoders need more dynamic shared memory than the default limit; an attribute, not an allocation
         CUDA_TRY(cudaFuncSetAttribute(rans_decode_kernel_t<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rans_smem_bytes(rans_l_entries(255)))));
         CUDA_TRY(cudaFuncSetAttribute(huffman_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HUF_SMEM));
+        CUDA_TRY(tans_allow_shared());
         CUDA_TRY(o1sac_allow_shared_rows());
         it = g_noalloc_ptr.emplace(device, static_cast<uint8_t*>(p)).first;
     }

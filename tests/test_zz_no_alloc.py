@@ -15,6 +15,9 @@ clear message.  The file sorts last so a run that stops at the first failure
 has already finished every other test.
 """
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -71,6 +74,31 @@ def test_noalloc_matches_regular_entry_point_twice_in_a_row():
             rc, got = _decode("ptwm_b200_decode_plane_noalloc", codec, payload, n, st, sv, stream=1)
             assert rc == n, (codec, attempt, rc, _lib.last_error())
             assert got == ref, (codec, attempt)  # decoded bytes and the untouched guard bytes behind them
+
+
+FIRST_CALL = """
+import sys
+sys.path[:0] = {path!r}
+import test_zz_no_alloc as t
+for codec, payload, n, st, sv, plane in t._cases_of_lengths({codec}):
+    rc, got = t._decode("ptwm_b200_decode_plane_noalloc", codec, payload, n, st, sv, stream=1)
+    assert rc == n and got[:n] == plane and got[n:] == bytes([0xCD]) * 32, (n, rc, t._lib.last_error())
+"""
+
+
+def _cases_of_lengths(codec):
+    for n in (2999, 3000, 70001):
+        plane = ((np.random.default_rng(n).normal(0, 3, n).astype(np.int64) + 120) % 120).astype(np.uint8).tobytes()
+        st, sv, payload = oracle.plane_encode(codec, plane, 0)
+        yield codec, payload, n, st, sv, plane
+
+
+@pytest.mark.parametrize("codec", [oracle.HUFFMAN, oracle.RANS, oracle.TANS, oracle.O1SAC])
+def test_noalloc_is_the_only_entry_point_of_a_process(codec):
+    # what the kernels need set up (their share of shared memory) cannot come from a call of another entry point
+    here = os.path.dirname(os.path.abspath(__file__))
+    res = subprocess.run([sys.executable, "-c", FIRST_CALL.format(path=[os.path.dirname(here), here], codec=int(codec))], capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
 
 
 def test_noalloc_refuses_a_state_beyond_its_scratch():
