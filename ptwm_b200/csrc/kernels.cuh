@@ -1635,7 +1635,8 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
             at -= group([](int, uint32_t) {});
             n += 16;
         }
-        while (int32_t(at - stop) > 0) {  // up to the first boundary at or below the node
+        bool over = false;
+        while (int32_t(at - stop) > 0 && !over) {  // up to the first boundary at or below the node
             refill();
             const uint32_t need = at - stop;
             uint32_t bits = 0, taken = 0, there = 0, symbols = 0;
@@ -1644,12 +1645,13 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
                 bits += e & 31u;
                 if (above) { taken = bits; there = entry; ++symbols; }
             });
-            if (symbols > most - n) {
-                set_aside(node - 1, n0);
-                if (walks == ALONE) sh.link[who] = TANS_DEAD;  // the right path: more symbols than the chunk has
-                return n - n0;
-            }
+            over = symbols > most - n;
             at -= taken; entry = there; n += symbols;
+        }
+        if (over) {
+            set_aside(node - 1, n0);
+            if (walks == ALONE) sh.link[who] = TANS_DEAD;  // the right path: more symbols than the chunk has
+            return n - n0;
         }
         stand = (stop - at) << 11 | entry >> 2;
         const uint32_t mine = 1u << 31 | who << 16 | stand;
