@@ -1309,7 +1309,8 @@ __global__ void __launch_bounds__(32) huffman_decode_kernel(const DecodeItem* __
 //
 // Table: one word per state, bit count (low five bits: what a funnel shift
 // takes of it) | symbol << 8 | byte offset of the baseline's entry << 16.
-constexpr uint32_t TANS_MIN_RUN = 64, TANS_SHORT = 3000, TANS_SHORT_RUN = 256;  // symbols per lane at least; in chunks shorter than TANS_SHORT, which are mostly serial
+constexpr uint32_t TANS_SHORT = 3000;          // chunks below this many symbols are mostly serial
+constexpr uint32_t TANS_FEW = 10240;           // chunks below this many have fewer runs than 32 or 64 lanes (tans_runs)
 constexpr uint32_t TANS_GATHER = 512;          // symbols between two looks at how many walks are left
 constexpr uint32_t TANS_GROUP_BITS = 8 * 11;  // a group of eight symbols takes at most this many
 
@@ -1320,6 +1321,17 @@ template <> struct TansShape<32> { static constexpr uint32_t SEGS = 2, SLOTS = 2
 template <> struct TansShape<64> { static constexpr uint32_t SEGS = 1, SLOTS = 4, BLOCKS = 12; };
 template <> struct TansShape<128> { static constexpr uint32_t SEGS = 1, SLOTS = 8, BLOCKS = 6; };
 template <> struct TansShape<256> { static constexpr uint32_t SEGS = 1, SLOTS = 8, BLOCKS = 4; };
+
+// Runs of a chunk.  32 and 64 lanes serve launches whose walks fill the GPU: there many walks of a short chunk cost more than they save, and
+// nodes that hold few paths each let them pass one another unmet.  us of 1184 chunks, bf16, 32 lanes with up to 32 / 16 / 8 runs: 2700
+// symbols 188 / 189 / 151; 4096: 395 / 258 / 189; 6000: 486 / 271 / 245; 8192: 482 / 278 / 310; 64 lanes with up to 64 / 32 / 16: 4096 417 / 180 /
+// 204; 8192: 344 / 227 / 287.
+template <int LANES>
+__device__ __forceinline__ uint32_t tans_runs(uint32_t n) {
+    const uint32_t runs = n / (LANES == 32 ? 256 : LANES == 64 ? 128 : n < TANS_SHORT ? 256 : 64);
+    const uint32_t most = n >= TANS_FEW || LANES > 64 ? LANES : LANES == 64 ? 32 : n < 5500 ? 8 : 16;
+    return runs > most ? most : runs;
+}
 
 template <int LANES>
 struct TansShared {
@@ -1520,8 +1532,7 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
 
     // ---- runs ----
     // LIFO reader (mod.rs:118-147): the stream is read from its last bit down.
-    uint32_t runs = it.n / (it.n < TANS_SHORT ? TANS_SHORT_RUN : TANS_MIN_RUN);
-    if (runs > LANES) runs = LANES;
+    uint32_t runs = tans_runs<LANES>(it.n);
     if (uint64_t(runs) * (32 * SEGS) > total_bits) runs = uint32_t(total_bits) / (32 * SEGS);  // nodes at least 32 bits apart
     if (runs < 1) runs = 1;
     const uint64_t apart = total_bits / (runs * SEGS);
@@ -2354,13 +2365,17 @@ inline void tans_launch_t(const DecodeItem* items, uint32_t n, const Bases& base
 // 2368: 1120 / 909 / 928 / 907; 16 Ki, 296: 231 / 187 / 267 / 489, 1184: 452 / 355 / 351 / 659, 2368: 796 / 525 / 511 / 626; 8 Ki, 1776:
 // 479 / 378 / 417 / 561.  Runs that are long against the way to a meeting (`apart`, in symbols of 1,400) need fewer walks: 128 Ki, 3552 chunks
 // 2344 / 2050 / 2052 / 1881; fp8, 64 Ki, 2368: 2011 / 1667 / 1565 / 1396; fp16, 8 Ki, 2368: 398 / 321 / 298 / 248.  In chunks that are mostly
-// serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 176, 32: 113.
+// serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 176, 32: 113.  Below TANS_FEW symbols the rounds of blocks count, 12 per SM
+// with 64 lanes and 16 with 32; 64 / 32 lanes: 3500 symbols, 1184 chunks 187 / 175, 1776 236 / 195 (fp16 137 / 163, 177 / 175); 6000: 1776 263 / 273,
+// 1900 304 / 261, 2368 356 / 287.
+constexpr uint32_t TANS_ROUND_64 = 148 * TansShape<64>::BLOCKS, TANS_ROUND_32 = 148 * TansShape<32>::BLOCKS;
 inline uint32_t tans_lanes(uint32_t chunks, uint32_t longest, double apart) {
     if (longest < TANS_SHORT) return chunks <= 4 * 148 ? 128 : 32;
     if (chunks <= (longest <= 4096 ? 148 : 2 * 148)) return 256;
     if (chunks <= 6 * 148) return 128;
-    if (chunks > 12 * 148 && longest > 65536 * apart) return 32;
-    return longest <= 8192 ? 128 : 64;
+    if (longest < 4000 && (apart > 0.5 || chunks > TANS_ROUND_64)) return 32;
+    if (longest < TANS_FEW) return chunks > TANS_ROUND_64 && chunks <= TANS_ROUND_32 ? 32 : 64;
+    return chunks > TANS_ROUND_64 && longest > 65536 * apart ? 32 : 64;
 }
 // `lanes` per chunk; 1: the kernel with a lane per stream.
 inline void tans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t lanes, cudaStream_t st) {

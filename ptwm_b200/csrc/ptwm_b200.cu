@@ -369,15 +369,21 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
 // tANS chunks of one launch, longest first: the kernel they go to, as tans_launch takes it.
 // The kernel with a lane per stream takes 148 us and 27 ns per symbol of the longest chunk for every 4736 chunks (148 SMs x 32), and up to
 // 3.3 times that per symbol where some lane in most rounds of 32 symbols has four in a row that take more than 32 bits (8 groups, 32
-// lanes) and all of them go back.  With several lanes per chunk a launch takes some 150 us and then its work: per chunk 16 to 28 ns,
+// lanes) and all of them go back.  With several lanes per chunk a launch takes a latency and then its work: per chunk 16 to 28 ns,
 // 10 ps per symbol of the first 8 Ki (paths meeting), and what placing a symbol costs.  Planes above four bits per symbol meet sooner,
-// and so do nibbles.  Chunks below TANS_SHORT are next to serial.
-// us, lane per stream / several lanes: bf16, 4 Ki: 1184 chunks 259 / 236, 1776 258 / 320; 8 Ki: 1184 363 / 327, 2368 365 / 513; 16 Ki: 2368
-// 590 / 511, 3552 592 / 741; 32 Ki: 3552 1034 / 864, 4736 1031 / 1021; 64 Ki: 4736 1902 / 1481; fp32, 32 Ki: 2368 1041 / 674, 4736 1038 / 1122;
-// fp16, 32 Ki, 4736 1078 / 765; fp8, 8 Ki, 2368 694 / 793; bf16, half of it zeros, 16 Ki: 4736 2606 / 1435.
+// and so do nibbles.  Below TANS_FEW symbols several lanes are the faster ones as long as one round of blocks holds the launch; after
+// that every round costs its latency again.
+// us, lane per stream / several lanes: bf16, 512: 3552 chunks 152 / 149; 1 Ki: 2368 166 / 116, 2700 165 / 185; 2 Ki: 2368 197 / 171, 2700 197 / 264;
+// 4 Ki: 2368 250 / 238, 2700 249 / 362; 8 Ki: 2368 360 / 359, 2700 360 / 430; 16 Ki: 2368 590 / 529; 32 Ki: 3552 1034 / 864, 4736 1031 / 1021;
+// 64 Ki: 4736 1902 / 1481; fp32, 32 Ki: 2368 1041 / 674, 4736 1038 / 1122; fp16, 8 Ki, 2700 386 / 308; 32 Ki, 4736 1078 / 765; fp8, 8 Ki, 2368 691 /
+// 577; bf16, half of it zeros, 16 Ki: 4736 2606 / 1435.
 uint32_t tans_kernel(const DecodeItem* items, size_t n) {
     constexpr size_t WAVE = 148 * TANS_CTA_CHUNKS;
-    double by_lanes = 0, wave = 0, work = n && items[0].n < TANS_SHORT ? 40 + 0.03 * items[0].n : 150, apart = 1;
+    const uint32_t longest = n ? items[0].n : 0;
+    const auto rounds = [n](uint32_t round) { return double((n + round - 1) / round); };
+    const bool one_warp = longest < 4000;  // as tans_lanes has it
+    double by_lanes = 0, wave = 0, work = one_warp ? rounds(TANS_ROUND_32) * (28 + 0.03 * longest) : longest < TANS_FEW ? 65 + 50 * rounds(TANS_ROUND_64) : 150, apart = 1;
+    const double meet = longest < TANS_FEW ? 7e-6 : 1e-5;
     bool placed = true;
     for (size_t k = 0; k < n && placed; ++k) {
         const DecodeItem& it = items[k];
@@ -388,11 +394,12 @@ uint32_t tans_kernel(const DecodeItem* items, size_t n) {
         if (k % WAVE == 0) { by_lanes += wave; wave = 0; }
         wave = std::max(wave, 148 + 0.0267 * len * (1 + 3.3 * back));
         if (k == 0) apart = fall * fall * (it.fused && eb == 1 ? 0.25 : 1);
-        work += it.n < TANS_SHORT ? 0.012 + 1.2e-5 * len
-                                  : 0.016 + 1.2e-5 * std::min(len, 1024.0) + 1e-5 * std::min(len, 8192 * fall) + len * (eb == 1 ? 2e-6 : eb == 2 ? 2.2e-6 : 2.6e-6);
+        work += one_warp ? 0.012 + (it.fused ? 1.2e-5 : 0.9e-5) * len
+                         : 0.016 + 1.2e-5 * std::min(len, 1024.0) + meet * std::min(len, 8192 * fall) + len * (eb == 1 ? 2e-6 : eb == 2 ? 2.2e-6 : 2.6e-6);
     }
-    if (placed && by_lanes + wave < work) return 1;
-    return tans_lanes(uint32_t(n), items[0].n, apart);
+    const bool one_round = longest < TANS_FEW && n <= TANS_ROUND_32;
+    if (placed && !one_round && by_lanes + wave < work) return 1;
+    return tans_lanes(uint32_t(n), longest, apart);
 }
 
 int codec_classes(const ptwm_b200_plan& pl) {

@@ -101,6 +101,13 @@ def test_tans_decode_with_many_lanes_per_chunk(dtype, chunk, chunks):
     check(specs, chunk_size=chunk, forced_codec=TANS)
 
 
+@pytest.mark.parametrize("dtype", ["u8", "bf16", "fp32", "fp8"])
+@pytest.mark.parametrize("chunk, chunks", [(2047, 600), (2999, 2369), (3999, 889), (4000, 889), (5499, 1777), (5500, 1777), (10239, 889), (10240, 889), (10240, 1777)])
+def test_tans_decode_runs_of_a_chunk(dtype, chunk, chunks):
+    # on either side of where a chunk gets fewer runs than lanes, with one round of blocks and one chunk more
+    test_tans_decode_with_many_lanes_per_chunk(dtype, chunk, chunks)
+
+
 @pytest.mark.parametrize("chunks", [1, 400, 1200])
 def test_tans_decode_of_uneven_streams(chunks):
     # nearly all of the symbols in a small part of the bits: walks that meet late or never, and paths that are followed by one lane alone
