@@ -136,10 +136,12 @@ class DecodePlan:
     def views(self, out: torch.Tensor) -> list[torch.Tensor]:
         """Typed, shaped views of the planned tensors inside the output arena."""
         # One torch call per tensor on one view of the arena per dtype, instead of a slice, a view and a reshape of each (a third of
-        # the time, and a pass waits for it).  What has no shape, or a dtype whose elements are not whole bytes, takes the general way.
+        # the time, and a pass waits for it).  What has no shape, a dtype whose elements are not whole bytes, or an arena other than
+        # out_bytes of contiguous bytes (as_strided looks at the storage alone) takes the general way.
         if self._view_specs is None:
             self._view_specs = [self.handle._view_spec(i, off) for i, off in zip(self.indices, self.out_offsets)]
-        whole = out.numel() % 16 == 0 and out.storage_offset() % 16 == 0
+        whole = (out.dim() == 1 and out.element_size() == 1 and out.is_contiguous() and out.numel() >= self.out_bytes and out.numel() % 16 == 0
+                 and out.storage_offset() % 16 == 0)
         typed, result = {}, []
         for i, off, spec in zip(self.indices, self.out_offsets, self._view_specs):
             if spec is None or not whole:

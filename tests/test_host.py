@@ -385,3 +385,23 @@ def test_views_of_a_plan_are_the_views_of_its_tensors(at):
     for i, off, got in zip(plan.indices, plan.out_offsets, plan.views(arena)):
         want = handle._view(i, arena, off)
         assert (got.dtype, got.shape, got.stride(), got.data_ptr()) == (want.dtype, want.shape, want.stride(), want.data_ptr())
+
+
+def test_views_of_an_arena_that_is_not_the_plans():
+    # shorter than the plan inside a larger buffer, every second byte of one, rows of bytes: what a slice, a view and a reshape of every tensor give or refuse
+    import torch
+    from _data import mixed_model
+    handle = ptwm_b200.ContainerHandle(oracle.write_container(mixed_model(), chunk_size=4096), device=0)
+    plan = handle.plan(None)
+    n = plan.out_bytes
+    large = torch.randint(0, 256, (2 * n + 512,), dtype=torch.uint8)
+
+    def outcome(f):
+        try:
+            return [(t.dtype, t.shape, t.stride(), t.data_ptr()) for t in f()]
+        except (RuntimeError, TypeError, IndexError) as e:
+            return type(e)
+
+    for arena in (large[:n - 256], large[:256], large[:0], large[:2 * n:2], large[:n].view(-1, 16), large[:n].view(torch.int32), large[:n].view(torch.int8)):
+        want = outcome(lambda: [handle._view(i, arena, off) for i, off in zip(plan.indices, plan.out_offsets)])
+        assert outcome(lambda: plan.views(arena)) == want, (arena.shape, arena.stride(), arena.dtype)
