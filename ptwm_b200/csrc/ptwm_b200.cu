@@ -371,12 +371,12 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
 // 3.3 times that per symbol where some lane in most rounds of 32 symbols has four in a row that take more than 32 bits (8 groups, 32
 // lanes) and all of them go back.  With several lanes per chunk a launch takes a latency and then its work: per chunk 16 to 28 ns,
 // 10 ps per symbol of the first 8 Ki (paths meeting), and what placing a symbol costs.  Planes above four bits per symbol meet sooner,
-// and so do nibbles.  Below TANS_FEW symbols several lanes are the faster ones as long as one round of blocks holds the launch; after
-// that every round costs its latency again.
+// and so do nibbles; below two bits they meet later.  Otherwise, below TANS_FEW symbols, several lanes are the faster ones as long as one round of
+// blocks holds the launch (fp32 from 4000 symbols on: of blocks of 64 lanes); after that every round costs its latency again.
 // us, lane per stream / several lanes: bf16, 512: 3552 chunks 152 / 149; 1 Ki: 2368 166 / 116, 2700 165 / 185; 2 Ki: 2368 197 / 171, 2700 197 / 264;
 // 4 Ki: 2368 250 / 238, 2700 249 / 362; 8 Ki: 2368 360 / 359, 2700 360 / 430; 16 Ki: 2368 590 / 529; 32 Ki: 3552 1034 / 864, 4736 1031 / 1021;
 // 64 Ki: 4736 1902 / 1481; fp32, 32 Ki: 2368 1041 / 674, 4736 1038 / 1122; fp16, 8 Ki, 2700 386 / 308; 32 Ki, 4736 1078 / 765; fp8, 8 Ki, 2368 691 /
-// 577; bf16, half of it zeros, 16 Ki: 4736 2606 / 1435.
+// 577; fp32, 6000, 2368 319 / 360; bf16, half of it zeros, 16 Ki: 4736 2606 / 1435; 99 % zeros, both planes: 32 Ki, 4000 2527 / 3162, 64 Ki, 1184 2793 / 1602.
 uint32_t tans_kernel(const DecodeItem* items, size_t n) {
     constexpr size_t WAVE = 148 * TANS_CTA_CHUNKS;
     const uint32_t longest = n ? items[0].n : 0;
@@ -385,19 +385,23 @@ uint32_t tans_kernel(const DecodeItem* items, size_t n) {
     double by_lanes = 0, wave = 0, work = one_warp ? rounds(TANS_ROUND_32) * (28 + 0.03 * longest) : longest < TANS_FEW ? 65 + 50 * rounds(TANS_ROUND_64) : 150, apart = 1;
     const double meet = longest < TANS_FEW ? 7e-6 : 1e-5;
     bool placed = true;
+    double symbols = 0, all_bits = 0;
     for (size_t k = 0; k < n && placed; ++k) {
         const DecodeItem& it = items[k];
         const uint32_t eb = it.fused ? uint32_t(kind_elem_bytes(it.kind)) : 1u;
         placed = eb != 4 || it.slot == 3;  // otherwise its decoding warp alone places the elements there
         const double len = it.n, bits = 8.0 * (it.src_len > 200 ? it.src_len - 100 : it.src_len) / std::max(len, 1.0);  // a header is some 100 bytes
         const double q = double(it.row_len >> 16) / 2048, back = std::min(1.0, 256 * q * q * q * q), f = 4.2 / std::max(bits, 4.2), fall = f * f * f * f;
+        const double late = std::sqrt(2 / std::min(2.0, std::max(bits, 1.0 / 64)));
+        symbols += len; all_bits += bits * len;
         if (k % WAVE == 0) { by_lanes += wave; wave = 0; }
         wave = std::max(wave, 148 + 0.0267 * len * (1 + 3.3 * back));
         if (k == 0) apart = fall * fall * (it.fused && eb == 1 ? 0.25 : 1);
         work += one_warp ? 0.012 + (it.fused ? 1.2e-5 : 0.9e-5) * len
-                         : 0.016 + 1.2e-5 * std::min(len, 1024.0) + meet * std::min(len, 8192 * fall) + len * (eb == 1 ? 2e-6 : eb == 2 ? 2.2e-6 : 2.6e-6);
+                         : 0.016 + 1.2e-5 * std::min(len, 1024.0) + meet * late * std::min(len, 8192 * fall) + len * (eb == 1 ? 2e-6 : eb == 2 ? 2.2e-6 : 2.6e-6);
     }
-    const bool one_round = longest < TANS_FEW && n <= TANS_ROUND_32;
+    const bool fp32 = n && items[0].fused && items[0].kind == K_M32;
+    const bool one_round = longest < TANS_FEW && n <= (fp32 && !one_warp ? TANS_ROUND_64 : TANS_ROUND_32) && all_bits >= 2 * symbols;
     if (placed && !one_round && by_lanes + wave < work) return 1;
     return tans_lanes(uint32_t(n), longest, apart);
 }
