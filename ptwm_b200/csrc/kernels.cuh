@@ -595,9 +595,9 @@ __host__ __device__ inline uint32_t rans_smem_bytes(uint32_t l_entries, bool per
 }
 
 // Chunks of a launch up to which the kernel with a table entry per slot is the faster one: what the GPU holds of it at once (six
-// blocks of four chunks per SM).  Chunks of 32 Ki symbols of a bf16 model, table per slot against rank tables: 1 chunk 447 / 736 us,
-// 592 chunks 455 / 771, 2368 506 / 783, 3552 609 / 786, and beyond that a second wave (4736: 1050 / 789).  fp32: 491 / 826, 621 /
-// 863, 650 / 867, 834 / 872.
+// blocks of four chunks per SM).  Chunks of 32 Ki symbols of a bf16 model, table per slot against rank tables: 1 chunk 430 / 736 us,
+// 592 chunks 442 / 771, 2368 474 / 783, 3552 583 / 786, and beyond that a second wave (4736: 1050 / 789).  fp32: 464 / 826, 595 /
+// 863, 619 / 867, 804 / 872.
 constexpr uint32_t RANS_DIRECT_CHUNKS = 6 * 4 * 148;
 constexpr uint32_t RANS_DIRECT_BYTES = 2048 * 4;  // per chunk
 __host__ __device__ inline uint32_t rans_direct_smem(uint32_t warp_chunks) { return warp_chunks * RANS_DIRECT_BYTES + RING_SMEM; }
@@ -1305,7 +1305,7 @@ __global__ void __launch_bounds__(32) huffman_decode_kernel(const DecodeItem* __
 // the latency of a step (54 cycles: the table read, two shifts, an add) times
 // those steps; in large ones shared memory (a look-up of 32 lanes takes 3.4
 // passes) and the issue slots, 2.7 to 4.3 look-ups per symbol.  A 4096 x 4096
-// bf16 tensor in 256 chunks: 607 -> 296 us.
+// bf16 tensor in 256 chunks: 607 -> 288 us.
 //
 // Table: one word per state, bit count (low five bits: what a funnel shift
 // takes of it) | symbol << 8 | byte offset of the baseline's entry << 16.
@@ -2366,11 +2366,11 @@ inline void tans_launch_t(const DecodeItem* items, uint32_t n, const Bases& base
     tans_decode_kernel<LANES><<<n, LANES, sizeof(TansShared<LANES>), st>>>(items, bases, status);
 }
 // Lanes per chunk: many shorten a chunk's latency and cost more walks per symbol, so as many as the GPU has room for.  us with
-// 256 / 128 / 64 / 32 lanes, bf16: 64 Ki symbols, 148 chunks 256 / 257 / 364 / 498, 592: 351 / 340 / 438 / 589, 1184: 607 / 585 / 576 / 686,
-// 2368: 1120 / 909 / 928 / 907; 16 Ki, 296: 231 / 187 / 267 / 489, 1184: 452 / 355 / 351 / 659, 2368: 796 / 525 / 511 / 626; 8 Ki, 1776:
-// 479 / 378 / 417 / 561.  Runs that are long against the way to a meeting (`apart`, in symbols of 1,400) need fewer walks: 128 Ki, 3552 chunks
-// 2344 / 2050 / 2052 / 1881; fp8, 64 Ki, 2368: 2011 / 1667 / 1565 / 1396; fp16, 8 Ki, 2368: 398 / 321 / 298 / 248.  In chunks that are mostly
-// serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 176, 32: 113.  Below TANS_FEW symbols the rounds of blocks count, 12 per SM
+// 256 / 128 / 64 / 32 lanes, bf16: 64 Ki symbols, 148 chunks 258 / 294 / 380 / 631, 592: 332 / 356 / 442 / 651, 1184: 593 / 592 / 507 / 669,
+// 2368: 1110 / 891 / 912 / 879; 16 Ki, 296: 214 / 233 / 220 / 528, 1184: 464 / 338 / 299 / 553, 2368: 809 / 510 / 526 / 717; 8 Ki, 1776:
+// 470 / 421 / 285 / 295.  Runs that are long against the way to a meeting (`apart`, in symbols of 1,400) need fewer walks: fp8, 64 Ki, 2368: 1993 /
+// 1597 / 1539 / 1327; fp16, 8 Ki, 2368: 398 / 316 / 280 / 221 (bf16, 128 Ki, 3552: 2291 / 2062 / 1933 / 2016).  In chunks that are mostly
+// serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 182, 32: 122.  Below TANS_FEW symbols the rounds of blocks count, 12 per SM
 // with 64 lanes and 16 with 32; 64 / 32 lanes: 3500 symbols, 1184 chunks 187 / 175, 1776 236 / 195 (fp16 137 / 163, 177 / 175); 6000: 1776 263 / 273,
 // 1900 304 / 261, 2368 356 / 287.
 constexpr uint32_t TANS_ROUND_64 = 148 * TansShape<64>::BLOCKS, TANS_ROUND_32 = 148 * TansShape<32>::BLOCKS;
