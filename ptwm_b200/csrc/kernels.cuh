@@ -591,15 +591,26 @@ constexpr uint32_t RANS_DENSE_SYMBOLS = 96;
 //    `l_entries` is then the number of rows and bounds the distinct symbols of
 //    a chunk; the host sends only chunks that fit.
 constexpr int RANS_RANK_BYTES = 512;
+// The kernel for narrow alphabets takes another table where all eight chunks of a warp allow it: an entry of two words for 32 slots,
+// the symbol that covers the first of them and the one that covers the last, so one read instead of two that wait for one another.
+// Exponent planes have their rare symbols at the ends of the slots, a few slots each, so the first 64 and the last 16 slots have an
+// entry each; elsewhere two symbols to 32 slots are all there are (normal, Laplace and Student-t weights, one sigma or one per row: every
+// chunk of some hundred; a plane half of zeros has more and keeps the rank table).  The number of a slot's entry is
+// max(min(slot, 62 + slot / 32), slot - 1906).  1136 bytes per chunk, 19 blocks per SM.
+constexpr uint32_t RANS_PAIR_LOW = 64, RANS_PAIR_HIGH = 16, RANS_PAIR_COARSE = RANS_PAIR_LOW - RANS_PAIR_LOW / 32;
+constexpr uint32_t RANS_PAIR_TOP = 2048 - RANS_PAIR_HIGH - (RANS_PAIR_COARSE + 64);  // slot minus entry, last slots
+constexpr uint32_t RANS_PAIR_ENTRIES = 2048 - RANS_PAIR_TOP;
+constexpr uint32_t RANS_PAIR_SMEM = RANS_WARP_CHUNKS * RANS_PAIR_ENTRIES * 8;
 __host__ __device__ inline uint32_t rans_l_entries(uint32_t max_sym) { return (max_sym + 3 + 3) & ~3u; }
 __host__ __device__ inline uint32_t rans_smem_bytes(uint32_t l_entries, bool per_lane = false) {
-    return RANS_WARP_CHUNKS * RANS_RANK_BYTES + (per_lane ? 128 * l_entries : RANS_WARP_CHUNKS * 4 * l_entries) + RING_SMEM;
+    const uint32_t rank = RANS_WARP_CHUNKS * RANS_RANK_BYTES + (per_lane ? 128 * l_entries : RANS_WARP_CHUNKS * 4 * l_entries);
+    return (per_lane && rank < RANS_PAIR_SMEM ? RANS_PAIR_SMEM : rank) + RING_SMEM;
 }
 
 // Chunks of a launch up to which the kernel with a table entry per slot is the faster one: what the GPU holds of it at once (six
-// blocks of four chunks per SM).  Chunks of 32 Ki symbols of a bf16 model, table per slot against rank tables: 1 chunk 430 / 736 us,
-// 592 chunks 442 / 771, 2368 474 / 783, 3552 583 / 786, and beyond that a second wave (4736: 1050 / 789).  fp32: 464 / 826, 595 /
-// 863, 619 / 867, 804 / 872.
+// blocks of four chunks per SM).  Chunks of 32 Ki symbols, us of a bf16 tensor, table per slot against tables of pairs: 1 to 592 chunks
+// 487 / 681, 2368 518 / 709, 3552 619 / 694, and beyond that a second wave (start of it, 4144: 832 / 694).  fp32: 507 / 739, 592 chunks 634 / 752,
+// 2368 667 / 758, 3552 855 / 780; fp16 (rank tables) 483 / 876, 3552 645 / 928.
 constexpr uint32_t RANS_DIRECT_CHUNKS = 6 * 4 * 148;
 constexpr uint32_t RANS_DIRECT_BYTES = 2048 * 4;  // per chunk
 __host__ __device__ inline uint32_t rans_direct_smem(uint32_t warp_chunks) { return warp_chunks * RANS_DIRECT_BYTES + RING_SMEM; }
@@ -698,6 +709,81 @@ __device__ __forceinline__ void rans_group8(const uint32_t* tab, const uint32_t*
     }
 }
 
+// The same on the table of pairs.  The state is kept doubled with the next bit of the stream below it, so that the bits it wants are
+// its leading zeros without their low three bits, and a slot is twelve bits: twice its number and that bit.  A word of an entry added to the
+// slot (on top, ones below) is the slot's distance from the symbol's first, doubled, << 20 | symbol << 12 | frequency * 2: all that
+// the update takes.  A symbol that starts behind the slot gives a distance that wraps, so the right one of two is the smaller sum.
+// The integer pipe (half an instruction per cycle and scheduler) is as busy as anything here, so what can be is a multiply-add with a
+// power of two that the compiler does not know, or a float multiply-add with truncation (2^23 + 2 * slot, divided by 64).
+// 8192 symbols of a stream: 850 -> 695 us up to four blocks per SM; the six-layer bf16 model, 3.2 rounds of 19 blocks, 4103 -> 3670 us:
+// POPC and a read less in the chain, 10.8 -> 9.0 passes of the load/store pipe per warp and symbol, 23 -> 20 integer instructions.
+// Tried: entries laid out so that the chunks of a read have banks of their own (6.3 -> 5.3 passes) 3822; byte count by comparisons 3982; the
+// window's second word left alone for four symbols 3668; sixteen symbols to a look at the ring 3913; streams in 32-byte blocks 3977.
+constexpr uint32_t RANS_PAIR_ONE = 0x4B000000u;   // 2^23
+struct RansPair { uint32_t base, two20, one, four, eight; };  // shared address of the chunk's first entry, for the float's bits; powers of two
+// `one` is 1 and not a constant.
+__device__ __forceinline__ RansPair rans_pair_at(const void* table, uint32_t one) {
+    return {uint32_t(__cvta_generic_to_shared(table)) - 4 * RANS_PAIR_ONE, one << 20, one, one * 4, one * 8};
+}
+__device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
+// One symbol of a state `xx` (doubled, see above): the sum; the symbol is in bits 12 to 19.
+__device__ __forceinline__ uint32_t rans_pair_lookup(const RansPair& p, uint32_t& xx) {
+    uint32_t m, q, first, second;
+    asm("lop3.b32 %0, %1, 0xFFE, 0x4B000000, 0xEA;" : "=r"(m) : "r"(xx));  // (xx & 0xFFE) | 2^23
+    const uint32_t c = __float_as_uint(__fmaf_rz(__uint_as_float(m), 0x1p-6f, 8388608.0f - 131072.0f));
+    const int low = int(mad_u32(m, p.four, p.base)), coarse = int(mad_u32(c, p.eight, p.base + 8 * RANS_PAIR_COARSE - 4 * RANS_PAIR_ONE));
+    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(first), "=r"(second) : "r"(max(min(low, coarse), low - int(8 * RANS_PAIR_TOP))));
+    const uint32_t slot = mad_u32(xx, p.two20, 0xFFFFFu);
+    asm("mul.hi.u32 %0, %1, %2;" : "=r"(q) : "r"(xx), "r"(p.two20));
+    const uint32_t d = min(mad_u32(first, p.one, slot), slot + second);
+    xx = (d & 0xFFFu) * q + (d >> 20);
+    return d;
+}
+// Up to eight symbols, byte by byte: `x` as in rans_short_group.
+__device__ __forceinline__ void rans_pair_short(const RansPair& p, const uint32_t* rw, uint32_t& x, uint32_t& rq, uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
+    s_lo = 0; s_hi = 0;
+    for (uint32_t j = 0; j < g; ++j) {
+        uint32_t xx = x << 1;
+        const uint32_t sym = (rans_pair_lookup(p, xx) >> 12) & 0xFFu;
+        x = xx >> 1;
+        if (j < 4) s_lo |= sym << (8 * j); else s_hi |= sym << (8 * (j - 4));
+        for (int k = 0; k < 3 && x < RANS_L; ++k) { x = (x << 8) | ring_byte(rw, rq); ++rq; }
+    }
+}
+__device__ __noinline__ uint4 rans_pair_short8(uint32_t base, const uint32_t* rw, uint32_t x, uint32_t rq) {
+    uint32_t s_lo, s_hi;
+    rans_pair_short(RansPair{base, 1u << 20, 1, 4, 8}, rw, x, rq, 8, s_lo, s_hi);
+    return make_uint4(x, rq, s_lo, s_hi);
+}
+__device__ __forceinline__ void rans_pair_group8(const RansPair& p, const uint32_t* rw, uint32_t& x, uint32_t& rq, uint32_t& s_lo, uint32_t& s_hi) {
+    uint32_t wh, wl, used = 0;
+    ring_window_be(rw, rq, wh, wl);
+    uint32_t xx = __funnelshift_l(wh, x, 1);
+    wh = __funnelshift_l(wl, wh, 1);
+    wl <<= 1;
+    s_lo = 0; s_hi = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const uint32_t e = rans_pair_lookup(p, xx) * 16;  // the symbol in the third byte
+        const uint32_t ins = (0x3210u & ~(0xFu << (4 * (j & 3)))) | (6u << (4 * (j & 3)));
+        if (j < 4) s_lo = __byte_perm(s_lo, e, ins); else s_hi = __byte_perm(s_hi, e, ins);
+        uint32_t zeros;
+        asm("bfind.shiftamt.u32 %0, %1;" : "=r"(zeros) : "r"(xx));
+        const uint32_t sh = zeros & 0x18u;
+        xx = __funnelshift_l(wh, xx, sh);
+        wh = __funnelshift_l(wl, wh, sh);
+        wl <<= sh;
+        used += sh;
+    }
+    if (used > 64) {
+        const uint4 again = rans_pair_short8(p.base, rw, x, rq);
+        x = again.x; rq = again.y; s_lo = again.z; s_hi = again.w;
+    } else {
+        x = xx >> 1;
+        rq += used >> 3;
+    }
+}
+
 // The same on a table with an entry per slot: slot's distance from the symbol's first << 20 | symbol << 12 | frequency, so that
 // both factors of the update are one step away.  From one state to the next it is a mask, one shared-memory read, a shift and a
 // multiply-add; renormalising moves the state shifted by one or two bytes over the state, two moves that hang on the comparisons
@@ -752,8 +838,7 @@ __device__ __forceinline__ uint32_t rans_direct_four(const uint32_t* tab, const 
 }
 
 // 20 blocks per SM lets the compiler use 96 registers (21 blocks), which the 32-bit rounds need to stay out of local
-// memory; shared memory allows 22, and more blocks than that gave nothing (the load/store pipe, the integer pipe and the
-// issue slots are each about 55-60 % busy there).
+// memory; shared memory allows 19, or 22 with rank tables of short lists, and more blocks than that gave nothing.
 //
 // DIRECT (chunks per warp, 0 = the rank tables above): a table entry per slot, 8 KiB per chunk, for launches that do not fill
 // the GPU, where the time from one symbol to the next is all that counts (rans_direct_four).
@@ -768,8 +853,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
     uint32_t* slots = reinterpret_cast<uint32_t*>(smem + RING_SMEM);                                  // DIRECT: [chunk][2048]
     uint32_t* ranktab = reinterpret_cast<uint32_t*>(smem);                                            // [8][128]
     uint32_t* symlist = reinterpret_cast<uint32_t*>(smem + (DIRECT ? 1 : CHUNKS) * RANS_RANK_BYTES);  // entry 0 of every list is a pad
-    const uint32_t list_bytes = PER_LANE ? 128 * l_entries : CHUNKS * 4 * l_entries;
-    Ring ring{reinterpret_cast<uint32_t*>(DIRECT ? smem : smem + CHUNKS * RANS_RANK_BYTES + list_bytes) + lane};
+    Ring ring{reinterpret_cast<uint32_t*>(DIRECT ? smem : smem + rans_smem_bytes(l_entries, PER_LANE) - RING_SMEM) + lane};
 
     const uint32_t item_idx = blockIdx.x * CHUNKS + c;
     const bool valid = c < CHUNKS && item_idx < n_items;
@@ -801,74 +885,100 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
 
     // tables: the whole warp builds one chunk's tables at a time
     bool dense = false;  // this lane's chunk is close to incompressible (see rans_group8)
-    for (uint32_t c2 = 0; c2 < CHUNKS; ++c2) {
-        const uint32_t leader = c2 * 4;
-        uintptr_t psrc = __shfl_sync(0xFFFFFFFFu, reinterpret_cast<uintptr_t>(src), leader);
-        uint32_t pms = __shfl_sync(0xFFFFFFFFu, max_sym, leader);
-        uint32_t perr = __shfl_sync(0xFFFFFFFFu, err, leader);
-        uint32_t pvalid = __shfl_sync(0xFFFFFFFFu, uint32_t(valid), leader);
-        if (!pvalid || perr) continue;
-        const uint8_t* ps = reinterpret_cast<const uint8_t*>(psrc);
-        uint32_t f[8], sum = 0, present = 0;
+    // The narrow kernel tries the tables of pairs first, with a chunk's rank table and symbol list in the place of the rings meanwhile.
+    bool pairs = PER_LANE;
+    if (PER_LANE) {  // states that rans_pair_group8 cannot take: see rans_group8, rans_direct_four
+        const uint32_t x = valid && !err && my_len >= 4 ? ld_u32_unaligned(src + my_off) : RANS_L;
+        pairs = !__any_sync(0xFFFFFFFFu, x >> 31 || x < RANS_L);
+    }
+    for (uint32_t pass = 0; pass < (PER_LANE ? 2u : 1u); ++pass) {  // 0: tables of pairs; 1: the others, also when a chunk does not fit the former
+        if (PER_LANE && (pass == 0) != pairs) continue;
+        for (uint32_t c2 = 0; c2 < CHUNKS; ++c2) {
+            const uint32_t leader = c2 * 4;
+            uintptr_t psrc = __shfl_sync(0xFFFFFFFFu, reinterpret_cast<uintptr_t>(src), leader);
+            uint32_t pms = __shfl_sync(0xFFFFFFFFu, max_sym, leader);
+            uint32_t perr = __shfl_sync(0xFFFFFFFFu, err, leader);
+            uint32_t pvalid = __shfl_sync(0xFFFFFFFFu, uint32_t(valid), leader);
+            if (!pvalid || perr) continue;
+            const uint8_t* ps = reinterpret_cast<const uint8_t*>(psrc);
+            uint32_t f[8], sum = 0, present = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            uint32_t sym = lane * 8 + k;
-            f[k] = sym <= pms ? uint32_t(ps[1 + 2 * sym]) | uint32_t(ps[2 + 2 * sym]) << 8 : 0u;
-            sum += f[k];
-            present += f[k] != 0;
-        }
-        uint32_t incl = sum, rincl = present;
+            for (int k = 0; k < 8; ++k) {
+                uint32_t sym = lane * 8 + k;
+                f[k] = sym <= pms ? uint32_t(ps[1 + 2 * sym]) | uint32_t(ps[2 + 2 * sym]) << 8 : 0u;
+                sum += f[k];
+                present += f[k] != 0;
+            }
+            uint32_t incl = sum, rincl = present;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d), r = __shfl_up_sync(0xFFFFFFFFu, rincl, d);
-            if (lane >= d) { incl += t; rincl += r; }
-        }
-        uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31), distinct = __shfl_sync(0xFFFFFFFFu, rincl, 31);
-        bool bad = total != 2048;  // decompress.rs:49-55
-        if (!PER_LANE && c == c2) dense = distinct >= RANS_DENSE_SYMBOLS;
-        if (distinct + 2 > l_entries) bad = true;  // the host sizes the list from the planned bytes; a blob that differs from them may not fit
-        if (bad) { if (c == c2) err = ST_BAD_HEADER; continue; }
-        uint32_t start = incl - sum, rank = rincl - present;
-        uint32_t* tab = DIRECT ? ranktab : ranktab + c2 * 128;
-        uint32_t* lst = DIRECT ? symlist : PER_LANE ? symlist + c2 * 4 : symlist + c2 * l_entries;
-        if (lane == 0) {
-            if (PER_LANE) *reinterpret_cast<uint4*>(lst) = make_uint4(0, 0, 0, 0); else lst[0] = 0;
-        }
-        *reinterpret_cast<uint4*>(tab + 4 * lane) = make_uint4(0, 0, 0, 0);
-        __syncwarp();
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            uint32_t sym = lane * 8 + k, fr = f[k];
-            if (!fr) continue;
-            uint32_t entry = sym | (fr << 8) | (start << 20);
-            if (PER_LANE) *reinterpret_cast<uint4*>(lst + (rank + 1) * 32) = make_uint4(entry, entry, entry, entry);  // the four lanes of the chunk
-            else lst[rank + 1] = entry;
-            atomicOr(&tab[start >> 4], 1u << (start & 15));
-            start += fr; ++rank;
-        }
-        __syncwarp();
-        // boundaries before each word: lane l owns words 4l .. 4l+3
-        uint4 bm = *reinterpret_cast<uint4*>(tab + 4 * lane);
-        uint32_t p0 = __popc(bm.x), p1 = __popc(bm.y), p2 = __popc(bm.z), p3 = __popc(bm.w), scan = p0 + p1 + p2 + p3;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            uint32_t t = __shfl_up_sync(0xFFFFFFFFu, scan, d);
-            if (lane >= d) scan += t;
-        }
-        uint32_t before = scan - (p0 + p1 + p2 + p3);
-        bm.x |= before << 16; before += p0;
-        bm.y |= before << 16; before += p1;
-        bm.z |= before << 16; before += p2;
-        bm.w |= before << 16;
-        *reinterpret_cast<uint4*>(tab + 4 * lane) = bm;
-        if (DIRECT) {
+            for (int d = 1; d < 32; d <<= 1) {
+                uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d), r = __shfl_up_sync(0xFFFFFFFFu, rincl, d);
+                if (lane >= d) { incl += t; rincl += r; }
+            }
+            uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31), distinct = __shfl_sync(0xFFFFFFFFu, rincl, 31);
+            bool bad = total != 2048;  // decompress.rs:49-55
+            if (!PER_LANE && c == c2) dense = distinct >= RANS_DENSE_SYMBOLS;
+            if (distinct + 2 > l_entries) bad = true;  // the host sizes the list from the planned bytes; a blob that differs from them may not fit
+            if (bad) { if (c == c2) err = ST_BAD_HEADER; continue; }
+            uint32_t start = incl - sum, rank = rincl - present;
+            uint32_t* tab = pairs ? ring.base - lane : DIRECT ? ranktab : ranktab + c2 * 128;
+            uint32_t* lst = pairs ? tab + 128 : DIRECT ? symlist : PER_LANE ? symlist + c2 * 4 : symlist + c2 * l_entries;
+            if (lane == 0) {
+                if (PER_LANE && !pairs) *reinterpret_cast<uint4*>(lst) = make_uint4(0, 0, 0, 0); else lst[0] = 0;
+            }
+            *reinterpret_cast<uint4*>(tab + 4 * lane) = make_uint4(0, 0, 0, 0);
             __syncwarp();
-#pragma unroll 8
-            for (uint32_t u = lane; u < 2048; u += 32) {
-                const uint32_t w = tab[u >> 4], e = lst[(w >> 16) + __popc(w << ((~u & 15u) | 16u))];
-                slots[c2 * 2048 + u] = (u - (e >> 20)) << 20 | (e & 0xFFu) << 12 | ((e >> 8) & 0xFFFu);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                uint32_t sym = lane * 8 + k, fr = f[k];
+                if (!fr) continue;
+                uint32_t entry = sym | (fr << 8) | (start << 20);
+                if (PER_LANE && !pairs) *reinterpret_cast<uint4*>(lst + (rank + 1) * 32) = make_uint4(entry, entry, entry, entry);  // the four lanes of the chunk
+                else lst[rank + 1] = entry;
+                atomicOr(&tab[start >> 4], 1u << (start & 15));
+                start += fr; ++rank;
             }
             __syncwarp();
+            // boundaries before each word: lane l owns words 4l .. 4l+3
+            uint4 bm = *reinterpret_cast<uint4*>(tab + 4 * lane);
+            uint32_t p0 = __popc(bm.x), p1 = __popc(bm.y), p2 = __popc(bm.z), p3 = __popc(bm.w), scan = p0 + p1 + p2 + p3;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                uint32_t t = __shfl_up_sync(0xFFFFFFFFu, scan, d);
+                if (lane >= d) scan += t;
+            }
+            uint32_t before = scan - (p0 + p1 + p2 + p3);
+            bm.x |= before << 16; before += p0;
+            bm.y |= before << 16; before += p1;
+            bm.z |= before << 16; before += p2;
+            bm.w |= before << 16;
+            *reinterpret_cast<uint4*>(tab + 4 * lane) = bm;
+            if (pairs) {
+                __syncwarp();
+                auto number = [&](uint32_t u) { const uint32_t w = tab[u >> 4]; return (w >> 16) + __popc(w << ((~u & 15u) | 16u)); };
+                auto entry = [&](uint32_t k) { const uint32_t e = lst[k]; return ((e & 0xFFu) << 12 | ((e >> 8) & 0xFFFu) * 2) - 0xFFFFFu - ((e >> 20) << 21); };
+                bool fits = distinct > 1;  // (a frequency of 2048 is one bit too long)
+                for (uint32_t k = lane; k < RANS_PAIR_ENTRIES; k += 32) {
+                    const bool coarse = k >= RANS_PAIR_LOW && k < RANS_PAIR_COARSE + 64;
+                    const uint32_t u = k < RANS_PAIR_LOW ? k : coarse ? (k - RANS_PAIR_COARSE) * 32 : k + RANS_PAIR_TOP;
+                    const uint32_t last = coarse ? (u + 31 < 2047 - RANS_PAIR_HIGH ? u + 31 : 2047 - RANS_PAIR_HIGH) : u;
+                    const uint32_t a = number(u), b = number(last);
+                    fits = fits && b - a <= 1;
+                    reinterpret_cast<uint2*>(smem)[c2 * RANS_PAIR_ENTRIES + k] = make_uint2(entry(a), entry(b));
+                }
+                pairs = __all_sync(0xFFFFFFFFu, fits);
+                __syncwarp();
+                if (!pairs) break;
+            }
+            if (DIRECT) {
+                __syncwarp();
+#pragma unroll 8
+                for (uint32_t u = lane; u < 2048; u += 32) {
+                    const uint32_t w = tab[u >> 4], e = lst[(w >> 16) + __popc(w << ((~u & 15u) | 16u))];
+                    slots[c2 * 2048 + u] = (u - (e >> 20)) << 20 | (e & 0xFFu) << 12 | ((e >> 8) & 0xFFFu);
+                }
+                __syncwarp();
+            }
         }
     }
     __syncwarp();
@@ -880,6 +990,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
         else {
             const uint32_t* tab = DIRECT == 1 ? slots : DIRECT ? slots + c * 2048 : ranktab + c * 128;
             const uint32_t* lst = PER_LANE ? symlist + lane : symlist + c * l_entries;
+            const RansPair pair = rans_pair_at(smem + c * RANS_PAIR_ENTRIES * 8, n_items ? 1u : 0u);
             const uint32_t* rw = ring.base;
             Epilogue ep = make_epilogue(bases, it);
             const uint8_t* st = src + my_off;
@@ -912,6 +1023,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
             uint32_t pos = seg_start, remaining = seg_len;
             auto short_group = [&](uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
                 if (DIRECT) rans_direct_short(tab, rw, x, rq, g, s_lo, s_hi);
+                else if (PER_LANE && pairs) rans_pair_short(pair, rw, x, rq, g, s_lo, s_hi);
                 else rans_short_group<LS>(tab, lst, rw, x, rq, g, s_lo, s_hi);
             };
             // head: a short group up to the next 8-element boundary of the destination
@@ -938,6 +1050,11 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
                     s_lo = rans_direct_four(tab, rw, x, rq, v, skip);
                     top_up_at(began, 40);
                     s_hi = rans_direct_four(tab, rw, x, rq, v, skip);
+                });
+            } else if (PER_LANE && pairs) {
+                fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {
+                    top_up();
+                    rans_pair_group8(pair, rw, x, rq, s_lo, s_hi);
                 });
             } else {
                 fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {

@@ -57,6 +57,42 @@ def test_decode_launch_sizes(codec, chunks, dtype):
     check(specs, chunk_size=67, forced_codec=codec)
 
 
+def counted(counts, rng, cluster=0):
+    """2048 symbols with exactly these counts, which are then the table's frequencies; the last `cluster` symbols put side by side."""
+    syms = np.repeat(np.arange(100, 100 + len(counts)), counts)
+    rng.shuffle(syms)
+    if cluster:
+        rare = np.flatnonzero(syms >= 100 + len(counts) - cluster)
+        rest = np.delete(syms, rare)
+        syms = np.concatenate([rest[:700], syms[rare], rest[700:]])
+    return syms.astype(np.uint8)
+
+
+@pytest.mark.parametrize("mix", ["fit", "mixed"])
+@pytest.mark.parametrize("dtype", ["u8", "bf16", "fp8"])
+def test_rans_decode_tables_of_pairs(dtype, mix):
+    # first slots of symbols on either side of where the parts of the table meet (64, 2032) and of 32 slots, one and two symbols, the longest
+    # list, rare symbols side by side (more than eight bytes to eight symbols); "mixed": eight chunks of which some have three symbols to 32 slots
+    rng = np.random.default_rng(5)
+    fit = [[1024, 1024], [1, 2047], [2047, 1], [63, 1969, 16], [64, 1968, 16], [65, 1966, 17], [64, 31, 1, 1952], [64, 32, 1, 1951], [1] * 35 + [30, 1967, 16],
+           [64, 1967] + [1] * 17, [32, 32, 31, 1, 31, 1, 32, 32, 1856], [2] * 32 + [1952, 8, 8, 8, 8], [4, 8, 16, 36, 70, 140, 300, 500, 700, 270, 3, 1]]
+    other = [[2048], [100, 5, 5, 1938], [70, 1, 1, 1976], [1000, 2, 2, 2, 1042], [2000, 20, 2, 2, 24], [54] * 36 + [104]]
+    chunks = []
+    for k in range(3600):
+        pick = other if mix == "mixed" and rng.random() < 0.05 else fit
+        counts = pick[rng.integers(len(pick))]
+        chunks.append(counted(counts, rng, 24 if len(counts) == 19 else 0))
+    raw = np.concatenate(chunks)[:-300]
+    if dtype == "u8":
+        spec = u8("p", raw.tobytes())
+    elif dtype == "bf16":
+        low = rng.integers(0, 256, len(raw)).astype(np.uint16)
+        spec = oracle.TensorSpec("p", oracle.DT_BF16, [len(raw)], ((low & 0x80) << 8 | raw.astype(np.uint16) << 7 | low & 0x7F).astype(np.uint16).tobytes())
+    else:
+        spec = oracle.TensorSpec("p", oracle.DT_E4M3, [len(raw)], (raw * 37 & 0xFF).astype(np.uint8).tobytes())
+    check([spec], chunk_size=2048, forced_codec=RANS)
+
+
 @pytest.mark.parametrize("alphabet", [2, 31, 33, 64, 256])
 @pytest.mark.parametrize("cols", [1, 5, 8, 9, 37, 0])
 def test_order1_scale_ac_shares_and_rows(alphabet, cols):
