@@ -259,6 +259,11 @@ __device__ __forceinline__ void stg256(void* p, uint4 a, uint4 b) {
     asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
                  : "memory");
 }
+// The same for bytes that the block reads again.
+__device__ __forceinline__ void stg256_kept(void* p, uint4 a, uint4 b) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
 // Aligned 32-byte block at `a`; bytes outside [lo, hi) read as zero and are not touched.
 __device__ __forceinline__ Block32 load_block_guarded(uintptr_t a, uintptr_t lo, uintptr_t hi) {
     if (a >= lo && a + 32 <= hi) return ldg256(reinterpret_cast<const void*>(a));
@@ -1439,7 +1444,7 @@ template <int LANES> struct TansShape;
 template <> struct TansShape<32> { static constexpr uint32_t SEGS = 2, SLOTS = 2, BLOCKS = 16; };
 template <> struct TansShape<64> { static constexpr uint32_t SEGS = 1, SLOTS = 4, BLOCKS = 12; };
 template <> struct TansShape<128> { static constexpr uint32_t SEGS = 1, SLOTS = 8, BLOCKS = 6; };
-template <> struct TansShape<256> { static constexpr uint32_t SEGS = 1, SLOTS = 8, BLOCKS = 4; };
+template <> struct TansShape<256> { static constexpr uint32_t SEGS = 1, SLOTS = 8, BLOCKS = 2; };  // launches of two chunks per SM at most: room for its registers
 
 // Runs of a chunk.  32 and 64 lanes serve launches whose walks fill the GPU: there many walks of a short chunk cost more than they save, and
 // nodes that hold few paths each let them pass one another unmet.  us of 1184 chunks, bf16, 32 lanes with up to 32 / 16 / 8 runs: 2700
@@ -1948,7 +1953,7 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
         };
         if (LANES > 32) {
             uint32_t g = uint32_t(8 - (reinterpret_cast<uintptr_t>(stage + pos) & 7));
-            while (remaining) {
+            auto some = [&]() {  // up to a boundary of eight bytes
                 if (g > remaining) g = remaining;
                 uint64_t syms = kept;
                 if (g > keep) {
@@ -1962,7 +1967,24 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
                 else for (uint32_t k = 0; k < g; ++k) to[k] = uint8_t(syms >> (8 * k));
                 pos += g; remaining -= g;
                 g = 8;
+            };
+#pragma unroll 1
+            do { if (remaining) some(); } while (remaining && (reinterpret_cast<uintptr_t>(stage + pos) & 31));
+            const uint32_t by = 8 * keep;
+#pragma unroll 1
+            for (; remaining >= 32; remaining -= 32, pos += 32) {  // whole sectors: a store by lanes that each walk a run of their own costs a pass per lane
+                uint64_t out[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint64_t next = more();
+                    out[k] = kept | next << by;
+                    kept = by ? next >> (64 - by) : 0;
+                }
+                stg256_kept(stage + pos, make_uint4(uint32_t(out[0]), uint32_t(out[0] >> 32), uint32_t(out[1]), uint32_t(out[1] >> 32)),
+                       make_uint4(uint32_t(out[2]), uint32_t(out[2] >> 32), uint32_t(out[3]), uint32_t(out[3] >> 32)));
             }
+#pragma unroll 1
+            while (remaining) some();
         } else {
             const Epilogue ep = make_epilogue(bases, it);
             auto dec8 = [&](uint32_t& s_lo, uint32_t& s_hi) {
