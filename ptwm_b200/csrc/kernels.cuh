@@ -1411,7 +1411,11 @@ __global__ void __launch_bounds__(32) huffman_decode_kernel(const DecodeItem* __
 //   pair first does not change what is decoded from it.
 // * Lane 0 starts in the right state.  Its path, then that of the lane it met,
 //   and so on is the right one; along it the state at every cut and the number
-//   of symbols before it are known.
+//   of symbols before it are known.  It is followed by jumps of doubling length
+//   (one by one it was 85 steps of 280 cycles with 256 lanes), and once it
+//   reaches the last run the walks that still go on are none of it and end:
+//   two tANS chunks of 4096 symbols 204 -> 150 us, 256 of 64 Ki 282 -> 258,
+//   4049 of 64 Ki 1375 -> 1326.
 // * Before it falls in, a lane can take many more symbols out of the same bits
 //   than the right path does (codes of rare symbols read out of step are mostly
 //   the frequent one).  So a lane that has met as many symbols as the chunk
@@ -1429,7 +1433,11 @@ __global__ void __launch_bounds__(32) huffman_decode_kernel(const DecodeItem* __
 // the latency of a step (54 cycles: the table read, two shifts, an add) times
 // those steps; in large ones shared memory (a look-up of 32 lanes takes 3.4
 // passes) and the issue slots, 2.7 to 4.3 look-ups per symbol.  A 4096 x 4096
-// bf16 tensor in 256 chunks: 607 -> 288 us.
+// bf16 tensor in 256 chunks: 607 -> 258 us.  A step is 45 cycles where nothing
+// but the group of eight goes on, 60 with the looks at the ring, more with many
+// warps.  Tried: loops without a branch that depends on a lane, the group at a
+// node decoded twice (317 against 282 us), the look at the ring in the middle
+// of every group (313).
 //
 // Table: one word per state, bit count (low five bits: what a funnel shift
 // takes of it) | symbol << 8 | byte offset of the baseline's entry << 16.
@@ -1472,7 +1480,7 @@ struct TansShared {
     uint32_t at[LANES];            // symbols before it
     uint32_t tally[LANES / 32];    // walks of each warp
 };
-constexpr uint32_t TANS_FINISHED = 0xFFFFFFFFu, TANS_DEAD = 0xFFFFFFFEu, TANS_ASIDE = 0x80000000u, TANS_NONE = 0xFFFFFFFFu;
+constexpr uint32_t TANS_FINISHED = 0xFFFFFFFFu, TANS_DEAD = 0xFFFFFFFEu, TANS_ASIDE = 0x80000000u, TANS_WALKING = 0xFFFFFFFDu, TANS_NONE = 0xFFFFFFFFu;
 
 // All lanes of a chunk.
 template <int LANES>
@@ -1660,8 +1668,9 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
     if (uint64_t(runs) * (32 * SEGS) > total_bits) runs = uint32_t(total_bits) / (32 * SEGS);  // nodes at least 32 bits apart
     if (runs < 1) runs = 1;
     const uint64_t apart = total_bits / (runs * SEGS);
-    uint32_t slots = SLOTS;  // short runs leave more paths to a node, and fewer nodes
-    while (slots < 32 && slots * 2 * runs <= SLOTS * LANES) slots *= 2;
+    uint32_t slot_bits = SLOTS == 8 ? 3 : SLOTS == 4 ? 2 : 1;  // short runs leave more paths to a node, and fewer nodes
+    while (slot_bits < 5 && (2u << slot_bits) * runs <= SLOTS * LANES) ++slot_bits;
+    const uint32_t slots = 1u << slot_bits;
     const uint32_t last_node = (runs - 1) * SEGS;  // start of the last run, whose symbols are what is left of the chunk's
     const uint64_t floor_bit = uint64_t(reinterpret_cast<uintptr_t>(bs)) * 8;  // bit address of the stream's first bit
     const uint64_t top_bit = floor_bit + total_bits;
@@ -1816,6 +1825,7 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
         sh.start[0] = start0; sh.at[0] = 0;
         if (!alive) { sh.link[0] = TANS_FINISHED; sh.met[0] = 0; }
     }
+    sh.link[l] = alive ? uint32_t(TANS_WALKING) : uint32_t(TANS_FINISHED);
     if (alive) take_up();
     // A damaged or very uneven stream can hold the whole chunk's symbols, or more, between any two nodes, and paths through a repeated pattern never
     // meet: once a warp has walked a quarter of the chunk's symbols the lanes only finish their runs, and the one with the right path goes on
@@ -1830,8 +1840,25 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
     // The right path is followed from lane 0's on, once nothing moves any more; walks set aside on it are taken up by lane 0.
     uint32_t lane = 0;
     bool too_many = false;
+    // The walk whose path the one of `lane` meets, or itself.
+    auto met_by = [&](uint32_t walk) -> uint32_t { const uint32_t link = sh.link[walk]; return link < TANS_ASIDE ? (sh.key[link] >> 16) & 0x3FFu : walk; };
+    // Whether the right path is known to the last run, in which case the walks still going are none of it: by jumps of doubling length.
+    auto complete = [&]() -> bool {
+        sh.from[l] = met_by(l);
+        tans_sync<LANES>();
+#pragma unroll 1
+        for (uint32_t d = 1; d < LANES; d *= 2) {
+            const uint32_t to = sh.from[sh.from[l]];
+            tans_sync<LANES>();
+            sh.from[l] = to;
+            tans_sync<LANES>();
+        }
+        const bool done = sh.link[sh.from[0]] == TANS_FINISHED;
+        tans_sync<LANES>();
+        return done;
+    };
     for (;;) {
-        const bool go = alive && (walks == ALL ? spent < budget && (warps == 1 || looks < every) : walks == ALONE || node < (who + 1) * SEGS);
+        const bool go = alive && (walks == ALL ? spent < budget && looks < every : walks == ALONE || node < (who + 1) * SEGS);
         if (__any_sync(0xFFFFFFFFu, go)) {
             uint32_t met = 0;
             if (go) met = segment();
@@ -1841,10 +1868,16 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
         }
         if (walks == ALL) {
             looks = 0;
-            if (LANES == 32) { walks = OWN_RUN; continue; }
+            if (LANES == 32) {
+                __syncwarp();
+                if (!__any_sync(0xFFFFFFFFu, alive) || spent >= budget) { walks = OWN_RUN; continue; }
+                if (complete()) alive = false;
+                continue;
+            }
             const uint32_t votes = __ballot_sync(0xFFFFFFFFu, alive);
             if (l % 32 == 0) sh.tally[l / 32] = __popc(votes);
             if (__syncthreads_or(spent >= budget)) { walks = OWN_RUN; continue; }
+            if (complete()) { alive = false; walks = OWN_RUN; continue; }
             uint32_t before = 0, total = 0;
 #pragma unroll
             for (uint32_t v = 0; v < LANES / 32; ++v) { if (v < l / 32) before += sh.tally[v]; total += sh.tally[v]; }
@@ -1866,21 +1899,57 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
             if (total == 0) walks = OWN_RUN;
             continue;
         }
+        uint32_t link;
         if (walks == OWN_RUN) {
             if (alive) set_aside(node, n);
-            sh.from[l] = TANS_NONE;
-            if (l == 0) { sh.from[0] = 0; sh.base[0] = 0; }
             walks = ALONE;
+            // The right path, the walks on it and the symbols before each, by jumps of doubling length: the jumps of every length are kept (the rings
+            // are not in use), sums go to the end of the path, and what lane 0 can reach is marked from the longest jump down.
+            constexpr uint32_t LOG = LANES == 32 ? 5 : LANES == 64 ? 6 : LANES == 128 ? 7 : 8;
+            uint32_t* jump = sh.ring;                                           // [length][lane]
+            int64_t* sum = reinterpret_cast<int64_t*>(sh.ring + LOG * LANES);  // [lane]: symbols from the start of this walk's part to the end
+            tans_sync<LANES>();
+            const uint32_t own = sh.link[l];
+            uint32_t to = met_by(l);
+            int64_t rest = own < TANS_ASIDE ? int64_t(sh.met[l]) - int64_t(sh.count[own]) : 0;
+#pragma unroll 1
+            for (uint32_t d = 0; d < LOG; ++d) {
+                jump[d * LANES + l] = to; sum[l] = rest;
+                tans_sync<LANES>();
+                rest += sum[to]; to = jump[d * LANES + to];
+                tans_sync<LANES>();
+            }
+            sum[l] = rest;
+            sh.from[l] = l == 0 ? 0 : TANS_NONE;
+            tans_sync<LANES>();
+            uint32_t end = 0;
+#pragma unroll 1
+            for (uint32_t d = LOG; d-- > 0;) {
+                if (sh.from[l] != TANS_NONE && jump[d * LANES + l] != l) sh.from[jump[d * LANES + l]] = 0;
+                end = jump[d * LANES + end];
+                tans_sync<LANES>();
+            }
+            const bool on = sh.from[l] != TANS_NONE;
+            const int64_t before = sum[0] - rest;
+            tans_sync<LANES>();
+            if (on) {
+                sh.base[l] = uint32_t(before);
+                too_many = own < TANS_ASIDE && before + int64_t(sh.met[l]) > int64_t(it.n);
+                if (own < TANS_ASIDE) sh.from[(sh.key[own] >> 16) & 0x3FFu] = own >> slot_bits;
+            }
+            too_many = LANES == 32 ? __any_sync(0xFFFFFFFFu, too_many) : __syncthreads_or(too_many);
+            lane = end;
+            base = sum[0] - sum[end];
+            tans_sync<LANES>();
         }
         tans_sync<LANES>();
-        uint32_t link;
         while ((link = sh.link[lane]) < TANS_ASIDE && !too_many) {
             base += sh.met[lane];
             if (base < 0) base += int64_t(1) << 32;  // (a walk taken up whose count went past 2^32)
             too_many = base > int64_t(it.n);
             base -= sh.count[link];
             lane = (sh.key[link] >> 16) & 0x3FFu;
-            if (l == 0) { sh.from[lane] = link / slots; sh.base[lane] = uint32_t(base); }
+            if (l == 0) { sh.from[lane] = link >> slot_bits; sh.base[lane] = uint32_t(base); }
         }
         const int64_t before = base + sh.met[lane];
         too_many = too_many || link == TANS_DEAD || before > int64_t(it.n);
@@ -1895,14 +1964,12 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
     }
     if (too_many) { if (l == 0) report(status, it.id, ST_NOT_CONSUMED); return; }  // more symbols than the chunk has
     tans_sync<LANES>();
-    if (sh.from[l] != TANS_NONE) {  // the lane's path is right between these nodes: where it enters the runs
-        const uint32_t link = sh.link[l], base = sh.base[l], end = link < TANS_ASIDE ? link / slots : last_node + 1;
-        for (uint32_t k = l == 0 ? 1 : (sh.from[l] + SEGS - 1) / SEGS; k * SEGS < end; ++k) {
-            for (uint32_t slot = k * SEGS * slots; slot < (k * SEGS + 1) * slots; ++slot) {
-                const uint32_t key = sh.key[slot];
-                if (key >> 16 == (0x8000u | l)) { sh.start[k] = key & 0x7FFFu; sh.at[k] = base + sh.count[slot]; }
-            }
-        }
+    // what walks of the right path entered where it is theirs: the starts of the runs
+    for (uint32_t slot = l; slot < (last_node + 1) << slot_bits; slot += LANES) {
+        const uint32_t key = sh.key[slot], walk = (key >> 16) & 0x3FFu, at_node = slot >> slot_bits;
+        if (key == 0 || at_node % SEGS != 0 || sh.from[walk] == TANS_NONE || at_node < sh.from[walk]) continue;
+        const uint32_t link = sh.link[walk];
+        if (at_node < (link < TANS_ASIDE ? link >> slot_bits : last_node + 1)) { sh.start[at_node / SEGS] = key & 0x7FFFu; sh.at[at_node / SEGS] = sh.base[walk] + sh.count[slot]; }
     }
     tans_sync<LANES>();
     // ---- last pass: the symbols to their places ----
