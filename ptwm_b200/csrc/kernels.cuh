@@ -1998,83 +1998,69 @@ __global__ void __launch_bounds__(LANES, TansShape<LANES>::BLOCKS) tans_decode_k
             at -= e & 31u;
             return (e >> 8) & 0xFFu;
         };
-        // Symbols are decoded eight at a time from the start of the run and handed out eight at a time from the first boundary of the
-        // output on; `kept` holds the `keep` between the two.  `todo` more belong to the run: a run that another one follows may go on
-        // past its end, the last one may not.
-        uint64_t kept = 0;
-        uint32_t keep = 0, todo = remaining;
-        auto more = [&]() -> uint64_t {
-            uint64_t syms = 0;
+        auto eight = [&](uint32_t& s_lo, uint32_t& s_hi) {
             refill();
-            if (at - floor_at >= TANS_GROUP_BITS && (todo >= 8 || !last)) {
+            if (at - floor_at >= TANS_GROUP_BITS) {
                 uint32_t s[8];
                 at -= group([&](int j, uint32_t e) { s[j] = e; });
-                syms = uint64_t(__byte_perm(__byte_perm(s[4], s[5], 0x0051), __byte_perm(s[6], s[7], 0x0051), 0x5410)) << 32 |
-                       __byte_perm(__byte_perm(s[0], s[1], 0x0051), __byte_perm(s[2], s[3], 0x0051), 0x5410);
-                todo = todo > 8 ? todo - 8 : 0;
+                s_lo = __byte_perm(__byte_perm(s[0], s[1], 0x0051), __byte_perm(s[2], s[3], 0x0051), 0x5410);
+                s_hi = __byte_perm(__byte_perm(s[4], s[5], 0x0051), __byte_perm(s[6], s[7], 0x0051), 0x5410);
             } else {
+                uint64_t syms = 0;
 #pragma unroll 1
-                for (int j = 0; j < 8 && todo; ++j, --todo) syms |= uint64_t(one_checked()) << (8 * j);
+                for (int j = 0; j < 8; ++j) syms |= uint64_t(one_checked()) << (8 * j);
+                s_lo = uint32_t(syms); s_hi = uint32_t(syms >> 32);
             }
+        };
+        auto few = [&](uint32_t count) -> uint64_t {  // less than eight, up to a boundary of the output or the end of the run
+            uint64_t syms = 0;
+            refill();
+            if (at - floor_at >= TANS_GROUP_BITS) {
+                uint32_t bits = 0, there = 0;
+                group([&](int j, uint32_t e) { if (uint32_t(j) < count) { bits += e & 31u; there = entry; syms |= uint64_t((e >> 8) & 0xFFu) << (8 * j); } });
+                at -= bits; entry = there;
+                return syms;
+            }
+#pragma unroll 1
+            for (uint32_t j = 0; j < count; ++j) syms |= uint64_t(one_checked()) << (8 * j);
             return syms;
         };
         if (LANES > 32) {
-            uint32_t g = uint32_t(8 - (reinterpret_cast<uintptr_t>(stage + pos) & 7));
-            auto some = [&]() {  // up to a boundary of eight bytes
-                if (g > remaining) g = remaining;
-                uint64_t syms = kept;
-                if (g > keep) {
-                    const uint64_t next = more();
-                    syms |= next << (8 * keep);
-                    kept = keep + 8 - g ? next >> (8 * (g - keep)) : 0;
-                    keep = keep + 8 - g;
-                } else { kept >>= 8 * g; keep -= g; }
-                uint8_t* to = stage + pos;
-                if (g == 8) *reinterpret_cast<uint64_t*>(to) = syms;
-                else for (uint32_t k = 0; k < g; ++k) to[k] = uint8_t(syms >> (8 * k));
-                pos += g; remaining -= g;
-                g = 8;
+            auto bytes = [&](uint32_t count) {
+                const uint64_t syms = few(count);
+                for (uint32_t k = 0; k < count; ++k) stage[pos + k] = uint8_t(syms >> (8 * k));
+                pos += count; remaining -= count;
             };
-#pragma unroll 1
-            do { if (remaining) some(); } while (remaining && (reinterpret_cast<uintptr_t>(stage + pos) & 31));
-            const uint32_t by = 8 * keep;
+            const uint32_t head = uint32_t(0u - reinterpret_cast<uintptr_t>(stage + pos)) & 7u;
+            if (head) bytes(head < remaining ? head : remaining);
+            while (remaining >= 8 && (reinterpret_cast<uintptr_t>(stage + pos) & 31)) {
+                uint2 a;
+                eight(a.x, a.y);
+                *reinterpret_cast<uint2*>(stage + pos) = a;
+                pos += 8; remaining -= 8;
+            }
 #pragma unroll 1
             for (; remaining >= 32; remaining -= 32, pos += 32) {  // whole sectors: a store by lanes that each walk a run of their own costs a pass per lane
-                uint64_t out[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint64_t next = more();
-                    out[k] = kept | next << by;
-                    kept = by ? next >> (64 - by) : 0;
-                }
-                stg256_kept(stage + pos, make_uint4(uint32_t(out[0]), uint32_t(out[0] >> 32), uint32_t(out[1]), uint32_t(out[1] >> 32)),
-                       make_uint4(uint32_t(out[2]), uint32_t(out[2] >> 32), uint32_t(out[3]), uint32_t(out[3] >> 32)));
+                uint4 a, b;
+                eight(a.x, a.y); eight(a.z, a.w); eight(b.x, b.y); eight(b.z, b.w);
+                stg256_kept(stage + pos, a, b);
             }
-#pragma unroll 1
-            while (remaining) some();
+            while (remaining >= 8) {
+                uint2 a;
+                eight(a.x, a.y);
+                *reinterpret_cast<uint2*>(stage + pos) = a;
+                pos += 8; remaining -= 8;
+            }
+            if (remaining) bytes(remaining);
         } else {
             const Epilogue ep = make_epilogue(bases, it);
-            auto dec8 = [&](uint32_t& s_lo, uint32_t& s_hi) {
-                const uint64_t next = more(), out = kept | next << (8 * keep);
-                if (keep) kept = next >> (64 - 8 * keep);
-                s_lo = uint32_t(out); s_hi = uint32_t(out >> 32);
-            };
             uint32_t g = remaining ? first_group(ep, pos, remaining) : 8;
-            if (g < 8) {
-                const uint64_t next = more();
-                emit(ep, pos, g, next);
-                kept = next >> (8 * g); keep = 8 - g;
-                pos += g; remaining -= g;
-            }
-            fast_groups(ep, it.n, pos, remaining, dec8);
+            if (g < 8) { emit(ep, pos, g, few(g)); pos += g; remaining -= g; }
+            fast_groups(ep, it.n, pos, remaining, eight);
             while (remaining) {
                 g = remaining < 8 ? remaining : 8;
-                uint64_t syms = kept;
-                if (g > keep) {
-                    const uint64_t next = more();
-                    syms |= next << (8 * keep);
-                    if (keep) kept = next >> (64 - 8 * keep);
-                }
+                uint64_t syms;
+                if (g == 8) { uint32_t lo, hi; eight(lo, hi); syms = lo | uint64_t(hi) << 32; } else syms = few(g);
                 emit(ep, pos, g, syms);
                 pos += g; remaining -= g;
             }
