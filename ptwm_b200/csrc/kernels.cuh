@@ -2620,20 +2620,28 @@ inline cudaError_t tans_allow_shared() {
 // can win again, so one look per eight symbols finds it and the eight are decoded again one by one; the end of a row is looked
 // for once per eight symbols too, and the stream's words for eight symbols are read at once, from a buffer in shared memory
 // that the warp fills 256 bytes at a time.  280 chunks of 32 Ki scales: 4.12 ms (247 cycles per symbol) with two maxima over
-// packed shares and everything else behind them, 4.00 with the lanes' own next states, 2.19 (131 cycles) without the branches.
+// packed shares and everything else behind them, 4.00 with the lanes' own next states, 2.14 without the branches, 2.09 (120 cycles) with
+// the next row asked for before the other two maxima and 64 bits of stream for four symbols instead of a window moved for each; 2400
+// chunks 5.88 -> 5.45.  Leading zeros instead of the two comparisons: 2.23, 5.12.
 constexpr uint32_t O1_ROW_BYTES = 32 * 12;  // per lane {minus the cumulative count, width}, then per lane the offset of the symbol's row << 8 | symbol
 constexpr uint32_t O1_HALF = 64;            // words in half of the stream buffer
 // Context rows of a chunk whose state has `state_len` bytes, the marginal's included (0 when the state is too short to hold any).
 inline uint32_t o1sac_tables(uint64_t state_len) { return state_len >= 32 + 512 ? uint32_t((state_len - 32 - 512) / 512) + 1 : 0; }
 
-__global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __restrict__ items, Bases bases, uint32_t* __restrict__ status, uint32_t smem_rows) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const uint32_t lane = threadIdx.x;
-    const DecodeItem it = items[blockIdx.x];
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) o1sac_decode_kernel(const DecodeItem* __restrict__ items, uint32_t n_items, Bases bases, uint32_t* __restrict__ status, uint32_t smem_rows) {
+    extern __shared__ __align__(16) uint8_t all_rows[];
+    __shared__ uint32_t all_bitmaps[WARPS][8], all_words[WARPS][2 * O1_HALF];
+    __shared__ uint16_t all_row_of[WARPS][256];
+    // (the maximum tells the compiler that the warp's number is the same for all lanes: 2213 -> 2012 us for a chunk)
+    const uint32_t lane = threadIdx.x % 32, warp = WARPS == 1 ? 0 : __reduce_max_sync(0xFFFFFFFFu, threadIdx.x / 32), chunk = blockIdx.x * WARPS + warp;
+    if (WARPS > 1 && chunk >= n_items) return;
+    uint8_t* smem = all_rows + warp * smem_rows * O1_ROW_BYTES;
+    const DecodeItem it = items[chunk];
     const uint8_t* st = rd(bases, it.state);
-    __shared__ uint32_t bitmap[8];      // contexts that have a row
-    __shared__ uint32_t words[2 * O1_HALF];  // the stream
-    __shared__ uint16_t row_of[256];    // the row a symbol leads to: 0 = marginal, 1 + rank of the context otherwise
+    uint32_t* bitmap = all_bitmaps[warp];   // contexts that have a row
+    uint32_t* words = all_words[warp];      // the stream
+    uint16_t* row_of = all_row_of[warp];    // the row a symbol leads to: 0 = marginal, 1 + rank of the context otherwise
     uint32_t err = it.state_version != 1 || it.state_len < 32 + 512 ? uint32_t(ST_BAD_STATE) : uint32_t(ST_OK);
     uint32_t rows = 1;
     if (!err) {
@@ -2736,26 +2744,36 @@ __global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __re
     uint32_t rpt = 0xFFFFFFFFu >> 12, row = 0;  // range / 4096; the context's row, in bytes
     const uint32_t row_len = it.row_len ? it.row_len : (it.n ? it.n : 1);
     uint32_t left_in_row = row_len;
-    // One symbol, by the 32 shares; rpt is 0 if none of them has it (and stays 0 if it was).  Returns the symbol, the bits taken and
-    // the next row: row << 8 | symbol, bits.
-    auto by_share = [&](uint32_t window, uint32_t& bits) -> uint32_t {
-        const uint2 mine = *reinterpret_cast<const uint2*>(smem + row + lane * 8);
-        const uint32_t lead = *reinterpret_cast<const uint32_t*>(smem + row + 256 + lane * 4);
+    const uint32_t shares = uint32_t(__cvta_generic_to_shared(smem)) + lane * 8, leads_at = uint32_t(__cvta_generic_to_shared(smem)) + 256 + lane * 4;
+    struct Share { uint32_t below, width, lead; };  // a lane's share of the row
+    // One symbol, by the 32 shares; rpt is 0 if none of them has it (and stays 0 if it was).  Returns the next row << 8 | symbol; `took` gets
+    // the bits taken in its low byte, which is also what a shift takes of it, and `mine` becomes the share of the next row.
+    auto load_share = [&]() -> Share {
+        Share v;
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.below), "=r"(v.width) : "r"(shares + row));
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v.lead) : "r"(leads_at + row));
+        return v;
+    };
+    auto most = [](uint32_t v) -> uint32_t { uint32_t r; asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v)); return r; };
+    auto by_share = [&](Share& mine, uint32_t window, uint32_t& took) -> uint32_t {
         // "cumulative count <= offset / rpt < count + width" without the division; the products fit 32 bits
-        const uint32_t rest = offset + mine.x * rpt, range = mine.y * rpt;
+        const uint32_t rest = offset + mine.below * rpt, range = mine.width * rpt;
         const bool won = rest < range;
-        const uint32_t got = __reduce_max_sync(0xFFFFFFFFu, won ? lead : 0u);
+        const uint32_t got = most(won ? mine.lead : 0u);
         const uint32_t b = range < (1u << 16) ? 16u : range < (1u << 24) ? 8u : 0u;  // rpt >= 2^12: two bytes at most
-        const uint32_t next = __reduce_max_sync(0xFFFFFFFFu, won ? (range << b) >> 12 | b << 24 : 0u);
-        offset = __reduce_max_sync(0xFFFFFFFFu, won ? __funnelshift_l(window, rest, b) : 0u);
-        rpt = next & 0xFFFFFFu;
-        bits = next >> 24;
+        const uint32_t next = won ? (range << b >> 4 & ~0xFFu) | b : 0u, low = won ? __funnelshift_l(window, rest, b) : 0u;
         row = got >> 8;
-        return got & 0xFFu;
+        mine = load_share();
+        took = most(next);
+        offset = most(low);
+        rpt = took >> 8;
+        return got;
     };
     auto one_symbol = [&]() -> uint32_t {
         const uint32_t was = offset, per = rpt, from = row, window = __funnelshift_l(word(1), word(0), uint32_t(bit));
-        uint32_t bits, sy = by_share(window, bits);
+        Share mine = load_share();
+        uint32_t bits, sy = by_share(mine, window, bits) & 0xFFu;
+        bits &= 0xFFu;
         if (rpt == 0) {
             // among all 256: the largest index whose count is <= min(offset / rpt, 4095) (order1_scale_ac.rs:474-486)
             uint32_t v[8], c = load_row(from / O1_ROW_BYTES, v), fit = 0, below = 0, w = 0;
@@ -2782,17 +2800,25 @@ __global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __re
         bool done = false;
         if (g == 8 && left_in_row > 8) {
             const uint32_t offset0 = offset, rpt0 = rpt, row0 = row;
-            uint32_t w0 = word(0), w1 = word(1), w2 = word(2), w3 = word(3), w4 = word(4), at = uint32_t(bit) & 31, used = 0;
+            // the next 64 bits are enough for four symbols: three before the last one take 48 and it needs 16 to go on
+            const uint32_t w0 = word(0), w1 = word(1), w2 = word(2), w3 = word(3), w4 = word(4), at = uint32_t(bit) & 31;
+            uint32_t hi = __funnelshift_l(w1, w0, at), lo = __funnelshift_l(w2, w1, at), used = 0;
+            Share mine = load_share();
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                uint32_t bits;
-                const uint32_t sy = by_share(__funnelshift_l(w1, w0, at), bits);
-                if (j < 4) s_lo |= sy << (8 * j); else s_hi |= sy << (8 * (j - 4));
-                at += bits; used += bits;
-                const bool over = at >= 32;
-                w0 = over ? w1 : w0; w1 = over ? w2 : w1; w2 = over ? w3 : w2; w3 = over ? w4 : w3;
-                at &= 31;
+                if (j == 4) {
+                    const uint32_t to = at + (used & 0xFFu);
+                    const bool one = to >= 32, two = to >= 64;
+                    const uint32_t a = two ? w2 : one ? w1 : w0, b = two ? w3 : one ? w2 : w1, c = two ? w4 : one ? w3 : w2;
+                    hi = __funnelshift_l(b, a, to); lo = __funnelshift_l(c, b, to);
+                }
+                uint32_t took;
+                const uint32_t got = by_share(mine, hi, took), ins = (0x3210u & ~(0xFu << (4 * (j & 3)))) | (4u << (4 * (j & 3)));
+                if (j < 4) s_lo = __byte_perm(s_lo, got, ins); else s_hi = __byte_perm(s_hi, got, ins);
+                hi = __funnelshift_l(lo, hi, took); lo = __funnelshift_l(0u, lo, took);
+                used += took;  // the low byte is the sum of the low bytes: 128 at most
             }
+            used &= 0xFFu;
             done = rpt != 0;
             if (done) { advance(used); left_in_row -= 8; }
             else { offset = offset0; rpt = rpt0; row = row0; s_lo = s_hi = 0; }
@@ -2810,15 +2836,22 @@ __global__ void __launch_bounds__(32) o1sac_decode_kernel(const DecodeItem* __re
     }
 }
 
-// `tables` = the most context rows among the items.
 constexpr uint32_t O1_MAX_ROWS = 257;
-inline void o1sac_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t tables, cudaStream_t st) {
+// The chain of a chunk is what a plan with block scales waits for, and it is a third longer with other decoders' warps on its scheduler.  So
+// where the plan says so (`alone`) four chunks go to a block, one to a scheduler, that takes an SM's shared memory whole, on half of the
+// SMs at most; the other decoders have the rest.  The MXFP4 / NVFP4 layer, 280 chunks of 32 Ki scales: 2799 -> 2188 us.
+constexpr uint32_t O1_ALONE_CHUNKS = 4 * 74, O1_ALONE_BYTES = 220 * 1024;
+// `tables` = the most context rows among the items.
+inline void o1sac_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t tables, bool alone, cudaStream_t st) {
     const uint32_t rows = tables < O1_MAX_ROWS ? tables : O1_MAX_ROWS;
-    o1sac_decode_kernel<<<n, 32, rows * O1_ROW_BYTES, st>>>(items, bases, status, rows);
+    if (alone && n <= O1_ALONE_CHUNKS && 4 * rows * O1_ROW_BYTES <= O1_ALONE_BYTES) o1sac_decode_kernel<4><<<(n + 3) / 4, 128, O1_ALONE_BYTES, st>>>(items, n, bases, status, rows);
+    else o1sac_decode_kernel<1><<<n, 32, rows * O1_ROW_BYTES, st>>>(items, n, bases, status, rows);
 }
 inline cudaError_t o1sac_allow_shared_rows() {
-    const cudaError_t e = cudaFuncSetAttribute(o1sac_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(O1_MAX_ROWS * O1_ROW_BYTES));
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(o1sac_decode_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaError_t e = cudaFuncSetAttribute(o1sac_decode_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(O1_ALONE_BYTES));
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(o1sac_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(O1_MAX_ROWS * O1_ROW_BYTES));
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(o1sac_decode_kernel<1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
 // ---- stand-alone merge / copy ---------------------------------------------

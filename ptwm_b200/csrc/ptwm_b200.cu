@@ -230,6 +230,7 @@ struct ptwm_b200_plan {
     bool merge_waits = false;  // a final merge reads scratch
     bool spread = false;       // few chunks: every coded plane to scratch at once, then a merge (see ptwm_b200_plan_create)
     bool join_small = false;   // the coded planes of small tensors go to scratch in the launch of the others, and a merge follows
+    bool o1_alone = false;     // Order1ScaleAC beside other codecs has SMs of its own
     uint64_t joined_bytes = 0;
     uint64_t slot_bytes[12] = {0};
     uint32_t slot_items[12] = {0};
@@ -464,6 +465,15 @@ void finish_lists(ptwm_b200_plan& pl) {
         pl.tiles[ph].push_back(tile);
         if (!m.empty()) pl.launches++;
     }
+    // Order1ScaleAC takes 63 ns per symbol of its longest chunk, the others 5 ps per symbol (tANS) or 1.6 (rANS, Huffman) and 1 ps per byte
+    // merged on the whole GPU: where they are done on half of it by then, they can do without the SMs it would otherwise share with them.
+    double chain = 0, rest = 0;
+    for (int ph = 0; ph < 2; ++ph) {
+        for (auto& it : pl.dec[ph][3]) chain = std::max(chain, 63e3 * it.n);
+        for (int cc = 0; cc < 3; ++cc) for (auto& it : pl.dec[ph][cc]) rest += it.n * (cc == 2 ? 5.0 : 1.6);
+        for (auto& it : pl.merges[ph]) rest += double(it.n) * kind_elem_bytes(int(it.kind));
+    }
+    pl.o1_alone = 2 * rest < chain;
     pl.post_tiles.clear();
     uint32_t tile = 0;
     bool delta = false;
@@ -568,7 +578,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
                 break;
             case 1: huffman_decode_kernel<<<(n + HUF_WARP_CHUNKS - 1) / HUF_WARP_CHUNKS, 32, HUF_SMEM, s>>>(it, n, bases, status); break;
             case 2: tans_launch(it, n, bases, status, r.size, s); break;
-            default: o1sac_launch(it, n, bases, status, r.size, s); break;
+            default: o1sac_launch(it, n, bases, status, r.size, s != st && pl.o1_alone, s); break;
         }
         CUDA_TRY(cudaGetLastError());
         return 0;
@@ -817,7 +827,7 @@ int64_t decode_plane_cuda(uint8_t sfv, const uint8_t* state, size_t state_len, c
         case C_RANS: rans_launch(d_it, 1, bases, d_status, true, false, 0, st); break;
         case C_HUFFMAN: huffman_decode_kernel<<<1, 32, HUF_SMEM, st>>>(d_it, 1, bases, d_status); break;
         case C_TANS: tans_launch(d_it, 1, bases, d_status, tans_lanes(1, uint32_t(decoded), 1), st); break;
-        default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), st); break;
+        default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), false, st); break;
     }
     CUDA_TRY(cudaGetLastError());
     uint32_t status = 0;

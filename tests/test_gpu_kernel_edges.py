@@ -106,6 +106,17 @@ def test_order1_scale_ac_shares_and_rows(alphabet, cols):
     check(specs, chunk_size=None if cols else 1500, forced_codec=oracle.O1SAC)
 
 
+@pytest.mark.parametrize("alphabet, chunks", [(3, 1), (3, 3), (3, 4), (3, 5), (3, 296), (3, 297), (200, 296)])
+def test_order1_scale_ac_beside_other_codecs(alphabet, chunks):
+    # four chunks to a block that has an SM to itself, a last block that is not full, one chunk too many for that, and tables too large for four
+    rng = np.random.default_rng(alphabet + chunks)
+    n = 30000 * (chunks - 1) + 27001
+    raw = ((np.cumsum(rng.random(n) < 0.05) * 7) % alphabet).astype(np.uint8).tobytes()  # runs: only the symbol before predicts them
+    specs, menu = [u8("s", raw, n), u8("p", plane("exponent", 3000))], (oracle.HUFFMAN, oracle.O1SAC)
+    assert oracle.write_container(specs[:1], chunk_size=30000, menu=menu) == oracle.write_container(specs[:1], chunk_size=30000, forced_codec=oracle.O1SAC)
+    check(specs, chunk_size=30000, menu=menu, emit_crc=True)
+
+
 @pytest.mark.parametrize("chunks", [1, 31, 33, 4735, 4736, 4737])
 @pytest.mark.parametrize("dtype", ["u8", "bf16", "fp32", "fp8"])
 def test_tans_decode_with_a_lane_per_stream(dtype, chunks):
