@@ -10,6 +10,8 @@
 //   O1SAC      codecs/order1_scale_ac.rs:620-663,963-1025, quantize.rs:13-45, range_coder.rs:16-113
 //   framing    compressor.rs:316-381, codecs/{huffman,rans,tans}.rs encode
 #pragma once
+#include <cooperative_groups.h>
+
 #include "encode_tables.cuh"
 #include "kernels.cuh"
 
@@ -705,8 +707,9 @@ __global__ void __launch_bounds__(32) rans_encode_kernel(const EncChunk* __restr
 // Huffman: the place of a symbol's bits follows from the lengths before it, so a warp codes a stream 512 symbols at a time:
 // every lane strings its sixteen codes together, a prefix sum over the lanes gives the bit each string starts at, and the
 // strings are put together in shared memory.  (One thread per stream took 107 ns per symbol.)
-// WARPS > 1, for launches that do not fill the GPU: that many warps to a stream, each with a share of its rounds.  They first
-// count the bits of their shares; a word that two shares meet in is kept by both and put together at the end.
+// WARPS > 1, for launches that do not fill the GPU: that many warps to a stream in each block of a cluster, every warp with a share of the
+// stream's rounds.  They first count the bits of their shares, which all blocks read of one another; a word that shares meet in
+// is kept by all of them and put together at the end by the one that fills it.
 constexpr uint32_t HENC_LANE = 16, HENC_WORDS = (32 * HENC_LANE * 11 + 31) / 32 + 2, HENC_ROUND = 32 * HENC_LANE;
 template <int WARPS>
 __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
@@ -719,7 +722,11 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
         uint32_t head_at[4][WARPS], head[4][WARPS], tail_at[4][WARPS], tail[4][WARPS];  // the words a share meets its neighbours in
     };
     __shared__ Shared sh;
-    const uint32_t ci = list[blockIdx.x], lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = warp / WARPS, part = warp % WARPS;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const uint32_t blocks = WARPS > 1 ? cluster.num_blocks() : 1, rank = WARPS > 1 ? cluster.block_rank() : 0;
+    const uint32_t ci = list[blockIdx.x / blocks], lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = warp / WARPS, mine = warp % WARPS;
+    const uint32_t part = rank * WARPS + mine, parts = blocks * WARPS;
+    auto of = [&](uint32_t q) -> const Shared* { return cluster.map_shared_rank(&sh, q / WARPS); };  // where share q is kept, at place q % WARPS
     const EncChunk c = chunks[ci];
     if (!c.n || !results[ci].coded) return;
     const uint32_t* g_codes = reinterpret_cast<const uint32_t*>(tables + c.table_off + 256);
@@ -733,7 +740,7 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
     uint8_t* slot = slots + c.slot_off + uint64_t(s) * c.slot_cap;
     uint32_t* out = reinterpret_cast<uint32_t*>(slot);
     const uint32_t rounds = (len + HENC_ROUND - 1) / HENC_ROUND;
-    const uint32_t from = uint32_t(uint64_t(rounds) * part / WARPS) * HENC_ROUND, to = part + 1 == WARPS ? len : uint32_t(uint64_t(rounds) * (part + 1) / WARPS) * HENC_ROUND;
+    const uint32_t from = uint32_t(uint64_t(rounds) * part / parts) * HENC_ROUND, to = part + 1 == parts ? len : uint32_t(uint64_t(rounds) * (part + 1) / parts) * HENC_ROUND;
     auto fetch = [&](uint32_t at, uint32_t n, uint64_t& a, uint64_t& b) {  // up to sixteen bytes from src + at
         a = b = 0;
         if (n == HENC_LANE) { a = ld8_unaligned(src + at); b = ld8_unaligned(src + at + 8); }
@@ -743,25 +750,27 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
     auto code_of = [&](uint64_t a, uint64_t b, uint32_t k) { return sh.codes[uint32_t((k < 8 ? a : b) >> (8 * (k & 7))) & 0xFFu]; };
     uint64_t na, nb, before_us = 0;
     if (WARPS > 1) {
-        uint64_t mine = 0;
+        uint64_t sum = 0;
         fetch(from + lane * HENC_LANE, count_at(from), na, nb);
         for (uint32_t base = from; base < to; base += HENC_ROUND) {
             const uint32_t n = count_at(base);
             const uint64_t ca = na, cb = nb;
             if (base + HENC_ROUND < to) fetch(base + HENC_ROUND + lane * HENC_LANE, count_at(base + HENC_ROUND), na, nb);
 #pragma unroll
-            for (uint32_t k = 0; k < HENC_LANE; ++k) mine += k < n ? code_of(ca, cb, k) >> 16 : 0u;
+            for (uint32_t k = 0; k < HENC_LANE; ++k) sum += k < n ? code_of(ca, cb, k) >> 16 : 0u;
         }
 #pragma unroll
-        for (int d = 16; d; d >>= 1) mine += __shfl_xor_sync(0xFFFFFFFFu, mine, d);
-        if (lane == 0) sh.bits[s][part] = mine;
-        __syncthreads();
-        for (uint32_t w = 0; w < part; ++w) before_us += sh.bits[s][w];
+        for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+        if (lane == 0) sh.bits[s][mine] = sum;
+        cluster.sync();
+        for (uint32_t q = lane; q < part; q += 32) before_us += of(q)->bits[s][q % WARPS];
+#pragma unroll
+        for (int d = 16; d; d >>= 1) before_us += __shfl_xor_sync(0xFFFFFFFFu, before_us, d);
     }
     uint32_t have = uint32_t(before_us) & 31;  // bits of the word that is not full yet, which stays in words[0]
     out += before_us >> 5;
     bool meets = have != 0;  // words[0] is the last one of the share before
-    if (WARPS > 1 && lane == 0) sh.head_at[s][part] = sh.tail_at[s][part] = 0xFFFFFFFFu;
+    if (WARPS > 1 && lane == 0) sh.head_at[s][mine] = sh.tail_at[s][mine] = 0xFFFFFFFFu;
     fetch(from + lane * HENC_LANE, count_at(from), na, nb);
     for (uint32_t base = from; base < to; base += HENC_ROUND) {
         const uint32_t n = count_at(base);
@@ -795,7 +804,7 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
         have = (have + total) & 31;
         const uint32_t rest = words[full];
         if (WARPS > 1 && meets && full) {
-            if (lane == 0) { sh.head_at[s][part] = uint32_t(out - reinterpret_cast<uint32_t*>(slot)); sh.head[s][part] = words[0]; }
+            if (lane == 0) { sh.head_at[s][mine] = uint32_t(out - reinterpret_cast<uint32_t*>(slot)); sh.head[s][mine] = words[0]; }
             for (uint32_t i = lane; i < full; i += 32) if (i) out[i] = words[i];
             meets = false;
         } else {
@@ -813,30 +822,46 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
         }
         return;
     }
-    if (lane == 0 && have) { sh.tail_at[s][part] = uint32_t(out - reinterpret_cast<uint32_t*>(slot)); sh.tail[s][part] = words[0]; }
-    __syncthreads();
-    if (part == 0 && lane == 0) {
-        uint64_t all = 0;
-        uint32_t at = 0xFFFFFFFFu, v = 0;
-        auto word = [&](uint32_t a, uint32_t x) {  // in ascending order; the same word more than once
-            if (a == 0xFFFFFFFFu) return;
-            if (at == a) { v |= x; return; }
-            if (at != 0xFFFFFFFFu) reinterpret_cast<uint32_t*>(slot)[at] = v;
-            at = a; v = x;
+    if (lane == 0 && have) { sh.tail_at[s][mine] = uint32_t(out - reinterpret_cast<uint32_t*>(slot)); sh.tail[s][mine] = words[0]; }
+    cluster.sync();
+    if (lane == 0) {
+        auto with_tails = [&](uint32_t w, uint32_t v) {  // and the bits of the shares before this one that end in word w
+            for (uint32_t q = part; q-- > 0;) {
+                const Shared* o = of(q);
+                if (o->tail_at[s][q % WARPS] == w) v |= o->tail[s][q % WARPS];
+                else if (o->bits[s][q % WARPS] != 0) break;
+            }
+            reinterpret_cast<uint32_t*>(slot)[w] = v;
         };
-        for (uint32_t w = 0; w < WARPS; ++w) { all += sh.bits[s][w]; word(sh.head_at[s][w], sh.head[s][w]); word(sh.tail_at[s][w], sh.tail[s][w]); }
-        if (at != 0xFFFFFFFFu) reinterpret_cast<uint32_t*>(slot)[at] = v;
-        results[ci].stream_len[s] = uint32_t((all + 7) / 8);
+        if (sh.head_at[s][mine] != 0xFFFFFFFFu) with_tails(sh.head_at[s][mine], sh.head[s][mine]);
+        if (part + 1 == parts) {
+            const uint64_t all = before_us + sh.bits[s][mine];
+            if (all & 31) with_tails(uint32_t(all >> 5), sh.tail_at[s][mine] == uint32_t(all >> 5) ? sh.tail[s][mine] : 0u);
+            results[ci].stream_len[s] = uint32_t((all + 7) / 8);
+        }
     }
+    cluster.sync();  // the other blocks' shared memory is read until here
 }
-// Chunks of a launch up to which eight warps take a stream.  us of a whole compress_model with one / eight warps: 64 Ki symbols, 1 chunk 194 /
-// 165, 148: 198 / 162, 592: 246 / 253; 16 Ki, 148: 158 / 146, 592: 174 / 185; 4 Ki, 148: 147 / 149, 296: 147 / 161.  A plane of 200,003 in a call of its
-// own: 243 -> 122.
+// Chunks of a launch up to which eight warps and more take a stream.  us of a whole compress_model with one / eight warps: 64 Ki symbols, 1 chunk 194 /
+// 165, 148: 198 / 162, 592: 246 / 253; 16 Ki, 148: 158 / 146, 592: 174 / 185; 4 Ki, 148: 147 / 149, 296: 147 / 161.  Launches that leave SMs
+// idle get two, four or eight blocks to a chunk: 200,003 symbols in a call of their own 65 -> 16 us, the call 139 -> 90, and 77 with the payload
+// gathered by several blocks that see for themselves whether it fits.
 constexpr uint32_t HENC_WIDE_CHUNKS = 148;
-inline void huffman_encode_launch(const EncChunk* chunks, const uint32_t* list, uint32_t n, const uint8_t* planes, const uint8_t* tables, uint8_t* slots, EncResult* results,
-                                  cudaStream_t st) {
-    if (n <= HENC_WIDE_CHUNKS) huffman_encode_kernel<8><<<n, 1024, 0, st>>>(chunks, list, n, planes, tables, slots, results);
-    else huffman_encode_kernel<1><<<n, 128, 0, st>>>(chunks, list, n, planes, tables, slots, results);
+inline cudaError_t huffman_encode_launch(const EncChunk* chunks, const uint32_t* list, uint32_t n, const uint8_t* planes, const uint8_t* tables, uint8_t* slots, EncResult* results,
+                                         cudaStream_t st) {
+    if (n > HENC_WIDE_CHUNKS) {
+        huffman_encode_kernel<1><<<n, 128, 0, st>>>(chunks, list, n, planes, tables, slots, results);
+        return cudaGetLastError();
+    }
+    uint32_t blocks = 8;
+    while (blocks > 1 && n * blocks > HENC_WIDE_CHUNKS) blocks /= 2;
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = blocks; cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(n * blocks); config.blockDim = dim3(1024); config.stream = st;
+    config.attrs = &cluster; config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, huffman_encode_kernel<8>, chunks, list, n, planes, tables, slots, results);
 }
 
 // tANS (entropy/tans/mod.rs:268-318): one serial stream per chunk, its symbols walked last to first, its bits going upward.
@@ -1007,10 +1032,9 @@ __device__ __forceinline__ void block_copy_reversed(uint8_t* d, const uint8_t* s
     const uint32_t i = blocks * 16 + t;
     if (i < n) d[i] = s[n - 1 - i];
 }
-// One chunk frame by the threads of a block: [state_version 0][state_len 0 u32] then the codec payload, at its final place.
+// One chunk frame by `nt` threads of whole warps, of which this is the `t`-th: [state_version 0][state_len 0 u32] then the codec payload, at its final place.
 __device__ __forceinline__ void gather_frame(uint8_t* d, const EncChunk& c, const EncResult& r, uint32_t form, const uint8_t* __restrict__ planes, const uint8_t* __restrict__ tables,
-                                             const uint8_t* __restrict__ slots) {
-    const uint32_t t = threadIdx.x;
+                                             const uint8_t* __restrict__ slots, uint32_t t, uint32_t nt) {
     const uint32_t mode = form & 0xFFu;
     const bool framed = !(form & (GATHER_BARE | GATHER_NOFRAME));
     if (framed) {
@@ -1020,7 +1044,7 @@ __device__ __forceinline__ void gather_frame(uint8_t* d, const EncChunk& c, cons
     if (mode <= 1) {
         if (mode == 1) { if (t == 0) d[0] = 0; d += 1; }
         const uint8_t* p = planes + c.plane_off;
-        block_copy(d, p, c.n, t, blockDim.x);
+        block_copy(d, p, c.n, t, nt);
         return;
     }
     const uint8_t* tab = tables + c.table_off;
@@ -1035,17 +1059,17 @@ __device__ __forceinline__ void gather_frame(uint8_t* d, const EncChunk& c, cons
                 fh[0] = 1; fh[1] = uint8_t(state_len); fh[2] = uint8_t(state_len >> 8); fh[3] = uint8_t(state_len >> 16); fh[4] = uint8_t(state_len >> 24);
             }
             if (t < 32) { uint32_t bits = 0; for (int k = 0; k < 8; ++k) bits |= uint32_t(present[8 * t + k] != 0) << k; d[t] = uint8_t(bits); }
-            for (uint32_t i = t; i < 256; i += blockDim.x) { d[32 + 2 * i] = uint8_t(pmf[i]); d[33 + 2 * i] = uint8_t(pmf[i] >> 8); }
+            for (uint32_t i = t; i < 256; i += nt) { d[32 + 2 * i] = uint8_t(pmf[i]); d[33 + 2 * i] = uint8_t(pmf[i] >> 8); }
             for (uint32_t ctx = 0; ctx < 256; ++ctx) {
                 if (!present[ctx]) continue;
                 uint8_t* row = d + 32 + 512 + 512 * uint32_t(rank[ctx]);
                 const uint16_t* pr = pmf + 256 * (1 + ctx);
-                for (uint32_t i = t; i < 256; i += blockDim.x) { row[2 * i] = uint8_t(pr[i]); row[2 * i + 1] = uint8_t(pr[i] >> 8); }
+                for (uint32_t i = t; i < 256; i += nt) { row[2 * i] = uint8_t(pr[i]); row[2 * i + 1] = uint8_t(pr[i] >> 8); }
             }
             d += state_len;
         }
         const uint8_t* sp = slots + c.slot_off;
-        block_copy(d, sp, r.stream_len[0], t, blockDim.x);
+        block_copy(d, sp, r.stream_len[0], t, nt);
         return;
     }
     if (t == 0) { d[0] = 1; d[1] = uint8_t(c.n); d[2] = uint8_t(c.n >> 8); d[3] = uint8_t(c.n >> 16); d[4] = uint8_t(c.n >> 24); }
@@ -1067,7 +1091,7 @@ __device__ __forceinline__ void gather_frame(uint8_t* d, const EncChunk& c, cons
         }
         d += 3 + 3 * r.hdr_n + 8;
         const uint8_t* sp = slots + c.slot_off;
-        block_copy(d, sp, r.stream_len[0], t, blockDim.x);
+        block_copy(d, sp, r.stream_len[0], t, nt);
         return;
     }
     uint32_t hdr;
@@ -1075,13 +1099,13 @@ __device__ __forceinline__ void gather_frame(uint8_t* d, const EncChunk& c, cons
         const uint16_t* freqs = reinterpret_cast<const uint16_t*>(tab);
         hdr = 1 + 2 * (r.hdr_n + 1);
         if (t == 0) d[0] = uint8_t(r.hdr_n);
-        for (uint32_t i = t; i <= r.hdr_n; i += blockDim.x) { d[1 + 2 * i] = uint8_t(freqs[i]); d[2 + 2 * i] = uint8_t(freqs[i] >> 8); }
+        for (uint32_t i = t; i <= r.hdr_n; i += nt) { d[1 + 2 * i] = uint8_t(freqs[i]); d[2 + 2 * i] = uint8_t(freqs[i] >> 8); }
     } else {
         const uint32_t nw = r.hdr_n;
         uint32_t hb = nw <= 127 ? 1 : 2;
         hdr = hb + (nw + 1) / 2;
         if (t == 0) { if (nw <= 127) d[0] = uint8_t(0x80 | nw); else { d[0] = 0x80; d[1] = uint8_t(nw); } }
-        for (uint32_t i = t; i < (nw + 1) / 2; i += blockDim.x) {
+        for (uint32_t i = t; i < (nw + 1) / 2; i += nt) {
             uint32_t lo = tab[2 * i] & 0x0F, hi = (2 * i + 1 < nw ? tab[2 * i + 1] : 0) & 0x0F;
             d[hb + i] = uint8_t(lo | (hi << 4));
         }
@@ -1090,7 +1114,7 @@ __device__ __forceinline__ void gather_frame(uint8_t* d, const EncChunk& c, cons
     if (t < 16) d[t] = uint8_t(r.stream_len[t >> 2] >> (8 * (t & 3)));
     d += 16;
     for (uint32_t s = 0; s < 4; ++s) {
-        block_copy_reversed(d, slots + c.slot_off + uint64_t(s) * c.slot_cap, r.stream_len[s], t, blockDim.x);
+        block_copy_reversed(d, slots + c.slot_off + uint64_t(s) * c.slot_cap, r.stream_len[s], t, nt);
         d += r.stream_len[s];
     }
 }
@@ -1107,11 +1131,16 @@ __global__ void __launch_bounds__(128) gather_kernel(const EncChunk* __restrict_
         e += put_varint_dev(e, place.frame);
         put_varint_dev(e, c.n);
     }
-    gather_frame(out + dst.frames + place.frame, c, results[blockIdx.x], place.mode, planes, tables, slots);
+    gather_frame(out + dst.frames + place.frame, c, results[blockIdx.x], place.mode, planes, tables, slots, threadIdx.x, blockDim.x);
 }
-__global__ void __launch_bounds__(512) gather_one_kernel(const EncChunk* __restrict__ chunk, const EncResult* __restrict__ result, uint32_t form, const uint8_t* __restrict__ planes,
-                                                         const uint8_t* __restrict__ tables, const uint8_t* __restrict__ slots, uint8_t* __restrict__ out) {
-    gather_frame(out, *chunk, *result, form, planes, tables, slots);
+// The payload of one plane, in the form its coded size calls for and without a frame, by all blocks; nothing where it does not fit.
+__global__ void __launch_bounds__(512) gather_one_kernel(const EncChunk* __restrict__ chunk, const EncResult* __restrict__ result, uint32_t codec, const uint8_t* __restrict__ planes,
+                                                         const uint8_t* __restrict__ tables, const uint8_t* __restrict__ slots, uint8_t* __restrict__ out, uint64_t out_cap) {
+    const EncChunk c = *chunk;
+    const EncResult r = *result;
+    uint32_t mode;
+    if (enc_payload(int(codec), false, c.n, r, mode) > out_cap) return;
+    gather_frame(out, c, r, mode | GATHER_BARE, planes, tables, slots, blockIdx.x * 512 + threadIdx.x, gridDim.x * 512);
 }
 
 // ---- ops between a byte split and a terminal (transforms/int_delta.rs:36-44, transforms/mantissa_zero.rs) ------

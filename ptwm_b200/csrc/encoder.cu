@@ -229,7 +229,7 @@ int64_t launch_encoders(const EncChunk* chunks, const uint32_t* lists, const uin
         if (k < LIST_HUFFMAN) {
             const uint32_t span = rans_list_span(k);
             rans_encode_kernel<<<(n[k] + RANS_WARP_CHUNKS - 1) / RANS_WARP_CHUNKS, 32, renc_smem_bytes(span), st>>>(chunks, lists, n[k], span, planes, tables, slots, results);
-        } else if (k == LIST_HUFFMAN) huffman_encode_launch(chunks, lists, n[k], planes, tables, slots, results, st);
+        } else if (k == LIST_HUFFMAN) CUDA_TRY(huffman_encode_launch(chunks, lists, n[k], planes, tables, slots, results, st));
         else tans_encode_kernel<<<n[k], 32, 0, st>>>(chunks, lists, n[k], planes, tables, slots, results);
         CUDA_TRY(cudaGetLastError());
         lists += n[k];
@@ -1015,8 +1015,11 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         hist_kernel<<<dim3(1, hist_blocks(n)), 256, 0, st>>>(&d->chunk, in, d->hist);
         table_kernel<<<1, 128, 0, st>>>(&d->plane, &d->chunk, 1, d->hist, area, &d->result);
         if (codec == C_RANS) rans_encode_kernel<<<1, 32, renc_smem_bytes(256), st>>>(&d->chunk, &d->list, 1, 256, in, area, area, &d->result);
-        else if (codec == C_HUFFMAN) huffman_encode_launch(&d->chunk, &d->list, 1, in, area, area, &d->result, st);
+        else if (codec == C_HUFFMAN) CUDA_TRY(huffman_encode_launch(&d->chunk, &d->list, 1, in, area, area, &d->result, st));
         else tans_encode_kernel<<<1, 32, 0, st>>>(&d->chunk, &d->list, 1, in, area, area, &d->result);
+        CUDA_TRY(cudaGetLastError());
+        // the form of the payload and whether it fits are seen on the device, so there is nothing to wait for in between
+        gather_one_kernel<<<unsigned(std::min<uint64_t>((n + 16383) / 16384, 148)), 512, 0, st>>>(&d->chunk, &d->result, uint32_t(codec), in, area, area, out, out_cap);
         CUDA_TRY(cudaGetLastError());
         EncResult r;
         CUDA_TRY(cudaMemcpyAsync(&r, &d->result, sizeof(r), cudaMemcpyDeviceToHost, st));
@@ -1024,15 +1027,11 @@ int64_t ptwm::encode_plane_cuda(int codec, const uint8_t* state, size_t state_le
         size = enc_payload(codec, false, uint32_t(n), r, mode);
     }
     if (need(size) > out_cap) return fail(PTWM_RC_BUFFER_TOO_SMALL, "output buffer too small");
-    if (mode == 1 && n > 0xFFFFFFFFull) {  // raw: tag byte, then the plane
+    if (n > 0xFFFFFFFFull) {  // raw: tag byte, then the plane
         CUDA_TRY(cudaMemsetAsync(out, 0, 1, st));
         CUDA_TRY(cudaMemcpyAsync(out + 1, in, n, cudaMemcpyDeviceToDevice, st));
-    } else {
-        Job* d = d_job.as<Job>();
-        gather_one_kernel<<<1, 512, 0, st>>>(&d->chunk, &d->result, mode | GATHER_BARE, in, d_job.as<uint8_t>(), d_job.as<uint8_t>(), out);
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamSynchronize(st));
     }
-    CUDA_TRY(cudaStreamSynchronize(st));
     return int64_t(size);
 }
 

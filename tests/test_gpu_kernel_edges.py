@@ -7,8 +7,10 @@ import torch
 
 import oracle
 import ptwm_b200
+from ptwm_b200 import _lib
 from ptwm_b200.compressor import CompressionConfig, HUFFMAN, IDENTITY, RANS, TANS, compress_model
 from _data import mixed_model, weights
+from test_gpu_decode import IDS
 
 pytestmark = pytest.mark.gpu
 
@@ -261,6 +263,29 @@ def test_huffman_encode_shares_of_a_stream(kind):
     lengths = [4 * 512 * k + d for k in (1, 7, 8, 9, 17) for d in (-5, 0, 1, 6)]
     encode_check([plane(kind, n) for n in lengths], None, HUFFMAN)
     encode_check([plane(kind, 600 * 149)], 600, HUFFMAN)
+
+
+@pytest.mark.parametrize("chunks", [1, 18, 19, 37, 38, 74, 75])
+@pytest.mark.parametrize("kind", ["exponent", "rare", "wide"])
+def test_huffman_encode_blocks_of_a_cluster(kind, chunks):
+    # eight, four, two blocks to a chunk and one: shares of all of them without a round, with one and with two, and streams of a few bits
+    for length in (5, 1029, 4 * 512 * 64 + 2051, 4 * 512 * 65 + 6):
+        encode_check([plane(kind, length * (chunks - 1) + length // 2 + 1)], length, HUFFMAN)
+
+
+@pytest.mark.parametrize("codec", [HUFFMAN, RANS, TANS])
+@pytest.mark.parametrize("n", [1, 16384, 16385, 70001, 600001])
+def test_plane_encode_gathers_where_it_fits(codec, n):
+    # several blocks put the payload together, coded or raw; a buffer one byte short stays as it is
+    for raw in (plane("exponent", n), np.random.default_rng(n).integers(0, 256, n, dtype=np.uint8).tobytes()):
+        want = oracle.plane_encode(codec, raw)[2]
+        src, out = torch.frombuffer(bytearray(raw), dtype=torch.uint8).cuda(), torch.full((len(want) + 32,), 0xCD, dtype=torch.uint8, device="cuda")
+        needed, ident = _lib.C.c_uint64(), bytes.fromhex(IDS[codec])
+        torch.cuda.synchronize()
+        for cap, rc in ((len(want) - 1, -2), (len(want), len(want))):
+            assert _lib.lib().ptwm_plane_codec_v1_encode_cuda(1, None, 0, ident, 32, src.data_ptr(), n, out.data_ptr(), cap, _lib.C.byref(needed), 0) == rc
+            assert out.cpu().numpy().tobytes() == (b"\xcd" * (len(want) + 32) if rc < 0 else want + b"\xcd" * 32)
+        assert needed.value == len(want)
 
 
 @pytest.mark.parametrize("span", [1, 2, 46, 47, 48, 63, 64, 127, 128, 200])
