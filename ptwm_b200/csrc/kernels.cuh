@@ -612,13 +612,22 @@ __host__ __device__ inline uint32_t rans_smem_bytes(uint32_t l_entries, bool per
     return (per_lane && rank < RANS_PAIR_SMEM ? RANS_PAIR_SMEM : rank) + RING_SMEM;
 }
 
+// Three kernels have a table entry per slot.  Launches of up to 592 chunks, one to a block: entries of four words, and the chunk's streams in shared
+// memory beside them where they fit, else through the rings.  Above that four chunks to a block, a word to an entry.  us of one chunk of 32 Ki
+// symbols / 64 Ki in a call of its own, bf16: a word to an entry 479 / 762, four words 460 / 725, streams in shared memory 412 / 630 (73 cycles per
+// symbol; the way from state to state alone is 47).  Tried: both byte counts from the table and one move chosen by them 415 / 652.
 // Chunks of a launch up to which the kernel with a table entry per slot is the faster one: what the GPU holds of it at once (six
 // blocks of four chunks per SM).  Chunks of 32 Ki symbols, us of a bf16 tensor, table per slot against tables of pairs: 1 to 592 chunks
-// 487 / 681, 2368 518 / 709, 3552 619 / 694, and beyond that a second wave (start of it, 4144: 832 / 694).  fp32: 507 / 739, 592 chunks 634 / 752,
+// 420 / 681, 2368 518 / 709, 3552 619 / 694, and beyond that a second wave (start of it, 4144: 832 / 694).  fp32: 445 / 739, 592 chunks 547 / 752,
 // 2368 667 / 758, 3552 855 / 780; fp16 (rank tables) 483 / 876, 3552 645 / 928.
 constexpr uint32_t RANS_DIRECT_CHUNKS = 6 * 4 * 148;
 constexpr uint32_t RANS_DIRECT_BYTES = 2048 * 4;  // per chunk
-__host__ __device__ inline uint32_t rans_direct_smem(uint32_t warp_chunks) { return warp_chunks * RANS_DIRECT_BYTES + RING_SMEM; }
+constexpr uint32_t RANS_WIDE_BYTES = 2048 * 16;   // with four words to an entry
+__host__ __device__ inline uint32_t rans_direct_smem(uint32_t warp_chunks) { return (warp_chunks == 1 ? RANS_WIDE_BYTES : warp_chunks * RANS_DIRECT_BYTES) + RING_SMEM; }
+// The same with a chunk's streams beside the table: up to fifteen bytes on either side of them, and 64 that a group may read too far.
+constexpr uint32_t RANS_STREAM_PAD = 64;
+__host__ __device__ inline uint32_t rans_resident_smem(uint32_t src_len) { return RANS_WIDE_BYTES + RING_SMEM + ((src_len + 32 + 15) & ~15u) + RANS_STREAM_PAD; }
+constexpr uint32_t RANS_RESIDENT_MOST = 220 * 1024;  // of a block; the blocks of an SM have 227 KiB, one of which each takes beside its own
 
 // Ring addressing: byte q of a lane's ring lives in word (q >> 2) & 15 of the
 // [word][lane] array, `rw` points at the lane's column.
@@ -792,7 +801,7 @@ __device__ __forceinline__ void rans_pair_group8(const RansPair& p, const uint32
 // The same on a table with an entry per slot: slot's distance from the symbol's first << 20 | symbol << 12 | frequency, so that
 // both factors of the update are one step away.  From one state to the next it is a mask, one shared-memory read, a shift and a
 // multiply-add; renormalising moves the state shifted by one or two bytes over the state, two moves that hang on the comparisons
-// alone (a chunk of 64 Ki symbols in a call of its own 778 -> 751 us).  A state that has been normalised once
+// alone.  A state that has been normalised once
 // never needs more than two bytes (an update leaves at least 2^12), so eight bytes of stream last for four symbols and nothing
 // is decoded twice.  A stream whose stored initial state is not normalised goes byte by byte.
 __device__ __forceinline__ uint32_t rans_direct_lookup(const uint32_t* tab, uint32_t& x) {
@@ -801,10 +810,15 @@ __device__ __forceinline__ uint32_t rans_direct_lookup(const uint32_t* tab, uint
     return e >> 12;
 }
 // The ring's words are kept with their first byte on top here.
+template <bool WIDE>
 __device__ __forceinline__ void rans_direct_short(const uint32_t* tab, const uint32_t* rw, uint32_t& x, uint32_t& rq, uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
     s_lo = 0; s_hi = 0;
     for (uint32_t j = 0; j < g; ++j) {
-        const uint32_t sym = rans_direct_lookup(tab, x) & 0xFFu;
+        uint32_t sym;
+        if (WIDE) {
+            const uint4 e = reinterpret_cast<const uint4*>(tab)[x & 2047u];
+            x = e.x * (x >> 11) + e.y; sym = e.w;
+        } else sym = rans_direct_lookup(tab, x) & 0xFFu;
         if (j < 4) s_lo |= sym << (8 * j); else s_hi |= sym << (8 * (j - 4));
         for (int k = 0; k < 3 && x < RANS_L; ++k) { x = (x << 8) | ring_byte(rw, rq ^ 3u); ++rq; }
     }
@@ -813,8 +827,20 @@ __device__ __forceinline__ void rans_direct_words(const uint32_t* rw, uint32_t r
 #pragma unroll
     for (uint32_t k = 0; k < 5; ++k) v[k] = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(rw) + (((rq << 5) + 0x80u * k) & 0x780u));
 }
+// One symbol with an entry of four words: frequency, slot's distance from the symbol's first, from which value of x >> 11 on the next state is
+// normalised, symbol.  The third is there so that the first byte need not wait for the state.
+__device__ __forceinline__ void rans_direct_step(const uint4& e, uint32_t wh, uint32_t& x, uint32_t& bits) {
+    asm("{\n\t.reg .pred some, more;\n\t.reg .u32 q, y;\n\t"
+        "shr.u32 q, %0, 11;\n\tsetp.lt.u32 some, q, %5;\n\t"
+        "mad.lo.u32 y, %3, q, %4;\n\tsetp.lt.u32 more, y, 0x8000;\n\t"
+        "mov.u32 %0, y;\n\tmov.u32 %1, 0;\n\t"
+        "@some prmt.b32 %0, y, %2, 0x2107;\n\t@some mov.u32 %1, 8;\n\t"
+        "@more prmt.b32 %0, y, %2, 0x1076;\n\t@more mov.u32 %1, 16;\n\t}"
+        : "+r"(x), "=&r"(bits) : "r"(wh), "r"(e.x), "r"(e.y), "r"(e.z));
+}
 // Four symbols.  `v` are five ring words read before the last four symbols were decoded, `skip` the bits of them that are used
-// up by now (88 at most).  The five words for the next four are requested here.
+// up by now (88 at most).  The five words for the next four are requested here.  WIDE: an entry of four words.
+template <bool WIDE>
 __device__ __forceinline__ uint32_t rans_direct_four(const uint32_t* tab, const uint32_t* rw, uint32_t& x, uint32_t& rq, uint32_t v[5], uint32_t& skip) {
     const bool one_off = skip >= 32, two_off = skip >= 64;
     const uint32_t a = two_off ? v[2] : one_off ? v[1] : v[0], b = two_off ? v[3] : one_off ? v[2] : v[1], c = two_off ? v[4] : one_off ? v[3] : v[2];
@@ -823,22 +849,72 @@ __device__ __forceinline__ uint32_t rans_direct_four(const uint32_t* tab, const 
     skip = (rq & 3u) * 8;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const uint32_t e = rans_direct_lookup(tab, x);
-        sy = __byte_perm(sy, e, (0x3210u & ~(0xFu << (4 * j))) | (4u << (4 * j)));
+        const uint32_t ins = (0x3210u & ~(0xFu << (4 * j))) | (4u << (4 * j));
         uint32_t bits;
-        asm("{\n\t.reg .pred some, more;\n\t.reg .u32 y;\n\t"
-            "setp.lt.u32 some, %0, 0x800000;\n\tsetp.lt.u32 more, %0, 0x8000;\n\t"
-            "mov.u32 y, %0;\n\tmov.u32 %1, 0;\n\t"
-            "@some prmt.b32 y, %0, %2, 0x2107;\n\t@some mov.u32 %1, 8;\n\t"
-            "@more prmt.b32 y, %0, %2, 0x1076;\n\t@more mov.u32 %1, 16;\n\t"
-            "mov.u32 %0, y;\n\t}"
-            : "+r"(x), "=&r"(bits) : "r"(wh));
+        if (WIDE) {
+            const uint4 e = reinterpret_cast<const uint4*>(tab)[x & 2047u];
+            rans_direct_step(e, wh, x, bits);
+            sy = __byte_perm(sy, e.w, ins);
+        } else {
+            const uint32_t e = rans_direct_lookup(tab, x);
+            sy = __byte_perm(sy, e, ins);
+            asm("{\n\t.reg .pred some, more;\n\t.reg .u32 y;\n\t"
+                "setp.lt.u32 some, %0, 0x800000;\n\tsetp.lt.u32 more, %0, 0x8000;\n\t"
+                "mov.u32 y, %0;\n\tmov.u32 %1, 0;\n\t"
+                "@some prmt.b32 y, %0, %2, 0x2107;\n\t@some mov.u32 %1, 8;\n\t"
+                "@more prmt.b32 y, %0, %2, 0x1076;\n\t@more mov.u32 %1, 16;\n\t"
+                "mov.u32 %0, y;\n\t}"
+                : "+r"(x), "=&r"(bits) : "r"(wh));
+        }
         wh = __funnelshift_l(wl, wh, bits);
         wl <<= bits;
         used += bits;
     }
     skip += used;
     rq += used >> 3;
+    return sy;
+}
+
+// The same on streams that lie in shared memory whole, words with their first byte on top: nothing to fill up and no ring to go round, so the
+// next words are four reads from one address.  `at` is a position in bits from `words` on, `last` the last word whose three successors
+// may be read (a damaged stream can lead anywhere).
+__device__ __forceinline__ void rans_resident_words(const uint32_t* words, uint32_t at, uint32_t last, uint32_t v[4]) {
+    const uint32_t k = min(at >> 5, last);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) v[j] = words[k + j];
+}
+__device__ __forceinline__ void rans_resident_short(const uint4* tab, const uint32_t* words, uint32_t last, uint32_t& x, uint32_t& at, uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
+    s_lo = 0; s_hi = 0;
+    for (uint32_t j = 0; j < g; ++j) {
+        const uint4 e = tab[x & 2047u];
+        x = e.x * (x >> 11) + e.y;
+        if (j < 4) s_lo |= e.w << (8 * j); else s_hi |= e.w << (8 * (j - 4));
+        for (int k = 0; k < 3 && x < RANS_L; ++k) { x = (x << 8) | ((words[min(at >> 5, last)] >> (24 - (at & 24u))) & 0xFFu); at += 8; }
+    }
+}
+// Four symbols.  `v` are words read when the last four were half done, `skip` the bits of them that are used up by now (below 64).
+__device__ __forceinline__ uint32_t rans_resident_four(const uint4* tab, const uint32_t* words, uint32_t last, uint32_t& x, uint32_t& at, uint32_t v[4], uint32_t& skip) {
+    const bool one_off = skip >= 32;
+    const uint32_t a = one_off ? v[1] : v[0], b = one_off ? v[2] : v[1], c = one_off ? v[3] : v[2];
+    uint32_t wh = __funnelshift_l(b, a, skip), wl = __funnelshift_l(c, b, skip), used = 0, sy = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j == 2) {
+            at += used;
+            rans_resident_words(words, at, last, v);
+            skip = at & 31u;
+            used = 0;
+        }
+        const uint4 e = tab[x & 2047u];
+        uint32_t bits;
+        rans_direct_step(e, wh, x, bits);
+        sy = __byte_perm(sy, e.w, (0x3210u & ~(0xFu << (4 * j))) | (4u << (4 * j)));
+        wh = __funnelshift_l(wl, wh, bits);
+        wl <<= bits;
+        used += bits;
+    }
+    at += used;
+    skip += used;
     return sy;
 }
 
@@ -851,7 +927,8 @@ template <bool PER_LANE, int DIRECT = 0>
 __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(const DecodeItem* __restrict__ items, uint32_t n_items, Bases bases, uint32_t* __restrict__ status,
                                                            uint32_t l_entries) {
     constexpr int LS = PER_LANE ? 32 : 1;
-    constexpr uint32_t CHUNKS = DIRECT ? DIRECT : RANS_WARP_CHUNKS;
+    constexpr bool RESIDENT = DIRECT == 2, WIDE = DIRECT == 1 || RESIDENT;
+    constexpr uint32_t CHUNKS = WIDE ? 1 : DIRECT ? DIRECT : RANS_WARP_CHUNKS;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t lane = threadIdx.x, c = lane >> 2, s = lane & 3;
     // DIRECT: the rings come first, and in their place, while the tables are built, one chunk's rank table and symbol list
@@ -980,10 +1057,38 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
 #pragma unroll 8
                 for (uint32_t u = lane; u < 2048; u += 32) {
                     const uint32_t w = tab[u >> 4], e = lst[(w >> 16) + __popc(w << ((~u & 15u) | 16u))];
-                    slots[c2 * 2048 + u] = (u - (e >> 20)) << 20 | (e & 0xFFu) << 12 | ((e >> 8) & 0xFFFu);
+                    const uint32_t f = (e >> 8) & 0xFFFu, d = u - (e >> 20);
+                    if (WIDE) reinterpret_cast<uint4*>(slots)[u] = make_uint4(f, d, (RANS_L - 1 - d) / f + 1, e & 0xFFu);
+                    else slots[c2 * 2048 + u] = d << 20 | (e & 0xFFu) << 12 | f;
                 }
                 __syncwarp();
             }
+        }
+    }
+    uint32_t* const words = slots + RANS_WIDE_BYTES / 4;  // RESIDENT: the chunk's streams, from the aligned 16 bytes on that hold their first one
+    uintptr_t words_from = 0;
+    uint32_t last_word = 0;
+    if (RESIDENT) {
+        const uintptr_t first = reinterpret_cast<uintptr_t>(rd(bases, items[blockIdx.x].src)) + __shfl_sync(0xFFFFFFFFu, hdr, 0) + 16;
+        const uintptr_t end = reinterpret_cast<uintptr_t>(rd(bases, items[blockIdx.x].src)) + items[blockIdx.x].src_len;
+        words_from = first & ~uintptr_t(15);
+        if (__shfl_sync(0xFFFFFFFFu, err, 0) == ST_OK) {  // the header fits, so first <= end
+            const uintptr_t lo16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_first) & ~uintptr_t(15);
+            const uintptr_t hi16 = (reinterpret_cast<uintptr_t>(bases.blob) + bases.blob_end + 15) & ~uintptr_t(15);
+            const uint32_t blocks = uint32_t((end - words_from + 15) >> 4);
+            last_word = 4 * blocks + RANS_STREAM_PAD / 4 - 4;
+            uint4* out = reinterpret_cast<uint4*>(words);
+            for (uint32_t b0 = 0; b0 < blocks; b0 += 8 * 32) {
+                uint4 v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = fetch16(words_from + 16 * uintptr_t(b0 + 32 * k + lane), lo16, hi16);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const uint32_t b = b0 + 32 * k + lane;
+                    if (b < blocks) out[b] = make_uint4(__byte_perm(v[k].x, 0, 0x0123), __byte_perm(v[k].y, 0, 0x0123), __byte_perm(v[k].z, 0, 0x0123), __byte_perm(v[k].w, 0, 0x0123));
+                }
+            }
+            if (lane < RANS_STREAM_PAD / 16) out[blocks + lane] = make_uint4(0, 0, 0, 0);
         }
     }
     __syncwarp();
@@ -993,7 +1098,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
     if (valid && !err && seg_len > 0) {
         if (my_len < 4) err = ST_STREAM_UNDERRUN;  // decompress.rs:82-86
         else {
-            const uint32_t* tab = DIRECT == 1 ? slots : DIRECT ? slots + c * 2048 : ranktab + c * 128;
+            const uint32_t* tab = WIDE ? slots : DIRECT ? slots + c * 2048 : ranktab + c * 128;
             const uint32_t* lst = PER_LANE ? symlist + lane : symlist + c * l_entries;
             const RansPair pair = rans_pair_at(smem + c * RANS_PAIR_ENTRIES * 8, n_items ? 1u : 0u);
             const uint32_t* rw = ring.base;
@@ -1001,6 +1106,33 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
             const uint8_t* st = src + my_off;
             uint32_t x = ld_u32_unaligned(st);
             const bool slow = x >> 31 || (DIRECT && x < RANS_L);  // see rans_group8, rans_direct_four
+            if (RESIDENT) {
+                const uint4* wide = reinterpret_cast<const uint4*>(slots);
+                uint32_t at = 8 * uint32_t(reinterpret_cast<uintptr_t>(st) + 4 - words_from), pos = seg_start, remaining = seg_len, s_lo, s_hi;
+                const uint32_t end_at = 8 * uint32_t(reinterpret_cast<uintptr_t>(st) + my_len - words_from);
+                const uint32_t g = first_group(ep, pos, remaining);
+                if (g < 8 || remaining < 16) {
+                    rans_resident_short(wide, words, last_word, x, at, g, s_lo, s_hi);
+                    emit(ep, pos, g, uint64_t(s_lo) | uint64_t(s_hi) << 32);
+                    pos += g; remaining -= g;
+                }
+                if (!slow) {
+                    uint32_t v[4], skip = at & 31u;
+                    rans_resident_words(words, at, last_word, v);
+                    fast_groups(ep, it.n, pos, remaining, [&](uint32_t& lo, uint32_t& hi) {
+                        lo = rans_resident_four(wide, words, last_word, x, at, v, skip);
+                        hi = rans_resident_four(wide, words, last_word, x, at, v, skip);
+                    });
+                }
+                while (remaining) {
+                    const uint32_t t = remaining < 8 ? remaining : 8;
+                    rans_resident_short(wide, words, last_word, x, at, t, s_lo, s_hi);
+                    emit(ep, pos, t, uint64_t(s_lo) | uint64_t(s_hi) << 32);
+                    pos += t; remaining -= t;
+                }
+                if (at > end_at) report(status, it.id, ST_STREAM_UNDERRUN);  // decompress.rs:99-104
+                return;
+            }
             // ring cursor as a 32-bit offset from the 16-byte aligned block that holds the first renorm byte
             const uintptr_t g0 = (reinterpret_cast<uintptr_t>(st) + 4) & ~uintptr_t(15);
             uint32_t rq = uint32_t(reinterpret_cast<uintptr_t>(st) + 4 - g0);
@@ -1027,7 +1159,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
 
             uint32_t pos = seg_start, remaining = seg_len;
             auto short_group = [&](uint32_t g, uint32_t& s_lo, uint32_t& s_hi) {
-                if (DIRECT) rans_direct_short(tab, rw, x, rq, g, s_lo, s_hi);
+                if (DIRECT) rans_direct_short<WIDE>(tab, rw, x, rq, g, s_lo, s_hi);
                 else if (PER_LANE && pairs) rans_pair_short(pair, rw, x, rq, g, s_lo, s_hi);
                 else rans_short_group<LS>(tab, lst, rw, x, rq, g, s_lo, s_hi);
             };
@@ -1052,9 +1184,9 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
                 rans_direct_words(rw, rq, v);
                 fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {
                     const uint32_t began = rq;
-                    s_lo = rans_direct_four(tab, rw, x, rq, v, skip);
+                    s_lo = rans_direct_four<WIDE>(tab, rw, x, rq, v, skip);
                     top_up_at(began, 40);
-                    s_hi = rans_direct_four(tab, rw, x, rq, v, skip);
+                    s_hi = rans_direct_four<WIDE>(tab, rw, x, rq, v, skip);
                 });
             } else if (PER_LANE && pairs) {
                 fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {
@@ -1064,7 +1196,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
             } else {
                 fast_groups(ep, it.n, pos, remaining, [&](uint32_t& s_lo, uint32_t& s_hi) {
                     top_up();
-                    if (DIRECT) rans_direct_short(tab, rw, x, rq, 8, s_lo, s_hi);
+                    if (DIRECT) rans_direct_short<WIDE>(tab, rw, x, rq, 8, s_lo, s_hi);
                     else rans_group8<LS, !PER_LANE>(tab, lst, rw, x, rq, s_lo, s_hi, dense, slow);
                 });
             }
@@ -1082,12 +1214,17 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
     if (err) report(status, it.id, err);
 }
 
-// `direct`: the launch takes the kernel with a table entry per slot.  Else `size` is the rows of the symbol lists (`narrow`) or the
-// most distinct symbols of a chunk.
+// `direct`: the launch takes a kernel with a table entry per slot, and `size` is the largest rans_direct_size.  Else `size` is the rows of the
+// symbol lists (`narrow`) or the most distinct symbols of a chunk.
+inline uint32_t rans_direct_size(const DecodeItem& it) { return it.n < 1u << 29 ? it.src_len : ~0u; }  // (positions in shared memory are 32-bit, in bits)
 inline void rans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, bool direct, bool narrow, uint32_t size, cudaStream_t st) {
     auto blocks = [n](uint32_t per) { return (n + per - 1) / per; };
-    if (direct && n <= 4 * 148) rans_decode_kernel_t<false, 1><<<n, 32, rans_direct_smem(1), st>>>(items, n, bases, status, rans_l_entries(255));
-    else if (direct) rans_decode_kernel_t<false, 4><<<blocks(4), 32, rans_direct_smem(4), st>>>(items, n, bases, status, rans_l_entries(255));
+    if (direct && n <= 4 * 148) {
+        // the streams go to shared memory where all blocks that an SM gets have room for theirs
+        const uint32_t per_sm = blocks(148), room = RANS_RESIDENT_MOST / per_sm;
+        if (size < room && rans_resident_smem(size) <= room) rans_decode_kernel_t<false, 2><<<n, 32, rans_resident_smem(size), st>>>(items, n, bases, status, rans_l_entries(255));
+        else rans_decode_kernel_t<false, 1><<<n, 32, rans_direct_smem(1), st>>>(items, n, bases, status, rans_l_entries(255));
+    } else if (direct) rans_decode_kernel_t<false, 4><<<blocks(4), 32, rans_direct_smem(4), st>>>(items, n, bases, status, rans_l_entries(255));
     else if (narrow) rans_decode_kernel_t<true><<<blocks(RANS_WARP_CHUNKS), 32, rans_smem_bytes(size + 2, true), st>>>(items, n, bases, status, size + 2);
     else {
         const uint32_t le = (size + 2 + 3) & ~3u;
@@ -1095,8 +1232,10 @@ inline void rans_launch(const DecodeItem* items, uint32_t n, const Bases& bases,
     }
 }
 inline cudaError_t rans_direct_allow_shared() {
-    const cudaError_t e = cudaFuncSetAttribute(rans_decode_kernel_t<false, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(rans_decode_kernel_t<false, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaError_t e = cudaFuncSetAttribute(rans_decode_kernel_t<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(RANS_RESIDENT_MOST));
+    for (auto k : {rans_decode_kernel_t<false, 1>, rans_decode_kernel_t<false, 2>, rans_decode_kernel_t<false, 4>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e;
 }
 
 // ---- canonical Huffman -----------------------------------------------------

@@ -220,7 +220,7 @@ struct ptwm_b200_plan {
     // per launch slot: 0-3 phase-0 decoders (rANS, Huffman, tANS, O1SAC), 4 scratch copies, 5-8 phase-1 decoders, 9 final merge, 10 CRC, 11 XXH64
     // One launch of a decoder: a run of items of a list.  Items of the second phase that read planes the first one puts into
     // scratch must wait for it, the others need not.  rANS chunks with few distinct symbols go to the kernel with a symbol list
-    // per lane; `size` is its rows there, the most distinct symbols of the run for the general kernel, the most cumulative
+    // per lane; `size` is its rows there, the most distinct symbols of the run for the general kernel, the coded bytes of a chunk for those with a table entry per slot, the most cumulative
     // tables of a chunk for Order1ScaleAC, and for tANS the kernel (tans_kernel).
     struct Launch { uint32_t first, count, size; bool waits, narrow; };
     std::vector<Launch> runs[2][4];
@@ -439,7 +439,7 @@ void finish_lists(ptwm_b200_plan& pl) {
             pl.slot_items[slot] = uint32_t(v.size());
             for (size_t k = 0; k < v.size(); ++k) {
                 const bool nw = !(order[k].first >> 33), w = order[k].first >> 32 & 1;
-                const uint32_t size = cc == 0 ? v[k].row_len >> 16 : cc == 3 ? o1sac_tables(v[k].state_len) : 0u;
+                const uint32_t size = cc == 0 ? (direct ? rans_direct_size(v[k]) : v[k].row_len >> 16) : cc == 3 ? o1sac_tables(v[k].state_len) : 0u;
                 auto add = [&](std::vector<ptwm_b200_plan::Launch>& to, bool cut) {
                     if (to.empty() || to.back().narrow != nw || (cut && to.back().waits != w)) to.push_back({uint32_t(k), 0, 0, w, nw});
                     to.back().count++;
@@ -824,7 +824,7 @@ int64_t decode_plane_cuda(uint8_t sfv, const uint8_t* state, size_t state_len, c
     const DecodeItem* d_it = reinterpret_cast<const DecodeItem*>(scratch + 64);
     uint32_t* d_status = reinterpret_cast<uint32_t*>(scratch) + 1;  // the summary word in front
     switch (codec) {
-        case C_RANS: rans_launch(d_it, 1, bases, d_status, true, false, 0, st); break;
+        case C_RANS: rans_launch(d_it, 1, bases, d_status, true, false, rans_direct_size(it), st); break;
         case C_HUFFMAN: huffman_decode_kernel<<<1, 32, HUF_SMEM, st>>>(d_it, 1, bases, d_status); break;
         case C_TANS: tans_launch(d_it, 1, bases, d_status, tans_lanes(1, uint32_t(decoded), 1), st); break;
         default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), false, st); break;

@@ -59,6 +59,18 @@ def test_decode_launch_sizes(codec, chunks, dtype):
     check(specs, chunk_size=67, forced_codec=codec)
 
 
+@pytest.mark.parametrize("n", [200_000, 233_000, 300_000, 600_001])
+@pytest.mark.parametrize("chunks", [1, 149, 445])
+def test_rans_decode_streams_in_shared_memory(n, chunks):
+    # streams that fit beside the table of a block, of two and of four blocks to an SM, and streams that go through the rings
+    n //= {1: 1, 149: 3, 445: 8}[chunks]
+    raw = plane("wide", n)
+    low = np.random.default_rng(n).integers(0, 256, n, dtype=np.uint8).astype(np.uint16)
+    wide = ((low & 0x80) << 8 | np.frombuffer(raw, np.uint8).astype(np.uint16) << 7 | low & 0x7F).astype(np.uint16)
+    check([u8("p", raw)] + [u8(f"q{k}", plane("wide", 100, k)) for k in range(chunks - 1)], chunk_size=1 << 20, forced_codec=RANS)
+    check([oracle.TensorSpec("p", oracle.DT_BF16, [n], wide.tobytes())], chunk_size=1 << 20, forced_codec=RANS, emit_crc=True)
+
+
 def counted(counts, rng, cluster=0):
     """2048 symbols with exactly these counts, which are then the table's frequencies; the last `cluster` symbols put side by side."""
     syms = np.repeat(np.arange(100, 100 + len(counts)), counts)
