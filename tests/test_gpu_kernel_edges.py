@@ -277,6 +277,16 @@ def test_huffman_encode_shares_of_a_stream(kind):
     encode_check([plane(kind, 600 * 149)], 600, HUFFMAN)
 
 
+@pytest.mark.parametrize("shift", [0, 1, 8, 16])
+def test_encode_split_of_a_view(shift):
+    # 16-bit elements from an address that is a multiple of 2, 16 and 32 bytes: single elements, two 128-bit loads, one of 256 bits
+    for n in (31, 32, 33, 5000, 70001):
+        w = weights(1, n + shift, n, False).to(torch.bfloat16).reshape(-1)
+        spec = oracle.TensorSpec("t", oracle.DT_BF16, [n], w[shift:].clone().view(torch.uint8).numpy().tobytes())
+        got = compress_model({"t": w.cuda()[shift:]}, CompressionConfig(streaming_chunk=4096, forced_codec=RANS)).to_bytes()
+        assert got == oracle.write_container([spec], chunk_size=4096, forced_codec=RANS), n
+
+
 @pytest.mark.parametrize("chunks", [1, 18, 19, 37, 38, 74, 75])
 @pytest.mark.parametrize("kind", ["exponent", "rare", "wide"])
 def test_huffman_encode_blocks_of_a_cluster(kind, chunks):
