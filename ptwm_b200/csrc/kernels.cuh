@@ -3329,9 +3329,11 @@ __global__ void __launch_bounds__(128) crc_planes_kernel(const VerifyTensor* __r
 // than that dependent chain allows.  Tensors hash concurrently, one per block, and the host lists the largest first: the
 // longest tensor is the critical path.  Two warps per block: lanes 0-3 of the first work through the stripes of one block of
 // words in shared memory and do nothing else; the second warp meanwhile brings the next block from memory and multiplies its
-// words by the second prime.  A step adds the next word's product inside the widening multiply of the low halves, the cross
-// products run beside that one, and a three-way add joins the high half: 24 cycles per stripe instead of 27 with the add in
-// front of the rotation.  59 MB, the largest tensor of a fp32 model: 28.2 ms with one warp that did all of it, 22.4 now.
+// words by the second prime.  A step adds the next word's product with the multiply of the low halves: its low word and carry
+// first, then the high word on top of the cross products, which it can take late.  20 cycles per stripe; 23 with a widening multiply
+// that adds both words at once (its high word takes 16), 24 to 38 with the high word, the carry or the cross products joined by adds of
+// their own, 27 with the add in front of the rotation.  59 MB, the largest tensor of a fp32 model: 28.2 ms with one warp that did all of
+// it, 22.4 with the widening multiply, 18.9 now.
 __device__ __forceinline__ uint64_t rotl64(uint64_t x, int r) { return (x << r) | (x >> (64 - r)); }
 __device__ __forceinline__ uint64_t ld_u64_unaligned(const uint8_t* p) { return uint64_t(ld_u32_unaligned(p)) | uint64_t(ld_u32_unaligned(p + 4)) << 32; }
 constexpr uint32_t XXH_BLOCK = 8192, XXH_THREADS = 64;
@@ -3340,8 +3342,10 @@ __device__ __forceinline__ uint64_t xxh_step(uint64_t s, uint64_t k) {
     constexpr uint64_t P1 = 11400714785074694791ull;
     const uint32_t a = uint32_t(s), b = uint32_t(s >> 32);
     const uint32_t lo = __funnelshift_l(b, a, 31), hi = __funnelshift_l(a, b, 31);
-    const uint64_t t = uint64_t(lo) * uint32_t(P1) + k;
-    return uint64_t(uint32_t(t >> 32) + lo * uint32_t(P1 >> 32) + hi * uint32_t(P1)) << 32 | uint32_t(t);
+    uint32_t l, h;
+    asm("{\n\t.reg .u32 u;\n\tmad.lo.u32 u, %3, %5, %7;\n\tmad.lo.u32 u, %2, %4, u;\n\tmad.lo.cc.u32 %0, %2, %5, %6;\n\tmadc.hi.u32 %1, %2, %5, u;\n\t}"
+        : "=&r"(l), "=&r"(h) : "r"(lo), "r"(hi), "r"(uint32_t(P1 >> 32)), "r"(uint32_t(P1)), "r"(uint32_t(k)), "r"(uint32_t(k >> 32)));
+    return uint64_t(h) << 32 | l;
 }
 
 __global__ void __launch_bounds__(XXH_THREADS) xxh64_kernel(const HashItem* __restrict__ items, uint32_t n_items, Bases bases, uint64_t* __restrict__ out) {
