@@ -2705,7 +2705,8 @@ inline void tans_launch_t(const DecodeItem* items, uint32_t n, const Bases& base
 // 1597 / 1539 / 1327; fp16, 8 Ki, 2368: 398 / 316 / 280 / 221 (bf16, 128 Ki, 3552: 2291 / 2062 / 1933 / 2016).  In chunks that are mostly
 // serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 182, 32: 122.  Below TANS_FEW symbols the rounds of blocks count, 12 per SM
 // with 64 lanes and 16 with 32; 64 / 32 lanes: 3500 symbols, 1184 chunks 187 / 175, 1776 236 / 195 (fp16 137 / 163, 177 / 175); 6000: 1776 263 / 273,
-// 1900 304 / 261, 2368 356 / 287.
+// 1900 304 / 261, 2368 356 / 287.  Where 32 lanes take as many rounds as 64 their longer ones only pay above 64 Ki symbols; 3330 chunks: fp8, 16 Ki
+// 1027 / 1288, 32 Ki 1274 / 1471, 64 Ki 1813 / 1935, 128 Ki 2950 / 2797; fp16, 32 Ki 593 / 621, 64 Ki 993 / 979; fp32, 32 Ki 834 / 1488.
 constexpr uint32_t TANS_ROUND_64 = 148 * TansShape<64>::BLOCKS, TANS_ROUND_32 = 148 * TansShape<32>::BLOCKS;
 inline uint32_t tans_lanes(uint32_t chunks, uint32_t longest, double apart) {
     if (longest < TANS_SHORT) return chunks <= 4 * 148 ? 128 : 32;
@@ -2713,7 +2714,8 @@ inline uint32_t tans_lanes(uint32_t chunks, uint32_t longest, double apart) {
     if (chunks <= 6 * 148) return 128;
     if (longest < 4000 && (apart > 0.5 || chunks > TANS_ROUND_64)) return 32;
     if (longest < TANS_FEW) return chunks > TANS_ROUND_64 && chunks <= TANS_ROUND_32 ? 32 : 64;
-    return chunks > TANS_ROUND_64 && longest > 65536 * apart ? 32 : 64;
+    const bool fewer_rounds = (chunks + TANS_ROUND_32 - 1) / TANS_ROUND_32 < (chunks + TANS_ROUND_64 - 1) / TANS_ROUND_64;
+    return chunks > TANS_ROUND_64 && longest > 65536 * (fewer_rounds ? apart : 1) ? 32 : 64;
 }
 // `lanes` per chunk; 1: the kernel with a lane per stream.
 inline void tans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t lanes, cudaStream_t st) {
@@ -3333,7 +3335,7 @@ __global__ void __launch_bounds__(128) crc_planes_kernel(const VerifyTensor* __r
 // first, then the high word on top of the cross products, which it can take late.  20 cycles per stripe; 23 with a widening multiply
 // that adds both words at once (its high word takes 16), 24 to 38 with the high word, the carry or the cross products joined by adds of
 // their own, 27 with the add in front of the rotation.  59 MB, the largest tensor of a fp32 model: 28.2 ms with one warp that did all of
-// it, 22.4 with the widening multiply, 18.9 now.
+// it, 22.4 with the widening multiply, 19.5 now.
 __device__ __forceinline__ uint64_t rotl64(uint64_t x, int r) { return (x << r) | (x >> (64 - r)); }
 __device__ __forceinline__ uint64_t ld_u64_unaligned(const uint8_t* p) { return uint64_t(ld_u32_unaligned(p)) | uint64_t(ld_u32_unaligned(p + 4)) << 32; }
 constexpr uint32_t XXH_BLOCK = 8192, XXH_THREADS = 64;
