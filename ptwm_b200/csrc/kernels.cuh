@@ -2980,13 +2980,20 @@ __global__ void __launch_bounds__(32 * WARPS) o1sac_decode_kernel(const DecodeIt
 constexpr uint32_t O1_MAX_ROWS = 257;
 // The chain of a chunk is what a plan with block scales waits for, and it is a third longer with other decoders' warps on its scheduler.  So
 // where the plan says so (`alone`) four chunks go to a block, one to a scheduler, that takes an SM's shared memory whole, on half of the
-// SMs at most; the other decoders have the rest.  The MXFP4 / NVFP4 layer, 280 chunks of 32 Ki scales: 2799 -> 2188 us.
+// SMs at most; the other decoders have the rest, and are let go a moment later (head_start_kernel): with a block on every SM
+// first they would keep these waiting.  The MXFP4 / NVFP4 layer, 280 chunks of 32 Ki scales: 2799 -> 2188 us.
 constexpr uint32_t O1_ALONE_CHUNKS = 4 * 74, O1_ALONE_BYTES = 220 * 1024;
 // `tables` = the most context rows among the items.
+inline bool o1sac_alone(uint32_t n, uint32_t tables) { return n <= O1_ALONE_CHUNKS && 4 * (tables < O1_MAX_ROWS ? tables : O1_MAX_ROWS) * O1_ROW_BYTES <= O1_ALONE_BYTES; }
 inline void o1sac_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t tables, bool alone, cudaStream_t st) {
     const uint32_t rows = tables < O1_MAX_ROWS ? tables : O1_MAX_ROWS;
-    if (alone && n <= O1_ALONE_CHUNKS && 4 * rows * O1_ROW_BYTES <= O1_ALONE_BYTES) o1sac_decode_kernel<4><<<(n + 3) / 4, 128, O1_ALONE_BYTES, st>>>(items, n, bases, status, rows);
+    if (alone && o1sac_alone(n, tables)) o1sac_decode_kernel<4><<<(n + 3) / 4, 128, O1_ALONE_BYTES, st>>>(items, n, bases, status, rows);
     else o1sac_decode_kernel<1><<<n, 32, rows * O1_ROW_BYTES, st>>>(items, n, bases, status, rows);
+}
+// A few microseconds on the stream whose event the other decoders wait for.
+__global__ void head_start_kernel() {
+    const long long from = clock64();
+    while (clock64() - from < 8000) {}
 }
 inline cudaError_t o1sac_allow_shared_rows() {
     cudaError_t e = cudaFuncSetAttribute(o1sac_decode_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(O1_ALONE_BYTES));

@@ -172,7 +172,7 @@ struct DevicePlan {
     uint32_t* acc = nullptr;
     uint64_t* hash_out = nullptr;
     cudaEvent_t ev[24] = {nullptr};   // begin/end per launch slot, created on first timed run
-    cudaEvent_t order[9] = {nullptr}; // fork, first phase done per codec class, all done per codec class; created on the first run that forks
+    cudaEvent_t order[10] = {nullptr}; // fork, first phase done per codec class, all done per codec class, behind Order1ScaleAC's head start; created on the first run that forks
     uint32_t* summary = nullptr;      // pinned: the largest status of the last run
     bool timed[12] = {false};
     uint8_t* arena = nullptr;          // everything above lives in this one block
@@ -657,10 +657,17 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
             ~Join() { if (!joined) for (cudaStream_t s : ds.side) cudaStreamSynchronize(s); }
         } join{ds, false};
         CUDA_TRY(cudaEventRecord(d.order[0], st));
+        // Order1ScaleAC that is to have SMs of its own must find them empty, so the others start some microseconds after it.
+        const bool o1_first = pl.o1_alone && !(pl.runs[0][3].empty() && pl.runs[1][3].empty());
+        if (o1_first) {
+            head_start_kernel<<<1, 1, 0, st>>>();
+            CUDA_TRY(cudaGetLastError());
+            CUDA_TRY(cudaEventRecord(d.order[9], st));
+        }
         for (int cc = 3; cc >= 0; --cc) {
             if (pl.runs[0][cc].empty() && pl.runs[1][cc].empty()) continue;
             cudaStream_t s = ds.side[cc];
-            CUDA_TRY(cudaStreamWaitEvent(s, d.order[0], 0));
+            CUDA_TRY(cudaStreamWaitEvent(s, d.order[cc != 3 && o1_first ? 9 : 0], 0));
             if ((rc = launch_class(0, cc, false, s)) < 0) return rc;
             if (waiting && !pl.runs[0][cc].empty()) { CUDA_TRY(cudaEventRecord(d.order[1 + cc], s)); CUDA_TRY(cudaStreamWaitEvent(st, d.order[1 + cc], 0)); }
             if ((rc = launch_class(1, cc, false, s)) < 0) return rc;
