@@ -729,7 +729,7 @@ __device__ __forceinline__ void rans_group8(const uint32_t* tab, const uint32_t*
 // the update takes.  A symbol that starts behind the slot gives a distance that wraps, so the right one of two is the smaller sum.
 // The integer pipe (half an instruction per cycle and scheduler) is as busy as anything here, so what can be is a multiply-add with a
 // power of two that the compiler does not know, or a float multiply-add with truncation (2^23 + 2 * slot, divided by 64).
-// 8192 symbols of a stream: 850 -> 695 us up to four blocks per SM; the six-layer bf16 model, 3.2 rounds of 19 blocks, 4103 -> 3670 us:
+// 8192 symbols of a stream: 830 -> 695 us up to four blocks per SM; the six-layer bf16 model, 3.2 rounds of 19 blocks, 4103 -> 3670 us:
 // POPC and a read less in the chain, 10.8 -> 9.0 passes of the load/store pipe per warp and symbol, 23 -> 20 integer instructions.
 // Tried: entries laid out so that the chunks of a read have banks of their own (6.3 -> 5.3 passes) 3822; byte count by comparisons 3982; the
 // window's second word left alone for four symbols 3668; sixteen symbols to a look at the ring 3913; streams in 32-byte blocks 3977.
