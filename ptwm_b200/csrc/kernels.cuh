@@ -921,8 +921,9 @@ __device__ __forceinline__ uint32_t rans_resident_four(const uint4* tab, const u
 // 20 blocks per SM lets the compiler use 96 registers (21 blocks), which the 32-bit rounds need to stay out of local
 // memory; shared memory allows 19, or 22 with rank tables of short lists, and more blocks than that gave nothing.
 //
-// DIRECT (chunks per warp, 0 = the rank tables above): a table entry per slot, 8 KiB per chunk, for launches that do not fill
-// the GPU, where the time from one symbol to the next is all that counts (rans_direct_four).
+// DIRECT: 0 the tables above; otherwise a table entry per slot, for launches that do not fill the GPU, where the time from one symbol to the
+// next is all that counts: 4 chunks per warp with a word to an entry (rans_direct_four), 1 chunk with four words to an entry, 2 the same with
+// the chunk's streams in shared memory (rans_resident_four).
 template <bool PER_LANE, int DIRECT = 0>
 __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(const DecodeItem* __restrict__ items, uint32_t n_items, Bases bases, uint32_t* __restrict__ status,
                                                            uint32_t l_entries) {
