@@ -722,7 +722,8 @@ __global__ void __launch_bounds__(32) rans_encode_kernel(const EncChunk* __restr
 // strings are put together in shared memory.  (One thread per stream took 107 ns per symbol.)
 // WARPS > 1, for launches that do not fill the GPU: that many warps to a stream in each block of a cluster, every warp with a share of the
 // stream's rounds.  They first count the bits of their shares, which all blocks read of one another; a word that shares meet in
-// is kept by all of them and put together at the end by the one that fills it.
+// is kept by all of them and put together at the end by the one that fills it.  It asks the shares before it one after the other, in other
+// blocks' shared memory, so a stream has no more shares than rounds: with empty ones 1000 symbols took 25.4 us, without 8.5.
 constexpr uint32_t HENC_LANE = 16, HENC_WORDS = (32 * HENC_LANE * 11 + 31) / 32 + 2, HENC_ROUND = 32 * HENC_LANE;
 template <int WARPS>
 __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncChunk* __restrict__ chunks, const uint32_t* __restrict__ list, uint32_t n_list,
@@ -738,7 +739,7 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const uint32_t blocks = WARPS > 1 ? cluster.num_blocks() : 1, rank = WARPS > 1 ? cluster.block_rank() : 0;
     const uint32_t ci = list[blockIdx.x / blocks], lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = warp / WARPS, mine = warp % WARPS;
-    const uint32_t part = rank * WARPS + mine, parts = blocks * WARPS;
+    const uint32_t part = rank * WARPS + mine;
     auto of = [&](uint32_t q) -> const Shared* { return cluster.map_shared_rank(&sh, q / WARPS); };  // where share q is kept, at place q % WARPS
     const EncChunk c = chunks[ci];
     if (!c.n || !results[ci].coded) return;
@@ -753,7 +754,9 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
     uint8_t* slot = slots + c.slot_off + uint64_t(s) * c.slot_cap;
     uint32_t* out = reinterpret_cast<uint32_t*>(slot);
     const uint32_t rounds = (len + HENC_ROUND - 1) / HENC_ROUND;
-    const uint32_t from = uint32_t(uint64_t(rounds) * part / parts) * HENC_ROUND, to = part + 1 == parts ? len : uint32_t(uint64_t(rounds) * (part + 1) / parts) * HENC_ROUND;
+    const uint32_t parts = min(blocks * WARPS, max(rounds, 1u));  // shares, a round or more each; the warps behind them have none
+    const uint32_t from = part < parts ? uint32_t(uint64_t(rounds) * part / parts) * HENC_ROUND : len;
+    const uint32_t to = part + 1 < parts ? uint32_t(uint64_t(rounds) * (part + 1) / parts) * HENC_ROUND : len;
     auto fetch = [&](uint32_t at, uint32_t n, uint64_t& a, uint64_t& b) {  // up to sixteen bytes from src + at
         a = b = 0;
         if (n == HENC_LANE) { a = ld8_unaligned(src + at); b = ld8_unaligned(src + at + 8); }
@@ -776,7 +779,7 @@ __global__ void __launch_bounds__(128 * WARPS) huffman_encode_kernel(const EncCh
         for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
         if (lane == 0) sh.bits[s][mine] = sum;
         cluster.sync();
-        for (uint32_t q = lane; q < part; q += 32) before_us += of(q)->bits[s][q % WARPS];
+        if (part < parts) for (uint32_t q = lane; q < part; q += 32) before_us += of(q)->bits[s][q % WARPS];
 #pragma unroll
         for (int d = 16; d; d >>= 1) before_us += __shfl_xor_sync(0xFFFFFFFFu, before_us, d);
     }
