@@ -74,10 +74,6 @@ __host__ __device__ inline uint32_t enc_table_bytes(int codec) {
     return codec == C_HUFFMAN ? ENC_HUFF_TABLE_BYTES : codec == C_O1SAC ? ENC_O1SAC_TABLE_BYTES : ENC_FREQ_TABLE_BYTES;
 }
 
-// A store of bytes that this kernel does not touch again, past the L1.
-__device__ __forceinline__ void stg128_past(void* p, uint4 a) {
-    asm volatile("st.global.L1::no_allocate.v4.b32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w) : "memory");
-}
 __device__ __forceinline__ uint32_t warp_prefix(uint32_t v, uint32_t lane) {  // exclusive
     uint32_t incl = v;
 #pragma unroll
@@ -89,8 +85,9 @@ __device__ __forceinline__ uint32_t warp_prefix(uint32_t v, uint32_t lane) {  //
 // SPLIT_TILE elements of a longer one), reads its elements once and writes the planes' bytes.  Sixteen elements per thread and
 // step where the source is 16-byte aligned: 128-bit loads, one 128-bit store per plane.  (Plane offsets are multiples of 16;
 // the groups start at multiples of 16 elements of the tensor, what lies outside them at either end of the block's range goes
-// element by element.)  Sixteen 16-bit elements are one 256-bit load where the source is 32-byte aligned, and neither loads nor stores take a
-// place in the L1: 798 -> 751 us for 1.74 GB of bf16, of which the bytes alone are 530 at the copy bandwidth.
+// element by element.)  Sixteen 16-bit elements are one 256-bit load where the source is 32-byte aligned: 203 -> 194 us for 0.44 GB of bf16, of
+// which the bytes alone are 133 at the copy bandwidth.  Stores that take no place in the L1 would save 2 us more of that, but where the
+// planes fit the L2 those who read them next lose more (bf16, 27 MB: rANS streams 613 -> 639 us, gather 15.5 -> 21.3).
 //
 // COPIES histograms per plane, laid out [symbol][copy], lane l counting in copy l mod COPIES: with 32 a lane has a bank of its
 // own and no atomic waits for another lane's (eight copies took three passes: the lanes that share a copy mostly meet in the
@@ -134,7 +131,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_kernel(const SplitItem* _
         }
     };
     auto put = [&](int p, uint64_t at, const uint32_t w[4]) {
-        stg128_past(planes + it.plane_off[p] + at, make_uint4(w[0], w[1], w[2], w[3]));
+        *reinterpret_cast<uint4*>(planes + it.plane_off[p] + at) = make_uint4(w[0], w[1], w[2], w[3]);
         count_words(p, w);
     };
     auto one = [&](uint64_t i) {
