@@ -612,10 +612,14 @@ __host__ __device__ inline uint32_t rans_smem_bytes(uint32_t l_entries, bool per
     return (per_lane && rank < RANS_PAIR_SMEM ? RANS_PAIR_SMEM : rank) + RING_SMEM;
 }
 
-// Three kernels have a table entry per slot.  Launches of up to 592 chunks, one to a block: entries of four words, and the chunk's streams in shared
+// Four kernels have a table entry per slot.  Launches of up to 592 chunks, one to a block: entries of four words, and the chunk's streams in shared
 // memory beside them where they fit, else through the rings.  Above that four chunks to a block, a word to an entry.  us of one chunk of 32 Ki
 // symbols / 64 Ki in a call of its own, bf16: a word to an entry 479 / 762, four words 460 / 725, streams in shared memory 412 / 630 (73 cycles per
 // symbol; the way from state to state alone is 47).  Tried: both byte counts from the table and one move chosen by them 415 / 652.
+// Chunks of few symbols, one to a block, take a word to an entry too: the larger table, with a division for each slot, takes longer to build than
+// so few gain.  Word / four words and streams, us, 100 chunks: 512 symbols of 32 values 34.0 / 34.4, 800 34.8 / 37.5, 1200 42.3 / 42.4, 2000 46.4 /
+// 46.6; bf16 512 40.7 / 44.4, 1200 46.4 / 54.3, 2000 58.5 / 57.2, 3000 68.9 / 66.5.
+constexpr uint32_t RANS_FEW = 1500;
 // Chunks of a launch up to which the kernel with a table entry per slot is the faster one: what the GPU holds of it at once (six
 // blocks of four chunks per SM).  Chunks of 32 Ki symbols, us of a bf16 tensor, table per slot against tables of pairs: 1 to 592 chunks
 // 420 / 681, 2368 518 / 709, 3552 619 / 694, and beyond that a second wave (start of it, 4144: 832 / 694).  fp32: 445 / 739, 592 chunks 547 / 752,
@@ -623,7 +627,7 @@ __host__ __device__ inline uint32_t rans_smem_bytes(uint32_t l_entries, bool per
 constexpr uint32_t RANS_DIRECT_CHUNKS = 6 * 4 * 148;
 constexpr uint32_t RANS_DIRECT_BYTES = 2048 * 4;  // per chunk
 constexpr uint32_t RANS_WIDE_BYTES = 2048 * 16;   // with four words to an entry
-__host__ __device__ inline uint32_t rans_direct_smem(uint32_t warp_chunks) { return (warp_chunks == 1 ? RANS_WIDE_BYTES : warp_chunks * RANS_DIRECT_BYTES) + RING_SMEM; }
+__host__ __device__ inline uint32_t rans_direct_smem(bool wide, uint32_t warp_chunks) { return (wide ? RANS_WIDE_BYTES : warp_chunks * RANS_DIRECT_BYTES) + RING_SMEM; }
 // The same with a chunk's streams beside the table: up to fifteen bytes on either side of them, and 64 that a group may read too far.
 constexpr uint32_t RANS_STREAM_PAD = 64;
 __host__ __device__ inline uint32_t rans_resident_smem(uint32_t src_len) { return RANS_WIDE_BYTES + RING_SMEM + ((src_len + 32 + 15) & ~15u) + RANS_STREAM_PAD; }
@@ -922,14 +926,14 @@ __device__ __forceinline__ uint32_t rans_resident_four(const uint4* tab, const u
 // memory; shared memory allows 19, or 22 with rank tables of short lists, and more blocks than that gave nothing.
 //
 // DIRECT: 0 the tables above; otherwise a table entry per slot, for launches that do not fill the GPU, where the time from one symbol to the
-// next is all that counts: 4 chunks per warp with a word to an entry (rans_direct_four), 1 chunk with four words to an entry, 2 the same with
-// the chunk's streams in shared memory (rans_resident_four).
+// next is all that counts: 4 chunks per warp with a word to an entry (rans_direct_four), 3 one chunk, 1 one chunk with four words to an entry, 2 the
+// same with the chunk's streams in shared memory (rans_resident_four).
 template <bool PER_LANE, int DIRECT = 0>
 __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(const DecodeItem* __restrict__ items, uint32_t n_items, Bases bases, uint32_t* __restrict__ status,
                                                            uint32_t l_entries) {
     constexpr int LS = PER_LANE ? 32 : 1;
     constexpr bool RESIDENT = DIRECT == 2, WIDE = DIRECT == 1 || RESIDENT;
-    constexpr uint32_t CHUNKS = WIDE ? 1 : DIRECT ? DIRECT : RANS_WARP_CHUNKS;
+    constexpr uint32_t CHUNKS = DIRECT == 0 ? RANS_WARP_CHUNKS : DIRECT == 4 ? 4 : 1;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t lane = threadIdx.x, c = lane >> 2, s = lane & 3;
     // DIRECT: the rings come first, and in their place, while the tables are built, one chunk's rank table and symbol list
@@ -1099,7 +1103,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
     if (valid && !err && seg_len > 0) {
         if (my_len < 4) err = ST_STREAM_UNDERRUN;  // decompress.rs:82-86
         else {
-            const uint32_t* tab = WIDE ? slots : DIRECT ? slots + c * 2048 : ranktab + c * 128;
+            const uint32_t* tab = DIRECT && CHUNKS == 1 ? slots : DIRECT ? slots + c * 2048 : ranktab + c * 128;
             const uint32_t* lst = PER_LANE ? symlist + lane : symlist + c * l_entries;
             const RansPair pair = rans_pair_at(smem + c * RANS_PAIR_ENTRIES * 8, n_items ? 1u : 0u);
             const uint32_t* rw = ring.base;
@@ -1217,15 +1221,16 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
 
 // `direct`: the launch takes a kernel with a table entry per slot, and `size` is the largest rans_direct_size.  Else `size` is the rows of the
 // symbol lists (`narrow`) or the most distinct symbols of a chunk.
-inline uint32_t rans_direct_size(const DecodeItem& it) { return it.n < 1u << 29 ? it.src_len : ~0u; }  // (positions in shared memory are 32-bit, in bits)
+inline uint32_t rans_direct_size(const DecodeItem& it) { return it.n < RANS_FEW ? 0 : it.n < 1u << 29 ? it.src_len : ~0u; }  // (positions in shared memory are 32-bit, in bits)
 inline void rans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, bool direct, bool narrow, uint32_t size, cudaStream_t st) {
     auto blocks = [n](uint32_t per) { return (n + per - 1) / per; };
     if (direct && n <= 4 * 148) {
         // the streams go to shared memory where all blocks that an SM gets have room for theirs
         const uint32_t per_sm = blocks(148), room = RANS_RESIDENT_MOST / per_sm;
-        if (size < room && rans_resident_smem(size) <= room) rans_decode_kernel_t<false, 2><<<n, 32, rans_resident_smem(size), st>>>(items, n, bases, status, rans_l_entries(255));
-        else rans_decode_kernel_t<false, 1><<<n, 32, rans_direct_smem(1), st>>>(items, n, bases, status, rans_l_entries(255));
-    } else if (direct) rans_decode_kernel_t<false, 4><<<blocks(4), 32, rans_direct_smem(4), st>>>(items, n, bases, status, rans_l_entries(255));
+        if (size == 0) rans_decode_kernel_t<false, 3><<<n, 32, rans_direct_smem(false, 1), st>>>(items, n, bases, status, rans_l_entries(255));
+        else if (size < room && rans_resident_smem(size) <= room) rans_decode_kernel_t<false, 2><<<n, 32, rans_resident_smem(size), st>>>(items, n, bases, status, rans_l_entries(255));
+        else rans_decode_kernel_t<false, 1><<<n, 32, rans_direct_smem(true, 1), st>>>(items, n, bases, status, rans_l_entries(255));
+    } else if (direct) rans_decode_kernel_t<false, 4><<<blocks(4), 32, rans_direct_smem(false, 4), st>>>(items, n, bases, status, rans_l_entries(255));
     else if (narrow) rans_decode_kernel_t<true><<<blocks(RANS_WARP_CHUNKS), 32, rans_smem_bytes(size + 2, true), st>>>(items, n, bases, status, size + 2);
     else {
         const uint32_t le = (size + 2 + 3) & ~3u;
@@ -1234,7 +1239,7 @@ inline void rans_launch(const DecodeItem* items, uint32_t n, const Bases& bases,
 }
 inline cudaError_t rans_direct_allow_shared() {
     cudaError_t e = cudaFuncSetAttribute(rans_decode_kernel_t<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(RANS_RESIDENT_MOST));
-    for (auto k : {rans_decode_kernel_t<false, 1>, rans_decode_kernel_t<false, 2>, rans_decode_kernel_t<false, 4>})
+    for (auto k : {rans_decode_kernel_t<false, 1>, rans_decode_kernel_t<false, 2>, rans_decode_kernel_t<false, 3>, rans_decode_kernel_t<false, 4>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     return e;
 }

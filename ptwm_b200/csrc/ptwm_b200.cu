@@ -220,7 +220,7 @@ struct ptwm_b200_plan {
     // per launch slot: 0-3 phase-0 decoders (rANS, Huffman, tANS, O1SAC), 4 scratch copies, 5-8 phase-1 decoders, 9 final merge, 10 CRC, 11 XXH64
     // One launch of a decoder: a run of items of a list.  Items of the second phase that read planes the first one puts into
     // scratch must wait for it, the others need not.  rANS chunks with few distinct symbols go to the kernel with a symbol list
-    // per lane; `size` is its rows there, the most distinct symbols of the run for the general kernel, the coded bytes of a chunk for those with a table entry per slot, the most cumulative
+    // per lane; `size` is its rows there, the most distinct symbols of the run for the general kernel, the coded bytes of a chunk for those with a table entry per slot (0: all short), the most cumulative
     // tables of a chunk for Order1ScaleAC, and for tANS the kernel (tans_kernel).
     struct Launch { uint32_t first, count, size; bool waits, narrow; };
     std::vector<Launch> runs[2][4];

@@ -6,6 +6,7 @@ import time
 import numpy as np
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 import oracle
 import ptwm_b200
@@ -71,6 +72,29 @@ def test_rans_decode_streams_in_shared_memory(n, chunks):
     wide = ((low & 0x80) << 8 | np.frombuffer(raw, np.uint8).astype(np.uint16) << 7 | low & 0x7F).astype(np.uint16)
     check([u8("p", raw)] + [u8(f"q{k}", plane("wide", 100, k)) for k in range(chunks - 1)], chunk_size=1 << 20, forced_codec=RANS)
     check([oracle.TensorSpec("p", oracle.DT_BF16, [n], wide.tobytes())], chunk_size=1 << 20, forced_codec=RANS, emit_crc=True)
+
+
+def launched(call):
+    """The kernels that `call` launches, by name."""
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    names = [e.key for e in p.key_averages() if "_kernel" in e.key]
+    if not names:
+        pytest.skip("no kernels seen: the profiler has no access to the device here")
+    return names
+
+
+@pytest.mark.parametrize("n, chunks, kernel", [(1499, 1, 3), (1499, 592, 3), (1500, 1, 2), (1500, 592, 2), (1499, 593, 4), (50_000, 592, 1)])
+def test_rans_decode_kernel_of_a_small_launch(n, chunks, kernel):
+    # short chunks: the table that is quickly built; then the one that is quickly read, with streams in shared memory where four blocks' fit
+    raw = plane("nibble", n * chunks)
+    blob = oracle.write_container([u8("p", raw)], chunk_size=n, forced_codec=RANS)
+    handle = ptwm_b200.ContainerHandle(blob, device=0)
+    assert any(f"rans_decode_kernel_t<false, {kernel}>" in k for k in launched(lambda: handle.decode("p")))
+    assert handle.decode("p").cpu().numpy().tobytes() == raw
 
 
 def counted(counts, rng, cluster=0):
