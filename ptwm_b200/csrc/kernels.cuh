@@ -1222,15 +1222,31 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
 // `direct`: the launch takes a kernel with a table entry per slot, and `size` is the largest rans_direct_size.  Else `size` is the rows of the
 // symbol lists (`narrow`) or the most distinct symbols of a chunk.
 inline uint32_t rans_direct_size(const DecodeItem& it) { return it.n < RANS_FEW ? 0 : it.n < 1u << 29 ? it.src_len : ~0u; }  // (positions in shared memory are 32-bit, in bits)
-inline void rans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, bool direct, bool narrow, uint32_t size, cudaStream_t st) {
+// What blocks of rans_launch may take of an SM's shared memory, all together.
+struct RansRoom { uint32_t resident, wide; };
+inline RansRoom rans_room_alone() { return {RANS_RESIDENT_MOST, RANS_RESIDENT_MOST}; }
+// Beside other codecs' decoders, whose blocks on an SM have `huffman` and `tans` bytes of shared memory: blocks that find no room wait until some of
+// the others have ended, and their streams are behind then.  Huffman's blocks stay for as long as their launch takes, so theirs is not to be had.
+// tANS blocks come and go, but too many large blocks keep them out in turn.  us by streams in shared memory / four words / four chunks to a block, u8
+// of 32 values in chunks of 64 Ki: 200 chunks beside 400 tANS chunks 671 / 764 / 819, 1776: 1082 / 1159 / 1206, 8000 Huffman chunks 1355 / 1306 / 1260;
+// 300 chunks 795 / 764 / 818, 1098 / 1171 / 1194, 1361 / 1310 / 1265; 444 chunks 905 / 770 / 822, 1610 / 1293 / 1211, 1847 / 1311 / 1268; 592 chunks (no
+// room for streams) - / 1009 / 826, - / 1328 / 1211, - / 1532 / 1269.  32 Ki, 300 chunks: 362 / 414 / 441, 642 / 684 / 704, 703 / 678 / 655; 370 beside 400: 450 / 416 / 441; 444: 469 / 418 /
+// 445, 666 / 762 / 706, 707 / 679 / 657.  256 Ki, 592 beside 100 tANS chunks, which leave room for all: - / 2796 / 3002.  A word to an entry and a chunk to
+// a block are the slower ones nearly everywhere (64 Ki, 592: 818, 1380, 1335).
+inline RansRoom rans_room_beside(uint32_t chunks, uint32_t huffman, uint32_t tans) {
+    auto without = [](uint32_t taken) { return taken < RANS_RESIDENT_MOST ? RANS_RESIDENT_MOST - taken : 0u; };
+    const uint32_t room = without(huffman) > 80u << 10 ? without(huffman) : 80u << 10;
+    return {chunks > 340 ? 0u : room, chunks <= 3 * 148 ? room : huffman ? 0u : without(tans)};
+}
+inline void rans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, bool direct, bool narrow, uint32_t size, RansRoom room, cudaStream_t st) {
     auto blocks = [n](uint32_t per) { return (n + per - 1) / per; };
-    if (direct && n <= 4 * 148) {
-        // the streams go to shared memory where all blocks that an SM gets have room for theirs
-        const uint32_t per_sm = blocks(148), room = RANS_RESIDENT_MOST / per_sm;
-        if (size == 0) rans_decode_kernel_t<false, 3><<<n, 32, rans_direct_smem(false, 1), st>>>(items, n, bases, status, rans_l_entries(255));
-        else if (size < room && rans_resident_smem(size) <= room) rans_decode_kernel_t<false, 2><<<n, 32, rans_resident_smem(size), st>>>(items, n, bases, status, rans_l_entries(255));
-        else rans_decode_kernel_t<false, 1><<<n, 32, rans_direct_smem(true, 1), st>>>(items, n, bases, status, rans_l_entries(255));
-    } else if (direct) rans_decode_kernel_t<false, 4><<<blocks(4), 32, rans_direct_smem(false, 4), st>>>(items, n, bases, status, rans_l_entries(255));
+    const uint32_t per_sm = blocks(148);
+    if (direct && n <= 4 * 148 && size == 0) rans_decode_kernel_t<false, 3><<<n, 32, rans_direct_smem(false, 1), st>>>(items, n, bases, status, rans_l_entries(255));
+    else if (direct && n <= 4 * 148 && size < room.resident && per_sm * rans_resident_smem(size) <= room.resident)
+        rans_decode_kernel_t<false, 2><<<n, 32, rans_resident_smem(size), st>>>(items, n, bases, status, rans_l_entries(255));
+    else if (direct && n <= 4 * 148 && per_sm * rans_direct_smem(true, 1) <= room.wide)
+        rans_decode_kernel_t<false, 1><<<n, 32, rans_direct_smem(true, 1), st>>>(items, n, bases, status, rans_l_entries(255));
+    else if (direct) rans_decode_kernel_t<false, 4><<<blocks(4), 32, rans_direct_smem(false, 4), st>>>(items, n, bases, status, rans_l_entries(255));
     else if (narrow) rans_decode_kernel_t<true><<<blocks(RANS_WARP_CHUNKS), 32, rans_smem_bytes(size + 2, true), st>>>(items, n, bases, status, size + 2);
     else {
         const uint32_t le = (size + 2 + 3) & ~3u;
@@ -2732,6 +2748,12 @@ inline void tans_launch(const DecodeItem* items, uint32_t n, const Bases& bases,
         case 32: tans_launch_t<32>(items, n, bases, status, st); break;
         default: tans_lanes_decode_kernel<<<(n + TANS_CTA_CHUNKS - 1) / TANS_CTA_CHUNKS, TANS_LANES_THREADS, TANS_LANES_SMEM, st>>>(items, n, bases, status);
     }
+}
+// Shared memory of an SM that the launch's blocks take there at once, if they all find room.
+inline uint64_t tans_shared(uint32_t n, uint32_t lanes) {
+    const uint64_t bytes = lanes == 256 ? sizeof(TansShared<256>) : lanes == 128 ? sizeof(TansShared<128>) : lanes == 64 ? sizeof(TansShared<64>) : lanes == 32 ? sizeof(TansShared<32>) : TANS_LANES_SMEM;
+    const uint64_t per_block = lanes == 1 ? TANS_CTA_CHUNKS : 1;
+    return (n + 148 * per_block - 1) / (148 * per_block) * (bytes + 1024);
 }
 template <int LANES>
 inline cudaError_t tans_allow_shared_t() {

@@ -564,6 +564,16 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
     for (bool& t : d.timed) t = false;
     if (timing) for (auto& e : d.ev) if (!e) CUDA_TRY(cudaEventCreate(&e));
     auto mark = [&](int slot, int end) -> cudaError_t { if (!timing) return cudaSuccess; d.timed[slot] = true; return cudaEventRecord(d.ev[2 * slot + end], st); };
+    // shared memory that the launches of a codec take of an SM, when they run beside others
+    auto taken = [&pl](int cc) -> uint32_t {
+        uint64_t most = 0;
+        for (int ph = 0; ph < 2; ++ph) {
+            uint64_t bytes = 0;
+            for (auto& r : pl.runs[ph][cc]) bytes += cc == 1 ? uint64_t((r.count + HUF_WARP_CHUNKS * 148 - 1) / (HUF_WARP_CHUNKS * 148)) * (HUF_SMEM + 1024) : tans_shared(r.count, r.size);
+            most = std::max(most, bytes);
+        }
+        return uint32_t(std::min<uint64_t>(most, RANS_RESIDENT_MOST));
+    };
     const DecodeItem* lists[2][4];
     {
         const DecodeItem* at = d.items;
@@ -574,7 +584,8 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         const uint32_t n = r.count;
         switch (cc) {
             case 0:
-                rans_launch(it, n, bases, status, pl.dec[ph][0].size() <= RANS_DIRECT_CHUNKS, r.narrow, r.size, s);
+                rans_launch(it, n, bases, status, pl.dec[ph][0].size() <= RANS_DIRECT_CHUNKS, r.narrow, r.size,
+                            s == st ? rans_room_alone() : rans_room_beside(n, taken(1), taken(2)), s);
                 break;
             case 1: huffman_decode_kernel<<<(n + HUF_WARP_CHUNKS - 1) / HUF_WARP_CHUNKS, 32, HUF_SMEM, s>>>(it, n, bases, status); break;
             case 2: tans_launch(it, n, bases, status, r.size, s); break;
@@ -831,7 +842,7 @@ int64_t decode_plane_cuda(uint8_t sfv, const uint8_t* state, size_t state_len, c
     const DecodeItem* d_it = reinterpret_cast<const DecodeItem*>(scratch + 64);
     uint32_t* d_status = reinterpret_cast<uint32_t*>(scratch) + 1;  // the summary word in front
     switch (codec) {
-        case C_RANS: rans_launch(d_it, 1, bases, d_status, true, false, rans_direct_size(it), st); break;
+        case C_RANS: rans_launch(d_it, 1, bases, d_status, true, false, rans_direct_size(it), rans_room_alone(), st); break;
         case C_HUFFMAN: huffman_decode_kernel<<<1, 32, HUF_SMEM, st>>>(d_it, 1, bases, d_status); break;
         case C_TANS: tans_launch(d_it, 1, bases, d_status, tans_lanes(1, uint32_t(decoded), 1), st); break;
         default: o1sac_launch(d_it, 1, bases, d_status, o1sac_tables(state_len), false, st); break;

@@ -97,6 +97,21 @@ def test_rans_decode_kernel_of_a_small_launch(n, chunks, kernel):
     assert handle.decode("p").cpu().numpy().tobytes() == raw
 
 
+@pytest.mark.parametrize("codec, others, chunks, kernel", [(TANS, 100, 592, 1), (TANS, 592, 340, 2), (TANS, 592, 341, 1), (TANS, 592, 444, 1), (TANS, 592, 445, 4), (TANS, 592, 593, 4),
+                                                           (HUFFMAN, 8000, 340, 2), (HUFFMAN, 8000, 341, 1), (HUFFMAN, 8000, 445, 4), (HUFFMAN, 19_000, 296, 2), (HUFFMAN, 19_000, 297, 4)])
+def test_rans_decode_kernel_beside_other_codecs(codec, others, chunks, kernel):
+    # a launch that would take most of an SM's shared memory takes less of it where other decoders want theirs
+    g, n = torch.Generator(device="cuda").manual_seed(chunks), 2048
+    skewed = (torch.rand(n * chunks, generator=g, device="cuda").clamp_min(1e-9).log() / -0.18).to(torch.int32).remainder(32).to(torch.uint8)
+    rest = (torch.randn(n * others, generator=g, device="cuda") * 0.02).bfloat16() if codec == TANS else torch.randint(0, 16, (n * others,), generator=g, device="cuda", dtype=torch.uint8)
+    enc = compress_model({"p": skewed, "q": rest}, CompressionConfig(streaming_chunk=n, codec_menu=(IDENTITY, RANS, codec)))
+    assert enc.plane_codecs["p"] == [RANS] and enc.plane_codecs["q"][-1] == codec
+    handle = ptwm_b200.ContainerHandle(enc.to_tensor())
+    assert any(f"rans_decode_kernel_t<false, {kernel}>" in k for k in launched(handle.decode_model))
+    got = dict(handle.decode_model())
+    assert torch.equal(got["p"], skewed) and torch.equal(got["q"].view(torch.uint8), rest.view(torch.uint8))
+
+
 def counted(counts, rng, cluster=0):
     """2048 symbols with exactly these counts, which are then the table's frequencies; the last `cluster` symbols put side by side."""
     syms = np.repeat(np.arange(100, 100 + len(counts)), counts)
