@@ -230,7 +230,7 @@ struct ptwm_b200_plan {
     bool merge_waits = false;  // a final merge reads scratch
     bool spread = false;       // few chunks: every coded plane to scratch at once, then a merge (see ptwm_b200_plan_create)
     bool join_small = false;   // the coded planes of small tensors go to scratch in the launch of the others, and a merge follows
-    bool o1_alone = false;     // Order1ScaleAC beside other codecs has SMs of its own
+    bool o1_alone = false;     // Order1ScaleAC beside other codecs has SMs of its own (a launch of it at least)
     uint64_t joined_bytes = 0;
     uint64_t slot_bytes[12] = {0};
     uint32_t slot_items[12] = {0};
@@ -468,12 +468,14 @@ void finish_lists(ptwm_b200_plan& pl) {
     // Order1ScaleAC takes 63 ns per symbol of its longest chunk, the others 5 ps per symbol (tANS) or 1.6 (rANS, Huffman) and 1 ps per byte
     // merged on the whole GPU: where they are done on half of it by then, they can do without the SMs it would otherwise share with them.
     double chain = 0, rest = 0;
+    bool fits = false;
     for (int ph = 0; ph < 2; ++ph) {
+        for (auto& r : pl.runs[ph][3]) fits |= o1sac_alone(r.count, r.size);
         for (auto& it : pl.dec[ph][3]) chain = std::max(chain, 63e3 * it.n);
         for (int cc = 0; cc < 3; ++cc) for (auto& it : pl.dec[ph][cc]) rest += it.n * (cc == 2 ? 5.0 : 1.6);
         for (auto& it : pl.merges[ph]) rest += double(it.n) * kind_elem_bytes(int(it.kind));
     }
-    pl.o1_alone = 2 * rest < chain;
+    pl.o1_alone = fits && 2 * rest < chain;
     pl.post_tiles.clear();
     uint32_t tile = 0;
     bool delta = false;
@@ -669,8 +671,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         } join{ds, false};
         CUDA_TRY(cudaEventRecord(d.order[0], st));
         // Order1ScaleAC that is to have SMs of its own must find them empty, so the others start some microseconds after it.
-        const bool o1_first = pl.o1_alone && !(pl.runs[0][3].empty() && pl.runs[1][3].empty());
-        if (o1_first) {
+        if (pl.o1_alone) {
             head_start_kernel<<<1, 1, 0, st>>>();
             CUDA_TRY(cudaGetLastError());
             CUDA_TRY(cudaEventRecord(d.order[9], st));
@@ -678,7 +679,7 @@ int64_t enqueue(ptwm_b200_plan& pl, DevicePlan& d, const Bases& bases, uint32_t 
         for (int cc = 3; cc >= 0; --cc) {
             if (pl.runs[0][cc].empty() && pl.runs[1][cc].empty()) continue;
             cudaStream_t s = ds.side[cc];
-            CUDA_TRY(cudaStreamWaitEvent(s, d.order[cc != 3 && o1_first ? 9 : 0], 0));
+            CUDA_TRY(cudaStreamWaitEvent(s, d.order[cc != 3 && pl.o1_alone ? 9 : 0], 0));
             if ((rc = launch_class(0, cc, false, s)) < 0) return rc;
             if (waiting && !pl.runs[0][cc].empty()) { CUDA_TRY(cudaEventRecord(d.order[1 + cc], s)); CUDA_TRY(cudaStreamWaitEvent(st, d.order[1 + cc], 0)); }
             if ((rc = launch_class(1, cc, false, s)) < 0) return rc;

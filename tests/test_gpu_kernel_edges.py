@@ -170,6 +170,9 @@ def test_order1_scale_ac_beside_other_codecs(alphabet, chunks):
     specs, menu = [u8("s", raw, n), u8("p", plane("exponent", 3000))], (oracle.HUFFMAN, oracle.O1SAC)
     assert oracle.write_container(specs[:1], chunk_size=30000, menu=menu) == oracle.write_container(specs[:1], chunk_size=30000, forced_codec=oracle.O1SAC)
     check(specs, chunk_size=30000, menu=menu, emit_crc=True)
+    names = launched(ptwm_b200.ContainerHandle(oracle.write_container(specs, chunk_size=30000, menu=menu), device=0).decode_model)
+    alone = alphabet == 3 and chunks <= 296  # the others wait a moment for that only then
+    assert any("head_start" in k for k in names) == alone and any(f"o1sac_decode_kernel<{4 if alone else 1}>" in k for k in names)
 
 
 @pytest.mark.parametrize("chunks", [1, 31, 33, 4735, 4736, 4737])
