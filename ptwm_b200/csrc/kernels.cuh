@@ -2727,8 +2727,13 @@ inline void tans_launch_t(const DecodeItem* items, uint32_t n, const Bases& base
 // 1597 / 1539 / 1327; fp16, 8 Ki, 2368: 398 / 316 / 280 / 221 (bf16, 128 Ki, 3552: 2291 / 2062 / 1933 / 2016).  In chunks that are mostly
 // serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 182, 32: 122.  Below TANS_FEW symbols the rounds of blocks count, 12 per SM
 // with 64 lanes and 16 with 32; 64 / 32 lanes: 3500 symbols, 1184 chunks 187 / 175, 1776 236 / 195 (fp16 137 / 163, 177 / 175); 6000: 1776 263 / 273,
-// 1900 304 / 261, 2368 356 / 287.  Where 32 lanes take as many rounds as 64 their longer ones only pay above 64 Ki symbols; 3330 chunks: fp8, 16 Ki
-// 1027 / 1288, 32 Ki 1274 / 1471, 64 Ki 1813 / 1935, 128 Ki 2950 / 2797; fp16, 32 Ki 593 / 621, 64 Ki 993 / 979; fp32, 32 Ki 834 / 1488.
+// 1900 304 / 261, 2368 356 / 287.  Where 32 lanes take as many rounds as 64 (2369 to 3552 chunks, 4737 to 5328) what counts is how the last round
+// ends: a few blocks of 32 lanes begin when the first ones of the round before end, some dozens take a round's latency, and the more of them the less
+// that matters.  64 / 32 lanes, fp16 (apart 0.08): 32 Ki, 2369 chunks 467 / 462, 2400 465 / 500, 3552 578 / 596, 4737 732 / 694, 4800 734 / 748, 5328 801 /
+// 819; 64 Ki, 2400 775 / 808, 2900 869 / 869, 3100 920 / 895, 3552 992 / 946, 4737 1299 / 1176, 5328 1423 / 1326.  fp8 (0.25): 20 Ki, 3330 976 / 1118, 4737
+// 1327 / 1400; 32 Ki, 2369 1015 / 956, 3000 1129 / 1192; 64 Ki, 3000 1657 / 1674, 3552 1854 / 1806, 4737 2403 / 2260; a layer of 3330 1829 / 1883.  Bytes of
+// 6.4 bits (0.04): 16 Ki, 3000 315 / 303, 4800 440 / 415; 32 Ki, 2376 387 / 388, 2700 405 / 451, 3552 467 / 481, 4737 603 / 555.  Over 588 launches of 8 Ki to 64 Ki
+// the rule is 1.004 times the better of the two (geometric mean; 64 always 1.015, 32 1.017), 1.05 at worst (64 1.23, 32 1.14).
 constexpr uint32_t TANS_ROUND_64 = 148 * TansShape<64>::BLOCKS, TANS_ROUND_32 = 148 * TansShape<32>::BLOCKS;
 inline uint32_t tans_lanes(uint32_t chunks, uint32_t longest, double apart) {
     if (longest < TANS_SHORT) return chunks <= 4 * 148 ? 128 : 32;
@@ -2736,8 +2741,12 @@ inline uint32_t tans_lanes(uint32_t chunks, uint32_t longest, double apart) {
     if (chunks <= 6 * 148) return 128;
     if (longest < 4000 && (apart > 0.5 || chunks > TANS_ROUND_64)) return 32;
     if (longest < TANS_FEW) return chunks > TANS_ROUND_64 && chunks <= TANS_ROUND_32 ? 32 : 64;
-    const bool fewer_rounds = (chunks + TANS_ROUND_32 - 1) / TANS_ROUND_32 < (chunks + TANS_ROUND_64 - 1) / TANS_ROUND_64;
-    return chunks > TANS_ROUND_64 && longest > 65536 * (fewer_rounds ? apart : 1) ? 32 : 64;
+    if (chunks <= TANS_ROUND_64 || longest <= 65536 * apart) return 64;
+    const uint32_t before = (chunks - 1) / TANS_ROUND_32, over = chunks - before * TANS_ROUND_32;  // whole rounds of 32 lanes, chunks in the one after them
+    if (longest > 65536 || before < (chunks - 1) / TANS_ROUND_64) return 32;
+    if (apart < 0.06) return before == 1 && over >= 32 && longest >= 24 << 10 ? 64 : 32;
+    if (before > 1) return (over >= 64 && longest <= 32 << 10) || (apart > 0.2 && longest <= 24 << 10) ? 64 : 32;
+    return over >= 4 && (apart > 0.2 || uint64_t(longest) * over <= 44u << 20) ? 64 : 32;
 }
 // `lanes` per chunk; 1: the kernel with a lane per stream.
 inline void tans_launch(const DecodeItem* items, uint32_t n, const Bases& bases, uint32_t* status, uint32_t lanes, cudaStream_t st) {

@@ -175,6 +175,19 @@ def test_order1_scale_ac_beside_other_codecs(alphabet, chunks):
     assert any("head_start" in k for k in names) == alone and any(f"o1sac_decode_kernel<{4 if alone else 1}>" in k for k in names)
 
 
+@pytest.mark.parametrize("dtype, n, chunks, lanes", [("fp16", 12, 2368, 32), ("fp16", 12, 2371, 32), ("fp16", 12, 2372, 64), ("fp16", 12, 3552, 64), ("fp16", 12, 3553, 32),
+                                                     ("fp16", 12, 4737, 32), ("fp16", 12, 4799, 32), ("fp16", 12, 4800, 64), ("fp16", 64, 2900, 64), ("fp16", 64, 3100, 32), ("fp8", 20, 2371, 32),
+                                                     ("fp8", 20, 2372, 64), ("fp8", 20, 4737, 64), ("bytes", 16, 3000, 32), ("bytes", 24, 2399, 32), ("bytes", 24, 2400, 64)])
+def test_tans_decode_lanes_where_both_take_as_many_rounds(dtype, n, chunks, lanes):
+    g, n = torch.Generator(device="cuda").manual_seed(chunks), 1024 * n
+    w = torch.randn(n * chunks, generator=g, device="cuda")
+    t = (w * 0.02).half() if dtype == "fp16" else (w * 40).to(torch.float8_e4m3fn) if dtype == "fp8" else (w * 20).round().clamp(-127, 127).to(torch.int8).view(torch.uint8)
+    handle = ptwm_b200.ContainerHandle(compress_model({"t": t}, CompressionConfig(streaming_chunk=n, forced_codec=TANS)).to_tensor())
+    names = launched(lambda: handle.decode("t"))  # (the first of two coded planes of fp8 takes 64 whatever the second does)
+    assert {k for k in (32, 64) if any(f"tans_decode_kernel<{k}>" in name for name in names)} == ({lanes, 64} if dtype == "fp8" else {lanes})
+    assert torch.equal(handle.decode("t").view(torch.uint8), t.view(torch.uint8))
+
+
 @pytest.mark.parametrize("chunks", [1, 31, 33, 4735, 4736, 4737])
 @pytest.mark.parametrize("dtype", ["u8", "bf16", "fp32", "fp8"])
 def test_tans_decode_with_a_lane_per_stream(dtype, chunks):
