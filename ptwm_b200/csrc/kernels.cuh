@@ -739,9 +739,12 @@ __device__ __forceinline__ void rans_group8(const uint32_t* tab, const uint32_t*
 // window's second word left alone for four symbols 3668; sixteen symbols to a look at the ring 3913; streams in 32-byte blocks 3977.
 constexpr uint32_t RANS_PAIR_ONE = 0x4B000000u;   // 2^23
 struct RansPair { uint32_t base, two20, one, four, eight; };  // shared address of the chunk's first entry, for the float's bits; powers of two
-// `one` is 1 and not a constant.
+// `one` is 1 and not a constant.  Called when the table is complete and changes no more: the reads name neither memory nor each other, so that the
+// compiler may order them as it likes, but none of them can come before the address, which is not known before all stores have been made.
 __device__ __forceinline__ RansPair rans_pair_at(const void* table, uint32_t one) {
-    return {uint32_t(__cvta_generic_to_shared(table)) - 4 * RANS_PAIR_ONE, one << 20, one, one * 4, one * 8};
+    uint32_t at = uint32_t(__cvta_generic_to_shared(table)) - 4 * RANS_PAIR_ONE;
+    asm volatile("" : "+r"(at) : : "memory");
+    return {at, one << 20, one, one * 4, one * 8};
 }
 __device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) { uint32_t d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
 // One symbol of a state `xx` (doubled, see above): the sum; the symbol is in bits 12 to 19.
@@ -1105,7 +1108,7 @@ __global__ void __launch_bounds__(32, DIRECT ? 1 : 20) rans_decode_kernel_t(cons
         else {
             const uint32_t* tab = DIRECT && CHUNKS == 1 ? slots : DIRECT ? slots + c * 2048 : ranktab + c * 128;
             const uint32_t* lst = PER_LANE ? symlist + lane : symlist + c * l_entries;
-            const RansPair pair = rans_pair_at(smem + c * RANS_PAIR_ENTRIES * 8, n_items ? 1u : 0u);
+            const RansPair pair = PER_LANE ? rans_pair_at(smem + c * RANS_PAIR_ENTRIES * 8, n_items ? 1u : 0u) : RansPair{};
             const uint32_t* rw = ring.base;
             Epilogue ep = make_epilogue(bases, it);
             const uint8_t* st = src + my_off;
@@ -2922,7 +2925,9 @@ __global__ void __launch_bounds__(32 * WARPS) o1sac_decode_kernel(const DecodeIt
     uint32_t rpt = 0xFFFFFFFFu >> 12, row = 0;  // range / 4096; the context's row, in bytes
     const uint32_t row_len = it.row_len ? it.row_len : (it.n ? it.n : 1);
     uint32_t left_in_row = row_len;
-    const uint32_t shares = uint32_t(__cvta_generic_to_shared(smem)) + lane * 8, leads_at = uint32_t(__cvta_generic_to_shared(smem)) + 256 + lane * 4;
+    uint32_t rows_at = uint32_t(__cvta_generic_to_shared(smem));
+    asm volatile("" : "+r"(rows_at) : : "memory");  // the rows are complete, and what reads them names no memory (rans_pair_at)
+    const uint32_t shares = rows_at + lane * 8, leads_at = rows_at + 256 + lane * 4;
     struct Share { uint32_t below, width, lead; };  // a lane's share of the row
     // One symbol, by the 32 shares; rpt is 0 if none of them has it (and stays 0 if it was).  Returns the next row << 8 | symbol; `took` gets
     // the bits taken in its low byte, which is also what a shift takes of it, and `mine` becomes the share of the next row.
