@@ -246,7 +246,7 @@ __device__ __forceinline__ void split_four_dev(uint32_t n, uint32_t s, uint32_t&
 // one 32-byte sector per instruction instead of half of one, which halves the
 // load/store-pipe cost of these scattered accesses.  Nothing in such a sector is touched twice, and with the tables taking the shared memory
 // little is left of the L1 that so many lanes' lines would go through: without a place there the six-layer bf16 rANS model takes 4103 instead of
-// 4775 us (loads alone 14 %, stores alone 12 %).  The 16-byte blocks of a stream do come from a sector twice and are kept.
+// 4775 us (loads alone 8 % less, stores alone 9 %).  The 16-byte blocks of a stream do come from a sector twice and are kept.
 struct Block32 { uint32_t w[8]; };
 __device__ __forceinline__ Block32 ldg256(const void* p) {
     Block32 b;
@@ -925,8 +925,9 @@ __device__ __forceinline__ uint32_t rans_resident_four(const uint4* tab, const u
     return sy;
 }
 
-// 20 blocks per SM lets the compiler use 96 registers (21 blocks), which the 32-bit rounds need to stay out of local
-// memory; shared memory allows 19, or 22 with rank tables of short lists, and more blocks than that gave nothing.
+// The bound of 20 blocks per SM lets the compiler use 96 registers, which the 32-bit rounds need to stay out of local memory; shared memory allows 19,
+// also where a warp that could not have tables of pairs takes rank tables after all.  Those had 22 before there were tables of pairs, and no less time
+// for it: 32 Ki, half of the weights zero, 3600 chunks 1543 us then and now, 7104: 1654 / 1641, 20,000: 3007 / 2894.
 //
 // DIRECT: 0 the tables above; otherwise a table entry per slot, for launches that do not fill the GPU, where the time from one symbol to the
 // next is all that counts: 4 chunks per warp with a word to an entry (rans_direct_four), 3 one chunk, 1 one chunk with four words to an entry, 2 the
@@ -2724,13 +2725,13 @@ inline void tans_launch_t(const DecodeItem* items, uint32_t n, const Bases& base
     tans_decode_kernel<LANES><<<n, LANES, sizeof(TansShared<LANES>), st>>>(items, bases, status);
 }
 // Lanes per chunk: many shorten a chunk's latency and cost more walks per symbol, so as many as the GPU has room for.  us with
-// 256 / 128 / 64 / 32 lanes, bf16: 64 Ki symbols, 148 chunks 258 / 294 / 380 / 631, 592: 332 / 356 / 442 / 651, 1184: 593 / 592 / 507 / 669,
-// 2368: 1110 / 891 / 912 / 879; 16 Ki, 296: 214 / 233 / 220 / 528, 1184: 464 / 338 / 299 / 553, 2368: 809 / 510 / 526 / 717; 8 Ki, 1776:
-// 470 / 421 / 285 / 295.  Runs that are long against the way to a meeting (`apart`, in symbols of 1,400) need fewer walks: fp8, 64 Ki, 2368: 1993 /
-// 1597 / 1539 / 1327; fp16, 8 Ki, 2368: 398 / 316 / 280 / 221 (bf16, 128 Ki, 3552: 2291 / 2062 / 1933 / 2016).  In chunks that are mostly
-// serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 182, 32: 122.  Below TANS_FEW symbols the rounds of blocks count, 12 per SM
-// with 64 lanes and 16 with 32; 64 / 32 lanes: 3500 symbols, 1184 chunks 187 / 175, 1776 236 / 195 (fp16 137 / 163, 177 / 175); 6000: 1776 263 / 273,
-// 1900 304 / 261, 2368 356 / 287.  Where 32 lanes take as many rounds as 64 (2369 to 3552 chunks, 4737 to 5328) what counts is how the last round
+// 256 / 128 / 64 / 32 lanes, bf16: 64 Ki symbols, 148 chunks 195 / 255 / 351 / 586, 592: 429 / 319 / 412 / 838, 1184: 791 / 543 / 568 / 876,
+// 2368: 1440 / 888 / 839 / 962; 16 Ki, 296: 184 / 172 / 228 / 491, 1184: 559 / 311 / 322 / 532, 2368: 1021 / 511 / 482 / 629; 8 Ki, 1776:
+// 594 / 347 / 271 / 326.  Runs that are long against the way to a meeting (`apart`, in symbols of 1,400) need fewer walks: fp8, 64 Ki, 2368: 2393 /
+// 1446 / 1430 / 1298; fp16, 8 Ki, 2368: 506 / 299 / 290 / 226 (bf16, 128 Ki, 3552: 2892 / 1834 / 1763 / 1687).  In chunks that are mostly
+// serial the other lanes only cost: 1024 symbols, 2368 chunks 128: 175, 32: 126.  Below TANS_FEW symbols the rounds of blocks count, 12 per SM
+// with 64 lanes and 16 with 32; 64 / 32 lanes: 3500 symbols, 1184 chunks 184 / 180, 1776 223 / 200 (fp16 150 / 155, 183 / 184); 6000: 1776 272 / 299,
+// 1900 294 / 307, 2368 380 / 315.  Where 32 lanes take as many rounds as 64 (2369 to 3552 chunks, 4737 to 5328) what counts is how the last round
 // ends: a few blocks of 32 lanes begin when the first ones of the round before end, some dozens take a round's latency, and the more of them the less
 // that matters.  64 / 32 lanes, fp16 (apart 0.08): 32 Ki, 2369 chunks 467 / 462, 2400 465 / 500, 3552 578 / 596, 4737 732 / 694, 4800 734 / 748, 5328 801 /
 // 819; 64 Ki, 2400 775 / 808, 2900 869 / 869, 3100 920 / 895, 3552 992 / 946, 4737 1299 / 1176, 5328 1423 / 1326.  fp8 (0.25): 20 Ki, 3330 976 / 1118, 4737
@@ -3023,7 +3024,7 @@ constexpr uint32_t O1_MAX_ROWS = 257;
 // The chain of a chunk is what a plan with block scales waits for, and it is a third longer with other decoders' warps on its scheduler.  So
 // where the plan says so (`alone`) four chunks go to a block, one to a scheduler, that takes an SM's shared memory whole, on half of the
 // SMs at most; the other decoders have the rest, and are let go a moment later (head_start_kernel): with a block on every SM
-// first they would keep these waiting.  The MXFP4 / NVFP4 layer, 280 chunks of 32 Ki scales: 2799 -> 2188 us.
+// first they would keep these waiting, which nothing but the time rules out.  The MXFP4 / NVFP4 layer, 280 chunks of 32 Ki scales: 2796 -> 2180 us.
 constexpr uint32_t O1_ALONE_CHUNKS = 4 * 74, O1_ALONE_BYTES = 220 * 1024;
 // `tables` = the most context rows among the items.
 inline bool o1sac_alone(uint32_t n, uint32_t tables) { return n <= O1_ALONE_CHUNKS && 4 * (tables < O1_MAX_ROWS ? tables : O1_MAX_ROWS) * O1_ROW_BYTES <= O1_ALONE_BYTES; }

@@ -374,10 +374,11 @@ void plan_tensor(ptwm_b200_plan& pl, uint32_t ti, const TensorDesc& t, uint64_t 
 // 10 ps per symbol of the first 8 Ki (paths meeting), and what placing a symbol costs.  Planes above four bits per symbol meet sooner,
 // and so do nibbles; below two bits they meet later.  Otherwise, below TANS_FEW symbols, several lanes are the faster ones as long as one round of
 // blocks holds the launch (fp32 from 4000 symbols on: of blocks of 64 lanes); after that every round costs its latency again.
-// us, lane per stream / several lanes: bf16, 512: 3552 chunks 152 / 149; 1 Ki: 2368 166 / 116, 2700 165 / 185; 2 Ki: 2368 197 / 171, 2700 197 / 264;
-// 4 Ki: 2368 250 / 238, 2700 249 / 362; 8 Ki: 2368 360 / 359, 2700 360 / 430; 16 Ki: 2368 590 / 529; 32 Ki: 3552 1034 / 864, 4736 1031 / 1021;
-// 64 Ki: 4736 1902 / 1481; fp32, 32 Ki: 2368 1041 / 674, 4736 1038 / 1122; fp16, 8 Ki, 2700 386 / 308; 32 Ki, 4736 1078 / 765; fp8, 8 Ki, 2368 691 /
-// 577; fp32, 6000, 2368 319 / 360; bf16, half of it zeros, 16 Ki: 4736 2606 / 1435; 99 % zeros, both planes: 32 Ki, 4000 2527 / 3162, 64 Ki, 1184 2793 / 1602.
+// us, lane per stream / several lanes: bf16, 512: 3552 chunks 156 / 155; 1 Ki: 2368 169 / 123, 2700 169 / 184; 2 Ki: 2368 198 / 179, 2700 200 / 273;
+// 4 Ki: 2368 254 / 244, 2700 255 / 320; 8 Ki: 2368 365 / 342, 2700 362 / 398; 16 Ki: 2368 588 / 478; 32 Ki: 3552 1019 / 726, 4736 1022 / 924;
+// 64 Ki: 4736 1883 / 1387; fp32, 32 Ki: 2368 1030 / 642, 4736 1027 / 991 (the one of these that the estimate, made for slower walks, sends to the wrong
+// kernel); fp16, 8 Ki, 2700 392 / 307; 32 Ki, 4736 1076 / 657; fp8, 8 Ki, 2368 695 / 584; fp32, 6000, 2368 328 / 342; bf16, both planes coded: half of it
+// zeros, 16 Ki, 4736 2613 / 1090; 99 % zeros, 32 Ki, 4000 2495 / 2994, 64 Ki, 1184 4202 / 1666.
 uint32_t tans_kernel(const DecodeItem* items, size_t n) {
     constexpr size_t WAVE = 148 * TANS_CTA_CHUNKS;
     const uint32_t longest = n ? items[0].n : 0;
