@@ -78,7 +78,7 @@ def launched(call):
     """The kernels that `call` launches, by name."""
     call()
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
         call()
         torch.cuda.synchronize()
     names = [e.key for e in p.key_averages() if "_kernel" in e.key]
